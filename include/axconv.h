@@ -125,6 +125,10 @@ int axc_depthwise_conv2d_output_dims(const axc_conv_desc *desc, int64_t out4[4])
  * (its first 256 bytes decide), only slower.  One buffer serves one stream at a time. */
 int axc_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
 int axc_depthwise_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
+/* Scratch with which a dense call takes the expanded-table kernels; 0 where the plan-based kernels are the better
+ * ones for the shape.  A call that brings at least this much is served by them (same results, no plan to build);
+ * nothing in the buffer outlives the call, so one buffer may serve all layers of a stream in turn. */
+int axc_conv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
 /* Reads back {rebuilt in the last call, fallback kernel in use, kernel status (0 = fine), schedule steps per
  * ideal step in per-mille} of the plan in a dense workspace.  Blocks until `stream` is idle.  Diagnostics only;
  * no counterpart in the reference. */

@@ -1,0 +1,85 @@
+"""GPU: the expanded-table kernels against the CPU checker, bit for bit, at the sizes where they can go wrong: edges of
+pixel tiles (256 to 3072 pixels), channel tiles (8 / 16), K chunks (16), codes in pixel order and as im2col rows, K split
+over CTAs, tables built by the CTAs and taken from global memory, and every form a table can be kept in."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def tables(ax):
+    rng = np.random.Generator(np.random.PCG64(8))
+    return {"exact": ax.exact_table(), "byte": ax.truncated_table(), "digits": rng.integers(0, 65280, 65536).astype(np.uint16),
+            "centred": ax.noisy_table(3), "neither": rng.integers(0, 65536, 65536).astype(np.uint16)}
+
+
+# n, h, w, c, kh, kw, cout, stride, dilation, padding
+SHAPES = [
+    (1, 7, 7, 512, 3, 3, 512, 1, 1, "SAME"),        # 49 pixels, K split over CTAs
+    (2, 32, 32, 16, 3, 3, 32, 1, 1, "SAME"),        # whole 16-byte pieces
+    (3, 27, 31, 150, 1, 1, 45, 1, 1, "SAME"),       # ragged channels on both sides
+    (1, 64, 64, 3, 7, 7, 64, 2, 1, "SAME"),         # im2col rows
+    (1, 112, 112, 8, 3, 3, 32, 1, 1, "SAME"),       # im2col rows, 16-byte input pixels
+    (2, 40, 37, 32, 3, 3, 24, 1, 2, "SAME"),        # dilation
+    (7, 33, 29, 20, 3, 3, 33, 2, 1, "VALID"),       # stride without padding
+    (1, 14, 14, 1024, 1, 1, 256, 2, 1, "SAME"),     # input pixels that no window reads
+    (4, 56, 57, 32, 3, 3, 64, 1, 1, "SAME"),        # enough pixels for tables in global memory
+    (9, 37, 37, 64, 1, 1, 72, 1, 1, "SAME"),
+]
+
+
+@pytest.mark.parametrize("kind", ["exact", "byte", "digits", "centred", "neither"])
+@pytest.mark.parametrize("shape", SHAPES, ids=["-".join(str(v) for v in s) for s in SHAPES])
+def test_expanded_tables_match_the_checker(built, shape, kind):
+    import torch
+    import tf_approximate_b200 as ax
+    from tf_approximate_b200 import ops
+    n, h, w, c, kh, kw, co, s, d, pad = shape
+    lut = tables(ax)[kind]
+    assert ops.fast_workspace_bytes((n, h, w, c), (kh, kw, c, co), [1, s, s, 1], pad, (1, d, d, 1)) > 0
+    rng = np.random.Generator(np.random.PCG64(sum(shape[:8])))
+    x = rng.uniform(-1, 1, (n, h, w, c)).astype(np.float32)
+    f = rng.normal(0, 0.1, (kh, kw, c, co)).astype(np.float32)
+    mm = (-0.7, 1.0, float(f.min()), float(f.max()))
+    ref = O.conv2d(O.desc(n, h, w, c, kh, kw, co, (s, s), (d, d), pad), lut, x, f, *mm, want=("out_exact", "acc"))
+    xd, fd, t = torch.from_numpy(x).cuda(), torch.from_numpy(f).cuda(), ax.Table(array=lut)
+    call = lambda *a, **kw_: ax.approx_conv2d_with_min_max_vars(xd, fd, *a, [1, s, s, 1], 8, t, pad, dilations=(1, d, d, 1), **kw_)  # noqa: E731
+    y, dbg = call(*mm, debug=True)
+    assert dbg["plan"]["status"] == 0
+    assert np.array_equal(dbg["acc"].cpu().numpy(), ref["acc"])
+    want = torch.from_numpy(ref["out_exact"]).cuda()
+    assert torch.equal(y.view(torch.int32), want.view(torch.int32))
+    # the plain call (another end of the kernel), ranges on the device, and what rides along with a call
+    assert torch.equal(call(*mm).view(torch.int32), want.view(torch.int32))
+    assert torch.equal(call(*[torch.tensor(v, device="cuda") for v in mm]).view(torch.int32), want.view(torch.int32))
+    g = torch.Generator(device="cuda").manual_seed(1)
+    bias, res = torch.randn(co, device="cuda", generator=g), torch.randn(want.shape, device="cuda", generator=g)
+    fused = call(*mm, bias=bias, residual=res, relu=True)
+    assert torch.equal(fused.view(torch.int32), torch.relu(want + bias + res).view(torch.int32))
+    # the plan-based kernels, which a workspace of the smaller size selects
+    ws = torch.zeros(ops.workspace_bytes((n, h, w, c), (kh, kw, c, co), [1, s, s, 1], pad, (1, d, d, 1)), dtype=torch.uint8, device="cuda")
+    if ws.numel() < ops.fast_workspace_bytes((n, h, w, c), (kh, kw, c, co), [1, s, s, 1], pad, (1, d, d, 1)):
+        a, b = call(*mm, input_relu=True), call(*mm, input_relu=True, workspace=ws)
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+def test_unusual_values_and_addresses(built):
+    """NaN, infinities and values outside the range; an input that starts 4 bytes past a 16-byte boundary; a one-value range."""
+    import torch
+    import tf_approximate_b200 as ax
+    from tf_approximate_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.rand((2, 40, 40, 32), device="cuda", generator=g) * 2 - 1
+    x.view(-1)[::997] = float("nan"); x.view(-1)[1::991] = float("inf"); x.view(-1)[2::983] = -float("inf"); x.view(-1)[3::977] = 7.0
+    f = torch.randn((3, 3, 32, 48), device="cuda", generator=g) * 0.1
+    t = ax.Table(array=ax.noisy_table(5))
+    odd = torch.empty(x.numel() + 1, device="cuda")[1:].view(x.shape).copy_(x)
+    for mm in [(-1.0, 1.0, -0.3, 0.3), (0.0, 0.0, -0.3, 0.3), (0.25, 0.75, 0.0, 0.0)]:
+        ws = torch.zeros(ops.workspace_bytes(x.shape, f.shape, [1, 1, 1, 1], "SAME"), dtype=torch.uint8, device="cuda")
+        want = ax.approx_conv2d_with_min_max_vars(x, f, *mm, [1, 1, 1, 1], 8, t, "SAME", workspace=ws)
+        for inp in (x, odd):
+            y = ax.approx_conv2d_with_min_max_vars(inp, f, *mm, [1, 1, 1, 1], 8, t, "SAME")
+            assert torch.equal(torch.isnan(y), torch.isnan(want))
+            assert torch.equal(torch.nan_to_num(y, 0.0).view(torch.int32), torch.nan_to_num(want, 0.0).view(torch.int32))

@@ -13,7 +13,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB = os.path.join(HERE, "libaxconv.so")
 LIB_CHECK = os.path.join(HERE, "libaxconv_check.so")
 OBJDIR = os.path.join(HERE, "build")
-SOURCES = ["axc_api.cu", "axc_conv.cu", "axc_sched.cu", "axc_depthwise.cu", "axc_probe.cu", "axc_qconv.cu", "axc_prologue.cu"]
+SOURCES = ["axc_api.cu", "axc_conv.cu", "axc_sched.cu", "axc_xtab.cu", "axc_depthwise.cu", "axc_probe.cu", "axc_qconv.cu", "axc_prologue.cu"]
 
 
 def needs_build(lib=LIB):

@@ -10,11 +10,14 @@
 
 #include "axc_internal.h"
 #include "axc_sched.h"
+#include "axc_xtab.h"
 
 struct axc_table {
     unsigned uid;
     uint32_t max_entry;          // largest entry
     int common_tz;               // trailing zero bits shared by all entries (16 for an all-zero table)
+    int e_min, e_max;            // smallest and largest distance of an entry from the exact product
+    int c_min, c_max;            // and of an entry from 128 (a + b)
     std::vector<uint16_t> host;  // 65536 entries, index (a << 8) | b
     std::mutex mu;
     std::vector<uint16_t *> dev;  // per-device replica, lazily created
@@ -39,6 +42,35 @@ void stamp(axc_table *t)
     int tz = 0;
     while (tz < 16 && ((ored >> tz) & 1u) == 0u) ++tz;
     t->common_tz = tz;
+    t->e_min = t->c_min = 1 << 20; t->e_max = t->c_max = -(1 << 20);
+    for (int i = 0; i < 65536; ++i) {
+        const int e = int(t->host[size_t(i)]) - (i >> 8) * (i & 255);
+        t->e_min = e < t->e_min ? e : t->e_min;
+        t->e_max = e > t->e_max ? e : t->e_max;
+        const int c = int(t->host[size_t(i)]) - 128 * ((i >> 8) + (i & 255));
+        t->c_min = c < t->c_min ? c : t->c_min;
+        t->c_max = c > t->c_max ? c : t->c_max;
+    }
+}
+
+void table_form(const axc_table *t, int *mode, int *centred, int *e_min)
+{
+    constexpr int kTwoDigits = 254 + 255 * 255;      // largest value of two digits to the base 255
+    const int span = t->e_max - t->e_min;
+    *centred = 0;
+    *e_min = 0;
+    if (span <= 255) {
+        *mode = span == 0 ? kXtabExact : kXtabByte;
+        *e_min = t->e_min;
+    } else if (int(t->max_entry) <= kTwoDigits) {
+        *mode = kXtabFull;
+    } else if (t->c_max - t->c_min <= kTwoDigits) {
+        *mode = kXtabFull;
+        *centred = 1;
+        *e_min = t->c_min;
+    } else {
+        *mode = kXtabNone;
+    }
 }
 
 bool table_sum_exact_in_fp32(const axc_table *t, long long K)
@@ -320,7 +352,7 @@ static int forward(bool depthwise, axc_table *table, const axc_conv_desc *desc, 
     const bool ref_order = !depthwise && ((g.accum == AXC_ACCUM_REFERENCE_F32 && !table_sum_exact_in_fp32(table, g.K)) ||
                                           !table_sum_fits_int32(table, g.K));
     rc = depthwise ? launch_depthwise(lut, g, q, input, filter, output, workspace, dbg, device, cudaStream_t(stream))
-                   : launch_dense(lut, table_uid(table), g, q, ranges_dev, input, filter, output, workspace, dbg, device,
+                   : launch_dense(lut, table, g, q, ranges_dev, input, filter, output, workspace, workspace_bytes, dbg, device,
                                   cudaStream_t(stream), ref_order);
     if (prev != device) cudaSetDevice(prev);
     return rc;
@@ -472,6 +504,19 @@ int axc_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes)
     return AXC_OK;
 }
 
+int axc_conv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_t *bytes)
+{
+    if (!bytes) return AXC_INVALID_ARGUMENT;
+    axc::Geom g;
+    int rc = axc::resolve_geometry(desc, false, &g);
+    if (rc) return rc;
+    *bytes = 0;
+    if (g.M * g.Cout == 0) return AXC_OK;
+    const size_t fast = axc::xtab_scratch_bytes(g), base = axc::dense_workspace_total(g.K, g.Cout, g.M);
+    if (fast > 0) *bytes = fast > base ? fast : base;
+    return AXC_OK;
+}
+
 int axc_depthwise_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes)
 {
     if (!bytes) return AXC_INVALID_ARGUMENT;
@@ -594,14 +639,15 @@ int axc_debug_bounds_record(int device, uint32_t out4[4])
     AXC_CUDA(cudaGetDevice(&prev));
     if (prev != device) AXC_CUDA(cudaSetDevice(device));
     cudaError_t e = cudaDeviceSynchronize();
-    unsigned parts[3][4] = {};
+    unsigned parts[4][4] = {};
     int rc = e == cudaSuccess ? AXC_OK : axc::cuda_failed(e);
     if (rc == AXC_OK) rc = axc::bounds_record_sched(parts[0]);
     if (rc == AXC_OK) rc = axc::bounds_record_conv(parts[1]);
     if (rc == AXC_OK) rc = axc::bounds_record_depthwise(parts[2]);
+    if (rc == AXC_OK) rc = axc::bounds_record_xtab(parts[3]);
     if (prev != device) cudaSetDevice(prev);
     out4[0] = out4[1] = out4[2] = out4[3] = 0;
-    for (int t = 0; t < 3; ++t) {
+    for (int t = 0; t < 4; ++t) {
         if (parts[t][0] != 0 && out4[0] == 0) { out4[1] = parts[t][1]; out4[2] = parts[t][2]; out4[3] = parts[t][3]; }
         out4[0] += parts[t][0];
     }

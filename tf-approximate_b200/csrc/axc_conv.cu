@@ -23,6 +23,7 @@
 
 #include "axc_internal.h"
 #include "axc_sched.h"
+#include "axc_xtab.h"
 
 namespace axc {
 
@@ -575,13 +576,39 @@ static int dense_variant()
     return v;
 }
 
-int launch_dense(const uint16_t *lut_dev, unsigned table_uid, const Geom &g, const Quant &q, const float *ranges_dev,
-                 const float *input, const float *filter, float *output, void *workspace, const axc_debug_out *dbg,
-                 int device, cudaStream_t stream, bool ref_order)
+static int launch_quantize_tap(const float *input, long long n, const DevQuant *dq, uint8_t *qinput, int input_relu, cudaStream_t stream)
+{
+    if (n <= 0) return AXC_OK;
+    const unsigned blocks = unsigned(n / 256 + 1 < 4096 ? n / 256 + 1 : 4096);
+    quantize_tensor_kernel<<<blocks, 256, 0, stream>>>(input, n, dq, qinput, input_relu ? 0.0f : -INFINITY);
+    AXC_CUDA(cudaGetLastError());
+    count_launch();
+    return AXC_OK;
+}
+
+int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g, const Quant &q, const float *ranges_dev,
+                 const float *input, const float *filter, float *output, void *workspace, size_t workspace_bytes,
+                 const axc_debug_out *dbg, int device, cudaStream_t stream, bool ref_order)
 {
     DeviceInfo di;
     int rc = device_info(device, &di);
     if (rc) return rc;
+    if (!ref_order && dense_variant() == 0 && di.max_smem_optin >= 232448 && di.smem_base <= 2048u && di.smem_end >= 233472u) {
+        const size_t need = xtab_scratch_bytes(g);
+        int mode, centred, e_min;
+        table_form(table, &mode, &centred, &e_min);
+        if (need > 0 && workspace_bytes >= need && mode != kXtabNone) {
+            if (dbg && dbg->qinput) {
+                rc = launch_quant(q, ranges_dev, g.K, static_cast<unsigned char *>(workspace), stream);
+                if (rc == AXC_OK)
+                    rc = launch_quantize_tap(input, (long long)g.N * g.H * g.W * g.C,
+                                             reinterpret_cast<const DevQuant *>(static_cast<unsigned char *>(workspace) + kDevQuantOffset),
+                                             dbg->qinput, g.ep.input_relu, stream);
+                if (rc) return rc;
+            }
+            return launch_xtab(lut_dev, mode, centred, e_min, g, q, ranges_dev, input, filter, output, static_cast<unsigned char *>(workspace), dbg, di, stream);
+        }
+    }
     // A caller that wants the integer sums only (output == NULL, the quantised entry point) gets the fp32 value written
     // to the same element of the accumulator tap first and the integer sum over it: the kernels need no test per store.
     const bool ints_only = output == nullptr;
@@ -608,17 +635,12 @@ int launch_dense(const uint16_t *lut_dev, unsigned table_uid, const Geom &g, con
 
     // the quantisation parameters reach the workspace with the first kernel of the plan check, or - without a
     // plan - with a kernel of their own
-    if (scheduled) rc = launch_plan(lut_dev, table_uid, g, q, ranges_dev, filter, plan, L, dbg ? dbg->qfilter : nullptr, stream);
+    if (scheduled) rc = launch_plan(lut_dev, table_uid(table), g, q, ranges_dev, filter, plan, L, dbg ? dbg->qfilter : nullptr, stream);
     else rc = launch_quant(q, ranges_dev, g.K, plan, stream);
     if (rc) return rc;
     if (dbg && dbg->qinput) {
-        const long long n = (long long)g.N * g.H * g.W * g.C;
-        if (n > 0) {
-            const unsigned blocks = unsigned(n / 256 + 1 < 4096 ? n / 256 + 1 : 4096);
-            quantize_tensor_kernel<<<blocks, 256, 0, stream>>>(input, n, dq, dbg->qinput, g.ep.input_relu ? 0.0f : -INFINITY);
-            AXC_CUDA(cudaGetLastError());
-            count_launch();
-        }
+        rc = launch_quantize_tap(input, (long long)g.N * g.H * g.W * g.C, dq, dbg->qinput, g.ep.input_relu, stream);
+        if (rc) return rc;
     }
     if (scheduled) {
         rc = launch_dense_sched(g, input, output, plan, L, dbg ? dbg->acc : nullptr, di, stream);

@@ -68,6 +68,7 @@ namespace axc {
 int bounds_record_sched(unsigned out4[4]);
 int bounds_record_conv(unsigned out4[4]);
 int bounds_record_depthwise(unsigned out4[4]);
+int bounds_record_xtab(unsigned out4[4]);
 
 // Quantisation state of one call: what the reference keeps in
 // BaseTableApproxOpType_t::quantProps (tf2/src/approx_ops_types.h:84-96).
@@ -144,6 +145,9 @@ unsigned table_uid(const axc_table *t);
 // sum is a multiple of 2^tz (tz = trailing zero bits common to all entries) and at most K * largest entry, and
 // fp32 holds every such multiple up to 2^(24 + tz).
 bool table_sum_exact_in_fp32(const axc_table *t, long long K);
+// How an entry is kept in an expanded table (XtabMode); whether it is stored less 128 (a + b) first (16-bit entries only); and
+// what every entry is stored less on top of that (8-bit entries and exact tables: of the exact product).
+void table_form(const axc_table *t, int *mode, int *centred, int *e_min);
 // True when K entries cannot overflow an int32 accumulator.
 bool table_sum_fits_int32(const axc_table *t, long long K);
 
@@ -175,9 +179,10 @@ Workspace depthwise_workspace(int KHW, int C, int mult);
 // ranges_dev: NULL, or {in_min, in_max, f_min, f_max} in device memory (then `q` is ignored).
 // ref_order: add the products up in K order with an fp32 running total (the reference's arithmetic) instead of
 // the exact integer sum.
-int launch_dense(const uint16_t *lut_dev, unsigned table_uid, const Geom &g, const Quant &q, const float *ranges_dev,
-                 const float *input, const float *filter, float *output, void *workspace, const axc_debug_out *dbg,
-                 int device, cudaStream_t stream, bool ref_order);
+// workspace_bytes: what the caller brought; from xtab_scratch_bytes() on the expanded-table kernels serve the call.
+int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g, const Quant &q, const float *ranges_dev,
+                 const float *input, const float *filter, float *output, void *workspace, size_t workspace_bytes,
+                 const axc_debug_out *dbg, int device, cudaStream_t stream, bool ref_order);
 // out = out (+ bias[channel]) (+ residual), then max(out, 0) if relu, in one pass; bias / residual may be NULL
 int launch_post(float *out, const float *bias, const float *residual, long long count, int channels, int relu,
                 const DeviceInfo &di, cudaStream_t stream);

@@ -22,6 +22,7 @@
 #include <cmath>
 
 #include "axc_internal.h"
+#include "axc_quant.cuh"
 #include "axc_sched.h"
 #include <vector>
 
@@ -109,35 +110,6 @@ __device__ __forceinline__ int slot_bank(int s) { return ((s & 127) >> 1) & 31; 
 // ------------------------------------------------------------------------------------------------
 // plan_check: quantisation parameters of the call, quantised filter vs. stored copy, structure of the stored plan
 // ------------------------------------------------------------------------------------------------
-// Range nudging on the device, operation by operation as on the host (axc_api.cu var_quant_props).
-__device__ void dev_var_quant(float min_v, float max_v, float *scale, float *inv, float *offset)
-{
-    float s = 0.0f, i = 0.0f, nudged_min = 0.0f;
-    if (min_v != 0.0f || max_v != 0.0f) {
-        s = __fdiv_rn(__fsub_rn(max_v, min_v), 255.0f);
-        const float zp_from_min = __fsub_rn(0.0f, __fdiv_rn(min_v, s));
-        float zp;
-        if (zp_from_min < 0.0f) zp = 0.0f;
-        else if (zp_from_min > 255.0f) zp = 255.0f;
-        else zp = roundf(zp_from_min);                       // half away from zero, like std::round
-        nudged_min = __fmul_rn(__fsub_rn(0.0f, zp), s);      // a true subtraction: +0.0 for zp == 0
-        i = __fdiv_rn(1.0f, s);
-    }
-    *scale = s; *inv = i; *offset = nudged_min;
-}
-
-__device__ DevQuant dev_quant_from_ranges(const float *__restrict__ ranges, int K)
-{
-    float s1, i1, o1, s2, i2, o2;
-    dev_var_quant(ranges[0], ranges[1], &s1, &i1, &o1);
-    dev_var_quant(ranges[2], ranges[3], &s2, &i2, &o2);
-    DevQuant q;
-    q.in_off = o1; q.in_inv = i1; q.f_off = o2; q.f_inv = i2;
-    q.s1s2 = __fmul_rn(s1, s2); q.m1 = o1; q.m2 = o2;
-    q.km1m2 = __fmul_rn(float(K), __fmul_rn(o1, o2));
-    return q;
-}
-
 // A program word is safe to execute when the shared-memory addresses the kernel forms from it stay inside the
 // table planes, the zero words and the activation buffers, and are aligned: plane byte 1 or 2 with an even column
 // byte, or the idle form (plane byte 3, bit 14 set, column byte a multiple of 4 below 128); activation row offset a
@@ -1202,7 +1174,7 @@ PlanLayout plan_layout(int K, int Cout)
     return L;
 }
 
-static DevQuant host_dev_quant(const Quant &q, int K)
+DevQuant host_dev_quant(const Quant &q, int K)
 {
     DevQuant d;
     d.in_off = q.in_off; d.in_inv = q.in_inv; d.f_off = q.f_off; d.f_inv = q.f_inv;
@@ -1361,6 +1333,7 @@ int plan_info(const void *workspace, int32_t out4[4], cudaStream_t stream)
     PlanHeader h;
     AXC_CUDA(cudaMemcpy(&h, workspace, sizeof(h), cudaMemcpyDeviceToHost));
     out4[0] = h.dirty; out4[1] = h.fallback; out4[2] = h.status; out4[3] = 0;
+    if (h.magic == kXtabMagic) out4[3] = 1000;      // expanded tables: every lookup is one step, there is nothing to build
     if (h.magic == kPlanMagic && h.G > 0 && h.NCH > 0 && h.G * h.NCH <= 65536) {
         const PlanLayout L = plan_layout(h.K, h.Cout);
         std::vector<int> steps(size_t(h.G) * h.NCH);

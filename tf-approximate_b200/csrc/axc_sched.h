@@ -11,6 +11,9 @@ struct Geom;
 struct Quant;
 struct DeviceInfo;
 
+// `magic` of the header that the expanded-table kernels leave in their scratch (axc_xtab.cu).
+constexpr uint32_t kXtabMagic = 0x41585430u;   // "AXT0"
+
 // K elements per schedule chunk: a program word addresses activation rows 0..1023 (8 zero rows + the chunk).
 constexpr int kMaxChunk = 1016;
 
@@ -49,6 +52,8 @@ __host__ __device__ inline bool plan_group_dual(int g, int G, int Cout, int K)
 {
     return g == G - 1 && (G % 4) == 1 && Cout - 32 * g <= 16 && (G == 1 || K <= 152);
 }
+
+DevQuant host_dev_quant(const Quant &q, int K);
 
 // Writes the DevQuant block of `plan`: from the host values `q`, or - when ranges_dev is given - on the device
 // from {in_min, in_max, f_min, f_max} read there (same arithmetic as the host: tf2/src/approx_ops_types.h:29-49,135-197).

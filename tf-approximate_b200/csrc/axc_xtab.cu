@@ -1,0 +1,1309 @@
+// Expanded-table dense convolution for sm_100a.
+//
+// Per K element a convolution looks the activations of its output pixels up in the table column of one weight per
+// output channel.  For a group of channels and 8 consecutive K elements those columns are laid side by side in shared
+// memory as an expanded table X[a][k][channel]: 256 rows of 8 x 16 bytes, where the 16 bytes at (a, k) are the entries of
+// 8 channels (16-bit entries) or 16 channels (8-bit entries).  One LDS.128 per lane then returns 8 or 16 lookups, and
+// since the 8 lanes of a quarter warp work on 8 different k, they read 8 different 16-byte bank groups whatever
+// the activations are: every load is conflict-free and carries 128 useful bytes per clock.  The sums are taken by the
+// tensor cores: the bytes of four lanes (four k of one pixel) are the A operand of an m16n8k32 u8 MMA against a constant
+// matrix that adds the bytes of a channel into its accumulator.
+//
+// What is looked up (whole numbers throughout, so the total is the same):
+//   8-bit entries    where the table differs from the exact product by values that span at most 255: that distance less its
+//                    minimum.  The exact products are added by further MMAs on the codes themselves (one per 16 K elements,
+//                    8 pixels and 16 channels).
+//   16-bit entries   two digits to the base 255, so that one MMA with the weights 1 and 255 adds both into a single
+//                    accumulator (256 does not fit a u8 operand; low and high bytes in accumulators of their own would
+//                    halve the pixels a tile can hold).  A table that reaches past 65279 is stored less 128 (a + b) and its
+//                    minimum; 128 times the sums of the activation and weight codes go back in at the end.
+//   nothing          for an exact table: only the products.
+//
+// Bound: the shared-memory pipe, 64 lookups (16-bit) or 128 lookups (8-bit) per clock and SM, less what the expansion costs:
+// 32 KiB read and 32 KiB written per 8 K elements and channel group, 512 clocks against one clock per pixel of the tile for the
+// lookups - hence tiles of up to 2048 pixels.  Measured on a B200: LDS.128 alone 4.02 clocks per warp instruction, LDS.128 + MMA
+// 4.05 (the MMA pipe is half idle), against 4.50 with eight dp2a in the MMA's place.  A 16-bit lookup per lane and
+// instruction (axc_sched.cu) cannot pass 32 per clock.
+//
+//   xprep_kernel   one pass over the input: 8-bit codes in pixel order (or the im2col rows where the channel count would
+//                  waste a quarter of the 16-byte pieces), the patch sums of the dequantisation in the reference's order
+//                  of additions; further blocks: quantised filter, transposed table, filter sums
+//   xtab_kernel    the convolution; the transposed table (one row per weight) stays in shared memory
+//   xfinal_kernel  only where K is split over CTAs: adds nothing, dequantises the integer sums
+//
+// Arithmetic (quantiser, table index, dequantisation) is the reference's, tf2/src/approx_nn_conv_kernels.cpp:167-296.
+#include <cmath>
+#include <type_traits>
+
+#include "axc_quant.cuh"
+#include "axc_sched.h"
+#include "axc_xtab.h"
+
+namespace axc {
+
+namespace {
+
+// Shared window of a CTA (the host checks that it starts below 2 KiB and reaches 228 KiB):
+//   [first byte, 3072)    barriers
+//   [3072, 35840)         codes of the tile's pixels for 16 elements of K (exact table: four of them, up to 134144)
+//   [35840, 65536)        transposed table, rows 0..57 (16-bit entries)
+//   [65536, 131072)       two expanded tables, interleaved: row a of stage s at a*256 + s*128, so that an address is
+//                         {offset in the row, a, 1, 0} and one byte permute puts the activation in
+//   [131072, 232960)      transposed table, the other rows (8-bit entries: all 257 rows)
+// With expanded tables from global memory: codes from 3072 up to 52224, tables of two chunks at 65536 and 131072, a chunk's
+// two octets interleaved like the two stages above.
+constexpr unsigned kCodes = 3072u;
+constexpr unsigned kRowsLow = 35840u;
+constexpr unsigned kTab = 65536u;
+constexpr unsigned kRowsHigh = 131072u;
+constexpr unsigned kWindowEnd = 233472u;
+constexpr int kLowRows = 58;
+constexpr int kWarps = 8;
+constexpr int kNull = 256;                     // table row of a weight that does not exist: all zeros
+static_assert(kRowsLow + kLowRows * 512u == kTab && kRowsHigh + (257u - kLowRows) * 512u <= kWindowEnd, "shared window");
+constexpr int kWaitPolls = 1 << 20;
+constexpr size_t kPartialMax = 64u << 20;      // integer sums of a call whose K is split over CTAs
+constexpr double kXtabMinLookups = 8e6;
+constexpr size_t kXtMax = 640u << 20;          // expanded tables in global memory
+constexpr int kModelSms = 148;                 // what the scratch size is computed for
+
+// ---- shared memory -----------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint4 lds128(unsigned addr)
+{
+    if (!AXC_SHARED_OK(addr, 16u, 0u, kWindowEnd, 301u)) return make_uint4(0, 0, 0, 0);
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void sts64(unsigned addr, unsigned x, unsigned y)
+{
+    if (!AXC_SHARED_OK(addr, 8u, 0u, kWindowEnd, 306u)) return;
+    asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(addr), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ unsigned lds32(unsigned addr)
+{
+    if (!AXC_SHARED_OK(addr, 4u, 0u, kWindowEnd, 302u)) return 0u;
+    unsigned v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void sts128(unsigned addr, uint4 v)
+{
+    if (!AXC_SHARED_OK(addr, 16u, 0u, kWindowEnd, 303u)) return;
+    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+// 16 bytes global -> shared, zeros where `bytes` is 0
+__device__ __forceinline__ void cp_async16(unsigned dst, const void *src, unsigned bytes)
+{
+    if (!AXC_SHARED_OK(dst, 16u, 0u, kWindowEnd, 304u)) return;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+// `bytes` (a multiple of 16) global -> shared by the bulk copy engine, counted on `bar`
+__device__ __forceinline__ void bulk_copy(unsigned dst, const void *src, unsigned bytes, unsigned bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Waits for the phase `parity`; gives up after about a second (`ok` stays false from then on, later waits return at once)
+__device__ __forceinline__ void mbar_wait(unsigned bar, unsigned parity, bool &ok)
+{
+    for (int it = 0; ok; ++it) {
+        unsigned done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        if (done) return;
+        if (it >= kWaitPolls) ok = false;
+    }
+}
+
+template <unsigned SEL>
+__device__ __forceinline__ unsigned prmt(unsigned a, unsigned b)
+{
+    unsigned d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "n"(SEL));
+    return d;
+}
+__device__ __forceinline__ unsigned prmt_r(unsigned a, unsigned b, unsigned sel)
+{
+    unsigned d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
+}
+__device__ __forceinline__ void mma_k32(int (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1)
+{
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// The 8-bit code of x: trunc((x - off) * inv + 0.5) with three separately rounded operations
+// (tf2/src/approx_nn_conv_kernels.cpp:293), clamped to 0..255, NaN -> 0.  Adding 2^23 with rounding towards minus infinity
+// leaves the integer part in the low mantissa bits: full-rate instructions in place of a conversion.
+__device__ __forceinline__ unsigned code_of(float x, float off, float inv)
+{
+    const float v = __fadd_rn(__fmul_rn(__fsub_rn(x, off), inv), 0.5f);
+    return __float_as_uint(__fadd_rd(fminf(fmaxf(v, 0.0f), 255.0f), 8388608.0f)) & 0xFFu;
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// preparation
+// ------------------------------------------------------------------------------------------------------------------
+struct XGeom {
+    int N, H, W, C, KH, KW, Cout, sh, sw, dh, dw, ph, pw, OH, OW, K, M;
+    int CC;             // 16-byte pieces of codes per pixel (im2col: per output pixel)
+    int chunks;         // 16-element steps of K: KH*KW*CC, or CC with im2col
+    int im2col;
+    int TNC;            // channels per tile: 8 (16-bit entries) or 16
+    int tiles_n;
+};
+
+struct PrepParams {
+    XGeom g;
+    const float *input, *filter;
+    const uint16_t *lut;
+    const float *ranges;
+    DevQuant host_q;
+    float in_floor;
+    int mode, centred, e_min;
+    int *acode, *bcode;         // sums of activation / weight codes (centred tables), else NULL
+    unsigned char *codes, *tt;
+    uint16_t *wrow;
+    uint2 *wb;
+    float *asum, *bsum;
+    uint8_t *qf_debug;
+    PlanHeader *hdr;
+    int blocks_sum, blocks_w, blocks_t;      // leading blocks; the rest are input tiles
+    int TH, TW, tiles_y, tiles_x, RH, RW, pitch, vec;
+};
+
+// channel of slot s in a piece: the order in which a lane's accumulators hold four neighbouring channels
+__device__ __forceinline__ int slot_channel(int mode, int s)
+{
+    if (mode == kXtabFull) return s;
+    return ((s >> 3) << 3) + ((s >> 1) & 1) * 4 + ((s >> 2) & 1) * 2 + (s & 1);     // 0 1 4 5 2 3 6 7 8 9 12 13 10 11 14 15
+}
+
+// shared-memory address of a row of the transposed table
+__device__ __forceinline__ unsigned row_address(int mode, unsigned row)
+{
+    if (mode != kXtabFull) return kRowsHigh + row * 256u;
+    return row < unsigned(kLowRows) ? kRowsLow + row * 512u : kRowsHigh + (row - kLowRows) * 512u;
+}
+
+// K index of element i of chunk ch, or -1 where there is none
+__device__ __forceinline__ int k_of(const XGeom &g, int ch, int i)
+{
+    if (g.im2col) {
+        const int k = ch * 16 + i;
+        return k < g.K ? k : -1;
+    }
+    const int tap = ch / g.CC, c = (ch - tap * g.CC) * 16 + i;
+    return c < g.C ? tap * g.C + c : -1;
+}
+
+// Filter sums in l order (tf2/src/approx_nn_conv_kernels.cpp:187-197), 32 channels per block: the whole block stages 256
+// rows at a time, one warp adds (a chain of K additions per channel; the staging hides the memory latency behind it).
+__device__ void prep_filter_sums(const PrepParams &P, const DevQuant &q, int block, float *stage)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = block * 32 + lane;
+    float acc = 0.0f;
+    int codes = 0;
+    float v[32];
+    auto fetch = [&](int l0) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+            const int l = l0 + e * 8 + warp;
+            v[e] = (l < P.g.K && j < P.g.Cout) ? __ldg(P.filter + (size_t)l * P.g.Cout + j) : 0.0f;
+        }
+    };
+    fetch(0);
+    for (int l0 = 0; l0 < P.g.K; l0 += 256) {
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+            stage[(e * 8 + warp) * 32 + lane] = v[e];
+            if (P.bcode && l0 + e * 8 + warp < P.g.K) codes += int(code_of(v[e], q.f_off, q.f_inv));
+        }
+        __syncthreads();
+        if (l0 + 256 < P.g.K) fetch(l0 + 256);
+        if (warp == 0) {
+            const int n = min(256, P.g.K - l0);
+            int l = 0;
+            for (; l + 16 <= n; l += 16) {
+                float u[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) u[e] = stage[(l + e) * 32 + lane];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) acc = __fadd_rn(acc, u[e]);
+            }
+            for (; l < n; ++l) acc = __fadd_rn(acc, stage[l * 32 + lane]);
+        }
+    }
+    if (warp == 0 && j < P.g.Cout) P.bsum[j] = acc;
+    if (P.bcode) {
+        int *sums = reinterpret_cast<int *>(stage);
+        __syncthreads();
+        sums[warp * 32 + lane] = codes;
+        __syncthreads();
+        if (warp == 0 && j < P.g.Cout) {
+            for (int w = 1; w < 8; ++w) codes += sums[w * 32 + lane];
+            P.bcode[j] = codes;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
+{
+    extern __shared__ __align__(16) float prep_smem[];
+    const XGeom &g = P.g;
+    const int tid = threadIdx.x;
+    const DevQuant q = P.ranges ? dev_quant_from_ranges(P.ranges, g.K) : P.host_q;
+    int b = int(blockIdx.x);
+    if (b == 0 && tid == 0) {
+        // header: the parameters of the call; every lookup is one conflict-free step, no plan to rebuild
+        *reinterpret_cast<DevQuant *>(reinterpret_cast<unsigned char *>(P.hdr) + kDevQuantOffset) = q;
+        P.hdr->magic = kXtabMagic;
+        P.hdr->dirty = 0; P.hdr->fallback = 0; P.hdr->status = 0;
+    }
+    if (b < P.blocks_sum) {
+        prep_filter_sums(P, q, b, prep_smem);
+        return;
+    }
+    b -= P.blocks_sum;
+    if (b < P.blocks_w) {
+        // wrow[tile][chunk][octet][k][slot]: where the table row of the slot's weight lies, in 16-byte units; wb[tile][chunk][lane]: the weight
+        // codes as B operand of the exact products
+        const int per_chunk = 16 * g.TNC;
+        const long long total = (long long)g.tiles_n * g.chunks * per_chunk;
+        for (long long x = (long long)b * 256 + tid; x < total; x += (long long)P.blocks_w * 256) {
+            const long long tc = x / per_chunk;
+            const int r = int(x - tc * per_chunk);
+            const int nt = int(tc / g.chunks), ch = int(tc - (long long)nt * g.chunks);
+            const int slot = r % g.TNC, kk = r / g.TNC;                          // kk = octet * 8 + t + 4p
+            const int i = ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);     // element 4t + 2*octet + p
+            const int j = nt * g.TNC + slot_channel(P.mode, slot), k = k_of(g, ch, i);
+            unsigned row = kNull;
+            if (k >= 0 && j < g.Cout) {
+                row = code_of(__ldg(P.filter + (size_t)k * g.Cout + j), q.f_off, q.f_inv);
+                if (P.qf_debug) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(row);
+            }
+            P.wrow[x] = uint16_t(row_address(P.mode, row) >> 4);
+            if (P.mode != kXtabFull) {
+                // B operand half h, column n: channel (n>>1)*4 + 2h + (n&1); lane (n, t) holds elements 4t..4t+3
+                const int cj = slot_channel(P.mode, slot), t = i >> 2, h = (cj >> 1) & 1, n = (cj >> 2) * 2 + (cj & 1);
+                unsigned char *w = reinterpret_cast<unsigned char *>(P.wb + tc * 32 + n * 4 + t) + h * 4 + (i & 3);
+                *w = row == kNull ? 0 : (unsigned char)row;
+            }
+        }
+        return;
+    }
+    b -= P.blocks_w;
+    const unsigned z = code_of(0.0f, q.in_off, q.in_inv);        // code of a tap outside the image; codes are stored xor z
+    if (b < P.blocks_t) {
+        // transposed table: row = weight, column = stored code; row 256 = zeros
+        const int total = 257 * 256;
+        for (int x = b * 256 + tid; x < total; x += P.blocks_t * 256) {
+            const int w = x >> 8, a = (x & 255) ^ int(z);
+            const int less = (P.mode == kXtabFull ? 128 * (a + w) * P.centred : a * w) + P.e_min;
+            const int v = w < 256 ? int(__ldg(P.lut + a * 256 + w)) - less : 0;
+            if (P.mode == kXtabFull) reinterpret_cast<uint16_t *>(P.tt)[x] = uint16_t(v % 255 + (v / 255) * 256);
+            else P.tt[x] = (unsigned char)v;
+        }
+        return;
+    }
+    b -= P.blocks_t;
+
+    // ---- an input tile: TH x TW output pixels of one image, the taps they read staged in shared memory ----------------
+    const int tx = b % P.tiles_x, rest = b / P.tiles_x;
+    const int ty = rest % P.tiles_y, n = rest / P.tiles_y;
+    const int oy0 = ty * P.TH, ox0 = tx * P.TW;
+    const int iy0 = oy0 * g.sh - g.ph, ix0 = ox0 * g.sw - g.pw;
+    // codes of the region's input pixels are written by the tile whose region starts closest before them
+    const int own_h = ty + 1 < P.tiles_y ? P.TH * g.sh : P.RH, own_w = tx + 1 < P.tiles_x ? P.TW * g.sw : P.RW;
+    const unsigned zz = z * 0x01010101u;
+    // codes[piece][pixel][16]: the pieces of neighbouring pixels lie side by side, so that the producers read whole lines
+    const int planes = g.N * g.H * g.W;
+    // centred tables: the sum of the codes of every staged pixel (z for one outside the image) behind the staged taps
+    int *pix_codes = reinterpret_cast<int *>(prep_smem + P.RH * P.RW * P.pitch);
+    if (P.acode && !g.im2col) {
+        for (int x = tid; x < P.RH * P.RW; x += 256) pix_codes[x] = 0;
+        __syncthreads();
+    }
+    if (P.vec) {
+        const int C4 = g.C >> 2;
+        int lp = 1;
+        while (lp < C4 && lp < 32) lp <<= 1;                      // lanes per pixel
+        const int px_step = 256 / lp, c_lane = tid & (lp - 1);
+        const int p = tid / lp;
+        int ry = p / P.RW, rx = p - ry * P.RW, c4 = c_lane;
+        const int step_y = px_step / P.RW, step_x = px_step - step_y * P.RW;
+        // eight pieces are requested before the first is used: the tile's load is a chain of memory latencies otherwise
+        // (cfg 56x56x64, 64 images: 63 us with one in flight)
+        constexpr int kBatch = 8;
+        while (ry < P.RH) {
+            float4 v[kBatch];
+            int at[kBatch];                                       // float offset in the staged region, -1: nothing
+            int code_at[kBatch];                                  // word offset of the codes, -1: not this tile's
+            int local[kBatch];                                    // pixel of the region
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                at[u] = -1; code_at[u] = -1; local[u] = 0;
+                if (ry < P.RH && c4 < C4) {
+                    const int iy = iy0 + ry, ix = ix0 + rx;
+                    local[u] = ry * P.RW + rx;
+                    at[u] = local[u] * P.pitch + c4 * 4;
+                    if (unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W)) {
+                        const int pix = (n * g.H + iy) * g.W + ix;
+                        v[u] = __ldg(reinterpret_cast<const float4 *>(P.input + (long long)pix * g.C) + c4);
+                        if (ry < own_h && rx < own_w && !g.im2col) code_at[u] = ((c4 >> 2) * planes + pix) * 4 + (c4 & 3);
+                    }
+                }
+                c4 += lp;
+                if (c4 >= C4) {
+                    c4 = c_lane;
+                    rx += step_x; ry += step_y;
+                    if (rx >= P.RW) { rx -= P.RW; ++ry; }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                v[u].x = max_keep_nan(v[u].x, P.in_floor); v[u].y = max_keep_nan(v[u].y, P.in_floor);
+                v[u].z = max_keep_nan(v[u].z, P.in_floor); v[u].w = max_keep_nan(v[u].w, P.in_floor);
+                if (at[u] >= 0) *reinterpret_cast<float4 *>(prep_smem + at[u]) = v[u];
+                if (code_at[u] >= 0 || (P.acode && at[u] >= 0 && !g.im2col)) {
+                    const unsigned w = code_of(v[u].x, q.in_off, q.in_inv) | code_of(v[u].y, q.in_off, q.in_inv) << 8 |
+                                       code_of(v[u].z, q.in_off, q.in_inv) << 16 | code_of(v[u].w, q.in_off, q.in_inv) << 24;
+                    if (code_at[u] >= 0) reinterpret_cast<unsigned *>(P.codes)[(unsigned)code_at[u]] = w ^ zz;
+                    if (P.acode) atomicAdd(pix_codes + local[u], int(__dp4a(w, 0x01010101u, 0u)));
+                }
+            }
+        }
+    } else {
+        const int row = P.RW * g.C;
+        for (int x = tid; x < P.RH * row; x += 256) {
+            const int ry = x / row, e = x - ry * row, rx = e / g.C, c = e - rx * g.C;
+            const int iy = iy0 + ry, ix = ix0 + rx;
+            const bool inside = unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W);
+            const long long pix = ((long long)n * g.H + iy) * g.W + ix;
+            float v = inside ? __ldg(P.input + pix * g.C + c) : 0.0f;
+            v = max_keep_nan(v, P.in_floor);
+            prep_smem[(ry * P.RW + rx) * P.pitch + c] = v;
+            if (P.acode && !g.im2col) atomicAdd(pix_codes + ry * P.RW + rx, int(code_of(v, q.in_off, q.in_inv)));
+            if (inside && ry < own_h && rx < own_w && !g.im2col)
+                P.codes[((long long)(c >> 4) * planes + pix) * 16 + (c & 15)] = (unsigned char)(code_of(v, q.in_off, q.in_inv) ^ z);
+        }
+    }
+    __syncthreads();
+    // patch sums (tf2/src/approx_nn_conv_kernels.cpp:272-295): the raw taps in K order, one thread per output pixel
+    for (int o = tid; o < P.TH * P.TW; o += 256) {
+        const int ly = o / P.TW, lx = o - ly * P.TW;
+        const int oy = oy0 + ly, ox = ox0 + lx;
+        if (oy >= g.OH || ox >= g.OW) continue;
+        const long long m = ((long long)n * g.OH + oy) * g.OW + ox;
+        float s = 0.0f;
+        int codes = 0;
+        if (!g.im2col) {
+            if (P.acode)
+                for (int ky = 0; ky < g.KH; ++ky)
+                    for (int kx = 0; kx < g.KW; ++kx) codes += pix_codes[(ly * g.sh + ky * g.dh) * P.RW + lx * g.sw + kx * g.dw];
+            for (int ky = 0; ky < g.KH; ++ky)
+                for (int kx = 0; kx < g.KW; ++kx) {
+                    const float *src = prep_smem + ((ly * g.sh + ky * g.dh) * P.RW + lx * g.sw + kx * g.dw) * P.pitch;
+                    if (P.vec) {
+#pragma unroll 4
+                        for (int c = 0; c < g.C; c += 4) {
+                            const float4 v = *reinterpret_cast<const float4 *>(src + c);
+                            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
+                        }
+                    } else {
+#pragma unroll 4
+                        for (int c = 0; c < g.C; ++c) s = __fadd_rn(s, src[c]);
+                    }
+                }
+        } else {
+            unsigned w[4] = {0, 0, 0, 0};
+            int i = 0;
+            uint4 *dst = reinterpret_cast<uint4 *>(P.codes) + m;
+            for (int ky = 0; ky < g.KH; ++ky)
+                for (int kx = 0; kx < g.KW; ++kx) {
+                    const float *src = prep_smem + ((ly * g.sh + ky * g.dh) * P.RW + lx * g.sw + kx * g.dw) * P.pitch;
+                    for (int c = 0; c < g.C; ++c) {
+                        const float v = src[c];
+                        s = __fadd_rn(s, v);
+                        const unsigned code = code_of(v, q.in_off, q.in_inv), byte = (code ^ z) << 24;
+                        codes += int(code);
+                        // four words shift along: the newest byte enters at the top of w[3]
+                        w[0] = __funnelshift_r(w[0], w[1], 8); w[1] = __funnelshift_r(w[1], w[2], 8);
+                        w[2] = __funnelshift_r(w[2], w[3], 8); w[3] = (w[3] >> 8) | byte;
+                        if (++i == 16) {
+                            *dst = make_uint4(w[0], w[1], w[2], w[3]);
+                            dst += g.M;
+                            i = 0;
+                        }
+                    }
+                }
+            if (i > 0) {
+                for (; i < 16; ++i) {
+                    w[0] = __funnelshift_r(w[0], w[1], 8); w[1] = __funnelshift_r(w[1], w[2], 8);
+                    w[2] = __funnelshift_r(w[2], w[3], 8); w[3] >>= 8;
+                }
+                *dst = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        }
+        P.asum[m] = s;
+        if (P.acode) P.acode[m] = codes;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// expanded tables in global memory, for calls with enough pixels to use each of them several times
+// ------------------------------------------------------------------------------------------------------------------
+struct ExpandParams {
+    XGeom g;
+    const float *filter;
+    const uint16_t *lut;
+    const float *ranges;
+    DevQuant host_q;
+    int centred, e_min;
+    unsigned char *xt;
+    uint2 *wb;
+    uint8_t *qf_debug;
+};
+
+// xt[channel tile][chunk][row a][piece kk][16 bytes], kk = octet * 8 + k.  The table as it is looked up (rows moved by xor z)
+// lies in shared memory; a thread gathers the entries of its piece's 8 or 16 weights and writes 16 bytes, 16 threads the
+// 256 bytes of a row.  Bound by the gathers (random banks) and, close behind, by the writes: 64 KiB per chunk.
+template <int MODE>
+__global__ void __launch_bounds__(256) xexpand_kernel(const ExpandParams P)
+{
+    constexpr int TNC = MODE == kXtabFull ? 8 : 16;
+    using Entry = typename std::conditional<MODE == kXtabFull, uint16_t, uint8_t>::type;
+    extern __shared__ __align__(16) unsigned char expand_smem[];
+    Entry *tab = reinterpret_cast<Entry *>(expand_smem);
+    const XGeom &g = P.g;
+    const int tid = threadIdx.x;
+    const DevQuant q = P.ranges ? dev_quant_from_ranges(P.ranges, g.K) : P.host_q;
+    const int z = int(code_of(0.0f, q.in_off, q.in_inv));
+    for (int x = tid; x < 8192; x += 256) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(P.lut) + x);
+        const unsigned w4[4] = {v.x, v.y, v.z, v.w};
+        const int a = x >> 5, b0 = (x & 31) * 8;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int entry = int((w4[e >> 1] >> (16 * (e & 1))) & 0xFFFFu), b = b0 + e;
+            const int d = entry - (MODE == kXtabFull ? 128 * (a + b) * P.centred : a * b) - P.e_min;
+            tab[(a ^ z) * 256 + b] = MODE == kXtabFull ? Entry(d % 255 + (d / 255) * 256) : Entry(d);
+        }
+    }
+    __syncthreads();
+    const int kk = tid & 15, a0 = tid >> 4;
+    const int i = ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);             // element 4t + 2*octet + p
+    const int total = g.tiles_n * g.chunks;
+    for (int tc = int(blockIdx.x); tc < total; tc += int(gridDim.x)) {
+        const int nt = tc / g.chunks, ch = tc - nt * g.chunks;
+        const int k = k_of(g, ch, i);
+        unsigned code[TNC];
+        unsigned mask = 0;
+#pragma unroll
+        for (int s = 0; s < TNC; ++s) {
+            const int j = nt * TNC + slot_channel(MODE, s);
+            code[s] = 0;
+            if (k >= 0 && j < g.Cout) {
+                code[s] = code_of(__ldg(P.filter + (size_t)k * g.Cout + j), q.f_off, q.f_inv);
+                mask |= 1u << s;
+                if (P.qf_debug && a0 == 0) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(code[s]);
+            }
+            if (MODE != kXtabFull && a0 == 0) {
+                const int cj = slot_channel(MODE, s), t = i >> 2, h = (cj >> 1) & 1, n = (cj >> 2) * 2 + (cj & 1);
+                reinterpret_cast<unsigned char *>(P.wb + (size_t)tc * 32 + n * 4 + t)[h * 4 + (i & 3)] = (unsigned char)code[s];
+            }
+        }
+        uint4 *dst = reinterpret_cast<uint4 *>(P.xt + (size_t)tc * 65536u) + kk;
+#pragma unroll 2
+        for (int a = a0; a < 256; a += 16) {
+            unsigned w[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int s = 0; s < TNC; ++s) {
+                const unsigned v = ((mask >> s) & 1u) ? unsigned(tab[a * 256 + code[s]]) : 0u;
+                w[s / (TNC / 4)] |= v << ((s % (TNC / 4)) * (128 / TNC));
+            }
+            dst[a * 16] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// the convolution
+// ------------------------------------------------------------------------------------------------------------------
+struct XParams {
+    XGeom g;
+    const unsigned char *codes, *tt;
+    const uint16_t *wrow;
+    const uint2 *wb;
+    const unsigned char *xt;    // expanded tables [channel tile][chunk][256][2 octets][8][16], or NULL: built by the CTAs
+    const float *asum, *bsum;
+    const PlanHeader *hdr;
+    float *output;              // NULL: integer sums only
+    int32_t *acc_out;
+    int32_t *partial;           // K split over CTAs: integer sums are added here
+    const float *bias, *residual;
+    float out_floor;
+    int plain;                  // fp32 output only, it and the shortcut at 16-byte boundaries
+    int k_e_min;                // K times what every entry was stored less
+    const int *acode, *bcode;   // centred tables: sums of codes, 128 of which every lookup was stored less; else NULL
+    int splits, chunks_per_split;
+    long long units;            // pixel tiles x channel tiles x splits
+};
+
+// ((S*s1s2 + m2*aSum) + m1*bSum) - K*m1m2, then what the op's callers add
+__device__ __forceinline__ float dequantise(const DevQuant &Q, int total, float a_sum, float t2)
+{
+    return __fsub_rn(__fadd_rn(__fadd_rn(__fmul_rn(float(total), Q.s1s2), __fmul_rn(Q.m2, a_sum)), t2), Q.km1m2);
+}
+
+// MODE: XtabMode.  NB: blocks of 8 pixels per warp (tile = 64*NB pixels).
+// Warp w holds the sums of pixels [w*8*NB, (w+1)*8*NB) x all channels of the tile in 2*NB (16-bit entries) or 4*NB registers
+// per lane.  Lane (g, t) = (lane / 4, lane % 4) looks pixel g of a block up at k = t and t + 4 of an octet; even and odd g take
+// the two in opposite order, so that a quarter warp covers all 8 k at once.
+// All warps are alike: each builds an eighth of the next octet's expanded table, in four rounds between its own lookups, and
+// fetches the codes of its own pixels.  Eight warps with 255 registers rather than sixteen with 128: the loads of the next two
+// block pairs are in flight while the MMAs of the last two run.
+// PRE: the expanded tables come from global memory (xexpand_kernel) by bulk copies, 64 KiB per 16 elements of K, which cost the
+// shared-memory pipe next to nothing (measured: 2 to 4 % beside a stream of LDS.128 + MMA); otherwise they are built here.
+template <int MODE, int NB, bool PRE>
+__global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
+{
+    constexpr int kPix = kWarps * 8 * NB;
+    constexpr int TNC = MODE == kXtabFull ? 8 : 16, HV = TNC / 8;
+    constexpr bool kTables = MODE != kXtabExact, kBuild = kTables && !PRE;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const XGeom &g = P.g;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned dyn0 = (unsigned)__cvta_generic_to_shared(smem_raw);
+    unsigned dyn_size;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_size));
+    const unsigned bars = (dyn0 + 15u) & ~15u;
+    const unsigned tab_full = bars, tab_empty = bars + 16u, rows_full = bars + 32u;
+    if (rows_full + 8u > kCodes || dyn0 + dyn_size < kWindowEnd) {
+        if (tid == 0) atomicExch(const_cast<int *>(&P.hdr->status), 2);
+        return;
+    }
+    if (tid == 0) {
+        for (int s = 0; s < 2; ++s) { mbar_init(tab_full + s * 8, PRE ? 1 : kWarps); mbar_init(tab_empty + s * 8, kWarps); }
+        mbar_init(rows_full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (kBuild) {
+            // the transposed table stays for the CTA's lifetime
+            constexpr unsigned low = MODE == kXtabFull ? kLowRows * 512u : 0u, high = MODE == kXtabFull ? (257u - kLowRows) * 512u : 257u * 256u;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(rows_full), "r"(low + high) : "memory");
+            if (low > 0) bulk_copy(kRowsLow, P.tt, low, rows_full);
+            bulk_copy(kRowsHigh, P.tt + low, high, rows_full);
+        }
+    }
+    __syncthreads();
+    bool ok = true;
+    const unsigned units = unsigned(P.units);
+
+    // unit number -> split of K, channel tile, first pixel, chunks
+    auto coords = [&](unsigned u, int &nt, int &m0, int &c_begin, int &c_end) {
+        const unsigned u2 = u / unsigned(P.splits), sp = u - u2 * unsigned(P.splits), mt = u2 / unsigned(g.tiles_n);
+        nt = int(u2 - mt * unsigned(g.tiles_n));
+        m0 = int(mt) * kPix;
+        c_begin = int(sp) * P.chunks_per_split;
+        c_end = min(g.chunks, c_begin + P.chunks_per_split);
+    };
+
+    // ---- codes: this warp's pixels, 16 elements of K at a time, one chunk ahead --------------------------------------
+    constexpr int PPL = (NB * 8 + 31) / 32;                        // pixels per lane
+    const int pieces = g.im2col ? g.M : g.N * g.H * g.W;           // distance of the 16-byte pieces of one pixel
+    const int eh = g.im2col ? 1 : g.H, ew = g.im2col ? 1 : g.W;
+    const unsigned my_codes = kCodes + unsigned(warp) * (NB * 8 * 16u);
+    int f_base[PPL], f_yx[PPL];                                    // pixel number of the patch origin, its row and column
+    unsigned f_unit = blockIdx.x;
+    int f_left = 0, f_cc = 0, f_ky = 0, f_kx = 0;
+    auto fetch_unit = [&]() {
+        int nt, m0, c_begin, c_end;
+        coords(f_unit, nt, m0, c_begin, c_end);
+        f_left = c_end - c_begin;
+        f_cc = c_begin; f_ky = 0; f_kx = 0;
+        if (!g.im2col) {
+            const int tap = c_begin / g.CC;
+            f_cc = c_begin - tap * g.CC;
+            f_ky = tap / g.KW;
+            f_kx = tap - f_ky * g.KW;
+        }
+#pragma unroll
+        for (int i = 0; i < PPL; ++i) {
+            const int m = m0 + warp * (NB * 8) + i * 32 + lane;
+            int b = 0, y = -32768, x = 0;                          // no pixel: every tap out of range
+            if (m < g.M && i * 32 + lane < NB * 8) {
+                b = m; y = 0;
+                if (!g.im2col) {
+                    const unsigned mm = unsigned(m), row = mm / unsigned(g.OW), n = row / unsigned(g.OH);
+                    y = int(row - n * unsigned(g.OH)) * g.sh - g.ph;
+                    x = int(mm - row * unsigned(g.OW)) * g.sw - g.pw;
+                    b = (int(n) * g.H + y) * g.W + x;
+                }
+            }
+            f_base[i] = b;
+            f_yx[i] = (y << 16) | (x & 0xFFFF);
+        }
+    };
+    // One chunk is asked for in PPL pieces (the caller spreads them over its lookups): fetch_begin() finds the chunk,
+    // fetch_pixel(i, dst) asks for the lane's i-th pixel.
+    bool f_active = false;
+    int f_off = 0, f_dy = 0, f_dx = 0;
+    auto fetch_begin = [&]() {
+        f_active = false;
+        if (f_left == 0) {
+            f_unit += gridDim.x;
+            if (f_unit >= units) return;
+            fetch_unit();
+        }
+        f_active = true;
+        f_dy = f_ky * g.dh; f_dx = f_kx * g.dw;
+        f_off = f_dy * g.W + f_dx + f_cc * pieces;
+        if (++f_cc == g.CC && !g.im2col) { f_cc = 0; if (++f_kx == g.KW) { f_kx = 0; ++f_ky; } }
+        --f_left;
+    };
+    auto fetch_pixel = [&](int i, unsigned dst) {
+        if (!f_active || (NB * 8 < 32 && lane >= NB * 8)) return;
+        const bool in = unsigned((f_yx[i] >> 16) + f_dy) < unsigned(eh) && unsigned(int(short(f_yx[i])) + f_dx) < unsigned(ew) &&
+                        AXC_GLOBAL_OK(f_base[i] + f_off, (long long)pieces * g.CC, 310u);
+        cp_async16(dst + unsigned(i * 32 + lane) * 16u, P.codes + (in ? (size_t)unsigned(f_base[i] + f_off) * 16u : 0u), in ? 16u : 0u);
+    };
+    auto fetch_chunk = [&](unsigned dst) {
+        fetch_begin();
+#pragma unroll
+        for (int i = 0; i < PPL; ++i) fetch_pixel(i, dst);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    // ---- expanded tables: this warp's eighth, one octet ahead ----------------------------------------------------------
+    // Round r: a lane reads one word of the rows of 8 weights of element kidx (two a of 16-bit entries, four a of 8-bit
+    // entries, whose 16 channels are shared by two lanes) and writes the expanded rows of those a.  The 32 lanes read 32
+    // different banks, whatever the weights, and write different bank groups.
+    const int kidx = lane & 7, sub = lane >> 3;
+    const int hf = MODE == kXtabByte ? sub & 1 : 0;
+    unsigned raw[8];
+    unsigned b_unit = blockIdx.x;
+    int b_left = 0;                                                // octets left to build in b_unit
+    const uint4 *b_rows = nullptr;
+    uint4 wq = make_uint4(0, 0, 0, 0), wq_next = wq;               // row lists of the octet being built and of the one after it
+    auto build_unit = [&]() {
+        int nt, m0, c_begin, c_end;
+        coords(b_unit, nt, m0, c_begin, c_end);
+        b_left = 2 * (c_end - c_begin);
+        b_rows = reinterpret_cast<const uint4 *>(P.wrow) + (((size_t)nt * g.chunks + c_begin) * 16 + kidx) * HV + hf;
+    };
+    auto build_next = [&]() {                                      // take the next octet's row list, request the one after it
+        wq = wq_next;
+        if (b_left == 0) {
+            b_unit += gridDim.x;
+            if (b_unit >= units) return;
+            build_unit();
+        }
+        wq_next = __ldg(b_rows);
+        b_rows += 8 * HV;
+        --b_left;
+    };
+    // Words of a row that the lane works on: 32 r + (4 (warp + kidx) + sub) mod 32 in round r (8-bit entries: 32 (r / 2) + .. with
+    // the two lanes that share a piece's channels swapped in odd rounds), so that a round is a constant offset.
+    const unsigned word0 = (4u * (unsigned(warp) + unsigned(kidx)) + unsigned(sub)) & 31u, word1 = word0 ^ 1u;
+    unsigned row_at[8];
+    auto build_rows = [&]() {
+        const unsigned w4[4] = {wq.x, wq.y, wq.z, wq.w};
+#pragma unroll
+        for (int s = 0; s < 8; ++s) row_at[s] = ((s & 1) ? w4[s >> 1] >> 16 : w4[s >> 1] & 0xFFFFu) * 16u + word0 * 4u;
+    };
+    auto build_load = [&](int r) {
+        const unsigned odd = MODE == kXtabByte && (r & 1) ? word1 * 4u - word0 * 4u : 0u;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) raw[s] = lds32(row_at[s] + odd + (MODE == kXtabByte ? unsigned(r >> 1) : unsigned(r)) * 128u);
+    };
+    auto build_store = [&](int r, unsigned st) {
+        const unsigned word = MODE == kXtabByte && (r & 1) ? word1 : word0;
+        const unsigned dst = kTab + st * 128u + unsigned(kidx) * 16u + unsigned(hf) * 8u +
+                             (MODE == kXtabFull ? word * 512u + unsigned(r) * 16384u : word * 1024u + unsigned(r >> 1) * 32768u);
+        if (MODE == kXtabFull) {
+            sts128(dst, make_uint4(prmt<0x5410>(raw[0], raw[1]), prmt<0x5410>(raw[2], raw[3]), prmt<0x5410>(raw[4], raw[5]), prmt<0x5410>(raw[6], raw[7])));
+            sts128(dst + 256u, make_uint4(prmt<0x7632>(raw[0], raw[1]), prmt<0x7632>(raw[2], raw[3]), prmt<0x7632>(raw[4], raw[5]), prmt<0x7632>(raw[6], raw[7])));
+        } else {
+            unsigned o[4][2];                                      // [row a][word]
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                const unsigned t0 = prmt<0x5140>(raw[4 * w], raw[4 * w + 1]), t1 = prmt<0x5140>(raw[4 * w + 2], raw[4 * w + 3]);
+                const unsigned t2 = prmt<0x7362>(raw[4 * w], raw[4 * w + 1]), t3 = prmt<0x7362>(raw[4 * w + 2], raw[4 * w + 3]);
+                o[0][w] = prmt<0x5410>(t0, t1); o[1][w] = prmt<0x7632>(t0, t1);
+                o[2][w] = prmt<0x5410>(t2, t3); o[3][w] = prmt<0x7632>(t2, t3);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sts64(dst + unsigned(i) * 256u, o[i][0], o[i][1]);
+        }
+    };
+
+    // ---- expanded tables from global memory: two chunks in flight, issued by one thread ------------------------------------
+    unsigned x_unit = blockIdx.x;
+    int x_left = 0;
+    const unsigned char *x_src = nullptr;
+    auto copy_table = [&](unsigned buf) {                          // the next chunk's table into buffer `buf`
+        if (x_left == 0) {
+            if (x_src) x_unit += gridDim.x;
+            if (x_unit >= units) return;
+            int nt, m0, c_begin, c_end;
+            coords(x_unit, nt, m0, c_begin, c_end);
+            x_left = c_end - c_begin;
+            x_src = P.xt + ((size_t)nt * g.chunks + c_begin) * 65536u;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tab_full + buf * 8), "r"(65536u) : "memory");
+        bulk_copy(kTab * (1u + buf), x_src, 65536u, tab_full + buf * 8);
+        x_src += 65536;
+        --x_left;
+    };
+
+    // ---- lookups ---------------------------------------------------------------------------------------------------------
+    const int gr = lane >> 2, t = lane & 3;
+    const DevQuant Q = *reinterpret_cast<const DevQuant *>(reinterpret_cast<const unsigned char *>(P.hdr) + kDevQuantOffset);
+    const unsigned zz = code_of(0.0f, Q.in_off, Q.in_inv) * 0x01010101u;
+    // Constant B operands.  A row of A has the words x, z of a piece, the row eight below it y, w.  8-bit entries: column n
+    // adds byte n of (x, z) resp. (y, w): 16 channels.  16-bit entries: digits 1 and 255 of the two channels of a word,
+    // in columns 0..3 for the first block of a pair, 4..7 for the second: one accumulator fragment serves both.
+    unsigned b00, b01, b10, b11;
+    if (MODE == kXtabFull) {
+        const unsigned digits = (gr & 1) ? 0xFF010000u : 0x0000FF01u;
+        b00 = (gr >> 1) == 0 ? digits : 0u; b01 = (gr >> 1) == 1 ? digits : 0u;
+        b10 = (gr >> 1) == 2 ? digits : 0u; b11 = (gr >> 1) == 3 ? digits : 0u;
+    } else {
+        b00 = b10 = gr < 4 ? 1u << (8 * gr) : 0u;
+        b01 = b11 = gr >= 4 ? 1u << (8 * (gr - 4)) : 0u;
+    }
+    // step s of an octet: even pixels take k = t + 4s, odd ones t + 4(1 - s)
+    const unsigned p0 = unsigned(gr & 1);
+    const unsigned lane_k0 = kTab + unsigned(t + 4 * p0) * 16u, lane_k1 = kTab + unsigned(t + 4 * (1 - p0)) * 16u;
+    constexpr int kAcc = NB * HV / 2;                              // accumulator fragments
+    int acc[kAcc][4];
+    unsigned cw[NB];
+    // Octet h (0 / 1) of the chunk, from the table of stage st; `more`: build the next octet's table into the other stage.
+    // Steps of two block pairs and one of their two k: the loads of a step are issued before the MMAs of the step before it,
+    // and no MMA waits for the one just issued (16-bit entries: two MMAs per pair and step add into one accumulator).
+    // Spread over the steps as well, so that the shared-memory pipe never waits for them (measured as bursts at the chunk's
+    // start: 830 clocks per octet of 2048 pixels): one MMA of the exact products per step; in octet 0 the requests for the next
+    // chunk's codes; in octet 1, where the last use of a code has passed, the loads of the next chunk's; four rounds of building.
+    constexpr int kSteps = NB / 2;
+    const unsigned code_src = my_codes + unsigned(gr) * 16u + unsigned(t) * 4u;
+    auto product = [&](int i, uint2 wb) {                          // both rows of a pixel hold its codes, each against half of the channels
+        const unsigned q = cw[i] ^ zz;
+        mma_k32(acc[i * HV / 2], q, 0u, 0u, q, wb.x, wb.y);
+    };
+    auto octet = [&](int h, unsigned toff, unsigned st, unsigned oct, bool more, uint2 wb) {
+        const unsigned l0 = lane_k0 + toff, l1 = lane_k1 + toff;
+        // address = {low byte of l, code byte, upper half of l}
+        const unsigned s0 = 0x3200u | ((4u + 2u * h + p0) << 4), s1 = 0x3200u | ((4u + 2u * h + 1u - p0) << 4);
+        uint4 x[2][4];
+        auto request = [&](int n, uint4 (&v)[4]) {
+            const int i = (n >> 1) * 2;                            // pairs i, i + 1
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = lds128((n & 1) ? prmt_r(l1, cw[2 * i + e], s1) : prmt_r(l0, cw[2 * i + e], s0));
+        };
+        request(0, x[0]);
+        if (h == 0) fetch_begin();
+        else {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+        }
+#pragma unroll
+        for (int n = 0; n < kSteps; ++n) {
+            if (n + 1 < kSteps) request(n + 1, x[(n + 1) & 1]);
+            const int i = (n >> 1) * 2;
+            uint4 (&v)[4] = x[n & 1];
+            // a loaded piece is an A operand as it is
+            mma_k32(acc[i * HV], v[0].x, v[0].y, v[0].z, v[0].w, b00, b01);
+            mma_k32(acc[(i + 1) * HV], v[2].x, v[2].y, v[2].z, v[2].w, b00, b01);
+            mma_k32(acc[i * HV + HV - 1], v[1].x, v[1].y, v[1].z, v[1].w, b10, b11);
+            mma_k32(acc[(i + 1) * HV + HV - 1], v[3].x, v[3].y, v[3].z, v[3].w, b10, b11);
+            if (MODE != kXtabFull) product(h * kSteps + n, wb);
+            if (h == 0) {
+#pragma unroll
+                for (int f = 0; f < PPL; ++f)
+                    if (n == f * kSteps / PPL) fetch_pixel(f, my_codes);
+            } else if (n & 1) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) cw[2 * (n - 1) + e] = lds32(code_src + unsigned(2 * (n - 1) + e) * 128u);
+            }
+            if (PRE && h == 0 && n == 1 && tid == 0 && oct > 0) {
+                // the other buffer's readers finished the chunk before this one: ask for the chunk after this one
+                mbar_wait(tab_empty + (st ^ 1u) * 8, ((oct - 1) >> 1) & 1u, ok);
+                copy_table(st ^ 1u);
+            }
+            if (kBuild && more) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    if (n == r * kSteps / 4) {
+                        if (r == 0) {
+                            build_next();
+                            // the stage's last readers worked on the octet before this one
+                            if (oct > 0) mbar_wait(tab_empty + (st ^ 1u) * 8, ((oct - 1) >> 1) & 1u, ok);
+                            build_rows();
+                        }
+                        build_load(r);
+                    }
+                    if (n == (kSteps < 4 ? r * kSteps / 4 : (r + 1) * kSteps / 4 - 1)) build_store(r, st ^ 1u);
+                }
+            }
+        }
+        __syncwarp();                                              // also: every lane has the codes before the next are asked for
+        if (lane == 0) {
+            if (kBuild && more) mbar_arrive(tab_full + (st ^ 1u) * 8);
+            if (kBuild || h == 1) mbar_arrive(tab_empty + st * 8);
+        }
+    };
+
+    unsigned oct = 0, oct_total = 0;                               // octets of this CTA so far, and all of them
+    constexpr int kBufs = kTables ? 1 : 4;                         // code buffers (only exact products: latency is all there is)
+    if (blockIdx.x < units) {
+        fetch_unit();
+#pragma unroll
+        for (int k = 0; k < (kTables ? 1 : kBufs - 1); ++k) fetch_chunk(my_codes + unsigned(k) * (kPix * 16u));
+    }
+    if (kTables && blockIdx.x < units) {
+        for (unsigned u = blockIdx.x; u < units; u += gridDim.x) {
+            int nt, m0, c_begin, c_end;
+            coords(u, nt, m0, c_begin, c_end);
+            oct_total += 2u * unsigned(c_end - c_begin);
+        }
+        if (PRE && tid == 0) {
+            copy_table(0u);
+            copy_table(1u);
+        }
+        if (kBuild) {
+            build_unit();
+            build_next();
+            build_next();
+            mbar_wait(rows_full, 0u, ok);
+            build_rows();
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                build_load(r);
+                build_store(r, 0u);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        if (kBuild && lane == 0) mbar_arrive(tab_full);
+#pragma unroll
+        for (int i = 0; i < NB; ++i) cw[i] = lds32(code_src + unsigned(i) * 128u);
+        __syncwarp();
+    }
+    unsigned chunk = 0;
+    for (unsigned u = blockIdx.x; u < units; u += gridDim.x) {
+        int nt, m0, c_begin, c_end;
+        coords(u, nt, m0, c_begin, c_end);
+#pragma unroll
+        for (int i = 0; i < kAcc; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][e] = 0;
+        const uint2 *wbp = P.wb + ((size_t)nt * g.chunks + c_begin) * 32 + lane;
+        uint2 wb_next = make_uint2(0, 0);
+        if (MODE != kXtabFull) wb_next = __ldg(wbp);
+        for (int c = c_begin; c < c_end; ++c, ++chunk) {
+            const uint2 wb = wb_next;
+            wbp += 32;
+            if (MODE != kXtabFull && c + 1 < c_end) wb_next = __ldg(wbp);
+            if (PRE) {
+                const unsigned st = chunk & 1u;
+                mbar_wait(tab_full + st * 8, (chunk >> 1) & 1u, ok);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) octet(h, st * kTab + unsigned(h) * 128u, st, chunk, true, wb);
+            } else if (kTables) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h, ++oct) {
+                    mbar_wait(tab_full + (oct & 1u) * 8, (oct >> 1) & 1u, ok);
+                    octet(h, (oct & 1u) * 128u, oct & 1u, oct, oct + 1 < oct_total, wb);
+                }
+            } else {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 2) : "memory");
+                __syncwarp();
+                const unsigned src = code_src + (chunk & (kBufs - 1)) * (kPix * 16u);
+#pragma unroll
+                for (int i = 0; i < NB; ++i) cw[i] = lds32(src + unsigned(i) * 128u);
+                __syncwarp();
+                fetch_chunk(my_codes + ((chunk + kBufs - 1) & (kBufs - 1)) * (kPix * 16u));
+#pragma unroll
+                for (int i = 0; i < NB; ++i) product(i, wb);
+            }
+        }
+        // ---- dequantise and store: a fragment is four neighbouring channels of one pixel -------------------------------
+        const int j0 = nt * TNC + 4 * (MODE == kXtabFull ? t & 1 : t);
+        float t2[4], bias[4];
+        int back[4];                                               // what the stored entries lack: per channel
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            t2[e] = (!P.partial && j0 + e < g.Cout) ? __fmul_rn(Q.m1, __ldg(P.bsum + j0 + e)) : 0.0f;
+            bias[e] = (P.bias && j0 + e < g.Cout) ? __ldg(P.bias + j0 + e) : 0.0f;
+            back[e] = P.k_e_min + (MODE == kXtabFull && P.bcode && j0 + e < g.Cout ? 128 * __ldg(P.bcode + j0 + e) : 0);
+        }
+        const bool whole = j0 + 4 <= g.Cout && (g.Cout & 3) == 0, chan = j0 < g.Cout;
+        constexpr int EB = kAcc < 4 ? kAcc : 4;
+        constexpr int kStep = MODE == kXtabFull ? 16 : 8;          // pixels from fragment to fragment
+        const int first = warp * (NB * 8) + gr + (MODE == kXtabFull ? (t >> 1) * 8 : 0);
+        const int left = chan ? g.M - m0 - first : 0;              // > kStep * i: fragment i has a pixel
+        const long long at0 = (long long)(m0 + first) * g.Cout + j0;
+        const int row = kStep * g.Cout;
+        if (P.plain && whole) {
+            // The common case on its own, in as few instructions as possible: the code is unrolled over the fragments and runs
+            // once per tile, so its length is paid in instruction fetches (one loop for all cases: 51 000 clocks per tile of
+            // 2048 pixels).  Four fragments at a time: what they read is requested before the first is finished.
+            const float *asum = P.asum + (m0 + first), *res = P.residual + at0;
+            float *out = P.output + at0;
+            const int *acode = P.acode + (m0 + first);
+#pragma unroll
+            for (int i0 = 0; i0 < kAcc; i0 += EB) {
+                float a_sum[EB];
+                int a_code[EB];
+                float4 r[EB];
+#pragma unroll
+                for (int i = 0; i < EB; ++i) a_code[i] = MODE == kXtabFull && P.acode && (i0 + i) * kStep < left ? 128 * __ldg(acode + (i0 + i) * kStep) : 0;
+#pragma unroll
+                for (int i = 0; i < EB; ++i) a_sum[i] = (i0 + i) * kStep < left ? __fmul_rn(Q.m2, __ldg(asum + (i0 + i) * kStep)) : 0.0f;
+                if (P.residual)
+#pragma unroll
+                    for (int i = 0; i < EB; ++i)
+                        if ((i0 + i) * kStep < left) r[i] = __ldg(reinterpret_cast<const float4 *>(res + (i0 + i) * row));
+#pragma unroll
+                for (int i = 0; i < EB; ++i) {
+                    float y[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        y[e] = __fsub_rn(__fadd_rn(__fadd_rn(__fmul_rn(float(acc[i0 + i][e] + back[e] + a_code[i]), Q.s1s2), a_sum[i]), t2[e]), Q.km1m2);
+                    if (P.bias)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) y[e] = __fadd_rn(y[e], bias[e]);
+                    if (P.residual) {
+                        y[0] = __fadd_rn(y[0], r[i].x); y[1] = __fadd_rn(y[1], r[i].y);
+                        y[2] = __fadd_rn(y[2], r[i].z); y[3] = __fadd_rn(y[3], r[i].w);
+                    }
+                    if ((i0 + i) * kStep < left && AXC_GLOBAL_OK(at0 + (i0 + i) * row + 3, (long long)g.M * g.Cout, 313u))
+                        *reinterpret_cast<float4 *>(out + (i0 + i) * row) =
+                            make_float4(max_keep_nan(y[0], P.out_floor), max_keep_nan(y[1], P.out_floor), max_keep_nan(y[2], P.out_floor), max_keep_nan(y[3], P.out_floor));
+                }
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kAcc; ++i) {
+                if (i * kStep >= left) continue;
+                const long long at = at0 + i * row;
+                if (!AXC_GLOBAL_OK(at, (long long)g.M * g.Cout, 314u)) continue;
+                const float a_sum = P.partial ? 0.0f : __ldg(P.asum + m0 + first + i * kStep);
+                const int a_code = MODE == kXtabFull && P.acode && !P.partial ? 128 * __ldg(P.acode + m0 + first + i * kStep) : 0;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (j0 + e >= g.Cout) continue;
+                    if (P.partial) {
+                        atomicAdd(P.partial + at + e, acc[i][e]);
+                        continue;
+                    }
+                    const int tot = acc[i][e] + back[e] + a_code;
+                    float y = dequantise(Q, tot, a_sum, t2[e]);
+                    if (P.bias) y = __fadd_rn(y, bias[e]);
+                    if (P.residual) y = __fadd_rn(y, __ldg(P.residual + at + e));
+                    if (P.output) P.output[at + e] = max_keep_nan(y, P.out_floor);
+                    if (P.acc_out) P.acc_out[at + e] = tot;
+                }
+            }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");               // nothing of this CTA is in flight when it ends
+    if (!ok && lane == 0) atomicExch(const_cast<int *>(&P.hdr->status), 3);
+}
+
+// The dequantisation of a call whose K was split over CTAs.
+__global__ void __launch_bounds__(256) xfinal_kernel(const XParams P)
+{
+    const DevQuant Q = *reinterpret_cast<const DevQuant *>(reinterpret_cast<const unsigned char *>(P.hdr) + kDevQuantOffset);
+    const long long total = (long long)P.g.M * P.g.Cout;
+    for (long long x = (long long)blockIdx.x * 256 + threadIdx.x; x < total; x += (long long)gridDim.x * 256) {
+        const int m = int(x / P.g.Cout), j = int(x - (long long)m * P.g.Cout);
+        const int tot = P.partial[x] + P.k_e_min + (P.acode ? 128 * (__ldg(P.acode + m) + __ldg(P.bcode + j)) : 0);
+        float y = dequantise(Q, tot, __ldg(P.asum + m), __fmul_rn(Q.m1, __ldg(P.bsum + j)));
+        if (P.bias) y = __fadd_rn(y, __ldg(P.bias + j));
+        if (P.residual) y = __fadd_rn(y, __ldg(P.residual + x));
+        if (P.output) P.output[x] = max_keep_nan(y, P.out_floor);
+        if (P.acc_out) P.acc_out[x] = tot;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// host
+// ------------------------------------------------------------------------------------------------------------------
+size_t r256(size_t v) { return (v + 255) & ~size_t(255); }
+
+struct XLayout {
+    size_t tt, wrow, wb, asum, bsum, acode, bcode, partial, codes, xt, xt_bytes, total;
+};
+
+constexpr size_t kPrepSmem = 72 * 1024;        // three preparation tiles per SM
+constexpr size_t kPrepSmemMax = 220 * 1024;
+
+struct PrepTile {
+    int TH, TW, RH, RW, pitch, vec;
+    size_t smem;
+};
+
+// Output pixels per preparation tile: at most 256 (one per thread), as wide as an output row allows, within the shared
+// memory of three CTAs per SM where that is possible.
+bool prep_tile(const Geom &g, int vec, bool im2col, PrepTile *out)
+{
+    PrepTile t;
+    t.vec = vec;
+    // an odd number of 16-byte pieces (floats) per pixel keeps the lanes of the patch sums on different banks
+    if (vec) t.pitch = ((g.C >> 2) | 1) * 4;
+    else t.pitch = im2col ? g.C : g.C | 1;
+    auto smem = [&](int th, int tw) {
+        const size_t rh = size_t(th - 1) * g.sh + size_t(g.KH - 1) * g.dh + 1, rw = size_t(tw - 1) * g.sw + size_t(g.KW - 1) * g.dw + 1;
+        return rh * rw * (t.pitch + 1) * 4;
+    };
+    t.TW = g.OW < 64 ? g.OW : 64;
+    while (t.TW > 1 && smem(1, t.TW) > kPrepSmem) t.TW = (t.TW + 1) / 2;
+    if (smem(1, t.TW) > kPrepSmemMax) return false;
+    t.TH = 1;
+    while (t.TH < g.OH && (t.TH + 1) * t.TW <= 256 && smem(t.TH + 1, t.TW) <= kPrepSmem) ++t.TH;
+    t.RH = (t.TH - 1) * g.sh + (g.KH - 1) * g.dh + 1;
+    t.RW = (t.TW - 1) * g.sw + (g.KW - 1) * g.dw + 1;
+    t.smem = smem(t.TH, t.TW);
+    if (t.smem < 32768) t.smem = 32768;        // the staging of the filter sums
+    *out = t;
+    return true;
+}
+
+// Codes per pixel in 16-byte pieces, or im2col rows where the padding of the channel count to 16 would add more than an
+// eighth to K.
+void code_layout(const Geom &g, int *CC, int *chunks, int *im2col)
+{
+    const int cc = (g.C + 15) / 16, taps = g.KH * g.KW;
+    const long long direct = (long long)taps * cc, rows = ((long long)g.K + 15) / 16;
+    *im2col = direct * 8 > rows * 9 ? 1 : 0;
+    *CC = *im2col ? int(rows) : cc;
+    *chunks = int(*im2col ? rows : direct);
+}
+
+bool xgeom(const Geom &g, XGeom *x)
+{
+    if (g.M >= (1ll << 30) || (long long)g.N * g.H * g.W >= (1ll << 30)) return false;
+    if (g.H >= 16384 || g.W >= 16384 || (long long)g.KH * g.dh >= 8192 || (long long)g.KW * g.dw >= 8192) return false;
+    if ((long long)g.OH * g.sh >= 16384 || (long long)g.OW * g.sw >= 16384) return false;
+    XGeom r;
+    r.N = g.N; r.H = g.H; r.W = g.W; r.C = g.C; r.KH = g.KH; r.KW = g.KW; r.Cout = g.Cout;
+    r.sh = g.sh; r.sw = g.sw; r.dh = g.dh; r.dw = g.dw; r.ph = g.ph; r.pw = g.pw; r.OH = g.OH; r.OW = g.OW; r.K = g.K; r.M = int(g.M);
+    code_layout(g, &r.CC, &r.chunks, &r.im2col);
+    const long long pieces = (r.im2col ? g.M : (long long)g.N * g.H * g.W) * r.CC;
+    if (pieces >= (1ll << 29)) return false;      // word offsets of the codes fit an int
+    // headroom for the piece number of a patch origin outside the image
+    if (!r.im2col && (long long)(g.ph + g.KH * g.dh + 1) * g.W * r.CC >= (1ll << 29)) return false;
+    r.TNC = 0; r.tiles_n = 0;
+    *x = r;
+    return true;
+}
+
+struct Config {
+    int nb, splits, chunks_per_split;
+    bool pre;
+};
+
+size_t xt_size(const XGeom &x, int mode) { return size_t((x.Cout + (mode == kXtabFull ? 7 : 15)) / (mode == kXtabFull ? 8 : 16)) * x.chunks * 65536u; }
+
+// Pixels per tile, splits of K, and where the expanded tables are made.  In clocks per octet: lookups and codes 1.09 per pixel,
+// about 130 for the waits around a table, 720 for building one (512 of them on the shared-memory pipe); a start and an end that
+// do not shrink with the tile; tables from global memory cost their writes (2.3 KiB per clock over the chip) and a launch.
+Config choose_config(int mode, const XGeom &x, int sms, bool may_split, size_t xt_bytes)
+{
+    const int tiles_n = (x.Cout + (mode == kXtabFull ? 7 : 15)) / (mode == kXtabFull ? 8 : 16);
+    Config best = {32, 1, x.chunks, false};
+    double best_cost = 1e300;
+    for (int pre = 0; pre < 2; ++pre) {
+        if (pre && (mode == kXtabExact || xt_size(x, mode) > xt_bytes)) continue;
+        for (int nb = mode == kXtabFull && pre ? 48 : 32; nb >= (pre ? 16 : 4); nb = nb == 48 ? 32 : nb >> 1) {
+            const int pix = kWarps * 8 * nb;
+            const long long tiles = ((long long)x.M + pix - 1) / pix * tiles_n;
+            const double octet = mode == kXtabExact ? 0.30 * pix + 100.0 : 1.09 * pix + (pre ? 130.0 : 850.0);
+            for (int sp = 1; sp <= 64 && sp <= x.chunks; sp *= 2) {
+                if (sp > 1 && (!may_split || tiles >= sms)) break;
+                const int cps = (x.chunks + sp - 1) / sp;
+                const int spe = (x.chunks + cps - 1) / cps;
+                const long long rounds = (tiles * spe + sms - 1) / sms;
+                double cost = double(rounds) * (2.0 * cps * octet + 2000.0 + 3.0 * pix * (spe > 1 ? 2.0 : 1.0)) + (spe > 1 ? 6000.0 : 0.0);
+                cost += pre ? double(xt_size(x, mode)) / 2300.0 + 8000.0 : 3000.0;
+                if (cost < best_cost) { best_cost = cost; best = {nb, spe, cps, pre != 0}; }
+            }
+        }
+    }
+    return best;
+}
+
+XLayout xlayout(const Geom &g, const XGeom &x)
+{
+    XLayout L;
+    const size_t cout16 = size_t((g.Cout + 15) / 16) * 16;
+    size_t off = 256;
+    L.tt = off;      off += r256(257 * 512);
+    L.wrow = off;    off += r256(cout16 * x.chunks * 32);
+    L.wb = off;      off += r256(cout16 * x.chunks * 16);
+    L.asum = off;    off += r256(size_t(g.M) * 4);
+    L.bsum = off;    off += r256(size_t(g.Cout) * 4);
+    L.acode = off;   off += r256(size_t(g.M) * 4);
+    L.bcode = off;   off += r256(size_t(g.Cout) * 4);
+    L.partial = off; off += r256(size_t(g.M) * g.Cout * 4 <= kPartialMax ? size_t(g.M) * g.Cout * 4 : 0);
+    L.codes = off;   off += r256((x.im2col ? size_t(g.M) : size_t(g.N) * g.H * g.W) * x.CC * 16);
+    // room for the expanded tables where a call would have them made in global memory
+    L.xt = off;
+    L.xt_bytes = 0;
+    for (int mode : {int(kXtabByte), int(kXtabFull)}) {
+        const size_t bytes = xt_size(x, mode);
+        if (bytes <= kXtMax && bytes > L.xt_bytes && choose_config(mode, x, kModelSms, size_t(g.M) * g.Cout * 4 <= kPartialMax, bytes).pre) L.xt_bytes = bytes;
+    }
+    off += L.xt_bytes;
+    L.total = off;
+    return L;
+}
+
+template <int MODE, int NB, bool PRE>
+int launch_variant(const XParams &P, const DeviceInfo &di, cudaStream_t stream)
+{
+    AXC_CUDA(cudaFuncSetAttribute(xtab_kernel<MODE, NB, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin));
+    const long long grid = P.units < di.sm_count ? P.units : di.sm_count;
+    xtab_kernel<MODE, NB, PRE><<<unsigned(grid), kWarps * 32, size_t(di.max_smem_optin), stream>>>(P);
+    AXC_CUDA(cudaGetLastError());
+    count_launch();
+    return AXC_OK;
+}
+
+template <int MODE>
+int launch_mode(const Config &cf, const XParams &P, const DeviceInfo &di, cudaStream_t stream)
+{
+    constexpr bool kPre = MODE != kXtabExact;
+    if (cf.pre) {
+        if (cf.nb == 48) return launch_variant<MODE, MODE == kXtabFull ? 48 : 32, kPre>(P, di, stream);
+        return cf.nb == 32 ? launch_variant<MODE, 32, kPre>(P, di, stream) : launch_variant<MODE, 16, kPre>(P, di, stream);
+    }
+    switch (cf.nb) {
+    case 32: return launch_variant<MODE, 32, false>(P, di, stream);
+    case 16: return launch_variant<MODE, 16, false>(P, di, stream);
+    case 8: return launch_variant<MODE, 8, false>(P, di, stream);
+    default: return launch_variant<MODE, 4, false>(P, di, stream);
+    }
+}
+
+template <int MODE>
+int launch_expand(const ExpandParams &E, const DeviceInfo &di, cudaStream_t stream)
+{
+    constexpr size_t smem = MODE == kXtabFull ? 131072 : 65536;
+    constexpr int per_sm = MODE == kXtabFull ? 1 : 3;
+    AXC_CUDA(cudaFuncSetAttribute(xexpand_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    const int total = E.g.tiles_n * E.g.chunks, grid = total < di.sm_count * per_sm ? total : di.sm_count * per_sm;
+    xexpand_kernel<MODE><<<unsigned(grid), 256, smem, stream>>>(E);
+    AXC_CUDA(cudaGetLastError());
+    count_launch();
+    return AXC_OK;
+}
+
+}  // namespace
+
+size_t xtab_scratch_bytes(const Geom &g)
+{
+    // Few lookups: the latency of preparation plus convolution is longer than the plan-based kernels' single pass over a
+    // filter that is already laid out.
+    if ((double)g.M * g.K * g.Cout < kXtabMinLookups) return 0;
+    XGeom x;
+    PrepTile t;
+    if (!xgeom(g, &x) || !prep_tile(g, g.C % 4 == 0, x.im2col != 0, &t) || !prep_tile(g, 0, x.im2col != 0, &t)) return 0;
+    return xlayout(g, x).total;
+}
+
+int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const Geom &g, const Quant &q, const float *ranges_dev,
+                const float *input, const float *filter, float *output, unsigned char *scratch, const axc_debug_out *dbg,
+                const DeviceInfo &di, cudaStream_t stream)
+{
+    PrepParams A;
+    if (!xgeom(g, &A.g)) return AXC_INTERNAL;
+    XGeom &x = A.g;
+    x.TNC = mode == kXtabFull ? 8 : 16;
+    x.tiles_n = (g.Cout + x.TNC - 1) / x.TNC;
+    const XLayout L = xlayout(g, x);
+    const size_t partial_bytes = size_t(g.M) * g.Cout * 4;
+    const Config cf = choose_config(mode, x, di.sm_count, partial_bytes <= kPartialMax, L.xt_bytes);
+    const int vec = (g.C % 4 == 0 && (reinterpret_cast<uintptr_t>(input) & 15u) == 0) ? 1 : 0;
+    PrepTile t;
+    if (!prep_tile(g, vec, x.im2col != 0, &t)) return AXC_INTERNAL;
+    A.input = input; A.filter = filter; A.lut = lut_dev; A.ranges = ranges_dev; A.host_q = host_dev_quant(q, g.K);
+    A.in_floor = g.ep.input_relu ? 0.0f : -INFINITY;
+    A.mode = mode; A.centred = centred; A.e_min = e_min;
+    A.acode = centred ? reinterpret_cast<int *>(scratch + L.acode) : nullptr;
+    A.bcode = centred ? reinterpret_cast<int *>(scratch + L.bcode) : nullptr;
+    A.codes = scratch + L.codes; A.tt = scratch + L.tt;
+    A.wrow = reinterpret_cast<uint16_t *>(scratch + L.wrow); A.wb = reinterpret_cast<uint2 *>(scratch + L.wb);
+    A.asum = reinterpret_cast<float *>(scratch + L.asum); A.bsum = reinterpret_cast<float *>(scratch + L.bsum);
+    A.qf_debug = dbg ? dbg->qfilter : nullptr;
+    A.hdr = reinterpret_cast<PlanHeader *>(scratch);
+    A.TH = t.TH; A.TW = t.TW; A.RH = t.RH; A.RW = t.RW; A.pitch = t.pitch; A.vec = t.vec;
+    A.tiles_y = (g.OH + t.TH - 1) / t.TH; A.tiles_x = (g.OW + t.TW - 1) / t.TW;
+    A.blocks_sum = (g.Cout + 31) / 32;
+    const long long w_items = (long long)x.tiles_n * x.chunks * 16 * x.TNC;
+    A.blocks_w = cf.pre ? 0 : int(w_items / 1024 + 1 < 592 ? w_items / 1024 + 1 : 592);
+    A.blocks_t = cf.pre ? 0 : 32;
+    const long long blocks = (long long)A.blocks_sum + A.blocks_w + A.blocks_t + (long long)g.N * A.tiles_y * A.tiles_x;
+    if (blocks >= (1ll << 31)) return AXC_INTERNAL;
+    AXC_CUDA(cudaFuncSetAttribute(xprep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPrepSmemMax)));
+    xprep_kernel<<<unsigned(blocks), 256, t.smem, stream>>>(A);
+    AXC_CUDA(cudaGetLastError());
+    count_launch();
+
+    if (cf.pre) {
+        ExpandParams E;
+        E.g = x; E.filter = filter; E.lut = lut_dev; E.ranges = ranges_dev; E.host_q = A.host_q; E.centred = centred; E.e_min = e_min;
+        E.xt = scratch + L.xt; E.wb = A.wb; E.qf_debug = A.qf_debug;
+        const int rc = mode == kXtabFull ? launch_expand<kXtabFull>(E, di, stream) : launch_expand<kXtabByte>(E, di, stream);
+        if (rc) return rc;
+    }
+
+    XParams P;
+    P.g = x;
+    P.xt = cf.pre ? scratch + L.xt : nullptr;
+    P.codes = A.codes; P.tt = A.tt; P.wrow = A.wrow; P.wb = A.wb; P.asum = A.asum; P.bsum = A.bsum; P.hdr = A.hdr;
+    P.output = output; P.acc_out = dbg ? dbg->acc : nullptr;
+    P.acode = A.acode; P.bcode = A.bcode;
+    P.bias = g.ep.bias; P.residual = g.ep.residual; P.out_floor = g.ep.relu ? 0.0f : -INFINITY;
+    P.k_e_min = int(unsigned(g.K) * unsigned(e_min));
+    P.splits = cf.splits; P.chunks_per_split = cf.chunks_per_split;
+    P.units = ((long long)x.M + kWarps * 8 * cf.nb - 1) / (kWarps * 8 * cf.nb) * x.tiles_n * cf.splits;
+    if (P.units >= (1ll << 31)) return AXC_INTERNAL;
+    P.partial = nullptr;
+    if (cf.splits > 1) {
+        P.partial = reinterpret_cast<int32_t *>(scratch + L.partial);
+        AXC_CUDA(cudaMemsetAsync(P.partial, 0, partial_bytes, stream));
+    }
+    P.plain = (output && !P.acc_out && !P.partial &&
+               ((reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(g.ep.residual)) & 15u) == 0) ? 1 : 0;
+    int rc = mode == kXtabFull ? launch_mode<kXtabFull>(cf, P, di, stream)
+             : mode == kXtabByte ? launch_mode<kXtabByte>(cf, P, di, stream) : launch_mode<kXtabExact>(cf, P, di, stream);
+    if (rc) return rc;
+    if (cf.splits > 1) {
+        const long long n = (g.M * g.Cout + 255) / 256;
+        xfinal_kernel<<<unsigned(n < 1184 ? n : 1184), 256, 0, stream>>>(P);
+        AXC_CUDA(cudaGetLastError());
+        count_launch();
+    }
+    return AXC_OK;
+}
+
+AXC_DEFINE_BOUNDS_READER(bounds_record_xtab)
+
+}  // namespace axc

@@ -187,6 +187,15 @@ def workspace_bytes(input_shape, filter_shape, strides, padding, dilations=(1, 1
     return int(wsz.value)
 
 
+def fast_workspace_bytes(input_shape, filter_shape, strides, padding, dilations=(1, 1, 1, 1)):
+    """Bytes of scratch with which a dense call is served by the expanded-table kernels (axc_conv2d_fast_workspace_bytes);
+    0 where the plan in a buffer of `workspace_bytes` serves the shape better."""
+    d = _desc(input_shape, filter_shape, strides, padding, "NHWC", list(dilations), [])
+    wsz = C.c_size_t()
+    raise_for_status(_lib.load().axc_conv2d_fast_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
+    return int(wsz.value)
+
+
 def _device_index(dev):
     """CUDA ordinal of a torch device; a device without an index means the current one."""
     return dev.index if dev.index is not None else torch.cuda.current_device()
@@ -218,9 +227,16 @@ def _forward(depthwise, input, filter, input_min, input_max, filter_min, filter_
     elif tuple(out.shape) != oshape or out.dtype != torch.float32 or not out.is_contiguous() or out.device != dev:
         raise InvalidArgumentError("out has the wrong shape, dtype, layout or device")
     wsz = C.c_size_t()
-    ws_fn = L.axc_depthwise_conv2d_workspace_bytes if depthwise else L.axc_conv2d_workspace_bytes
-    raise_for_status(ws_fn(C.byref(d), C.byref(wsz)), "workspace size")
-    if workspace is not None:
+    if workspace is None and not depthwise:
+        raise_for_status(L.axc_conv2d_fast_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
+    fast = wsz.value > 0
+    if not fast:
+        ws_fn = L.axc_depthwise_conv2d_workspace_bytes if depthwise else L.axc_conv2d_workspace_bytes
+        raise_for_status(ws_fn(C.byref(d), C.byref(wsz)), "workspace size")
+    if fast:
+        # scratch of this call alone: torch's allocator hands it to later work of the same stream only
+        ws = torch.empty(wsz.value, dtype=torch.uint8, device=dev)
+    elif workspace is not None:
         if (workspace.dtype != torch.uint8 or workspace.device != dev or not workspace.is_contiguous()
                 or workspace.numel() < wsz.value or workspace.data_ptr() % 256):
             raise InvalidArgumentError("workspace must be a contiguous uint8 tensor on the input's device, 256-byte "
