@@ -275,6 +275,8 @@ int axc_depthwise_conv2d_forward_noalloc(axc_table *table, const axc_conv_desc *
  * than the window by two or more, :153-163) return AXC_UNIMPLEMENTED.  The table sums are computed by the kernels
  * of axc_conv2d_forward; the workspace additionally holds an fp32 image of both operands. */
 int axc_qconv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
+/* Scratch with which a quantised call takes the expanded-table kernels (see axc_conv2d_fast_workspace_bytes); 0: none. */
+int axc_qconv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
 int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, const uint8_t *qinput, const uint8_t *qfilter,
                         int32_t input_offset, int32_t filter_offset, int32_t *output, void *workspace,
                         size_t workspace_bytes, int device, void *stream);

@@ -83,3 +83,29 @@ def test_unusual_values_and_addresses(built):
             y = ax.approx_conv2d_with_min_max_vars(inp, f, *mm, [1, 1, 1, 1], 8, t, "SAME")
             assert torch.equal(torch.isnan(y), torch.isnan(want))
             assert torch.equal(torch.nan_to_num(y, 0.0).view(torch.int32), torch.nan_to_num(want, 0.0).view(torch.int32))
+
+
+Q_SHAPES = [  # n, h, w, c, k, cout, stride, padding, input range, filter range
+    (2, 28, 28, 64, 3, 96, 1, "SAME", (-1.0, 2.0), (-0.5, 0.5)),
+    (3, 21, 23, 30, 3, 45, 2, "SAME", (0.5, 2.0), (-0.5, 0.25)),        # zero point of the input below 0: padded taps wrap
+    (1, 50, 50, 3, 5, 50, 1, "VALID", (0.0, 1.0), (0.0, 1.0)),          # im2col rows, no zero-point terms
+    (5, 50, 51, 32, 3, 64, 1, "SAME", (-3.0, -1.0), (-1.0, 3.0)),
+]
+
+
+@pytest.mark.parametrize("kind", ["exact", "byte", "digits", "centred"])
+@pytest.mark.parametrize("shape", Q_SHAPES, ids=["-".join(str(v) for v in s[:8]) for s in Q_SHAPES])
+def test_quantised_operands(built, shape, kind):
+    """uint8 operands on the expanded tables, the zero-point terms added at the end, against the checker's functor."""
+    import torch
+    import tf_approximate_b200 as ax
+    n, h, w, c, k, co, s, pad, ri, rf = shape
+    lut = tables(ax)[kind]
+    rng = np.random.Generator(np.random.PCG64(77 + c))
+    a = rng.integers(0, 256, (n, h, w, c)).astype(np.uint8)
+    b = rng.integers(0, 256, (k, k, c, co)).astype(np.uint8)
+    zi, zf = O.quantized_zero_point(*ri), O.quantized_zero_point(*rf)
+    ref = O.qconv2d(O.desc(n, h, w, c, k, k, co, (s, s), (1, 1), pad), lut, a, b, zi, zf)
+    y, _, _ = ax.ax_conv2d(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), *ri, *rf, [1, s, s, 1], pad, table=ax.Table(array=lut),
+                           ax_tune=False)
+    assert np.array_equal(y.cpu().numpy(), ref)

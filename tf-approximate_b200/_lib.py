@@ -15,7 +15,7 @@ SYMBOLS = [
     "axc_depthwise_conv2d_forward_noalloc", "axc_depthwise_conv2d_status",
     "axc_quant_props", "axc_status_string", "axc_last_cuda_error", "axc_launch_count", "axc_measure_lookup_peak", "axc_debug_bounds_record",
     "axc_add_residual", "axc_max_pool_same", "axc_conv2d_forward_fused", "axc_depthwise_conv2d_forward_fused", "axc_tensor_range", "axc_fake_quant", "axc_conv2d_forward_sharded", "axc_gather_outputs",
-    "axc_qconv2d_workspace_bytes", "axc_qconv2d_forward", "axc_quantized_zero_point", "axc_quantized_output_range",
+    "axc_qconv2d_workspace_bytes", "axc_qconv2d_fast_workspace_bytes", "axc_qconv2d_forward", "axc_quantized_zero_point", "axc_quantized_output_range",
 ]
 
 
@@ -76,6 +76,7 @@ def load():
     L.axc_depthwise_conv2d_forward_noalloc.argtypes = [C.c_void_p, C.POINTER(ConvDesc), C.c_void_p, C.c_void_p, C.c_float,
                                                        C.c_float, C.c_float, C.c_float, C.c_void_p, C.c_int, C.c_void_p]
     L.axc_depthwise_conv2d_status.argtypes = [C.POINTER(ConvDesc), C.c_void_p, C.POINTER(C.c_int32), C.c_int, C.c_void_p]
+    L.axc_qconv2d_fast_workspace_bytes.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
     L.axc_qconv2d_workspace_bytes.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
     L.axc_qconv2d_forward.argtypes = [C.c_void_p, C.POINTER(ConvDesc), C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p,
                                       C.c_void_p, C.c_size_t, C.c_int, C.c_void_p]

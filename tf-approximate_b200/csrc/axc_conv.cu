@@ -593,7 +593,7 @@ int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g,
     DeviceInfo di;
     int rc = device_info(device, &di);
     if (rc) return rc;
-    if (!ref_order && dense_variant() == 0 && di.max_smem_optin >= 232448 && di.smem_base <= 2048u && di.smem_end >= 233472u) {
+    if (!ref_order && dense_variant() == 0 && xtab_device_ok(di)) {
         const size_t need = xtab_scratch_bytes(g);
         int mode, centred, e_min;
         table_form(table, &mode, &centred, &e_min);

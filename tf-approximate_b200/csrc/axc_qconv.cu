@@ -12,6 +12,7 @@
 // caller's output; a second pass subtracts the zero-point terms.
 #include "axc_internal.h"
 #include "axc_sched.h"
+#include "axc_xtab.h"
 
 namespace axc {
 
@@ -134,6 +135,19 @@ extern "C" int axc_qconv2d_workspace_bytes(const axc_conv_desc *desc, size_t *by
     return AXC_OK;
 }
 
+extern "C" int axc_qconv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_t *bytes)
+{
+    if (!bytes) return AXC_INVALID_ARGUMENT;
+    axc::Geom g;
+    int rc = axc::resolve_geometry(desc, false, &g);
+    if (rc) return rc;
+    *bytes = 0;
+    if (g.M * g.Cout == 0) return AXC_OK;
+    const size_t fast = axc::xtab_scratch_bytes(g), base = axc::qconv_layout(g).total;
+    if (fast > 0) *bytes = fast > base ? fast : base;
+    return AXC_OK;
+}
+
 extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, const uint8_t *qinput, const uint8_t *qfilter,
                                    int32_t input_offset, int32_t filter_offset, int32_t *output, void *workspace,
                                    size_t workspace_bytes, int device, void *stream)
@@ -168,6 +182,26 @@ extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, 
     if (prev != device) AXC_CUDA(cudaSetDevice(device));
     cudaStream_t s = cudaStream_t(stream);
     unsigned char *ws = static_cast<unsigned char *>(workspace);
+    {
+        // enough scratch for the expanded-table kernels: they take the bytes as they are and add the zero-point terms at the end
+        DeviceInfo di;
+        rc = device_info(device, &di);
+        const size_t need = xtab_scratch_bytes(g);
+        int mode, centred, e_min;
+        table_form(table, &mode, &centred, &e_min);
+        if (rc == AXC_OK && need > 0 && workspace_bytes >= need && mode != kXtabNone && xtab_device_ok(di)) {
+            const QuantisedOperands u8 = {qinput, qfilter, input_offset, filter_offset};
+            const axc_debug_out ints = {nullptr, nullptr, output};
+            rc = launch_xtab(lut, mode, centred, e_min, g, make_quant(float(-pad_code), float(255 - pad_code), 0.0f, 255.0f), nullptr, nullptr, nullptr,
+                             nullptr, ws, &ints, di, s, &u8);
+            if (prev != device) cudaSetDevice(prev);
+            return rc;
+        }
+        if (rc) {
+            if (prev != device) cudaSetDevice(prev);
+            return rc;
+        }
+    }
     float *xin = reinterpret_cast<float *>(ws + L.xin_off);
     float *xf = reinterpret_cast<float *>(ws + L.xf_off);
     int *bsum = reinterpret_cast<int *>(ws + L.bsum_off);

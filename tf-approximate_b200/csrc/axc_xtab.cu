@@ -166,12 +166,14 @@ struct XGeom {
 struct PrepParams {
     XGeom g;
     const float *input, *filter;
+    const uint8_t *input_u8, *filter_u8;      // quantised operands (then the fp32 pointers are NULL): the code c counts as c - pad
+    int pad;                                  // resp. c, which the call's ranges map back to c
     const uint16_t *lut;
     const float *ranges;
     DevQuant host_q;
     float in_floor;
     int mode, centred, e_min;
-    int *acode, *bcode;         // sums of activation / weight codes (centred tables), else NULL
+    int *acode, *bcode;         // sums of activation / weight codes where the end of the call needs them, else NULL
     unsigned char *codes, *tt;
     uint16_t *wrow;
     uint2 *wb;
@@ -195,6 +197,8 @@ __device__ __forceinline__ unsigned row_address(int mode, unsigned row)
     if (mode != kXtabFull) return kRowsHigh + row * 256u;
     return row < unsigned(kLowRows) ? kRowsLow + row * 512u : kRowsHigh + (row - kLowRows) * 512u;
 }
+
+__device__ __forceinline__ float filter_value(const float *f, const uint8_t *u8, size_t at) { return u8 ? float(__ldg(u8 + at)) : __ldg(f + at); }
 
 // K index of element i of chunk ch, or -1 where there is none
 __device__ __forceinline__ int k_of(const XGeom &g, int ch, int i)
@@ -220,7 +224,7 @@ __device__ void prep_filter_sums(const PrepParams &P, const DevQuant &q, int blo
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
             const int l = l0 + e * 8 + warp;
-            v[e] = (l < P.g.K && j < P.g.Cout) ? __ldg(P.filter + (size_t)l * P.g.Cout + j) : 0.0f;
+            v[e] = (l < P.g.K && j < P.g.Cout) ? filter_value(P.filter, P.filter_u8, (size_t)l * P.g.Cout + j) : 0.0f;
         }
     };
     fetch(0);
@@ -291,7 +295,7 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
             const int j = nt * g.TNC + slot_channel(P.mode, slot), k = k_of(g, ch, i);
             unsigned row = kNull;
             if (k >= 0 && j < g.Cout) {
-                row = code_of(__ldg(P.filter + (size_t)k * g.Cout + j), q.f_off, q.f_inv);
+                row = code_of(filter_value(P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
                 if (P.qf_debug) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(row);
             }
             P.wrow[x] = uint16_t(row_address(P.mode, row) >> 4);
@@ -362,7 +366,10 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
                     at[u] = local[u] * P.pitch + c4 * 4;
                     if (unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W)) {
                         const int pix = (n * g.H + iy) * g.W + ix;
-                        v[u] = __ldg(reinterpret_cast<const float4 *>(P.input + (long long)pix * g.C) + c4);
+                        if (P.input_u8) {
+                            const uchar4 w = __ldg(reinterpret_cast<const uchar4 *>(P.input_u8 + (long long)pix * g.C) + c4);
+                            v[u] = make_float4(float(int(w.x) - P.pad), float(int(w.y) - P.pad), float(int(w.z) - P.pad), float(int(w.w) - P.pad));
+                        } else v[u] = __ldg(reinterpret_cast<const float4 *>(P.input + (long long)pix * g.C) + c4);
                         if (ry < own_h && rx < own_w && !g.im2col) code_at[u] = ((c4 >> 2) * planes + pix) * 4 + (c4 & 3);
                     }
                 }
@@ -393,7 +400,7 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
             const int iy = iy0 + ry, ix = ix0 + rx;
             const bool inside = unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W);
             const long long pix = ((long long)n * g.H + iy) * g.W + ix;
-            float v = inside ? __ldg(P.input + pix * g.C + c) : 0.0f;
+            float v = !inside ? 0.0f : P.input_u8 ? float(int(__ldg(P.input_u8 + pix * g.C + c)) - P.pad) : __ldg(P.input + pix * g.C + c);
             v = max_keep_nan(v, P.in_floor);
             prep_smem[(ry * P.RW + rx) * P.pitch + c] = v;
             if (P.acode && !g.im2col) atomicAdd(pix_codes + ry * P.RW + rx, int(code_of(v, q.in_off, q.in_inv)));
@@ -469,6 +476,7 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
 struct ExpandParams {
     XGeom g;
     const float *filter;
+    const uint8_t *filter_u8;
     const uint16_t *lut;
     const float *ranges;
     DevQuant host_q;
@@ -517,7 +525,7 @@ __global__ void __launch_bounds__(256) xexpand_kernel(const ExpandParams P)
             const int j = nt * TNC + slot_channel(MODE, s);
             code[s] = 0;
             if (k >= 0 && j < g.Cout) {
-                code[s] = code_of(__ldg(P.filter + (size_t)k * g.Cout + j), q.f_off, q.f_inv);
+                code[s] = code_of(filter_value(P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
                 mask |= 1u << s;
                 if (P.qf_debug && a0 == 0) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(code[s]);
             }
@@ -556,9 +564,10 @@ struct XParams {
     int32_t *partial;           // K split over CTAs: integer sums are added here
     const float *bias, *residual;
     float out_floor;
-    int plain;                  // fp32 output only, it and the shortcut at 16-byte boundaries
+    int plain;                  // one output (fp32 or the integer sums), it and the shortcut at 16-byte boundaries
     int k_e_min;                // K times what every entry was stored less
-    const int *acode, *bcode;   // centred tables: sums of codes, 128 of which every lookup was stored less; else NULL
+    const int *acode, *bcode;   // sums of codes (or NULL) and what they enter the total with: 128 for a centred table, less
+    int a_coef, b_coef;         // the zero points of a quantised call
     int splits, chunks_per_split;
     long long units;            // pixel tiles x channel tiles x splits
 };
@@ -950,7 +959,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         for (int e = 0; e < 4; ++e) {
             t2[e] = (!P.partial && j0 + e < g.Cout) ? __fmul_rn(Q.m1, __ldg(P.bsum + j0 + e)) : 0.0f;
             bias[e] = (P.bias && j0 + e < g.Cout) ? __ldg(P.bias + j0 + e) : 0.0f;
-            back[e] = P.k_e_min + (MODE == kXtabFull && P.bcode && j0 + e < g.Cout ? 128 * __ldg(P.bcode + j0 + e) : 0);
+            back[e] = P.k_e_min + (P.bcode && j0 + e < g.Cout ? P.b_coef * __ldg(P.bcode + j0 + e) : 0);
         }
         const bool whole = j0 + 4 <= g.Cout && (g.Cout & 3) == 0, chan = j0 < g.Cout;
         constexpr int EB = kAcc < 4 ? kAcc : 4;
@@ -959,7 +968,16 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         const int left = chan ? g.M - m0 - first : 0;              // > kStep * i: fragment i has a pixel
         const long long at0 = (long long)(m0 + first) * g.Cout + j0;
         const int row = kStep * g.Cout;
-        if (P.plain && whole) {
+        if (P.plain && whole && P.acc_out) {
+            int32_t *ints = P.acc_out + at0;
+#pragma unroll
+            for (int i = 0; i < kAcc; ++i) {
+                if (i * kStep >= left || !AXC_GLOBAL_OK(at0 + i * row + 3, (long long)g.M * g.Cout, 315u)) continue;
+                const int a_code = P.acode ? P.a_coef * __ldg(P.acode + m0 + first + i * kStep) : 0;
+                *reinterpret_cast<int4 *>(ints + i * row) = make_int4(acc[i][0] + back[0] + a_code, acc[i][1] + back[1] + a_code,
+                                                                      acc[i][2] + back[2] + a_code, acc[i][3] + back[3] + a_code);
+            }
+        } else if (P.plain && whole) {
             // The common case on its own, in as few instructions as possible: the code is unrolled over the fragments and runs
             // once per tile, so its length is paid in instruction fetches (one loop for all cases: 51 000 clocks per tile of
             // 2048 pixels).  Four fragments at a time: what they read is requested before the first is finished.
@@ -972,7 +990,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
                 int a_code[EB];
                 float4 r[EB];
 #pragma unroll
-                for (int i = 0; i < EB; ++i) a_code[i] = MODE == kXtabFull && P.acode && (i0 + i) * kStep < left ? 128 * __ldg(acode + (i0 + i) * kStep) : 0;
+                for (int i = 0; i < EB; ++i) a_code[i] = MODE == kXtabFull && P.acode && (i0 + i) * kStep < left ? P.a_coef * __ldg(acode + (i0 + i) * kStep) : 0;
 #pragma unroll
                 for (int i = 0; i < EB; ++i) a_sum[i] = (i0 + i) * kStep < left ? __fmul_rn(Q.m2, __ldg(asum + (i0 + i) * kStep)) : 0.0f;
                 if (P.residual)
@@ -1004,7 +1022,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
                 const long long at = at0 + i * row;
                 if (!AXC_GLOBAL_OK(at, (long long)g.M * g.Cout, 314u)) continue;
                 const float a_sum = P.partial ? 0.0f : __ldg(P.asum + m0 + first + i * kStep);
-                const int a_code = MODE == kXtabFull && P.acode && !P.partial ? 128 * __ldg(P.acode + m0 + first + i * kStep) : 0;
+                const int a_code = P.acode && !P.partial ? P.a_coef * __ldg(P.acode + m0 + first + i * kStep) : 0;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     if (j0 + e >= g.Cout) continue;
@@ -1033,7 +1051,7 @@ __global__ void __launch_bounds__(256) xfinal_kernel(const XParams P)
     const long long total = (long long)P.g.M * P.g.Cout;
     for (long long x = (long long)blockIdx.x * 256 + threadIdx.x; x < total; x += (long long)gridDim.x * 256) {
         const int m = int(x / P.g.Cout), j = int(x - (long long)m * P.g.Cout);
-        const int tot = P.partial[x] + P.k_e_min + (P.acode ? 128 * (__ldg(P.acode + m) + __ldg(P.bcode + j)) : 0);
+        const int tot = P.partial[x] + P.k_e_min + (P.acode ? P.a_coef * __ldg(P.acode + m) + P.b_coef * __ldg(P.bcode + j) : 0);
         float y = dequantise(Q, tot, __ldg(P.asum + m), __fmul_rn(Q.m1, __ldg(P.bsum + j)));
         if (P.bias) y = __fadd_rn(y, __ldg(P.bias + j));
         if (P.residual) y = __fadd_rn(y, __ldg(P.residual + x));
@@ -1230,9 +1248,10 @@ size_t xtab_scratch_bytes(const Geom &g)
 
 int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const Geom &g, const Quant &q, const float *ranges_dev,
                 const float *input, const float *filter, float *output, unsigned char *scratch, const axc_debug_out *dbg,
-                const DeviceInfo &di, cudaStream_t stream)
+                const DeviceInfo &di, cudaStream_t stream, const QuantisedOperands *u8)
 {
     PrepParams A;
+    XParams P;
     if (!xgeom(g, &A.g)) return AXC_INTERNAL;
     XGeom &x = A.g;
     x.TNC = mode == kXtabFull ? 8 : 16;
@@ -1240,14 +1259,18 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     const XLayout L = xlayout(g, x);
     const size_t partial_bytes = size_t(g.M) * g.Cout * 4;
     const Config cf = choose_config(mode, x, di.sm_count, partial_bytes <= kPartialMax, L.xt_bytes);
-    const int vec = (g.C % 4 == 0 && (reinterpret_cast<uintptr_t>(input) & 15u) == 0) ? 1 : 0;
+    const int vec = (g.C % 4 == 0 && (u8 ? (reinterpret_cast<uintptr_t>(u8->input) & 3u) : (reinterpret_cast<uintptr_t>(input) & 15u)) == 0) ? 1 : 0;
     PrepTile t;
     if (!prep_tile(g, vec, x.im2col != 0, &t)) return AXC_INTERNAL;
+    A.input_u8 = u8 ? u8->input : nullptr; A.filter_u8 = u8 ? u8->filter : nullptr; A.pad = u8 ? u8->input_offset & 255 : 0;
     A.input = input; A.filter = filter; A.lut = lut_dev; A.ranges = ranges_dev; A.host_q = host_dev_quant(q, g.K);
     A.in_floor = g.ep.input_relu ? 0.0f : -INFINITY;
     A.mode = mode; A.centred = centred; A.e_min = e_min;
-    A.acode = centred ? reinterpret_cast<int *>(scratch + L.acode) : nullptr;
-    A.bcode = centred ? reinterpret_cast<int *>(scratch + L.bcode) : nullptr;
+    P.a_coef = 128 * centred - (u8 ? u8->filter_offset : 0);
+    P.b_coef = 128 * centred - (u8 ? u8->input_offset : 0);
+    const bool sums = P.a_coef != 0 || P.b_coef != 0;
+    A.acode = sums ? reinterpret_cast<int *>(scratch + L.acode) : nullptr;
+    A.bcode = sums ? reinterpret_cast<int *>(scratch + L.bcode) : nullptr;
     A.codes = scratch + L.codes; A.tt = scratch + L.tt;
     A.wrow = reinterpret_cast<uint16_t *>(scratch + L.wrow); A.wb = reinterpret_cast<uint2 *>(scratch + L.wb);
     A.asum = reinterpret_cast<float *>(scratch + L.asum); A.bsum = reinterpret_cast<float *>(scratch + L.bsum);
@@ -1268,20 +1291,19 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
 
     if (cf.pre) {
         ExpandParams E;
-        E.g = x; E.filter = filter; E.lut = lut_dev; E.ranges = ranges_dev; E.host_q = A.host_q; E.centred = centred; E.e_min = e_min;
+        E.g = x; E.filter = filter; E.filter_u8 = A.filter_u8; E.lut = lut_dev; E.ranges = ranges_dev; E.host_q = A.host_q; E.centred = centred; E.e_min = e_min;
         E.xt = scratch + L.xt; E.wb = A.wb; E.qf_debug = A.qf_debug;
         const int rc = mode == kXtabFull ? launch_expand<kXtabFull>(E, di, stream) : launch_expand<kXtabByte>(E, di, stream);
         if (rc) return rc;
     }
 
-    XParams P;
     P.g = x;
     P.xt = cf.pre ? scratch + L.xt : nullptr;
     P.codes = A.codes; P.tt = A.tt; P.wrow = A.wrow; P.wb = A.wb; P.asum = A.asum; P.bsum = A.bsum; P.hdr = A.hdr;
     P.output = output; P.acc_out = dbg ? dbg->acc : nullptr;
     P.acode = A.acode; P.bcode = A.bcode;
     P.bias = g.ep.bias; P.residual = g.ep.residual; P.out_floor = g.ep.relu ? 0.0f : -INFINITY;
-    P.k_e_min = int(unsigned(g.K) * unsigned(e_min));
+    P.k_e_min = int(unsigned(g.K) * (unsigned(e_min) + (u8 ? unsigned(u8->input_offset) * unsigned(u8->filter_offset) : 0u)));
     P.splits = cf.splits; P.chunks_per_split = cf.chunks_per_split;
     P.units = ((long long)x.M + kWarps * 8 * cf.nb - 1) / (kWarps * 8 * cf.nb) * x.tiles_n * cf.splits;
     if (P.units >= (1ll << 31)) return AXC_INTERNAL;
@@ -1290,8 +1312,8 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
         P.partial = reinterpret_cast<int32_t *>(scratch + L.partial);
         AXC_CUDA(cudaMemsetAsync(P.partial, 0, partial_bytes, stream));
     }
-    P.plain = (output && !P.acc_out && !P.partial &&
-               ((reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(g.ep.residual)) & 15u) == 0) ? 1 : 0;
+    P.plain = ((output != nullptr) != (P.acc_out != nullptr) && !P.partial &&
+               ((reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(P.acc_out) | reinterpret_cast<uintptr_t>(g.ep.residual)) & 15u) == 0) ? 1 : 0;
     int rc = mode == kXtabFull ? launch_mode<kXtabFull>(cf, P, di, stream)
              : mode == kXtabByte ? launch_mode<kXtabByte>(cf, P, di, stream) : launch_mode<kXtabExact>(cf, P, di, stream);
     if (rc) return rc;

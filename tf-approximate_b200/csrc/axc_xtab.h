@@ -11,11 +11,21 @@ namespace axc {
 // What an expanded entry holds (table_form): two digits to the base 255, one byte, or nothing (only the exact products).
 enum XtabMode { kXtabFull = 16, kXtabByte = 8, kXtabExact = 0, kXtabNone = -1 };
 
+// The fixed shared-window addresses of the kernels fit this device.
+inline bool xtab_device_ok(const DeviceInfo &di) { return di.max_smem_optin >= 232448 && di.smem_base <= 2048u && di.smem_end >= 233472u; }
+
 // Scratch bytes of the expanded-table route for this shape; 0 where the plan-based kernels serve the shape.
 size_t xtab_scratch_bytes(const Geom &g);
 
+// Operands of the quantised entry point and their zero points: the int32 result carries the terms
+// K in_off f_off - f_off sum(a) - in_off sum(b); a tap outside the image has the code input_offset modulo 256.
+struct QuantisedOperands {
+    const uint8_t *input, *filter;
+    int input_offset, filter_offset;
+};
+
 int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const Geom &g, const Quant &q, const float *ranges_dev,
                 const float *input, const float *filter, float *output, unsigned char *scratch, const axc_debug_out *dbg,
-                const DeviceInfo &di, cudaStream_t stream);
+                const DeviceInfo &di, cudaStream_t stream, const QuantisedOperands *u8 = nullptr);
 
 }  // namespace axc

@@ -371,8 +371,12 @@ def ax_conv2d(input, filter, min_input, max_input, min_filter, max_filter, strid
     raise_for_status(L.axc_quantized_zero_point(float(min_input), float(max_input), C.byref(off_in)), "input offset")
     raise_for_status(L.axc_quantized_zero_point(float(min_filter), float(max_filter), C.byref(off_f)), "filter offset")
     wsz = C.c_size_t()
-    raise_for_status(L.axc_qconv2d_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
-    ws = _workspace(dev, wsz.value, (f.data_ptr(), tuple(f.shape), id(tab), "q"))
+    raise_for_status(L.axc_qconv2d_fast_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
+    if wsz.value > 0:
+        ws = torch.empty(wsz.value, dtype=torch.uint8, device=dev)      # scratch of this call alone
+    else:
+        raise_for_status(L.axc_qconv2d_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
+        ws = _workspace(dev, wsz.value, (f.data_ptr(), tuple(f.shape), id(tab), "q"))
     dev_index = dev.index if dev.index is not None else torch.cuda.current_device()
     st = L.axc_qconv2d_forward(tab.handle, C.byref(d), x.data_ptr(), f.data_ptr(), off_in.value, off_f.value,
                                out.data_ptr(), ws.data_ptr(), ws.numel(), dev_index,
