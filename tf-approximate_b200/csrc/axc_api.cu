@@ -226,6 +226,26 @@ Workspace depthwise_workspace(int KHW, int C, int mult)
     return w;
 }
 
+// The rows of the expanded tables' form behind the native image.
+static void append_rows(const axc_table *t, std::vector<uint16_t> *image)
+{
+    int mode, centred, e_min;
+    table_form(t, &mode, &centred, &e_min);
+    const size_t at = image->size();
+    image->resize(at + 257 * 256, 0);
+    uint16_t *digits = image->data() + at;
+    uint8_t *bytes = reinterpret_cast<uint8_t *>(digits);
+    if (mode != kXtabFull && mode != kXtabByte) return;
+    for (int a = 0; a < 256; ++a) {
+        const uint16_t *row = t->host.data() + a * 256;
+        for (int b = 0; b < 256; ++b) {
+            const unsigned d = unsigned(int(row[b]) - (mode == kXtabByte ? a * b : centred * 128 * (a + b)) - e_min);
+            if (mode == kXtabByte) bytes[b * 256 + a] = uint8_t(d);
+            else digits[b * 256 + a] = uint16_t(d + d / 255u);     // (d mod 255) + 256 (d div 255)
+        }
+    }
+}
+
 const uint16_t *table_device_ptr(axc_table *t, int device, int *status)
 {
     *status = AXC_OK;
@@ -248,9 +268,11 @@ const uint16_t *table_device_ptr(axc_table *t, int device, int *status)
     int prev = 0;
     cudaGetDevice(&prev);
     uint16_t *p = nullptr;
+    std::vector<uint16_t> image(t->host);
+    append_rows(t, &image);
     e = cudaSetDevice(device);
-    if (e == cudaSuccess) e = cudaMalloc(&p, 65536 * sizeof(uint16_t));
-    if (e == cudaSuccess) e = cudaMemcpy(p, t->host.data(), 65536 * sizeof(uint16_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&p, image.size() * sizeof(uint16_t));
+    if (e == cudaSuccess) e = cudaMemcpy(p, image.data(), image.size() * sizeof(uint16_t), cudaMemcpyHostToDevice);
     // A copy from pageable host memory returns once the data is staged; the transfer itself is ordered on the legacy
     // stream only.  The caller's stream may be a non-blocking one, which does not wait for the legacy stream: wait
     // here until the replica is complete (once per table and device).

@@ -33,7 +33,6 @@
 //
 // Arithmetic (quantiser, table index, dequantisation) is the reference's, tf2/src/approx_nn_conv_kernels.cpp:167-296.
 #include <cmath>
-#include <type_traits>
 
 #include "axc_quant.cuh"
 #include "axc_sched.h"
@@ -123,6 +122,11 @@ __device__ __forceinline__ void mbar_wait(unsigned bar, unsigned parity, bool &o
         if (it >= kWaitPolls) ok = false;
     }
 }
+
+// Programmatic dependent launch: the three kernels of a call are launched so that each may start while the one before it
+// runs.  pdl_trigger: the next kernel may be brought in; pdl_wait: everything before this kernel is complete and visible.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <unsigned SEL>
 __device__ __forceinline__ unsigned prmt(unsigned a, unsigned b)
@@ -266,6 +270,7 @@ __device__ void prep_filter_sums(const PrepParams &P, const DevQuant &q, int blo
 __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
 {
     extern __shared__ __align__(16) float prep_smem[];
+    pdl_trigger();
     const XGeom &g = P.g;
     const int tid = threadIdx.x;
     const DevQuant q = P.ranges ? dev_quant_from_ranges(P.ranges, g.K) : P.host_q;
@@ -473,79 +478,102 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
 // ------------------------------------------------------------------------------------------------------------------
 // expanded tables in global memory, for calls with enough pixels to use each of them several times
 // ------------------------------------------------------------------------------------------------------------------
+constexpr int kExpandThreads = 512;
+
 struct ExpandParams {
     XGeom g;
     const float *filter;
     const uint8_t *filter_u8;
-    const uint16_t *lut;
+    const unsigned char *rows;      // table_rows_device: one row of entries per weight, row 256 all zeros
     const float *ranges;
     DevQuant host_q;
-    int centred, e_min;
     unsigned char *xt;
     uint2 *wb;
     uint8_t *qf_debug;
 };
 
-// xt[channel tile][chunk][row a][piece kk][16 bytes], kk = octet * 8 + k.  The table as it is looked up (rows moved by xor z)
-// lies in shared memory; a thread gathers the entries of its piece's 8 or 16 weights and writes 16 bytes, 16 threads the
-// 256 bytes of a row.  Bound by the gathers (random banks) and, close behind, by the writes: 64 KiB per chunk.
+// xt[channel tile][chunk][row a][piece kk][16 bytes], kk = octet * 8 + k.  The table's rows (one per weight) lie in shared memory.
+// A lane reads the same word (two or four a) of the rows of its piece's 8 or 16 weights, transposes in registers and writes
+// whole pieces; the 32 lanes (8 k x 4 words) read 32 different banks whatever the weights are, and write 128-byte runs.
+// Bound by the writes, 64 KiB per chunk (gathering entry by entry with random banks took 12 700 clocks per chunk, this 1500).
 template <int MODE>
-__global__ void __launch_bounds__(256) xexpand_kernel(const ExpandParams P)
+__global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const ExpandParams P)
 {
     constexpr int TNC = MODE == kXtabFull ? 8 : 16;
-    using Entry = typename std::conditional<MODE == kXtabFull, uint16_t, uint8_t>::type;
+    constexpr unsigned kRow = MODE == kXtabFull ? 512u : 256u;     // bytes of a table row
+    constexpr int kRounds = MODE == kXtabFull ? 64 : 32;           // warp rounds per chunk
     extern __shared__ __align__(16) unsigned char expand_smem[];
-    Entry *tab = reinterpret_cast<Entry *>(expand_smem);
     const XGeom &g = P.g;
-    const int tid = threadIdx.x;
-    const DevQuant q = P.ranges ? dev_quant_from_ranges(P.ranges, g.K) : P.host_q;
-    const int z = int(code_of(0.0f, q.in_off, q.in_inv));
-    for (int x = tid; x < 8192; x += 256) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(P.lut) + x);
-        const unsigned w4[4] = {v.x, v.y, v.z, v.w};
-        const int a = x >> 5, b0 = (x & 31) * 8;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int entry = int((w4[e >> 1] >> (16 * (e & 1))) & 0xFFFFu), b = b0 + e;
-            const int d = entry - (MODE == kXtabFull ? 128 * (a + b) * P.centred : a * b) - P.e_min;
-            tab[(a ^ z) * 256 + b] = MODE == kXtabFull ? Entry(d % 255 + (d / 255) * 256) : Entry(d);
-        }
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned tab = (unsigned)__cvta_generic_to_shared(expand_smem), lists = tab + 257u * kRow, bar = lists + 2u * 16u * TNC * 2u;
+    pdl_trigger();
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(257u * kRow) : "memory");
+        bulk_copy(tab, P.rows, 257u * kRow, bar);
     }
     __syncthreads();
-    const int kk = tid & 15, a0 = tid >> 4;
-    const int i = ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);             // element 4t + 2*octet + p
+    const DevQuant q = P.ranges ? dev_quant_from_ranges(P.ranges, g.K) : P.host_q;
+    const unsigned z = code_of(0.0f, q.in_off, q.in_inv);
+    bool ok = true;
+    mbar_wait(bar, 0u, ok);
+    // thread (kk, slot) of the first 16*TNC prepares the list of table rows of a chunk
+    const int kk = tid / TNC, slot = tid % TNC;
+    const int elem = ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);           // element 4t + 2*octet + p
     const int total = g.tiles_n * g.chunks;
-    for (int tc = int(blockIdx.x); tc < total; tc += int(gridDim.x)) {
-        const int nt = tc / g.chunks, ch = tc - nt * g.chunks;
-        const int k = k_of(g, ch, i);
-        unsigned code[TNC];
-        unsigned mask = 0;
-#pragma unroll
-        for (int s = 0; s < TNC; ++s) {
-            const int j = nt * TNC + slot_channel(MODE, s);
-            code[s] = 0;
+    const int kidx = lane & 7, sub = lane >> 3;
+    unsigned parity = 0;
+    for (int tc = int(blockIdx.x); tc < total; tc += int(gridDim.x), parity ^= 1u) {
+        if (tid < 16 * TNC) {
+            const int nt = tc / g.chunks, ch = tc - nt * g.chunks;
+            const int k = k_of(g, ch, elem), cj = slot_channel(MODE, slot), j = nt * TNC + cj;
+            unsigned row = kNull;
             if (k >= 0 && j < g.Cout) {
-                code[s] = code_of(filter_value(P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
-                mask |= 1u << s;
-                if (P.qf_debug && a0 == 0) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(code[s]);
+                row = code_of(filter_value(P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
+                if (P.qf_debug) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(row);
             }
-            if (MODE != kXtabFull && a0 == 0) {
-                const int cj = slot_channel(MODE, s), t = i >> 2, h = (cj >> 1) & 1, n = (cj >> 2) * 2 + (cj & 1);
-                reinterpret_cast<unsigned char *>(P.wb + (size_t)tc * 32 + n * 4 + t)[h * 4 + (i & 3)] = (unsigned char)code[s];
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(lists + parity * (16u * TNC * 2u) + unsigned(kk * TNC + slot) * 2u), "h"((unsigned short)row) : "memory");
+            if (MODE != kXtabFull) {
+                // exact products, B operand half h, column n: channel (n>>1)*4 + 2h + (n&1); lane (n, t) holds elements 4t..4t+3
+                const int t = elem >> 2, h = (cj >> 1) & 1, n = (cj >> 2) * 2 + (cj & 1);
+                reinterpret_cast<unsigned char *>(P.wb + (size_t)tc * 32 + n * 4 + t)[h * 4 + (elem & 3)] = row == kNull ? 0 : (unsigned char)row;
             }
         }
-        uint4 *dst = reinterpret_cast<uint4 *>(P.xt + (size_t)tc * 65536u) + kk;
-#pragma unroll 2
-        for (int a = a0; a < 256; a += 16) {
-            unsigned w[4] = {0, 0, 0, 0};
+        __syncthreads();                                           // (the other list's readers are a chunk behind this barrier)
+        for (int r = warp; r < kRounds; r += kExpandThreads / 32) {
+            const int o = r / (kRounds / 2), x = r % (kRounds / 2);                  // octet, round
+            const unsigned word = unsigned((x >> 3) * 32 + ((4 * ((x & 7) + kidx) + sub) & 31));
+            const unsigned list = lists + parity * (16u * TNC * 2u) + unsigned((o * 8 + kidx) * TNC) * 2u;
+            unsigned v[TNC];
 #pragma unroll
-            for (int s = 0; s < TNC; ++s) {
-                const unsigned v = ((mask >> s) & 1u) ? unsigned(tab[a * 256 + code[s]]) : 0u;
-                w[s / (TNC / 4)] |= v << ((s % (TNC / 4)) * (128 / TNC));
+            for (int s4 = 0; s4 < TNC / 8; ++s4) {
+                const uint4 l = lds128(list + unsigned(s4) * 16u);
+                const unsigned l4[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+                for (int s = 0; s < 8; ++s) v[s4 * 8 + s] = lds32(tab + ((s & 1) ? l4[s >> 1] >> 16 : l4[s >> 1] & 0xFFFFu) * kRow + word * 4u);
             }
-            dst[a * 16] = make_uint4(w[0], w[1], w[2], w[3]);
+            uint4 *dst = reinterpret_cast<uint4 *>(P.xt + (size_t)tc * 65536u) + o * 8 + kidx;
+            if (MODE == kXtabFull) {
+                const unsigned a = word * 2u;
+                dst[(a ^ z) * 16u] = make_uint4(prmt<0x5410>(v[0], v[1]), prmt<0x5410>(v[2], v[3]), prmt<0x5410>(v[4], v[5]), prmt<0x5410>(v[6], v[7]));
+                dst[((a + 1u) ^ z) * 16u] = make_uint4(prmt<0x7632>(v[0], v[1]), prmt<0x7632>(v[2], v[3]), prmt<0x7632>(v[4], v[5]), prmt<0x7632>(v[6], v[7]));
+            } else {
+                unsigned w4[4][4];                                 // [row a][word]
+#pragma unroll
+                for (int w = 0; w < TNC / 4; ++w) {
+                    const unsigned t0 = prmt<0x5140>(v[4 * w], v[4 * w + 1]), t1 = prmt<0x5140>(v[4 * w + 2], v[4 * w + 3]);
+                    const unsigned t2 = prmt<0x7362>(v[4 * w], v[4 * w + 1]), t3 = prmt<0x7362>(v[4 * w + 2], v[4 * w + 3]);
+                    w4[0][w] = prmt<0x5410>(t0, t1); w4[1][w] = prmt<0x7632>(t0, t1);
+                    w4[2][w] = prmt<0x5410>(t2, t3); w4[3][w] = prmt<0x7632>(t2, t3);
+                }
+#pragma unroll
+                for (unsigned i = 0; i < 4; ++i) dst[((word * 4u + i) ^ z) * 16u] = make_uint4(w4[i][0], w4[i][1], w4[i][2], w4[i][TNC / 4 - 1]);
+            }
         }
     }
+    pdl_wait();                                                    // the kernel after this one waits for this one only
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -605,6 +633,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         if (tid == 0) atomicExch(const_cast<int *>(&P.hdr->status), 2);
         return;
     }
+    pdl_wait();
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) { mbar_init(tab_full + s * 8, PRE ? 1 : kWarps); mbar_init(tab_empty + s * 8, kWarps); }
         mbar_init(rows_full, 1);
@@ -1153,8 +1182,9 @@ Config choose_config(int mode, const XGeom &x, int sms, bool may_split, size_t x
             const int pix = kWarps * 8 * nb;
             const long long tiles = ((long long)x.M + pix - 1) / pix * tiles_n;
             const double octet = mode == kXtabExact ? 0.30 * pix + 100.0 : 1.09 * pix + (pre ? 130.0 : 850.0);
-            for (int sp = 1; sp <= 64 && sp <= x.chunks; sp *= 2) {
-                if (sp > 1 && (!may_split || tiles >= sms)) break;
+            for (int r = 0; r <= 4; ++r) {                         // no split, or as many as fill one to four rounds
+                if (r > 0 && (!may_split || tiles >= sms)) break;
+                const int sp = r == 0 ? 1 : int(r * (long long)sms / tiles < x.chunks ? r * (long long)sms / tiles : x.chunks);
                 const int cps = (x.chunks + sp - 1) / sp;
                 const int spe = (x.chunks + cps - 1) / cps;
                 const long long rounds = (tiles * spe + sms - 1) / sms;
@@ -1193,15 +1223,27 @@ XLayout xlayout(const Geom &g, const XGeom &x)
     return L;
 }
 
+// launch of a kernel that calls pdl_wait() before it touches what earlier kernels of the stream leave
+template <typename Kernel, typename Params>
+int launch_dependent(Kernel kernel, unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const Params &P)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    AXC_CUDA(cudaLaunchKernelEx(&cfg, kernel, P));
+    count_launch();
+    return AXC_OK;
+}
+
 template <int MODE, int NB, bool PRE>
 int launch_variant(const XParams &P, const DeviceInfo &di, cudaStream_t stream)
 {
     AXC_CUDA(cudaFuncSetAttribute(xtab_kernel<MODE, NB, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin));
     const long long grid = P.units < di.sm_count ? P.units : di.sm_count;
-    xtab_kernel<MODE, NB, PRE><<<unsigned(grid), kWarps * 32, size_t(di.max_smem_optin), stream>>>(P);
-    AXC_CUDA(cudaGetLastError());
-    count_launch();
-    return AXC_OK;
+    return launch_dependent(xtab_kernel<MODE, NB, PRE>, unsigned(grid), kWarps * 32, size_t(di.max_smem_optin), stream, P);
 }
 
 template <int MODE>
@@ -1223,14 +1265,11 @@ int launch_mode(const Config &cf, const XParams &P, const DeviceInfo &di, cudaSt
 template <int MODE>
 int launch_expand(const ExpandParams &E, const DeviceInfo &di, cudaStream_t stream)
 {
-    constexpr size_t smem = MODE == kXtabFull ? 131072 : 65536;
-    constexpr int per_sm = MODE == kXtabFull ? 1 : 3;
+    constexpr size_t smem = MODE == kXtabFull ? 257 * 512 + 2 * 16 * 8 * 2 + 16 : 257 * 256 + 2 * 16 * 16 * 2 + 16;
+    constexpr int per_sm = 1;
     AXC_CUDA(cudaFuncSetAttribute(xexpand_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const int total = E.g.tiles_n * E.g.chunks, grid = total < di.sm_count * per_sm ? total : di.sm_count * per_sm;
-    xexpand_kernel<MODE><<<unsigned(grid), 256, smem, stream>>>(E);
-    AXC_CUDA(cudaGetLastError());
-    count_launch();
-    return AXC_OK;
+    return launch_dependent(xexpand_kernel<MODE>, unsigned(grid), kExpandThreads, smem, stream, E);
 }
 
 }  // namespace
@@ -1284,6 +1323,11 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     A.blocks_t = cf.pre ? 0 : 32;
     const long long blocks = (long long)A.blocks_sum + A.blocks_w + A.blocks_t + (long long)g.N * A.tiles_y * A.tiles_x;
     if (blocks >= (1ll << 31)) return AXC_INTERNAL;
+    P.partial = nullptr;
+    if (cf.splits > 1) {
+        P.partial = reinterpret_cast<int32_t *>(scratch + L.partial);
+        AXC_CUDA(cudaMemsetAsync(P.partial, 0, partial_bytes, stream));
+    }
     AXC_CUDA(cudaFuncSetAttribute(xprep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPrepSmemMax)));
     xprep_kernel<<<unsigned(blocks), 256, t.smem, stream>>>(A);
     AXC_CUDA(cudaGetLastError());
@@ -1291,7 +1335,7 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
 
     if (cf.pre) {
         ExpandParams E;
-        E.g = x; E.filter = filter; E.filter_u8 = A.filter_u8; E.lut = lut_dev; E.ranges = ranges_dev; E.host_q = A.host_q; E.centred = centred; E.e_min = e_min;
+        E.g = x; E.filter = filter; E.filter_u8 = A.filter_u8; E.rows = reinterpret_cast<const unsigned char *>(lut_dev + 65536); E.ranges = ranges_dev; E.host_q = A.host_q;
         E.xt = scratch + L.xt; E.wb = A.wb; E.qf_debug = A.qf_debug;
         const int rc = mode == kXtabFull ? launch_expand<kXtabFull>(E, di, stream) : launch_expand<kXtabByte>(E, di, stream);
         if (rc) return rc;
@@ -1307,11 +1351,6 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     P.splits = cf.splits; P.chunks_per_split = cf.chunks_per_split;
     P.units = ((long long)x.M + kWarps * 8 * cf.nb - 1) / (kWarps * 8 * cf.nb) * x.tiles_n * cf.splits;
     if (P.units >= (1ll << 31)) return AXC_INTERNAL;
-    P.partial = nullptr;
-    if (cf.splits > 1) {
-        P.partial = reinterpret_cast<int32_t *>(scratch + L.partial);
-        AXC_CUDA(cudaMemsetAsync(P.partial, 0, partial_bytes, stream));
-    }
     P.plain = ((output != nullptr) != (P.acc_out != nullptr) && !P.partial &&
                ((reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(P.acc_out) | reinterpret_cast<uintptr_t>(g.ep.residual)) & 15u) == 0) ? 1 : 0;
     int rc = mode == kXtabFull ? launch_mode<kXtabFull>(cf, P, di, stream)
