@@ -125,10 +125,11 @@ int axc_depthwise_conv2d_output_dims(const axc_conv_desc *desc, int64_t out4[4])
  * (its first 256 bytes decide), only slower.  One buffer serves one stream at a time. */
 int axc_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
 int axc_depthwise_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
-/* Scratch with which a dense call takes the expanded-table kernels; 0 where the plan-based kernels are the better
- * ones for the shape.  A call that brings at least this much is served by them (same results, no plan to build);
- * nothing in the buffer outlives the call, so one buffer may serve all layers of a stream in turn. */
-int axc_conv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
+/* Scratch with which a dense call on `table` takes the expanded-table kernels; 0 where other kernels serve the shape, the table
+ * or the mode of accumulation.  table == NULL: enough for every table (a call that then does not take them falls back to the
+ * plan-based kernels if the buffer has axc_conv2d_workspace_bytes).  Same results, no plan to build; nothing in the buffer
+ * outlives the call, so one buffer may serve all layers of a stream in turn. */
+int axc_conv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc *desc, size_t *bytes);
 /* Reads back {rebuilt in the last call, fallback kernel in use, kernel status (0 = fine), schedule steps per
  * ideal step in per-mille} of the plan in a dense workspace.  Blocks until `stream` is idle.  Diagnostics only;
  * no counterpart in the reference. */
@@ -276,7 +277,7 @@ int axc_depthwise_conv2d_forward_noalloc(axc_table *table, const axc_conv_desc *
  * of axc_conv2d_forward; the workspace additionally holds an fp32 image of both operands. */
 int axc_qconv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
 /* Scratch with which a quantised call takes the expanded-table kernels (see axc_conv2d_fast_workspace_bytes); 0: none. */
-int axc_qconv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
+int axc_qconv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc *desc, size_t *bytes);
 int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, const uint8_t *qinput, const uint8_t *qfilter,
                         int32_t input_offset, int32_t filter_offset, int32_t *output, void *workspace,
                         size_t workspace_bytes, int device, void *stream);

@@ -38,13 +38,15 @@ def test_expanded_tables_match_the_checker(built, shape, kind):
     from tf_approximate_b200 import ops
     n, h, w, c, kh, kw, co, s, d, pad = shape
     lut = tables(ax)[kind]
-    assert ops.fast_workspace_bytes((n, h, w, c), (kh, kw, c, co), [1, s, s, 1], pad, (1, d, d, 1)) > 0
+    t = ax.Table(array=lut)
+    fast = ops.fast_workspace_bytes((n, h, w, c), (kh, kw, c, co), [1, s, s, 1], pad, (1, d, d, 1), t)
+    assert (fast > 0) == (kind != "neither")
     rng = np.random.Generator(np.random.PCG64(sum(shape[:8])))
     x = rng.uniform(-1, 1, (n, h, w, c)).astype(np.float32)
     f = rng.normal(0, 0.1, (kh, kw, c, co)).astype(np.float32)
     mm = (-0.7, 1.0, float(f.min()), float(f.max()))
     ref = O.conv2d(O.desc(n, h, w, c, kh, kw, co, (s, s), (d, d), pad), lut, x, f, *mm, want=("out_exact", "acc"))
-    xd, fd, t = torch.from_numpy(x).cuda(), torch.from_numpy(f).cuda(), ax.Table(array=lut)
+    xd, fd = torch.from_numpy(x).cuda(), torch.from_numpy(f).cuda()
     call = lambda *a, **kw_: ax.approx_conv2d_with_min_max_vars(xd, fd, *a, [1, s, s, 1], 8, t, pad, dilations=(1, d, d, 1), **kw_)  # noqa: E731
     y, dbg = call(*mm, debug=True)
     assert dbg["plan"]["status"] == 0
@@ -58,11 +60,23 @@ def test_expanded_tables_match_the_checker(built, shape, kind):
     bias, res = torch.randn(co, device="cuda", generator=g), torch.randn(want.shape, device="cuda", generator=g)
     fused = call(*mm, bias=bias, residual=res, relu=True)
     assert torch.equal(fused.view(torch.int32), torch.relu(want + bias + res).view(torch.int32))
-    # the plan-based kernels, which a workspace of the smaller size selects
+    # the plan-based kernels, which a workspace of their size selects (unless it has room for the expanded tables as well)
     ws = torch.zeros(ops.workspace_bytes((n, h, w, c), (kh, kw, c, co), [1, s, s, 1], pad, (1, d, d, 1)), dtype=torch.uint8, device="cuda")
-    if ws.numel() < ops.fast_workspace_bytes((n, h, w, c), (kh, kw, c, co), [1, s, s, 1], pad, (1, d, d, 1)):
-        a, b = call(*mm, input_relu=True), call(*mm, input_relu=True, workspace=ws)
-        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    a, b = call(*mm, input_relu=True), call(*mm, input_relu=True, workspace=ws)
+    assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+def test_a_table_without_a_form_keeps_its_plan(built):
+    """A table that fits none of the forms is served by the plan-based kernels, whose plan survives from call to call."""
+    import torch
+    import tf_approximate_b200 as ax
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.rand((2, 40, 40, 32), device="cuda", generator=g)
+    f = torch.randn((3, 3, 32, 48), device="cuda", generator=g)
+    t = ax.Table(array=tables(ax)["neither"])
+    rebuilt = [ax.approx_conv2d_with_min_max_vars(x, f, 0.0, 1.0, -3.0, 3.0, [1, 1, 1, 1], 8, t, "SAME", debug=True)[1]["plan"]["rebuilt"]
+               for _ in range(3)]
+    assert rebuilt == [1, 0, 0]
 
 
 def test_unusual_values_and_addresses(built):

@@ -65,7 +65,7 @@ def load():
     L.axc_conv2d_output_dims.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_int64)]
     L.axc_depthwise_conv2d_output_dims.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_int64)]
     L.axc_conv2d_workspace_bytes.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
-    L.axc_conv2d_fast_workspace_bytes.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
+    L.axc_conv2d_fast_workspace_bytes.argtypes = [C.c_void_p, C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
     L.axc_depthwise_conv2d_workspace_bytes.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
     L.axc_conv2d_plan_info.argtypes = [C.c_void_p, C.POINTER(C.c_int32), C.c_int, C.c_void_p]
     L.axc_conv2d_forward.argtypes = fwd
@@ -76,7 +76,7 @@ def load():
     L.axc_depthwise_conv2d_forward_noalloc.argtypes = [C.c_void_p, C.POINTER(ConvDesc), C.c_void_p, C.c_void_p, C.c_float,
                                                        C.c_float, C.c_float, C.c_float, C.c_void_p, C.c_int, C.c_void_p]
     L.axc_depthwise_conv2d_status.argtypes = [C.POINTER(ConvDesc), C.c_void_p, C.POINTER(C.c_int32), C.c_int, C.c_void_p]
-    L.axc_qconv2d_fast_workspace_bytes.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
+    L.axc_qconv2d_fast_workspace_bytes.argtypes = [C.c_void_p, C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
     L.axc_qconv2d_workspace_bytes.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
     L.axc_qconv2d_forward.argtypes = [C.c_void_p, C.POINTER(ConvDesc), C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p,
                                       C.c_void_p, C.c_size_t, C.c_int, C.c_void_p]

@@ -85,6 +85,13 @@ bool table_sum_fits_int32(const axc_table *t, long long K)
     return K * (long long)t->max_entry <= 0x7FFFFFFFll;
 }
 
+// The sum is taken in K order with an fp32 running total: asked for and not provably equal to the exact sum, or too large for
+// an int32.
+static bool sums_in_reference_order(const axc_table *t, const Geom &g)
+{
+    return (g.accum == AXC_ACCUM_REFERENCE_F32 && !table_sum_exact_in_fp32(t, g.K)) || !table_sum_fits_int32(t, g.K);
+}
+
 int cuda_failed(cudaError_t e)
 {
     g_last_cuda_error = int(e);
@@ -357,7 +364,14 @@ static int forward(bool depthwise, axc_table *table, const axc_conv_desc *desc, 
     const long long out_c = depthwise ? (long long)g.C * g.Cout : g.Cout;
     if (g.M * out_c == 0) return AXC_OK;  // empty output: nothing to do
     if (!input || !filter || !output) return AXC_INVALID_ARGUMENT;
-    const size_t ws_total = depthwise ? depthwise_workspace(g.K, g.C, g.Cout).total : dense_workspace_total(g.K, g.Cout, g.M);
+    size_t ws_total = depthwise ? depthwise_workspace(g.K, g.C, g.Cout).total : dense_workspace_total(g.K, g.Cout, g.M);
+    if (!depthwise && workspace_bytes < ws_total && !sums_in_reference_order(table, g)) {
+        // the expanded-table kernels may need less than a plan
+        int mode, centred, e_min;
+        table_form(table, &mode, &centred, &e_min);
+        const size_t fast = xtab_scratch_bytes(g, mode);
+        if (fast > 0 && fast < ws_total) ws_total = fast;
+    }
     if (!workspace || workspace_bytes < ws_total) return AXC_INTERNAL;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return AXC_INVALID_ARGUMENT;
 
@@ -371,8 +385,7 @@ static int forward(bool depthwise, axc_table *table, const axc_conv_desc *desc, 
     const Quant q = make_quant(in_min, in_max, f_min, f_max);
     // The reference's fp32 running total is served by the integer kernels whenever it provably equals the exact
     // sum; a sum that could overflow an int32 accumulator is always added up the reference's way.
-    const bool ref_order = !depthwise && ((g.accum == AXC_ACCUM_REFERENCE_F32 && !table_sum_exact_in_fp32(table, g.K)) ||
-                                          !table_sum_fits_int32(table, g.K));
+    const bool ref_order = !depthwise && sums_in_reference_order(table, g);
     rc = depthwise ? launch_depthwise(lut, g, q, input, filter, output, workspace, dbg, device, cudaStream_t(stream))
                    : launch_dense(lut, table, g, q, ranges_dev, input, filter, output, workspace, workspace_bytes, dbg, device,
                                   cudaStream_t(stream), ref_order);
@@ -526,7 +539,7 @@ int axc_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes)
     return AXC_OK;
 }
 
-int axc_conv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_t *bytes)
+int axc_conv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc *desc, size_t *bytes)
 {
     if (!bytes) return AXC_INVALID_ARGUMENT;
     axc::Geom g;
@@ -534,8 +547,12 @@ int axc_conv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_t *bytes)
     if (rc) return rc;
     *bytes = 0;
     if (g.M * g.Cout == 0) return AXC_OK;
-    const size_t fast = axc::xtab_scratch_bytes(g), base = axc::dense_workspace_total(g.K, g.Cout, g.M);
-    if (fast > 0) *bytes = fast > base ? fast : base;
+    int mode = axc::kXtabAny, centred, e_min;
+    if (table) {
+        axc::table_form(table, &mode, &centred, &e_min);
+        if (axc::sums_in_reference_order(table, g)) return AXC_OK;
+    }
+    *bytes = axc::xtab_scratch_bytes(g, mode);
     return AXC_OK;
 }
 

@@ -594,10 +594,10 @@ int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g,
     int rc = device_info(device, &di);
     if (rc) return rc;
     if (!ref_order && dense_variant() == 0 && xtab_device_ok(di)) {
-        const size_t need = xtab_scratch_bytes(g);
         int mode, centred, e_min;
         table_form(table, &mode, &centred, &e_min);
-        if (need > 0 && workspace_bytes >= need && mode != kXtabNone) {
+        const size_t need = xtab_scratch_bytes(g, mode);
+        if (need > 0 && workspace_bytes >= need) {
             if (dbg && dbg->qinput) {
                 rc = launch_quant(q, ranges_dev, g.K, static_cast<unsigned char *>(workspace), stream);
                 if (rc == AXC_OK)

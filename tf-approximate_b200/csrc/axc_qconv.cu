@@ -135,7 +135,7 @@ extern "C" int axc_qconv2d_workspace_bytes(const axc_conv_desc *desc, size_t *by
     return AXC_OK;
 }
 
-extern "C" int axc_qconv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_t *bytes)
+extern "C" int axc_qconv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc *desc, size_t *bytes)
 {
     if (!bytes) return AXC_INVALID_ARGUMENT;
     axc::Geom g;
@@ -143,8 +143,9 @@ extern "C" int axc_qconv2d_fast_workspace_bytes(const axc_conv_desc *desc, size_
     if (rc) return rc;
     *bytes = 0;
     if (g.M * g.Cout == 0) return AXC_OK;
-    const size_t fast = axc::xtab_scratch_bytes(g), base = axc::qconv_layout(g).total;
-    if (fast > 0) *bytes = fast > base ? fast : base;
+    int mode = axc::kXtabAny, centred, e_min;
+    if (table) axc::table_form(table, &mode, &centred, &e_min);
+    *bytes = axc::xtab_scratch_bytes(g, mode);
     return AXC_OK;
 }
 
@@ -171,7 +172,13 @@ extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, 
     if (!same_window_as_reference(g, desc->padding)) return AXC_UNIMPLEMENTED;
     if (!table_sum_fits_int32(table, g.K)) return AXC_INVALID_ARGUMENT;
     const QLayout L = qconv_layout(g);
-    if (!workspace || workspace_bytes < L.total) return AXC_INTERNAL;
+    {
+        // the expanded-table kernels may need less than the passes of the general route
+        int mode, centred, e_min;
+        table_form(table, &mode, &centred, &e_min);
+        const size_t fast = xtab_scratch_bytes(g, mode);
+        if (!workspace || workspace_bytes < (fast > 0 && fast < L.total ? fast : L.total)) return AXC_INTERNAL;
+    }
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return AXC_INVALID_ARGUMENT;
     int status = AXC_OK;
     const uint16_t *lut = table_device_ptr(table, device, &status);
@@ -186,10 +193,10 @@ extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, 
         // enough scratch for the expanded-table kernels: they take the bytes as they are and add the zero-point terms at the end
         DeviceInfo di;
         rc = device_info(device, &di);
-        const size_t need = xtab_scratch_bytes(g);
         int mode, centred, e_min;
         table_form(table, &mode, &centred, &e_min);
-        if (rc == AXC_OK && need > 0 && workspace_bytes >= need && mode != kXtabNone && xtab_device_ok(di)) {
+        const size_t need = xtab_scratch_bytes(g, mode);
+        if (rc == AXC_OK && need > 0 && workspace_bytes >= need && xtab_device_ok(di)) {
             const QuantisedOperands u8 = {qinput, qfilter, input_offset, filter_offset};
             const axc_debug_out ints = {nullptr, nullptr, output};
             rc = launch_xtab(lut, mode, centred, e_min, g, make_quant(float(-pad_code), float(255 - pad_code), 0.0f, 255.0f), nullptr, nullptr, nullptr,

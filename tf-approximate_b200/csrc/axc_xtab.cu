@@ -1197,7 +1197,7 @@ Config choose_config(int mode, const XGeom &x, int sms, bool may_split, size_t x
     return best;
 }
 
-XLayout xlayout(const Geom &g, const XGeom &x)
+XLayout xlayout(const Geom &g, const XGeom &x, int mode)
 {
     XLayout L;
     const size_t cout16 = size_t((g.Cout + 15) / 16) * 16;
@@ -1214,9 +1214,9 @@ XLayout xlayout(const Geom &g, const XGeom &x)
     // room for the expanded tables where a call would have them made in global memory
     L.xt = off;
     L.xt_bytes = 0;
-    for (int mode : {int(kXtabByte), int(kXtabFull)}) {
-        const size_t bytes = xt_size(x, mode);
-        if (bytes <= kXtMax && bytes > L.xt_bytes && choose_config(mode, x, kModelSms, size_t(g.M) * g.Cout * 4 <= kPartialMax, bytes).pre) L.xt_bytes = bytes;
+    for (int m : {int(kXtabByte), int(kXtabFull)}) {
+        const size_t bytes = xt_size(x, m);
+        if ((mode == m || mode == kXtabAny) && bytes <= kXtMax && bytes > L.xt_bytes && choose_config(m, x, kModelSms, size_t(g.M) * g.Cout * 4 <= kPartialMax, bytes).pre) L.xt_bytes = bytes;
     }
     off += L.xt_bytes;
     L.total = off;
@@ -1274,15 +1274,16 @@ int launch_expand(const ExpandParams &E, const DeviceInfo &di, cudaStream_t stre
 
 }  // namespace
 
-size_t xtab_scratch_bytes(const Geom &g)
+size_t xtab_scratch_bytes(const Geom &g, int mode)
 {
+    if (mode == kXtabNone) return 0;
     // Few lookups: the latency of preparation plus convolution is longer than the plan-based kernels' single pass over a
     // filter that is already laid out.
     if ((double)g.M * g.K * g.Cout < kXtabMinLookups) return 0;
     XGeom x;
     PrepTile t;
     if (!xgeom(g, &x) || !prep_tile(g, g.C % 4 == 0, x.im2col != 0, &t) || !prep_tile(g, 0, x.im2col != 0, &t)) return 0;
-    return xlayout(g, x).total;
+    return xlayout(g, x, mode).total;
 }
 
 int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const Geom &g, const Quant &q, const float *ranges_dev,
@@ -1295,7 +1296,7 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     XGeom &x = A.g;
     x.TNC = mode == kXtabFull ? 8 : 16;
     x.tiles_n = (g.Cout + x.TNC - 1) / x.TNC;
-    const XLayout L = xlayout(g, x);
+    const XLayout L = xlayout(g, x, mode);
     const size_t partial_bytes = size_t(g.M) * g.Cout * 4;
     const Config cf = choose_config(mode, x, di.sm_count, partial_bytes <= kPartialMax, L.xt_bytes);
     const int vec = (g.C % 4 == 0 && (u8 ? (reinterpret_cast<uintptr_t>(u8->input) & 3u) : (reinterpret_cast<uintptr_t>(input) & 15u)) == 0) ? 1 : 0;

@@ -9,13 +9,14 @@
 namespace axc {
 
 // What an expanded entry holds (table_form): two digits to the base 255, one byte, or nothing (only the exact products).
-enum XtabMode { kXtabFull = 16, kXtabByte = 8, kXtabExact = 0, kXtabNone = -1 };
+enum XtabMode { kXtabFull = 16, kXtabByte = 8, kXtabExact = 0, kXtabNone = -1, kXtabAny = -2 };
 
 // The fixed shared-window addresses of the kernels fit this device.
 inline bool xtab_device_ok(const DeviceInfo &di) { return di.max_smem_optin >= 232448 && di.smem_base <= 2048u && di.smem_end >= 233472u; }
 
-// Scratch bytes of the expanded-table route for this shape; 0 where the plan-based kernels serve the shape.
-size_t xtab_scratch_bytes(const Geom &g);
+// Scratch bytes of the expanded-table route for this shape and a table kept as `mode` (kXtabAny: enough for every table); 0
+// where the plan-based kernels serve the call.
+size_t xtab_scratch_bytes(const Geom &g, int mode);
 
 // Operands of the quantised entry point and their zero points: the int32 result carries the terms
 // K in_off f_off - f_off sum(a) - in_off sum(b); a tap outside the image has the code input_offset modulo 256.

@@ -112,12 +112,12 @@ class FakeApproxConv2D(torch.nn.Module):
         self._ranges = None
         self._workspace = None
 
-    def _own_buffers(self, inputs, strides4, dilations4):
+    def _own_buffers(self, inputs, strides4, dilations4, table):
         dev = inputs.device
         if self._ranges is None or self._ranges.device != dev:
             self._ranges = torch.empty(4, dtype=torch.float32, device=dev)
             self._workspace = None
-        if ops.fast_workspace_bytes(inputs.shape, self.kernel.shape, strides4, self.padding, dilations4) > 0:
+        if ops.fast_workspace_bytes(inputs.shape, self.kernel.shape, strides4, self.padding, dilations4, table) > 0:
             return self._ranges, None            # the op's scratch for this shape holds nothing between calls
         need = ops.workspace_bytes(inputs.shape, self.kernel.shape, strides4, self.padding, dilations4)
         if self._workspace is None or self._workspace.numel() < need:
@@ -143,7 +143,8 @@ class FakeApproxConv2D(torch.nn.Module):
             raise ops.InvalidArgumentError("only num_bits == 8 is supported")
         strides4 = (1, self.strides[0], self.strides[1], 1)
         dilations4 = (1, self.dilation_rate[0], self.dilation_rate[1], 1)
-        ranges, workspace = self._own_buffers(inputs, strides4, dilations4)
+        table = ops._table_for(self.mul_map_file, self.num_bits)
+        ranges, workspace = self._own_buffers(inputs, strides4, dilations4, table)
         # per-batch ranges: one reduction kernel each, written where the op reads them - no host round trip
         ops.tensor_range(inputs.detach(), ranges[0:2])
         ops.tensor_range(self.kernel.detach(), ranges[2:4])
@@ -151,7 +152,7 @@ class FakeApproxConv2D(torch.nn.Module):
         q_k = _FakeQuantFn.apply(self.kernel, ranges[2:4])
         # while the weights are being trained they change every step: no lookup plan then (nothing to rebuild)
         plan = "none" if (self.training and self.kernel.requires_grad) else "keep"
-        y = _ApproxConvFn.apply(q_in, q_k, ranges, strides4, self.padding, self.mul_map_file, self.num_bits, dilations4,
+        y = _ApproxConvFn.apply(q_in, q_k, ranges, strides4, self.padding, table, self.num_bits, dilations4,
                                 plan, workspace)
         if self.bias is not None:
             y = y + self.bias

@@ -187,12 +187,12 @@ def workspace_bytes(input_shape, filter_shape, strides, padding, dilations=(1, 1
     return int(wsz.value)
 
 
-def fast_workspace_bytes(input_shape, filter_shape, strides, padding, dilations=(1, 1, 1, 1)):
-    """Bytes of scratch with which a dense call is served by the expanded-table kernels (axc_conv2d_fast_workspace_bytes);
-    0 where the plan in a buffer of `workspace_bytes` serves the shape better."""
+def fast_workspace_bytes(input_shape, filter_shape, strides, padding, dilations=(1, 1, 1, 1), table=None):
+    """Bytes of scratch with which a dense call on `table` (None: any table) is served by the expanded-table kernels
+    (axc_conv2d_fast_workspace_bytes); 0 where a buffer of `workspace_bytes` serves the call."""
     d = _desc(input_shape, filter_shape, strides, padding, "NHWC", list(dilations), [])
     wsz = C.c_size_t()
-    raise_for_status(_lib.load().axc_conv2d_fast_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
+    raise_for_status(_lib.load().axc_conv2d_fast_workspace_bytes(table.handle if table is not None else None, C.byref(d), C.byref(wsz)), "workspace size")
     return int(wsz.value)
 
 
@@ -228,7 +228,7 @@ def _forward(depthwise, input, filter, input_min, input_max, filter_min, filter_
         raise InvalidArgumentError("out has the wrong shape, dtype, layout or device")
     wsz = C.c_size_t()
     if workspace is None and not depthwise:
-        raise_for_status(L.axc_conv2d_fast_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
+        raise_for_status(L.axc_conv2d_fast_workspace_bytes(table.handle, C.byref(d), C.byref(wsz)), "workspace size")
     fast = wsz.value > 0
     if not fast:
         ws_fn = L.axc_depthwise_conv2d_workspace_bytes if depthwise else L.axc_conv2d_workspace_bytes
@@ -371,7 +371,7 @@ def ax_conv2d(input, filter, min_input, max_input, min_filter, max_filter, strid
     raise_for_status(L.axc_quantized_zero_point(float(min_input), float(max_input), C.byref(off_in)), "input offset")
     raise_for_status(L.axc_quantized_zero_point(float(min_filter), float(max_filter), C.byref(off_f)), "filter offset")
     wsz = C.c_size_t()
-    raise_for_status(L.axc_qconv2d_fast_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
+    raise_for_status(L.axc_qconv2d_fast_workspace_bytes(tab.handle, C.byref(d), C.byref(wsz)), "workspace size")
     if wsz.value > 0:
         ws = torch.empty(wsz.value, dtype=torch.uint8, device=dev)      # scratch of this call alone
     else:

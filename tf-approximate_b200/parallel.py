@@ -68,7 +68,7 @@ def forward_sharded(x_slabs, filters, table, ranges, strides, padding, gather_to
         oshape = ops.conv2d_output_shape(x.shape, f.shape, strides, padding)
         y = torch.empty(oshape, dtype=torch.float32, device=dev)
         ws = torch.zeros(max(ops.workspace_bytes(x.shape, f.shape, strides, padding),
-                             ops.fast_workspace_bytes(x.shape, f.shape, strides, padding)), dtype=torch.uint8, device=dev)
+                             ops.fast_workspace_bytes(x.shape, f.shape, strides, padding, table=tab)), dtype=torch.uint8, device=dev)
         xs, fs = x.contiguous(), f.contiguous()
         keep += [xs, fs, ws]
         outs.append(y)
