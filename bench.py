@@ -26,7 +26,7 @@ if ROOT not in sys.path:
 import numpy as np  # noqa: E402
 
 SM_COUNT = 148
-LOOKUPS_PER_CLK_PER_SM = 32   # one 32-bit shared-memory bank transaction per lane per clock
+SMEM_BYTES_PER_CLK_PER_SM = 128   # shared-memory bandwidth: what bounds the table lookups
 NCU_DRAM_OVER_ALGORITHMIC = (205.0 + 162.1) / 411.2
 
 
@@ -363,10 +363,14 @@ def run_gpu(args):
     io_bytes = sum(W.conv_io_bytes(s, h, batch) for s, h in net.convs if not s.depthwise)
     sm_mhz = clocks["sm_mhz"] or 1965.0
     achieved = dense_macs / (dense_ms * 1e-3)
-    peak = SM_COUNT * LOOKUPS_PER_CLK_PER_SM * sm_mhz * 1e6
-    # the same peak measured on this GPU: conflict-free 16-bit shared-memory loads per clock and SM (one short kernel)
+    # bytes of a looked-up entry: one where the table differs from the exact product by a byte's span, else two
+    err = runner.tables[0].numpy().astype(np.int64) - ax.exact_table().astype(np.int64)
+    entry_bytes = 1 if int(err.max() - err.min()) <= 255 else 2
+    lookups_per_clk = SMEM_BYTES_PER_CLK_PER_SM // entry_bytes
+    peak = SM_COUNT * lookups_per_clk * sm_mhz * 1e6
+    # the same peak measured on this GPU: conflict-free shared-memory wavefronts per clock and SM (one short kernel, 32 lanes each)
     measured_per_clk = ax.measure_lookup_peak(dev)
-    peak_measured = SM_COUNT * measured_per_clk * sm_mhz * 1e6
+    peak_measured = SM_COUNT * measured_per_clk / 32 * lookups_per_clk * sm_mhz * 1e6
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -379,15 +383,16 @@ def run_gpu(args):
     traffic = NCU_DRAM_OVER_ALGORITHMIC * io_bytes / dense_launches
     slowest = sorted(per_layer.items(), key=lambda kv: -kv[1])[:3]
     roofline = {
-        "kernel": "dense_sched_kernel (table convolution, %d convolution calls per step)" % dense_launches,
+        "kernel": "xtab_kernel (table convolution, %d convolution calls per step)" % dense_launches,
         "bound": "smem_lookup",
         "achieved": achieved / 1e9, "peak": peak / 1e9, "unit": "GLUT-MAC/s", "frac": achieved / peak,
-        "peak_basis": "148 SMs x 32 shared-memory lookups/clk x %.0f MHz (median SM clock sampled during this run); "
-                      "%.0f GLUT-MAC/s at the 1965 MHz maximum" % (sm_mhz, SM_COUNT * 32 * 1965e6 / 1e9),
+        "peak_basis": "148 SMs x 128 bytes of shared memory per clock / %d byte(s) per looked-up entry x %.0f MHz (median SM "
+                      "clock sampled during this run); %.0f GLUT-MAC/s at the 1965 MHz maximum"
+                      % (entry_bytes, sm_mhz, SM_COUNT * lookups_per_clk * 1965e6 / 1e9),
         "peak_measured": peak_measured / 1e9, "frac_of_measured": achieved / peak_measured,
-        "peak_measured_basis": "%.2f conflict-free 16-bit shared-memory loads per clock and SM, measured in this run "
-                               "by axc_measure_lookup_peak (512 threads per SM, 16 independent loads per thread and "
-                               "iteration), x 148 SMs x the sampled clock" % measured_per_clk,
+        "peak_measured_basis": "%.3f conflict-free shared-memory wavefronts per clock and SM, measured in this run by "
+                               "axc_measure_lookup_peak (512 threads per SM, 16 independent loads per thread and "
+                               "iteration), x %d entries x 148 SMs x the sampled clock" % (measured_per_clk / 32, lookups_per_clk),
         "units_per_launch": dense_macs / dense_launches, "ms_per_launch": dense_ms / dense_launches,
         "traffic": traffic, "traffic_unit": "bytes per launch (scaled from an ncu capture of one layer)",
         "hbm": {"algorithmic_bytes_per_step": io_bytes, "achieved_gbs": io_bytes / (dense_ms * 1e-3) / 1e9,
