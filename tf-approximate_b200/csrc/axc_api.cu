@@ -92,6 +92,17 @@ static bool sums_in_reference_order(const axc_table *t, const Geom &g)
     return (g.accum == AXC_ACCUM_REFERENCE_F32 && !table_sum_exact_in_fp32(t, g.K)) || !table_sum_fits_int32(t, g.K);
 }
 
+size_t expanded_scratch_bytes(const axc_table *table, const Geom &g)
+{
+    if (dense_variant() != 0) return 0;
+    int mode = kXtabAny, centred, e_min;
+    if (table) {
+        if (sums_in_reference_order(table, g)) return 0;
+        table_form(table, &mode, &centred, &e_min);
+    }
+    return xtab_scratch_bytes(g, mode);
+}
+
 int cuda_failed(cudaError_t e)
 {
     g_last_cuda_error = int(e);
@@ -364,15 +375,10 @@ static int forward(bool depthwise, axc_table *table, const axc_conv_desc *desc, 
     const long long out_c = depthwise ? (long long)g.C * g.Cout : g.Cout;
     if (g.M * out_c == 0) return AXC_OK;  // empty output: nothing to do
     if (!input || !filter || !output) return AXC_INVALID_ARGUMENT;
-    size_t ws_total = depthwise ? depthwise_workspace(g.K, g.C, g.Cout).total : dense_workspace_total(g.K, g.Cout, g.M);
-    if (!depthwise && workspace_bytes < ws_total && !sums_in_reference_order(table, g)) {
-        // the expanded-table kernels may need less than a plan
-        int mode, centred, e_min;
-        table_form(table, &mode, &centred, &e_min);
-        const size_t fast = xtab_scratch_bytes(g, mode);
-        if (fast > 0 && fast < ws_total) ws_total = fast;
-    }
-    if (!workspace || workspace_bytes < ws_total) return AXC_INTERNAL;
+    const size_t fast = depthwise ? 0 : expanded_scratch_bytes(table, g);
+    const bool expanded = fast > 0 && workspace_bytes >= fast;
+    const size_t ws_total = depthwise ? depthwise_workspace(g.K, g.C, g.Cout).total : dense_workspace_total(g.K, g.Cout, g.M);
+    if (!workspace || (!expanded && workspace_bytes < ws_total)) return AXC_INTERNAL;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return AXC_INVALID_ARGUMENT;
 
     int status = AXC_OK;
@@ -387,7 +393,7 @@ static int forward(bool depthwise, axc_table *table, const axc_conv_desc *desc, 
     // sum; a sum that could overflow an int32 accumulator is always added up the reference's way.
     const bool ref_order = !depthwise && sums_in_reference_order(table, g);
     rc = depthwise ? launch_depthwise(lut, g, q, input, filter, output, workspace, dbg, device, cudaStream_t(stream))
-                   : launch_dense(lut, table, g, q, ranges_dev, input, filter, output, workspace, workspace_bytes, dbg, device,
+                   : launch_dense(lut, table, g, q, ranges_dev, input, filter, output, workspace, expanded, dbg, device,
                                   cudaStream_t(stream), ref_order);
     if (prev != device) cudaSetDevice(prev);
     return rc;
@@ -547,12 +553,7 @@ int axc_conv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc 
     if (rc) return rc;
     *bytes = 0;
     if (g.M * g.Cout == 0) return AXC_OK;
-    int mode = axc::kXtabAny, centred, e_min;
-    if (table) {
-        axc::table_form(table, &mode, &centred, &e_min);
-        if (axc::sums_in_reference_order(table, g)) return AXC_OK;
-    }
-    *bytes = axc::xtab_scratch_bytes(g, mode);
+    *bytes = axc::expanded_scratch_bytes(table, g);
     return AXC_OK;
 }
 

@@ -563,11 +563,9 @@ int launch_post(float *out, const float *bias, const float *residual, long long 
     return AXC_OK;
 }
 
-// 0 = bank-scheduled kernel with the common-K kernel as its device-side fallback (default),
-// 1 = common-K kernel only.  Read once from AXC_DENSE_VARIANT.
 AXC_DEFINE_BOUNDS_READER(bounds_record_conv)
 
-static int dense_variant()
+int dense_variant()
 {
     static const int v = [] {
         const char *e = getenv("AXC_DENSE_VARIANT");
@@ -587,27 +585,28 @@ static int launch_quantize_tap(const float *input, long long n, const DevQuant *
 }
 
 int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g, const Quant &q, const float *ranges_dev,
-                 const float *input, const float *filter, float *output, void *workspace, size_t workspace_bytes,
+                 const float *input, const float *filter, float *output, void *workspace, bool expanded,
                  const axc_debug_out *dbg, int device, cudaStream_t stream, bool ref_order)
 {
     DeviceInfo di;
     int rc = device_info(device, &di);
     if (rc) return rc;
-    if (!ref_order && dense_variant() == 0 && xtab_device_ok(di)) {
+    // The kernels are laid out for the 227 KiB of sm_100 and address the table by absolute window addresses: refuse
+    // to launch where the probed window of this device does not start early enough or does not reach 228 KiB
+    // (a kernel that found its layout broken would leave the output unwritten).
+    if (!window_ok(di)) return AXC_INTERNAL;
+    if (expanded) {
         int mode, centred, e_min;
         table_form(table, &mode, &centred, &e_min);
-        const size_t need = xtab_scratch_bytes(g, mode);
-        if (need > 0 && workspace_bytes >= need) {
-            if (dbg && dbg->qinput) {
-                rc = launch_quant(q, ranges_dev, g.K, static_cast<unsigned char *>(workspace), stream);
-                if (rc == AXC_OK)
-                    rc = launch_quantize_tap(input, (long long)g.N * g.H * g.W * g.C,
-                                             reinterpret_cast<const DevQuant *>(static_cast<unsigned char *>(workspace) + kDevQuantOffset),
-                                             dbg->qinput, g.ep.input_relu, stream);
-                if (rc) return rc;
-            }
-            return launch_xtab(lut_dev, mode, centred, e_min, g, q, ranges_dev, input, filter, output, static_cast<unsigned char *>(workspace), dbg, di, stream);
+        if (dbg && dbg->qinput) {
+            rc = launch_quant(q, ranges_dev, g.K, static_cast<unsigned char *>(workspace), stream);
+            if (rc == AXC_OK)
+                rc = launch_quantize_tap(input, (long long)g.N * g.H * g.W * g.C,
+                                         reinterpret_cast<const DevQuant *>(static_cast<unsigned char *>(workspace) + kDevQuantOffset),
+                                         dbg->qinput, g.ep.input_relu, stream);
+            if (rc) return rc;
         }
+        return launch_xtab(lut_dev, mode, centred, e_min, g, q, ranges_dev, input, filter, output, static_cast<unsigned char *>(workspace), dbg, di, stream);
     }
     // A caller that wants the integer sums only (output == NULL, the quantised entry point) gets the fp32 value written
     // to the same element of the accumulator tap first and the integer sum over it: the kernels need no test per store.
@@ -616,10 +615,6 @@ int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g,
         if (!dbg || !dbg->acc) return AXC_INVALID_ARGUMENT;
         output = reinterpret_cast<float *>(dbg->acc);
     }
-    // The kernels are laid out for the 227 KiB of sm_100 and address the table by absolute window addresses: refuse
-    // to launch where the probed window of this device does not start early enough or does not reach 228 KiB
-    // (a kernel that found its layout broken would leave the output unwritten).
-    if (di.max_smem_optin < 232448 || di.smem_base > 2048u || di.smem_end < 233472u) return AXC_INTERNAL;
     // the scheduled kernel divides by C and KW with 40-bit reciprocals, exact while K * max(C, KW) < 2^40; it
     // lets every lane walk K in an order of its own, so a sum that has to be taken in K order is not its job
     const bool scheduled = !ref_order && g.plan == AXC_PLAN_KEEP && dense_variant() == 0 && (long long)g.K * (g.C > g.KW ? g.C : g.KW) < (1ll << 40);

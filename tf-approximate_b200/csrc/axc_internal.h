@@ -151,6 +151,10 @@ bool table_sum_exact_in_fp32(const axc_table *t, long long K);
 void table_form(const axc_table *t, int *mode, int *centred, int *e_min);
 // True when K entries cannot overflow an int32 accumulator.
 bool table_sum_fits_int32(const axc_table *t, long long K);
+// Scratch of a dense or quantised call on the expanded-table kernels; 0 where other kernels serve the table (NULL: any
+// table), the shape, the order of additions or the process (dense_variant).  The size queries and the entry points all ask
+// here, so that a buffer is never accepted for one route and used by another.
+size_t expanded_scratch_bytes(const axc_table *table, const Geom &g);
 
 struct DeviceInfo {
     int sm_count;
@@ -180,10 +184,13 @@ Workspace depthwise_workspace(int KHW, int C, int mult);
 // ranges_dev: NULL, or {in_min, in_max, f_min, f_max} in device memory (then `q` is ignored).
 // ref_order: add the products up in K order with an fp32 running total (the reference's arithmetic) instead of
 // the exact integer sum.
-// workspace_bytes: what the caller brought; from xtab_scratch_bytes() on the expanded-table kernels serve the call.
+// expanded: the call takes the expanded-table kernels and `workspace` has expanded_scratch_bytes(); else it has
+// dense_workspace_total().  The caller has checked that.
 int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g, const Quant &q, const float *ranges_dev,
-                 const float *input, const float *filter, float *output, void *workspace, size_t workspace_bytes,
+                 const float *input, const float *filter, float *output, void *workspace, bool expanded,
                  const axc_debug_out *dbg, int device, cudaStream_t stream, bool ref_order);
+// 0 = all kernels (default), 1 = the common-K kernel for every dense call.  Read once from AXC_DENSE_VARIANT.
+int dense_variant();
 // out = out (+ bias[channel]) (+ residual), then max(out, 0) if relu, in one pass; bias / residual may be NULL
 int launch_post(float *out, const float *bias, const float *residual, long long count, int channels, int relu,
                 const DeviceInfo &di, cudaStream_t stream);

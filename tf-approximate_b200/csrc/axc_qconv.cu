@@ -141,11 +141,10 @@ extern "C" int axc_qconv2d_fast_workspace_bytes(const axc_table *table, const ax
     axc::Geom g;
     int rc = axc::resolve_geometry(desc, false, &g);
     if (rc) return rc;
+    g.accum = AXC_ACCUM_EXACT_I32;
     *bytes = 0;
     if (g.M * g.Cout == 0) return AXC_OK;
-    int mode = axc::kXtabAny, centred, e_min;
-    if (table) axc::table_form(table, &mode, &centred, &e_min);
-    *bytes = axc::xtab_scratch_bytes(g, mode);
+    *bytes = axc::expanded_scratch_bytes(table, g);
     return AXC_OK;
 }
 
@@ -158,6 +157,7 @@ extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, 
     Geom g;
     int rc = resolve_geometry(desc, false, &g);
     if (rc) return rc;
+    g.accum = AXC_ACCUM_EXACT_I32;
     if (g.M * g.Cout == 0) return AXC_OK;
     if (!qinput || !qfilter || !output) return AXC_INVALID_ARGUMENT;
     {
@@ -172,13 +172,9 @@ extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, 
     if (!same_window_as_reference(g, desc->padding)) return AXC_UNIMPLEMENTED;
     if (!table_sum_fits_int32(table, g.K)) return AXC_INVALID_ARGUMENT;
     const QLayout L = qconv_layout(g);
-    {
-        // the expanded-table kernels may need less than the passes of the general route
-        int mode, centred, e_min;
-        table_form(table, &mode, &centred, &e_min);
-        const size_t fast = xtab_scratch_bytes(g, mode);
-        if (!workspace || workspace_bytes < (fast > 0 && fast < L.total ? fast : L.total)) return AXC_INTERNAL;
-    }
+    const size_t fast = expanded_scratch_bytes(table, g);
+    const bool expanded = fast > 0 && workspace_bytes >= fast;
+    if (!workspace || (!expanded && workspace_bytes < L.total)) return AXC_INTERNAL;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return AXC_INVALID_ARGUMENT;
     int status = AXC_OK;
     const uint16_t *lut = table_device_ptr(table, device, &status);
@@ -189,25 +185,21 @@ extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, 
     if (prev != device) AXC_CUDA(cudaSetDevice(device));
     cudaStream_t s = cudaStream_t(stream);
     unsigned char *ws = static_cast<unsigned char *>(workspace);
-    {
-        // enough scratch for the expanded-table kernels: they take the bytes as they are and add the zero-point terms at the end
-        DeviceInfo di;
-        rc = device_info(device, &di);
+    DeviceInfo di;
+    rc = device_info(device, &di);
+    if (rc == AXC_OK && !window_ok(di)) rc = AXC_INTERNAL;
+    if (rc == AXC_OK && expanded) {
+        // the expanded-table kernels take the bytes as they are and add the zero-point terms at the end
         int mode, centred, e_min;
         table_form(table, &mode, &centred, &e_min);
-        const size_t need = xtab_scratch_bytes(g, mode);
-        if (rc == AXC_OK && need > 0 && workspace_bytes >= need && xtab_device_ok(di)) {
-            const QuantisedOperands u8 = {qinput, qfilter, input_offset, filter_offset};
-            const axc_debug_out ints = {nullptr, nullptr, output};
-            rc = launch_xtab(lut, mode, centred, e_min, g, make_quant(float(-pad_code), float(255 - pad_code), 0.0f, 255.0f), nullptr, nullptr, nullptr,
-                             nullptr, ws, &ints, di, s, &u8);
-            if (prev != device) cudaSetDevice(prev);
-            return rc;
-        }
-        if (rc) {
-            if (prev != device) cudaSetDevice(prev);
-            return rc;
-        }
+        const QuantisedOperands u8 = {qinput, qfilter, input_offset, filter_offset};
+        const axc_debug_out ints = {nullptr, nullptr, output};
+        rc = launch_xtab(lut, mode, centred, e_min, g, make_quant(float(-pad_code), float(255 - pad_code), 0.0f, 255.0f), nullptr, nullptr, nullptr,
+                         nullptr, ws, &ints, di, s, &u8);
+    }
+    if (rc != AXC_OK || expanded) {
+        if (prev != device) cudaSetDevice(prev);
+        return rc;
     }
     float *xin = reinterpret_cast<float *>(ws + L.xin_off);
     float *xf = reinterpret_cast<float *>(ws + L.xf_off);
@@ -222,10 +214,7 @@ extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, 
         // scale 1, zero point = pad_code: the op's quantiser returns the caller's bytes, and pad_code for a padded tap
         const Quant q = make_quant(float(-pad_code), float(255 - pad_code), 0.0f, 255.0f);
         axc_debug_out taps = {nullptr, nullptr, output};
-        Geom ge = g;
-        ge.accum = AXC_ACCUM_EXACT_I32;
-        ge.plan = g.plan;
-        rc = launch_dense(lut, table, ge, q, nullptr, xin, xf, nullptr, ws, L.dense_bytes, &taps, device, s, false);
+        rc = launch_dense(lut, table, g, q, nullptr, xin, xf, nullptr, ws, false, &taps, device, s, false);
     }
     if (e == cudaSuccess && rc == AXC_OK && (input_offset != 0 || filter_offset != 0)) {
         qfilter_sum_kernel<<<unsigned((g.Cout + 127) / 128), 128, 0, s>>>(qfilter, g.K, g.Cout, bsum);
