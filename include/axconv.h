@@ -53,9 +53,10 @@ enum { AXC_FORMAT_NHWC = 0, AXC_FORMAT_NCHW = 1 };
 enum { AXC_ACCUM_EXACT_I32 = 0, AXC_ACCUM_REFERENCE_F32 = 1 };
 /* Whether the dense op prepares a per-filter lookup plan (kept in the workspace, built in 3-90 ms, reused while the
  * filter is unchanged) or serves the call without one.
- * AXC_PLAN_KEEP (default): inference - the plan makes every table lookup conflict-free (about 1.8 x the speed).
- * AXC_PLAN_NONE: filters that change from call to call (training steps): the kernel that walks K in order serves
- *   the call, nothing is prepared and nothing has to be rebuilt.  Same results bit for bit. */
+ * AXC_PLAN_KEEP (default): the buffer may hold a plan from one call to the next.
+ * AXC_PLAN_NONE: nothing in the buffer is kept: the expanded-table kernels serve the call where the buffer suffices for them
+ *   (axc_conv2d_fast_workspace_bytes), else the kernel that walks K in order; nothing is prepared and nothing has to be rebuilt
+ *   (filters that change from call to call, scratch that is borrowed for one call).  Same results bit for bit. */
 enum { AXC_PLAN_KEEP = 0, AXC_PLAN_NONE = 1 };
 
 /* Geometry of one call: what ApproxConv2DParameters + ApproxConv2DDimensions carry
@@ -121,15 +122,28 @@ int axc_depthwise_conv2d_output_dims(const axc_conv_desc *desc, int64_t out4[4])
  * For the dense op it holds the filter's lookup plan (quantised filter copy, table image, per-lane lookup
  * schedule, filter sums) and the fallback kernel's filter program.  The plan is rebuilt only when the buffer does not
  * already hold the plan of this very filter (values, ranges, table): keep one buffer per layer between
- * calls, leave it untouched, and the preparation is paid once; a fresh or recycled buffer is always safe
- * (its first 256 bytes decide), only slower.  One buffer serves one stream at a time. */
+ * calls, leave it untouched, and the preparation is paid once - whatever the batch sizes of the calls; a fresh or
+ * recycled buffer is always safe (its first 256 bytes decide), only slower.  One buffer serves one stream at a time. */
 int axc_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
 int axc_depthwise_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
-/* Scratch with which a dense call on `table` takes the expanded-table kernels; 0 where other kernels serve the shape, the table
+/* Buffer with which a dense call on `table` takes the expanded-table kernels; 0 where other kernels serve the shape, the table
  * or the mode of accumulation.  table == NULL: enough for every table (a call that then does not take them falls back to the
- * plan-based kernels if the buffer has axc_conv2d_workspace_bytes).  Same results, no plan to build; nothing in the buffer
- * outlives the call, so one buffer may serve all layers of a stream in turn. */
+ * plan-based kernels if the buffer has axc_conv2d_workspace_bytes).  Same results, no plan to build; nothing that these kernels
+ * write outlives the call, so one buffer may serve all layers of a stream in turn.
+ * With desc->plan == AXC_PLAN_NONE that is their scratch alone, and they use the buffer from its start.  With AXC_PLAN_KEEP a
+ * buffer of axc_conv2d_workspace_bytes or more belongs to the plan: they leave its first axc_conv2d_workspace_bytes alone,
+ * and the size reported here includes those where their scratch is not smaller than them anyway. */
 int axc_conv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc *desc, size_t *bytes);
+/* Which kernels serve a dense call with a buffer of `workspace_bytes` (what the call itself decides by):
+ * out4 = {AXC_ROUTE_*, and for AXC_ROUTE_EXPANDED the output pixels per tile, the splits of K, and 1 where the tables come from
+ * global memory, on a GPU of 148 SMs}.  Diagnostics only; no counterpart in the reference. */
+enum {
+    AXC_ROUTE_NONE = 0,      /* nothing to do, or a buffer that the call refuses (AXC_INTERNAL) */
+    AXC_ROUTE_PLAN = 1,      /* lookups scheduled by the plan in the buffer */
+    AXC_ROUTE_COMMON_K = 2,  /* all lanes at the same K index, no plan */
+    AXC_ROUTE_EXPANDED = 3   /* expanded tables */
+};
+int axc_conv2d_route(const axc_table *table, const axc_conv_desc *desc, size_t workspace_bytes, int32_t out4[4]);
 /* Reads back {rebuilt in the last call, fallback kernel in use, kernel status (0 = fine), schedule steps per
  * ideal step in per-mille} of the plan in a dense workspace.  Blocks until `stream` is idle.  Diagnostics only;
  * no counterpart in the reference. */
@@ -276,8 +290,10 @@ int axc_depthwise_conv2d_forward_noalloc(axc_table *table, const axc_conv_desc *
  * than the window by two or more, :153-163) return AXC_UNIMPLEMENTED.  The table sums are computed by the kernels
  * of axc_conv2d_forward; the workspace additionally holds an fp32 image of both operands. */
 int axc_qconv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes);
-/* Scratch with which a quantised call takes the expanded-table kernels (see axc_conv2d_fast_workspace_bytes); 0: none. */
+/* Buffer with which a quantised call takes the expanded-table kernels (as axc_conv2d_fast_workspace_bytes, with
+ * axc_qconv2d_workspace_bytes in the place of axc_conv2d_workspace_bytes); 0: none.  axc_qconv2d_route: see axc_conv2d_route. */
 int axc_qconv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc *desc, size_t *bytes);
+int axc_qconv2d_route(const axc_table *table, const axc_conv_desc *desc, size_t workspace_bytes, int32_t out4[4]);
 int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, const uint8_t *qinput, const uint8_t *qfilter,
                         int32_t input_offset, int32_t filter_offset, int32_t *output, void *workspace,
                         size_t workspace_bytes, int device, void *stream);

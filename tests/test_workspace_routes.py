@@ -99,3 +99,102 @@ print("served")
 @pytest.mark.gpu
 def test_switch_to_the_common_k_kernel_serves_the_calls(built):
     assert "served" in child(COMMON_K, AXC_DENSE_VARIANT="1")
+
+
+def routes(fn, table, shape, nbytes, plan):
+    import ctypes as C
+    from tf_approximate_b200 import _lib
+    n, h, w, c, k, cout = shape
+    out = (C.c_int32 * 4)()
+    d = _lib.ConvDesc(n, h, w, c, k, k, c, cout, 1, 1, 1, 1, 0, 0, 0, plan)
+    assert getattr(_lib.load(), fn)(table.handle, C.byref(d), nbytes, out) == 0
+    return out[0]
+
+
+def sizes(fn, table, shape, plan):
+    import ctypes as C
+    from tf_approximate_b200 import _lib
+    n, h, w, c, k, cout = shape
+    b = C.c_size_t()
+    d = _lib.ConvDesc(n, h, w, c, k, k, c, cout, 1, 1, 1, 1, 0, 0, 0, plan)
+    args = (C.byref(d), C.byref(b)) if table is None else (table.handle, C.byref(d), C.byref(b))
+    assert getattr(_lib.load(), fn)(*args) == 0
+    return b.value
+
+
+@pytest.mark.parametrize("op", ["axc_conv2d", "axc_qconv2d"])
+@pytest.mark.parametrize("layer", [(7, 7, 512, 3, 512), (28, 28, 64, 3, 64), (14, 14, 256, 1, 1024)])
+def test_a_buffer_that_can_hold_a_plan_is_the_plans(built, op, layer):
+    """A kept buffer of the documented size goes to the plan whatever the batch; the sizes that the queries name for the
+    expanded tables lead there, one byte less does not; and with no plan to keep their scratch alone is enough."""
+    import tf_approximate_b200 as ax
+    NONE, PLAN, COMMON_K, EXPANDED = range(4)
+    t = ax.Table(array=ax.noisy_table(3))
+    below = above = 0
+    for n in (1, 2, 8, 64, 128, 256):
+        s = (n,) + layer
+        general, keep, none = sizes(op + "_workspace_bytes", None, s, 0), sizes(op + "_fast_workspace_bytes", t, s, 0), sizes(op + "_fast_workspace_bytes", t, s, 1)
+        assert routes(op + "_route", t, s, general, 0) == PLAN and none > 0
+        below += none < general
+        above += none >= general
+        assert keep == (none if none < general else general + none)
+        assert routes(op + "_route", t, s, keep, 0) == EXPANDED and routes(op + "_route", t, s, none, 1) == EXPANDED
+        assert routes(op + "_route", t, s, keep - 1, 0) == (NONE if keep < general else PLAN)
+        assert routes(op + "_route", t, s, none - 1, 1) == (NONE if none - 1 < general else COMMON_K)
+    assert above or op == "axc_qconv2d"
+    assert below or layer != (7, 7, 512, 3, 512)
+
+
+@pytest.mark.gpu
+def test_a_kept_plan_survives_every_batch_size(built):
+    """One buffer per layer, called with full and ragged batches and with device ranges: the plan is built once.  A buffer with
+    room for the expanded tables behind the plan takes them and leaves the plan alone."""
+    import ctypes as C
+    import torch
+    import tf_approximate_b200 as ax
+    from tf_approximate_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(6)
+    t = ax.Table(array=ax.noisy_table(4))
+    f = torch.randn((3, 3, 128, 128), device="cuda", generator=g) * 0.05
+    one = [1, 1, 1, 1]
+    plan_bytes = ops.workspace_bytes((1, 7, 7, 128), f.shape, one, "SAME")
+    both = ops.fast_workspace_bytes((128, 7, 7, 128), f.shape, one, "SAME", table=t, plan="keep")
+    assert both > plan_bytes
+    for size, last in ((plan_bytes, "plan"), (both, "expanded")):
+        ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
+        rebuilt = []
+        for n in (8, 64, 128, 8):
+            x = torch.rand((n, 7, 7, 128), device="cuda", generator=g) * 2 - 1
+            y, dbg = ax.approx_conv2d_with_min_max_vars(x, f, -1.0, 1.0, -0.2, 0.2, one, 8, t, "SAME", workspace=ws, debug=True)
+            if n == 128:
+                assert dbg["route"]["kernels"] == last
+            if dbg["route"]["kernels"] == "plan":
+                rebuilt.append(dbg["plan"]["rebuilt"])
+            want = ax.approx_conv2d_with_min_max_vars(x, f, -1.0, 1.0, -0.2, 0.2, one, 8, t, "SAME")
+            assert torch.equal(y.view(torch.int32), want.view(torch.int32))
+        assert rebuilt[:1] in ([1], []) and not any(rebuilt[1:])
+        if size == plan_bytes:
+            assert rebuilt == [1, 0, 0, 0]
+    # the quantised entry point keeps the plan in the same place
+    L = _lib.load()
+    ws, word = None, (C.c_int32 * 4)()
+    b = torch.randint(0, 256, (3, 3, 128, 128), device="cuda", generator=g, dtype=torch.uint8)
+    zero = [C.c_int32(), C.c_int32()]
+    assert L.axc_quantized_zero_point(-1.0, 2.0, C.byref(zero[0])) == 0 and L.axc_quantized_zero_point(-0.5, 0.5, C.byref(zero[1])) == 0
+    rebuilt = []
+    for n in (128, 8, 128):
+        a = torch.randint(0, 256, (n, 7, 7, 128), device="cuda", generator=g, dtype=torch.uint8)
+        d = _lib.ConvDesc(n, 7, 7, 128, 3, 3, 128, 128, 1, 1, 1, 1, 0, 0, 0, 0)
+        if ws is None:
+            need = C.c_size_t()
+            assert L.axc_qconv2d_workspace_bytes(C.byref(d), C.byref(need)) == 0
+            ws = torch.zeros(need.value, dtype=torch.uint8, device="cuda")
+        y = torch.empty((n, 7, 7, 128), dtype=torch.int32, device="cuda")
+        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert L.axc_qconv2d_forward(t.handle, C.byref(d), a.data_ptr(), b.data_ptr(), zero[0].value, zero[1].value, y.data_ptr(), ws.data_ptr(),
+                                     sizes("axc_qconv2d_workspace_bytes", None, (n, 7, 7, 128, 3, 128), 0), 0, stream) == 0
+        assert L.axc_conv2d_plan_info(ws.data_ptr(), word, 0, stream) == 0
+        rebuilt.append(word[0])
+        want, _, _ = ax.ax_conv2d(a, b, -1.0, 2.0, -0.5, 0.5, one, "SAME", table=t, ax_tune=False)
+        assert torch.equal(y, want)
+    assert rebuilt == [1, 0, 0]

@@ -10,12 +10,12 @@ SYMBOLS = [
     "axc_table_create_from_file", "axc_table_create_from_memory", "axc_table_create_exact",
     "axc_table_destroy", "axc_table_tune_weights", "axc_table_host_data", "axc_table_ensure_device",
     "axc_conv2d_output_dims", "axc_depthwise_conv2d_output_dims",
-    "axc_conv2d_workspace_bytes", "axc_conv2d_fast_workspace_bytes", "axc_depthwise_conv2d_workspace_bytes", "axc_conv2d_plan_info",
+    "axc_conv2d_workspace_bytes", "axc_conv2d_fast_workspace_bytes", "axc_conv2d_route", "axc_depthwise_conv2d_workspace_bytes", "axc_conv2d_plan_info",
     "axc_conv2d_forward", "axc_conv2d_forward_device_ranges", "axc_depthwise_conv2d_forward",
     "axc_depthwise_conv2d_forward_noalloc", "axc_depthwise_conv2d_status",
     "axc_quant_props", "axc_status_string", "axc_last_cuda_error", "axc_launch_count", "axc_measure_lookup_peak", "axc_debug_bounds_record",
     "axc_add_residual", "axc_max_pool_same", "axc_conv2d_forward_fused", "axc_depthwise_conv2d_forward_fused", "axc_tensor_range", "axc_fake_quant", "axc_conv2d_forward_sharded", "axc_gather_outputs",
-    "axc_qconv2d_workspace_bytes", "axc_qconv2d_fast_workspace_bytes", "axc_qconv2d_forward", "axc_quantized_zero_point", "axc_quantized_output_range",
+    "axc_qconv2d_workspace_bytes", "axc_qconv2d_fast_workspace_bytes", "axc_qconv2d_route", "axc_qconv2d_forward", "axc_quantized_zero_point", "axc_quantized_output_range",
 ]
 
 
@@ -66,6 +66,8 @@ def load():
     L.axc_depthwise_conv2d_output_dims.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_int64)]
     L.axc_conv2d_workspace_bytes.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
     L.axc_conv2d_fast_workspace_bytes.argtypes = [C.c_void_p, C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
+    L.axc_conv2d_route.argtypes = [C.c_void_p, C.POINTER(ConvDesc), C.c_size_t, C.POINTER(C.c_int32)]
+    L.axc_qconv2d_route.argtypes = L.axc_conv2d_route.argtypes
     L.axc_depthwise_conv2d_workspace_bytes.argtypes = [C.POINTER(ConvDesc), C.POINTER(C.c_size_t)]
     L.axc_conv2d_plan_info.argtypes = [C.c_void_p, C.POINTER(C.c_int32), C.c_int, C.c_void_p]
     L.axc_conv2d_forward.argtypes = fwd

@@ -103,6 +103,40 @@ size_t expanded_scratch_bytes(const axc_table *table, const Geom &g)
     return xtab_scratch_bytes(g, mode);
 }
 
+Route choose_route(const axc_table *table, const Geom &g, size_t bytes, size_t general)
+{
+    const size_t fast = expanded_scratch_bytes(table, g);
+    if (fast > 0) {
+        if (g.plan == AXC_PLAN_NONE || bytes < general) {
+            if (bytes >= fast) return {true, true, 0};
+        } else if (bytes - general >= fast) return {true, true, general};
+    }
+    return {bytes >= general, false, 0};
+}
+
+size_t fast_buffer_bytes(const axc_table *table, const Geom &g, size_t general)
+{
+    const size_t fast = expanded_scratch_bytes(table, g);
+    return fast == 0 || fast < general || g.plan == AXC_PLAN_NONE ? fast : general + fast;
+}
+
+int describe_route(const axc_table *table, const Geom &g, size_t bytes, size_t general, int32_t out4[4])
+{
+    out4[0] = AXC_ROUTE_NONE;
+    out4[1] = out4[2] = out4[3] = 0;
+    const Route r = choose_route(table, g, bytes, general);
+    if (g.M * g.Cout == 0 || !r.enough) return AXC_OK;
+    if (!r.expanded) {
+        out4[0] = plan_serves(g, sums_in_reference_order(table, g)) ? AXC_ROUTE_PLAN : AXC_ROUTE_COMMON_K;
+        return AXC_OK;
+    }
+    int mode, centred, e_min;
+    table_form(table, &mode, &centred, &e_min);
+    out4[0] = AXC_ROUTE_EXPANDED;
+    xtab_config(g, mode, out4 + 1);
+    return AXC_OK;
+}
+
 int cuda_failed(cudaError_t e)
 {
     g_last_cuda_error = int(e);
@@ -375,10 +409,9 @@ static int forward(bool depthwise, axc_table *table, const axc_conv_desc *desc, 
     const long long out_c = depthwise ? (long long)g.C * g.Cout : g.Cout;
     if (g.M * out_c == 0) return AXC_OK;  // empty output: nothing to do
     if (!input || !filter || !output) return AXC_INVALID_ARGUMENT;
-    const size_t fast = depthwise ? 0 : expanded_scratch_bytes(table, g);
-    const bool expanded = fast > 0 && workspace_bytes >= fast;
-    const size_t ws_total = depthwise ? depthwise_workspace(g.K, g.C, g.Cout).total : dense_workspace_total(g.K, g.Cout, g.M);
-    if (!workspace || (!expanded && workspace_bytes < ws_total)) return AXC_INTERNAL;
+    const Route route = depthwise ? Route{workspace_bytes >= depthwise_workspace(g.K, g.C, g.Cout).total, false, 0}
+                                  : choose_route(table, g, workspace_bytes, dense_workspace_total(g.K, g.Cout, g.M));
+    if (!workspace || !route.enough) return AXC_INTERNAL;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return AXC_INVALID_ARGUMENT;
 
     int status = AXC_OK;
@@ -392,8 +425,9 @@ static int forward(bool depthwise, axc_table *table, const axc_conv_desc *desc, 
     // The reference's fp32 running total is served by the integer kernels whenever it provably equals the exact
     // sum; a sum that could overflow an int32 accumulator is always added up the reference's way.
     const bool ref_order = !depthwise && sums_in_reference_order(table, g);
+    workspace = static_cast<unsigned char *>(workspace) + route.scratch;
     rc = depthwise ? launch_depthwise(lut, g, q, input, filter, output, workspace, dbg, device, cudaStream_t(stream))
-                   : launch_dense(lut, table, g, q, ranges_dev, input, filter, output, workspace, expanded, dbg, device,
+                   : launch_dense(lut, table, g, q, ranges_dev, input, filter, output, workspace, route.expanded, dbg, device,
                                   cudaStream_t(stream), ref_order);
     if (prev != device) cudaSetDevice(prev);
     return rc;
@@ -553,8 +587,17 @@ int axc_conv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc 
     if (rc) return rc;
     *bytes = 0;
     if (g.M * g.Cout == 0) return AXC_OK;
-    *bytes = axc::expanded_scratch_bytes(table, g);
+    *bytes = axc::fast_buffer_bytes(table, g, axc::dense_workspace_total(g.K, g.Cout, g.M));
     return AXC_OK;
+}
+
+int axc_conv2d_route(const axc_table *table, const axc_conv_desc *desc, size_t workspace_bytes, int32_t out4[4])
+{
+    if (!table || !out4) return AXC_INVALID_ARGUMENT;
+    axc::Geom g;
+    int rc = axc::resolve_geometry(desc, false, &g);
+    if (rc) return rc;
+    return axc::describe_route(table, g, workspace_bytes, axc::dense_workspace_total(g.K, g.Cout, g.M), out4);
 }
 
 int axc_depthwise_conv2d_workspace_bytes(const axc_conv_desc *desc, size_t *bytes)

@@ -574,6 +574,13 @@ int dense_variant()
     return v;
 }
 
+bool plan_serves(const Geom &g, bool ref_order)
+{
+    // the scheduled kernel divides by C and KW with 40-bit reciprocals, exact while K * max(C, KW) < 2^40; it
+    // lets every lane walk K in an order of its own, so a sum that has to be taken in K order is not its job
+    return !ref_order && g.plan == AXC_PLAN_KEEP && dense_variant() == 0 && (long long)g.K * (g.C > g.KW ? g.C : g.KW) < (1ll << 40);
+}
+
 static int launch_quantize_tap(const float *input, long long n, const DevQuant *dq, uint8_t *qinput, int input_relu, cudaStream_t stream)
 {
     if (n <= 0) return AXC_OK;
@@ -615,9 +622,7 @@ int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g,
         if (!dbg || !dbg->acc) return AXC_INVALID_ARGUMENT;
         output = reinterpret_cast<float *>(dbg->acc);
     }
-    // the scheduled kernel divides by C and KW with 40-bit reciprocals, exact while K * max(C, KW) < 2^40; it
-    // lets every lane walk K in an order of its own, so a sum that has to be taken in K order is not its job
-    const bool scheduled = !ref_order && g.plan == AXC_PLAN_KEEP && dense_variant() == 0 && (long long)g.K * (g.C > g.KW ? g.C : g.KW) < (1ll << 40);
+    const bool scheduled = plan_serves(g, ref_order);
     const PlanLayout L = plan_layout(g.K, g.Cout);
     const Workspace ws = dense_workspace(g.K, g.Cout);
     unsigned char *plan = static_cast<unsigned char *>(workspace);

@@ -155,6 +155,19 @@ bool table_sum_fits_int32(const axc_table *t, long long K);
 // table), the shape, the order of additions or the process (dense_variant).  The size queries and the entry points all ask
 // here, so that a buffer is never accepted for one route and used by another.
 size_t expanded_scratch_bytes(const axc_table *table, const Geom &g);
+// How a call with a buffer of `bytes` is served; `general` = what the other kernels need.  A buffer that can hold a plan
+// is the plan's (AXC_PLAN_KEEP: building one takes 3-90 ms, so it must survive calls of every batch size): the expanded
+// tables then use only what lies behind it.
+struct Route {
+    bool enough;            // false: the buffer is too small for any route, nothing is launched
+    bool expanded;
+    size_t scratch;         // where the expanded-table kernels' scratch starts
+};
+Route choose_route(const axc_table *table, const Geom &g, size_t bytes, size_t general);
+// Smallest buffer with which choose_route takes the expanded tables, 0 where none does.
+size_t fast_buffer_bytes(const axc_table *table, const Geom &g, size_t general);
+// Body of axc_conv2d_route / axc_qconv2d_route.
+int describe_route(const axc_table *table, const Geom &g, size_t bytes, size_t general, int32_t out4[4]);
 
 struct DeviceInfo {
     int sm_count;
@@ -184,13 +197,15 @@ Workspace depthwise_workspace(int KHW, int C, int mult);
 // ranges_dev: NULL, or {in_min, in_max, f_min, f_max} in device memory (then `q` is ignored).
 // ref_order: add the products up in K order with an fp32 running total (the reference's arithmetic) instead of
 // the exact integer sum.
-// expanded: the call takes the expanded-table kernels and `workspace` has expanded_scratch_bytes(); else it has
-// dense_workspace_total().  The caller has checked that.
+// expanded: the call takes the expanded-table kernels and `workspace` is their scratch; else it has dense_workspace_total().
+// The caller has checked that.
 int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g, const Quant &q, const float *ranges_dev,
                  const float *input, const float *filter, float *output, void *workspace, bool expanded,
                  const axc_debug_out *dbg, int device, cudaStream_t stream, bool ref_order);
 // 0 = all kernels (default), 1 = the common-K kernel for every dense call.  Read once from AXC_DENSE_VARIANT.
 int dense_variant();
+// The lookups follow a plan (device-side fallback: the common-K kernel); else the common-K kernel serves the call outright.
+bool plan_serves(const Geom &g, bool ref_order);
 // out = out (+ bias[channel]) (+ residual), then max(out, 0) if relu, in one pass; bias / residual may be NULL
 int launch_post(float *out, const float *bias, const float *residual, long long count, int channels, int relu,
                 const DeviceInfo &di, cudaStream_t stream);

@@ -144,8 +144,18 @@ extern "C" int axc_qconv2d_fast_workspace_bytes(const axc_table *table, const ax
     g.accum = AXC_ACCUM_EXACT_I32;
     *bytes = 0;
     if (g.M * g.Cout == 0) return AXC_OK;
-    *bytes = axc::expanded_scratch_bytes(table, g);
+    *bytes = axc::fast_buffer_bytes(table, g, axc::qconv_layout(g).total);
     return AXC_OK;
+}
+
+extern "C" int axc_qconv2d_route(const axc_table *table, const axc_conv_desc *desc, size_t workspace_bytes, int32_t out4[4])
+{
+    if (!table || !out4) return AXC_INVALID_ARGUMENT;
+    axc::Geom g;
+    int rc = axc::resolve_geometry(desc, false, &g);
+    if (rc) return rc;
+    g.accum = AXC_ACCUM_EXACT_I32;
+    return axc::describe_route(table, g, workspace_bytes, axc::qconv_layout(g).total, out4);
 }
 
 extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, const uint8_t *qinput, const uint8_t *qfilter,
@@ -172,9 +182,8 @@ extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, 
     if (!same_window_as_reference(g, desc->padding)) return AXC_UNIMPLEMENTED;
     if (!table_sum_fits_int32(table, g.K)) return AXC_INVALID_ARGUMENT;
     const QLayout L = qconv_layout(g);
-    const size_t fast = expanded_scratch_bytes(table, g);
-    const bool expanded = fast > 0 && workspace_bytes >= fast;
-    if (!workspace || (!expanded && workspace_bytes < L.total)) return AXC_INTERNAL;
+    const Route route = choose_route(table, g, workspace_bytes, L.total);
+    if (!workspace || !route.enough) return AXC_INTERNAL;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return AXC_INVALID_ARGUMENT;
     int status = AXC_OK;
     const uint16_t *lut = table_device_ptr(table, device, &status);
@@ -188,16 +197,16 @@ extern "C" int axc_qconv2d_forward(axc_table *table, const axc_conv_desc *desc, 
     DeviceInfo di;
     rc = device_info(device, &di);
     if (rc == AXC_OK && !window_ok(di)) rc = AXC_INTERNAL;
-    if (rc == AXC_OK && expanded) {
+    if (rc == AXC_OK && route.expanded) {
         // the expanded-table kernels take the bytes as they are and add the zero-point terms at the end
         int mode, centred, e_min;
         table_form(table, &mode, &centred, &e_min);
         const QuantisedOperands u8 = {qinput, qfilter, input_offset, filter_offset};
         const axc_debug_out ints = {nullptr, nullptr, output};
         rc = launch_xtab(lut, mode, centred, e_min, g, make_quant(float(-pad_code), float(255 - pad_code), 0.0f, 255.0f), nullptr, nullptr, nullptr,
-                         nullptr, ws, &ints, di, s, &u8);
+                         nullptr, ws + route.scratch, &ints, di, s, &u8);
     }
-    if (rc != AXC_OK || expanded) {
+    if (rc != AXC_OK || route.expanded) {
         if (prev != device) cudaSetDevice(prev);
         return rc;
     }

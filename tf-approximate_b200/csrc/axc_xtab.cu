@@ -1286,6 +1286,14 @@ size_t xtab_scratch_bytes(const Geom &g, int mode)
     return xlayout(g, x, mode).total;
 }
 
+void xtab_config(const Geom &g, int mode, int32_t out3[3])
+{
+    XGeom x;
+    xgeom(g, &x);
+    const Config cf = choose_config(mode, x, kModelSms, size_t(g.M) * g.Cout * 4 <= kPartialMax, xlayout(g, x, mode).xt_bytes);
+    out3[0] = kWarps * 8 * cf.nb; out3[1] = cf.splits; out3[2] = cf.pre ? 1 : 0;
+}
+
 int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const Geom &g, const Quant &q, const float *ranges_dev,
                 const float *input, const float *filter, float *output, unsigned char *scratch, const axc_debug_out *dbg,
                 const DeviceInfo &di, cudaStream_t stream, const QuantisedOperands *u8)

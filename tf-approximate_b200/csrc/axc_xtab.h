@@ -17,6 +17,8 @@ inline bool window_ok(const DeviceInfo &di) { return di.max_smem_optin >= 232448
 // Scratch bytes of the expanded-table route for this shape and a table kept as `mode` (kXtabAny: enough for every table); 0
 // where the plan-based kernels serve the call.
 size_t xtab_scratch_bytes(const Geom &g, int mode);
+// {pixels per tile, splits of K, tables from global memory} of a call that these kernels serve, on 148 SMs (diagnostics).
+void xtab_config(const Geom &g, int mode, int32_t out3[3]);
 
 // Operands of the quantised entry point and their zero points: the int32 result carries the terms
 // K in_off f_off - f_off sum(a) - in_off sum(b); a tap outside the image has the code input_offset modulo 256.

@@ -187,13 +187,19 @@ def workspace_bytes(input_shape, filter_shape, strides, padding, dilations=(1, 1
     return int(wsz.value)
 
 
-def fast_workspace_bytes(input_shape, filter_shape, strides, padding, dilations=(1, 1, 1, 1), table=None):
-    """Bytes of scratch with which a dense call on `table` (None: any table) is served by the expanded-table kernels
-    (axc_conv2d_fast_workspace_bytes); 0 where a buffer of `workspace_bytes` serves the call."""
-    d = _desc(input_shape, filter_shape, strides, padding, "NHWC", list(dilations), [])
+def fast_workspace_bytes(input_shape, filter_shape, strides, padding, dilations=(1, 1, 1, 1), table=None, plan="none"):
+    """Bytes of a buffer with which a dense call on `table` (None: any table) is served by the expanded-table kernels
+    (axc_conv2d_fast_workspace_bytes): scratch of one call, or with plan="keep" a caller's own `workspace=` that keeps its
+    plan besides; 0 where a buffer of `workspace_bytes` serves the call."""
+    d = _desc(input_shape, filter_shape, strides, padding, "NHWC", list(dilations), [], plan=plan)
     wsz = C.c_size_t()
     raise_for_status(_lib.load().axc_conv2d_fast_workspace_bytes(table.handle if table is not None else None, C.byref(d), C.byref(wsz)), "workspace size")
     return int(wsz.value)
+
+
+def _route(out4):
+    return {"kernels": ("none", "plan", "common-k", "expanded")[out4[0]], "tile": int(out4[1]), "splits": int(out4[2]),
+            "tables_in_global_memory": bool(out4[3])}
 
 
 def _device_index(dev):
@@ -228,13 +234,15 @@ def _forward(depthwise, input, filter, input_min, input_max, filter_min, filter_
         raise InvalidArgumentError("out has the wrong shape, dtype, layout or device")
     wsz = C.c_size_t()
     if workspace is None and not depthwise:
+        d.plan = _PLAN["none"]              # scratch of this call alone: nothing in it is kept
         raise_for_status(L.axc_conv2d_fast_workspace_bytes(table.handle, C.byref(d), C.byref(wsz)), "workspace size")
     fast = wsz.value > 0
     if not fast:
+        d.plan = _PLAN[plan]
         ws_fn = L.axc_depthwise_conv2d_workspace_bytes if depthwise else L.axc_conv2d_workspace_bytes
         raise_for_status(ws_fn(C.byref(d), C.byref(wsz)), "workspace size")
     if fast:
-        # scratch of this call alone: torch's allocator hands it to later work of the same stream only
+        # torch's allocator hands it to later work of the same stream only
         ws = torch.empty(wsz.value, dtype=torch.uint8, device=dev)
     elif workspace is not None:
         if (workspace.dtype != torch.uint8 or workspace.device != dev or not workspace.is_contiguous()
@@ -295,6 +303,8 @@ def _forward(depthwise, input, filter, input_min, input_max, filter_min, filter_
             raise_for_status(L.axc_conv2d_plan_info(ws.data_ptr(), info, dev_index, C.c_void_p(stream)), "plan info")
             dbg_t["plan"] = {"rebuilt": int(info[0]), "fallback": int(info[1]), "status": int(info[2]),
                              "steps_per_mille": int(info[3])}
+            raise_for_status(L.axc_conv2d_route(table.handle, C.byref(d), ws.numel(), info), "route")
+            dbg_t["route"] = _route(info)
         else:
             word = C.c_int32(-1)
             raise_for_status(L.axc_depthwise_conv2d_status(C.byref(d), ws.data_ptr(), C.byref(word), dev_index,
@@ -371,10 +381,12 @@ def ax_conv2d(input, filter, min_input, max_input, min_filter, max_filter, strid
     raise_for_status(L.axc_quantized_zero_point(float(min_input), float(max_input), C.byref(off_in)), "input offset")
     raise_for_status(L.axc_quantized_zero_point(float(min_filter), float(max_filter), C.byref(off_f)), "filter offset")
     wsz = C.c_size_t()
+    d.plan = _PLAN["none"]
     raise_for_status(L.axc_qconv2d_fast_workspace_bytes(tab.handle, C.byref(d), C.byref(wsz)), "workspace size")
     if wsz.value > 0:
         ws = torch.empty(wsz.value, dtype=torch.uint8, device=dev)      # scratch of this call alone
     else:
+        d.plan = _PLAN["keep"]
         raise_for_status(L.axc_qconv2d_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
         ws = _workspace(dev, wsz.value, (f.data_ptr(), tuple(f.shape), id(tab), "q"))
     dev_index = dev.index if dev.index is not None else torch.cuda.current_device()

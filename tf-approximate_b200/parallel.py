@@ -63,12 +63,14 @@ def forward_sharded(x_slabs, filters, table, ranges, strides, padding, gather_to
     d = ops._desc(x_slabs[0].shape, filters[0].shape, strides, padding, "NHWC", [1, 1, 1, 1], [])
     shards = (_lib.Shard * len(x_slabs))()
     outs, keep = [], []
+    fast = [ops.fast_workspace_bytes(x.shape, f.shape, strides, padding, table=tab) for x, f in zip(x_slabs, filters)]
+    if any(fast):
+        d.plan = ops._PLAN["none"]          # the buffers are this call's own: nothing in them is kept
     for i, (x, f) in enumerate(zip(x_slabs, filters)):
         dev = x.device
         oshape = ops.conv2d_output_shape(x.shape, f.shape, strides, padding)
         y = torch.empty(oshape, dtype=torch.float32, device=dev)
-        ws = torch.zeros(max(ops.workspace_bytes(x.shape, f.shape, strides, padding),
-                             ops.fast_workspace_bytes(x.shape, f.shape, strides, padding, table=tab)), dtype=torch.uint8, device=dev)
+        ws = torch.zeros(max(ops.workspace_bytes(x.shape, f.shape, strides, padding), fast[i]), dtype=torch.uint8, device=dev)
         xs, fs = x.contiguous(), f.contiguous()
         keep += [xs, fs, ws]
         outs.append(y)
