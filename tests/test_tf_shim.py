@@ -143,6 +143,38 @@ def test_shim_compute_reproduces_the_reference(harness, tmp_path, case):
 
 
 @pytest.mark.gpu
+def test_shim_takes_the_expanded_tables(harness, tmp_path):
+    """A call that they serve goes to the expanded-table kernels with temporary scratch (as many launches as the Python call, which
+    reports its kernels), whatever the size of the plan's workspace; a small call in between keeps the op's plan."""
+    import torch
+    import tf_approximate_b200 as ax
+    path = str(tmp_path / "table.bin")
+    ax.write_table(path, ax.noisy_table(5))
+    g = torch.Generator(device="cuda").manual_seed(3)
+    f = torch.randn((3, 3, 128, 128), device="cuda", generator=g) * 0.05
+    mm = (-1.0, 1.0, -0.2, 0.2)
+    op, code, msg = _create(harness, path.encode())
+    assert op is not None, (code, msg)
+    launches = {}
+    try:
+        for n, hw, kernels in ((16, 14, "expanded"), (1, 5, "plan"), (128, 7, "expanded"), (1, 5, "plan")):
+            x = torch.rand((n, hw, hw, 128), device="cuda", generator=g) * 2 - 1
+            before = ax.launch_count()
+            code, msg, dims, out = _compute(harness, op, x, f, mm, (n, hw, hw, 128))
+            assert code == 0, msg
+            mid = ax.launch_count()
+            want = ax.approx_conv2d_with_min_max_vars(x, f, *mm, [1, 1, 1, 1], 8, path, "SAME")
+            assert mid - before == ax.launch_count() - mid
+            launches.setdefault(kernels, set()).add(mid - before)
+            assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+            _, dbg = ax.approx_conv2d_with_min_max_vars(x, f, *mm, [1, 1, 1, 1], 8, path, "SAME", debug=True)
+            assert dbg["route"]["kernels"] == kernels
+        assert not launches["expanded"] & launches["plan"]
+    finally:
+        harness.shimtest_destroy(op)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("case", cases.DEPTHWISE_CASES, ids=[c[0] for c in cases.DEPTHWISE_CASES])
 def test_depthwise_shim_compute_matches_the_checker(harness, tmp_path, case):
     import torch

@@ -90,14 +90,22 @@ public:
         OP_REQUIRES_OK(ctx, ctx->allocate_output(0, ShapeFromFormat(format_, dims[0], dims[1], dims[2], dims[3]), &output));
         if (output->NumElements() == 0) return;             // as the reference: nothing to do (:449-450)
 
-        // The workspace keeps the filter's lookup plan between calls, so it belongs to the op instance: allocated
-        // on first use (and when a larger input needs more), then reused.  A buffer taken from allocate_temp on
-        // every call would work too - the library checks what it finds - but would rebuild the plan every time.
-        size_t ws_bytes = 0;
-        OP_REQUIRES_OK(ctx, FromAxc(axc_conv2d_workspace_bytes(&d, &ws_bytes)));
-        if (ws_bytes > ws_bytes_) {
-            OP_REQUIRES_OK(ctx, ctx->allocate_temp(DT_UINT8, TensorShape({static_cast<int64>(ws_bytes)}), &workspace_));
-            ws_bytes_ = ws_bytes;
+        // Where the expanded-table kernels serve the call, their scratch holds nothing afterwards: a temporary.  Otherwise (or
+        // where that much memory is not to be had) the workspace keeps the filter's lookup plan between calls, so it
+        // belongs to the op instance: allocated on first use (and when a larger input needs more), then reused.
+        Tensor scratch;
+        size_t bytes = 0;
+        d.plan = AXC_PLAN_NONE;
+        OP_REQUIRES_OK(ctx, FromAxc(axc_conv2d_fast_workspace_bytes(table_, &d, &bytes)));
+        if (bytes == 0 || !ctx->allocate_temp(DT_UINT8, TensorShape({static_cast<int64>(bytes)}), &scratch).ok()) {
+            d.plan = AXC_PLAN_KEEP;
+            OP_REQUIRES_OK(ctx, FromAxc(axc_conv2d_workspace_bytes(&d, &bytes)));
+            if (bytes > ws_bytes_) {
+                OP_REQUIRES_OK(ctx, ctx->allocate_temp(DT_UINT8, TensorShape({static_cast<int64>(bytes)}), &workspace_));
+                ws_bytes_ = bytes;
+            }
+            scratch = workspace_;
+            bytes = ws_bytes_;
         }
         int device = 0;
         OP_REQUIRES(ctx, cudaGetDevice(&device) == cudaSuccess, errors::Internal("No GPU device is current."));
@@ -106,7 +114,7 @@ public:
         const int st = axc_conv2d_forward(table_, &d, input.flat<float>().data(), filter.flat<float>().data(),
                                           ctx->input(2).scalar<float>()(), ctx->input(3).scalar<float>()(),
                                           ctx->input(4).scalar<float>()(), ctx->input(5).scalar<float>()(),
-                                          output->flat<float>().data(), workspace_.flat<uint8>().data(), ws_bytes_, nullptr,
+                                          output->flat<float>().data(), scratch.flat<uint8>().data(), bytes, nullptr,
                                           device, stream);
         OP_REQUIRES_OK(ctx, FromAxc(st));
     }

@@ -61,7 +61,7 @@ public:
 
     ~AxconvAxConv2DOp() override
     {
-        for (Buffer *b : {&in_, &filter_, &out_, &ws_}) cudaFree(b->ptr);
+        for (Buffer *b : {&in_, &filter_, &out_, &ws_, &scratch_}) cudaFree(b->ptr);
         if (stream_) cudaStreamDestroy(stream_);
         axc_table_destroy(table_);
     }
@@ -103,16 +103,25 @@ public:
         const size_t n_in = static_cast<size_t>(input.NumElements()), n_f = static_cast<size_t>(filter.NumElements());
         const size_t n_out = static_cast<size_t>(output->NumElements());
         if (n_out != 0) {
+            // scratch of the expanded-table kernels where they serve the call and it is to be had; else the workspace, which
+            // keeps the filter's lookup plan between calls and is therefore a buffer of its own
+            Buffer *ws = &scratch_;
             size_t ws_bytes = 0;
-            OP_REQUIRES(context, axc_qconv2d_workspace_bytes(&d, &ws_bytes) == AXC_OK, errors::InvalidArgument("AxConv2D: invalid shapes"));
+            d.plan = AXC_PLAN_NONE;
+            OP_REQUIRES(context, axc_qconv2d_fast_workspace_bytes(table_, &d, &ws_bytes) == AXC_OK, errors::InvalidArgument("AxConv2D: invalid shapes"));
+            if (ws_bytes == 0 || !scratch_.reserve(ws_bytes)) {
+                ws = &ws_;
+                d.plan = AXC_PLAN_KEEP;
+                OP_REQUIRES(context, axc_qconv2d_workspace_bytes(&d, &ws_bytes) == AXC_OK, errors::InvalidArgument("AxConv2D: invalid shapes"));
+            }
             int device = 0;
             OP_REQUIRES(context, cudaGetDevice(&device) == cudaSuccess, errors::Internal("No GPU device is current."));
-            OP_REQUIRES(context, in_.reserve(n_in) && filter_.reserve(n_f) && out_.reserve(n_out * 4) && ws_.reserve(ws_bytes),
+            OP_REQUIRES(context, in_.reserve(n_in) && filter_.reserve(n_f) && out_.reserve(n_out * 4) && ws->reserve(ws_bytes),
                         errors::Internal("AxConv2D: device allocation failed"));
             cudaMemcpyAsync(in_.ptr, input.flat<quint8>().data(), n_in, cudaMemcpyHostToDevice, stream_);
             cudaMemcpyAsync(filter_.ptr, filter.flat<quint8>().data(), n_f, cudaMemcpyHostToDevice, stream_);
             const int st = axc_qconv2d_forward(table_, &d, static_cast<const uint8_t *>(in_.ptr), static_cast<const uint8_t *>(filter_.ptr),
-                                               offset_input, offset_filter, static_cast<int32_t *>(out_.ptr), ws_.ptr, ws_.bytes, device,
+                                               offset_input, offset_filter, static_cast<int32_t *>(out_.ptr), ws->ptr, ws->bytes, device,
                                                stream_);
             OP_REQUIRES(context, st == AXC_OK,
                         st == AXC_UNIMPLEMENTED ? errors::Unimplemented("AxConv2D: window placement not supported for this stride")
@@ -141,7 +150,11 @@ private:
             cudaFree(ptr);
             ptr = nullptr;
             bytes = 0;
-            if (cudaMalloc(&ptr, want) != cudaSuccess) return false;
+            if (cudaMalloc(&ptr, want) != cudaSuccess) {
+                ptr = nullptr;
+                cudaGetLastError();                       // not an error of the launches that follow
+                return false;
+            }
             bytes = want;
             return true;
         }
@@ -150,7 +163,7 @@ private:
     Padding padding_ = SAME;
     axc_table *table_ = nullptr;
     cudaStream_t stream_ = nullptr;
-    Buffer in_, filter_, out_, ws_;
+    Buffer in_, filter_, out_, ws_, scratch_;
 };
 
 REGISTER_KERNEL_BUILDER(Name("AxConv2D")
