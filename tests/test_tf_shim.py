@@ -168,7 +168,7 @@ def test_shim_takes_the_expanded_tables(harness, tmp_path):
             launches.setdefault(kernels, set()).add(mid - before)
             assert torch.equal(out.view(torch.int32), want.view(torch.int32))
             _, dbg = ax.approx_conv2d_with_min_max_vars(x, f, *mm, [1, 1, 1, 1], 8, path, "SAME", debug=True)
-            assert dbg["route"]["kernels"] == kernels
+            assert dbg["plan"]["route"]["kernels"] == kernels
         assert not launches["expanded"] & launches["plan"]
     finally:
         harness.shimtest_destroy(op)

@@ -167,8 +167,8 @@ def test_a_kept_plan_survives_every_batch_size(built):
             x = torch.rand((n, 7, 7, 128), device="cuda", generator=g) * 2 - 1
             y, dbg = ax.approx_conv2d_with_min_max_vars(x, f, -1.0, 1.0, -0.2, 0.2, one, 8, t, "SAME", workspace=ws, debug=True)
             if n == 128:
-                assert dbg["route"]["kernels"] == last
-            if dbg["route"]["kernels"] == "plan":
+                assert dbg["plan"]["route"]["kernels"] == last
+            if dbg["plan"]["route"]["kernels"] == "plan":
                 rebuilt.append(dbg["plan"]["rebuilt"])
             want = ax.approx_conv2d_with_min_max_vars(x, f, -1.0, 1.0, -0.2, 0.2, one, 8, t, "SAME")
             assert torch.equal(y.view(torch.int32), want.view(torch.int32))

@@ -304,7 +304,7 @@ def _forward(depthwise, input, filter, input_min, input_max, filter_min, filter_
             dbg_t["plan"] = {"rebuilt": int(info[0]), "fallback": int(info[1]), "status": int(info[2]),
                              "steps_per_mille": int(info[3])}
             raise_for_status(L.axc_conv2d_route(table.handle, C.byref(d), ws.numel(), info), "route")
-            dbg_t["route"] = _route(info)
+            dbg_t["plan"]["route"] = _route(info)
         else:
             word = C.c_int32(-1)
             raise_for_status(L.axc_depthwise_conv2d_status(C.byref(d), ws.data_ptr(), C.byref(word), dev_index,
