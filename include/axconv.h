@@ -146,7 +146,11 @@ enum {
 int axc_conv2d_route(const axc_table *table, const axc_conv_desc *desc, size_t workspace_bytes, int32_t out4[4]);
 /* Reads back {rebuilt in the last call, fallback kernel in use, kernel status (0 = fine), schedule steps per
  * ideal step in per-mille} of the plan in a dense workspace.  Blocks until `stream` is idle.  Diagnostics only;
- * no counterpart in the reference. */
+ * no counterpart in the reference.
+ * Calls that the expanded-table kernels served leave a header of their own at the start of their scratch (0, 0, status, 1000):
+ * status 2 = the shared-memory layout was broken, 3 = a copy or a barrier inside a kernel did not come within about a
+ * second; the output is then not valid.  The calls are asynchronous and return AXC_OK all the same: this is the only place
+ * where it shows (in a buffer that keeps a plan besides: axc_conv2d_workspace_bytes behind its start). */
 int axc_conv2d_plan_info(const void *workspace, int32_t out4[4], int device, void *stream);
 
 /* ---- forward: ApproxConv2DOp::Compute + LaunchApproxConv2DOp<GPUDevice>
@@ -340,6 +344,11 @@ uint64_t axc_launch_count(void);
  * reading clears the record.  Blocks until the device is idle.  In the normal build: AXC_UNIMPLEMENTED.  No
  * counterpart in the reference. */
 int axc_debug_bounds_record(int device, uint32_t out4[4]);
+
+/* Debug flavour only, as above: polls after which a wait inside the expanded-table kernels gives up (the kernel that makes the
+ * tables in global memory, and the convolution); negative: the built-in limit of about a second.  With 0 every wait runs
+ * out at once: the kernels finish, the outputs are not valid, and axc_conv2d_plan_info reports status 3. */
+int axc_debug_wait_polls(int device, int32_t expand, int32_t convolution);
 
 /* Measures what one SM sustains in conflict-free 16-bit shared-memory loads - the operation a table MAC of the
  * dense kernels costs (the reference does the same lookup through a texture fetch,

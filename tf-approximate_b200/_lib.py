@@ -13,7 +13,7 @@ SYMBOLS = [
     "axc_conv2d_workspace_bytes", "axc_conv2d_fast_workspace_bytes", "axc_conv2d_route", "axc_depthwise_conv2d_workspace_bytes", "axc_conv2d_plan_info",
     "axc_conv2d_forward", "axc_conv2d_forward_device_ranges", "axc_depthwise_conv2d_forward",
     "axc_depthwise_conv2d_forward_noalloc", "axc_depthwise_conv2d_status",
-    "axc_quant_props", "axc_status_string", "axc_last_cuda_error", "axc_launch_count", "axc_measure_lookup_peak", "axc_debug_bounds_record",
+    "axc_quant_props", "axc_status_string", "axc_last_cuda_error", "axc_launch_count", "axc_measure_lookup_peak", "axc_debug_bounds_record", "axc_debug_wait_polls",
     "axc_add_residual", "axc_max_pool_same", "axc_conv2d_forward_fused", "axc_depthwise_conv2d_forward_fused", "axc_tensor_range", "axc_fake_quant", "axc_conv2d_forward_sharded", "axc_gather_outputs",
     "axc_qconv2d_workspace_bytes", "axc_qconv2d_fast_workspace_bytes", "axc_qconv2d_route", "axc_qconv2d_forward", "axc_quantized_zero_point", "axc_quantized_output_range",
 ]

@@ -738,6 +738,22 @@ int axc_debug_bounds_record(int device, uint32_t out4[4])
 #endif
 }
 
+int axc_debug_wait_polls(int device, int32_t expand, int32_t convolution)
+{
+#ifndef AXC_BOUNDS_CHECK
+    (void)device; (void)expand; (void)convolution;
+    return AXC_UNIMPLEMENTED;
+#else
+    int prev = 0;
+    AXC_CUDA(cudaGetDevice(&prev));
+    if (prev != device) AXC_CUDA(cudaSetDevice(device));
+    cudaError_t e = cudaDeviceSynchronize();
+    const int rc = e == cudaSuccess ? axc::set_wait_polls(expand, convolution) : axc::cuda_failed(e);
+    if (prev != device) cudaSetDevice(prev);
+    return rc;
+#endif
+}
+
 int axc_quant_props(float min_value, float max_value, float out3[3])
 {
     if (!out3) return AXC_INVALID_ARGUMENT;

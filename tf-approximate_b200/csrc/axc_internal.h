@@ -69,6 +69,7 @@ int bounds_record_sched(unsigned out4[4]);
 int bounds_record_conv(unsigned out4[4]);
 int bounds_record_depthwise(unsigned out4[4]);
 int bounds_record_xtab(unsigned out4[4]);
+int set_wait_polls(int expand, int convolution);      // debug flavour only
 
 // Quantisation state of one call: what the reference keeps in
 // BaseTableApproxOpType_t::quantProps (tf2/src/approx_ops_types.h:84-96).

@@ -111,16 +111,32 @@ __device__ __forceinline__ void mbar_arrive(unsigned bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Waits for the phase `parity`; gives up after about a second (`ok` stays false from then on, later waits return at once)
-__device__ __forceinline__ void mbar_wait(unsigned bar, unsigned parity, bool &ok)
+// Polls after which a wait gives up, about a second.  The debug flavour reads them from device memory, so that a test can make
+// the waits of one kernel run out: {xexpand_kernel, xtab_kernel}.
+#ifdef AXC_BOUNDS_CHECK
+__device__ int g_wait_polls[2] = {kWaitPolls, kWaitPolls};
+#define AXC_WAIT_POLLS(kernel) (*(volatile int *)&g_wait_polls[kernel])
+#else
+#define AXC_WAIT_POLLS(kernel) kWaitPolls
+#endif
+// Waits for the phase `parity`; gives up after `polls` (`ok` stays false from then on, later waits return at once).
+// A kernel whose wait gave up starts no further copy, finishes with whatever is in shared memory (every address is in bounds
+// whatever the tables hold), waits for its own copies in flight and leaves 3 in the header's status.
+__device__ __forceinline__ void mbar_wait(unsigned bar, unsigned parity, bool &ok, int polls)
 {
     for (int it = 0; ok; ++it) {
+        if (it >= polls) { ok = false; return; }
         unsigned done;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
         if (done) return;
-        if (it >= kWaitPolls) ok = false;
     }
+}
+// The end of a kernel that gave up: the phase that a copy in flight completes.
+__device__ __forceinline__ void mbar_drain(unsigned bar, unsigned parity)
+{
+    bool ok = true;
+    mbar_wait(bar, parity, ok, kWaitPolls);
 }
 
 // Programmatic dependent launch: the three kernels of a call are launched so that each may start while the one before it
@@ -490,6 +506,7 @@ struct ExpandParams {
     unsigned char *xt;
     uint2 *wb;
     uint8_t *qf_debug;
+    PlanHeader *hdr;
 };
 
 // xt[channel tile][chunk][row a][piece kk][16 bytes], kk = octet * 8 + k.  The table's rows (one per weight) lie in shared memory.
@@ -518,7 +535,7 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
     const DevQuant q = P.ranges ? dev_quant_from_ranges(P.ranges, g.K) : P.host_q;
     const unsigned z = code_of(0.0f, q.in_off, q.in_inv);
     bool ok = true;
-    mbar_wait(bar, 0u, ok);
+    mbar_wait(bar, 0u, ok, AXC_WAIT_POLLS(0));
     // thread (kk, slot) of the first 16*TNC prepares the list of table rows of a chunk
     const int kk = tid / TNC, slot = tid % TNC;
     const int elem = ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);           // element 4t + 2*octet + p
@@ -574,6 +591,10 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
         }
     }
     pdl_wait();                                                    // the kernel after this one waits for this one only
+    if (!ok) {
+        if (tid == 0) mbar_drain(bar, 0u);
+        atomicExch(&P.hdr->status, 3);                             // (xprep_kernel, which clears it, is complete)
+    }
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -628,13 +649,14 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
     unsigned dyn_size;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_size));
     const unsigned bars = (dyn0 + 15u) & ~15u;
-    const unsigned tab_full = bars, tab_empty = bars + 16u, rows_full = bars + 32u;
-    if (rows_full + 8u > kCodes || dyn0 + dyn_size < kWindowEnd) {
-        if (tid == 0) atomicExch(const_cast<int *>(&P.hdr->status), 2);
+    const unsigned tab_full = bars, tab_empty = bars + 16u, rows_full = bars + 32u, copies = bars + 40u;
+    pdl_wait();
+    if (copies + 4u > kCodes || dyn0 + dyn_size < kWindowEnd) {
+        if (tid == 0) atomicExch(const_cast<int *>(&P.hdr->status), 2);      // (xprep_kernel, which clears it, is complete)
         return;
     }
-    pdl_wait();
     if (tid == 0) {
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(copies), "r"(0u) : "memory");
         for (int s = 0; s < 2; ++s) { mbar_init(tab_full + s * 8, PRE ? 1 : kWarps); mbar_init(tab_empty + s * 8, kWarps); }
         mbar_init(rows_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -794,6 +816,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
     int x_left = 0;
     const unsigned char *x_src = nullptr;
     auto copy_table = [&](unsigned buf) {                          // the next chunk's table into buffer `buf`
+        if (!ok) return;                                           // the buffer's last copy may still be in flight
         if (x_left == 0) {
             if (x_src) x_unit += gridDim.x;
             if (x_unit >= units) return;
@@ -805,6 +828,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tab_full + buf * 8), "r"(65536u) : "memory");
         bulk_copy(kTab * (1u + buf), x_src, 65536u, tab_full + buf * 8);
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(copies), "r"(lds32(copies) + 1u) : "memory");
         x_src += 65536;
         --x_left;
     };
@@ -880,7 +904,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
             }
             if (PRE && h == 0 && n == 1 && tid == 0 && oct > 0) {
                 // the other buffer's readers finished the chunk before this one: ask for the chunk after this one
-                mbar_wait(tab_empty + (st ^ 1u) * 8, ((oct - 1) >> 1) & 1u, ok);
+                mbar_wait(tab_empty + (st ^ 1u) * 8, ((oct - 1) >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
                 copy_table(st ^ 1u);
             }
             if (kBuild && more) {
@@ -890,7 +914,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
                         if (r == 0) {
                             build_next();
                             // the stage's last readers worked on the octet before this one
-                            if (oct > 0) mbar_wait(tab_empty + (st ^ 1u) * 8, ((oct - 1) >> 1) & 1u, ok);
+                            if (oct > 0) mbar_wait(tab_empty + (st ^ 1u) * 8, ((oct - 1) >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
                             build_rows();
                         }
                         build_load(r);
@@ -927,7 +951,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
             build_unit();
             build_next();
             build_next();
-            mbar_wait(rows_full, 0u, ok);
+            mbar_wait(rows_full, 0u, ok, AXC_WAIT_POLLS(1));
             build_rows();
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
@@ -959,13 +983,13 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
             if (MODE != kXtabFull && c + 1 < c_end) wb_next = __ldg(wbp);
             if (PRE) {
                 const unsigned st = chunk & 1u;
-                mbar_wait(tab_full + st * 8, (chunk >> 1) & 1u, ok);
+                mbar_wait(tab_full + st * 8, (chunk >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
 #pragma unroll
                 for (int h = 0; h < 2; ++h) octet(h, st * kTab + unsigned(h) * 128u, st, chunk, true, wb);
             } else if (kTables) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h, ++oct) {
-                    mbar_wait(tab_full + (oct & 1u) * 8, (oct >> 1) & 1u, ok);
+                    mbar_wait(tab_full + (oct & 1u) * 8, (oct >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
                     octet(h, (oct & 1u) * 128u, oct & 1u, oct, oct + 1 < oct_total, wb);
                 }
             } else {
@@ -1070,7 +1094,16 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");               // nothing of this CTA is in flight when it ends
-    if (!ok && lane == 0) atomicExch(const_cast<int *>(&P.hdr->status), 3);
+    if (!ok) {
+        // thread 0 issued all bulk copies and, had every wait of its own come true, would have seen each of them arrive
+        if (tid == 0) {
+            if (kBuild) mbar_drain(rows_full, 0u);
+            const unsigned n = PRE ? lds32(copies) : 0u;
+            if (n > 1) mbar_drain(tab_full + (n & 1u) * 8, ((n - 2) >> 1) & 1u);
+            if (n > 0) mbar_drain(tab_full + ((n - 1) & 1u) * 8, ((n - 1) >> 1) & 1u);
+        }
+        atomicExch(const_cast<int *>(&P.hdr->status), 3);
+    }
 }
 
 // The dequantisation of a call whose K was split over CTAs.
@@ -1345,7 +1378,7 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     if (cf.pre) {
         ExpandParams E;
         E.g = x; E.filter = filter; E.filter_u8 = A.filter_u8; E.rows = reinterpret_cast<const unsigned char *>(lut_dev + 65536); E.ranges = ranges_dev; E.host_q = A.host_q;
-        E.xt = scratch + L.xt; E.wb = A.wb; E.qf_debug = A.qf_debug;
+        E.xt = scratch + L.xt; E.wb = A.wb; E.qf_debug = A.qf_debug; E.hdr = A.hdr;
         const int rc = mode == kXtabFull ? launch_expand<kXtabFull>(E, di, stream) : launch_expand<kXtabByte>(E, di, stream);
         if (rc) return rc;
     }
@@ -1375,5 +1408,14 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
 }
 
 AXC_DEFINE_BOUNDS_READER(bounds_record_xtab)
+
+#ifdef AXC_BOUNDS_CHECK
+int set_wait_polls(int expand, int convolution)
+{
+    const int polls[2] = {expand < 0 ? kWaitPolls : expand, convolution < 0 ? kWaitPolls : convolution};
+    AXC_CUDA(cudaMemcpyToSymbol(g_wait_polls, polls, sizeof(polls)));
+    return AXC_OK;
+}
+#endif
 
 }  // namespace axc
