@@ -108,3 +108,21 @@ def test_sharded_entry_point_on_the_devices_present(built):
     assert st == 13 and failed.value == 1
     lo, hi = parallel.shard_bounds(x.shape[0], nshards, 0)
     assert torch.equal(outs[0].view(torch.int32), want[lo:hi].to(outs[0].device).view(torch.int32))
+
+
+def test_sharded_call_fills_no_scratch(built, monkeypatch):
+    """Scratch of the expanded tables (up to hundreds of MB) is taken as it comes: nothing is set to zero first."""
+    import torch
+    import tf_approximate_b200 as ax
+    from tf_approximate_b200 import parallel
+    g = torch.Generator(device="cuda").manual_seed(11)
+    f = torch.randn((3, 3, 32, 64), device="cuda", generator=g) * 0.1
+    x = torch.rand((6, 40, 40, 32), device="cuda", generator=g)
+    table = ax.Table(array=ax.truncated_table())
+    filled = []
+    zeros = torch.zeros
+    monkeypatch.setattr(torch, "zeros", lambda *a, **k: filled.append(a) or zeros(*a, **k))
+    y = parallel.forward_sharded([x[:2], x[2:]], [f, f], table, (0.0, 1.0, -0.4, 0.4), [1, 1, 1, 1], "SAME", gather_to="cuda:0")
+    assert not filled
+    want = ax.approx_conv2d_with_min_max_vars(x, f, 0.0, 1.0, -0.4, 0.4, [1, 1, 1, 1], 8, table, "SAME")
+    assert torch.equal(y.view(torch.int32), want.view(torch.int32))

@@ -70,7 +70,10 @@ def forward_sharded(x_slabs, filters, table, ranges, strides, padding, gather_to
         dev = x.device
         oshape = ops.conv2d_output_shape(x.shape, f.shape, strides, padding)
         y = torch.empty(oshape, dtype=torch.float32, device=dev)
-        ws = torch.zeros(max(ops.workspace_bytes(x.shape, f.shape, strides, padding), fast[i]), dtype=torch.uint8, device=dev)
+        if fast[i]:
+            ws = torch.empty(fast[i], dtype=torch.uint8, device=dev)
+        else:
+            ws = torch.zeros(ops.workspace_bytes(x.shape, f.shape, strides, padding), dtype=torch.uint8, device=dev)
         xs, fs = x.contiguous(), f.contiguous()
         keep += [xs, fs, ws]
         outs.append(y)
