@@ -198,3 +198,40 @@ def test_a_kept_plan_survives_every_batch_size(built):
         want, _, _ = ax.ax_conv2d(a, b, -1.0, 2.0, -0.5, 0.5, one, "SAME", table=t, ax_tune=False)
         assert torch.equal(y, want)
     assert rebuilt == [1, 0, 0]
+
+
+@pytest.mark.gpu
+def test_a_device_without_room_for_the_scratch_still_serves_the_call(built, monkeypatch):
+    """Where the expanded tables' scratch cannot be allocated the call runs on the kernels that need a plan's workspace only:
+    same bits, no error - the op, the layer-level caller, the quantised op and the sharded call."""
+    import torch
+    import tf_approximate_b200 as ax
+    from tf_approximate_b200 import parallel
+    g = torch.Generator(device="cuda").manual_seed(12)
+    t = ax.Table(array=ax.noisy_table(6))
+    x = torch.rand((8, 28, 28, 64), device="cuda", generator=g)
+    f = torch.randn((3, 3, 64, 64), device="cuda", generator=g) * 0.1
+    a = torch.randint(0, 256, x.shape, device="cuda", generator=g, dtype=torch.uint8)
+    b = torch.randint(0, 256, f.shape, device="cuda", generator=g, dtype=torch.uint8)
+    layer = ax.FakeApproxConv2D(64, 64, 3, padding="same", mul_map_file=t).cuda().eval()
+    one = [1, 1, 1, 1]
+
+    def calls():
+        with torch.no_grad():
+            return [ax.approx_conv2d_with_min_max_vars(x, f, 0.0, 1.0, -0.4, 0.4, one, 8, t, "SAME"), layer(x),
+                    ax.ax_conv2d(a, b, -1.0, 2.0, -0.5, 0.5, one, "SAME", table=t, ax_tune=False)[0],
+                    parallel.forward_sharded([x[:5], x[5:]], [f, f], t, (0.0, 1.0, -0.4, 0.4), one, "SAME", gather_to="cuda:0")]
+    want = calls()
+    empty, refused = torch.empty, []
+
+    def full(*args, **kw):
+        if kw.get("dtype") == torch.uint8:
+            refused.append(args)
+            raise torch.OutOfMemoryError("out of memory")
+        return empty(*args, **kw)
+    monkeypatch.setattr(torch, "empty", full)
+    got = calls()
+    monkeypatch.undo()
+    assert len(refused) == 5
+    for w, y in zip(want, got):
+        assert torch.equal(w.view(torch.int32), y.view(torch.int32))

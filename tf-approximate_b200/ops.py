@@ -202,6 +202,17 @@ def _route(out4):
             "tables_in_global_memory": bool(out4[3])}
 
 
+def _scratch(dev, nbytes):
+    """Scratch of one call on the expanded tables, or None where the device has not that much memory left (up to hundreds of
+    MB; the other kernels need a plan's workspace only).  torch's allocator hands it to later work of the same stream only."""
+    if nbytes == 0:
+        return None
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def _device_index(dev):
     """CUDA ordinal of a torch device; a device without an index means the current one."""
     return dev.index if dev.index is not None else torch.cuda.current_device()
@@ -233,25 +244,23 @@ def _forward(depthwise, input, filter, input_min, input_max, filter_min, filter_
     elif tuple(out.shape) != oshape or out.dtype != torch.float32 or not out.is_contiguous() or out.device != dev:
         raise InvalidArgumentError("out has the wrong shape, dtype, layout or device")
     wsz = C.c_size_t()
+    ws = None
     if workspace is None and not depthwise:
         d.plan = _PLAN["none"]              # scratch of this call alone: nothing in it is kept
         raise_for_status(L.axc_conv2d_fast_workspace_bytes(table.handle, C.byref(d), C.byref(wsz)), "workspace size")
-    fast = wsz.value > 0
-    if not fast:
+        ws = _scratch(dev, wsz.value)
+    if ws is None:
         d.plan = _PLAN[plan]
         ws_fn = L.axc_depthwise_conv2d_workspace_bytes if depthwise else L.axc_conv2d_workspace_bytes
         raise_for_status(ws_fn(C.byref(d), C.byref(wsz)), "workspace size")
-    if fast:
-        # torch's allocator hands it to later work of the same stream only
-        ws = torch.empty(wsz.value, dtype=torch.uint8, device=dev)
-    elif workspace is not None:
-        if (workspace.dtype != torch.uint8 or workspace.device != dev or not workspace.is_contiguous()
+        if workspace is None:
+            ws = _workspace(dev, wsz.value, (f.data_ptr(), tuple(f.shape), id(table), depthwise))
+        elif (workspace.dtype != torch.uint8 or workspace.device != dev or not workspace.is_contiguous()
                 or workspace.numel() < wsz.value or workspace.data_ptr() % 256):
             raise InvalidArgumentError("workspace must be a contiguous uint8 tensor on the input's device, 256-byte "
                                        "aligned, of at least %d bytes" % wsz.value)
-        ws = workspace
-    else:
-        ws = _workspace(dev, wsz.value, (f.data_ptr(), tuple(f.shape), id(table), depthwise))
+        else:
+            ws = workspace
     dbg_ptr = None
     dbg_t = None
     if debug:
@@ -383,9 +392,8 @@ def ax_conv2d(input, filter, min_input, max_input, min_filter, max_filter, strid
     wsz = C.c_size_t()
     d.plan = _PLAN["none"]
     raise_for_status(L.axc_qconv2d_fast_workspace_bytes(tab.handle, C.byref(d), C.byref(wsz)), "workspace size")
-    if wsz.value > 0:
-        ws = torch.empty(wsz.value, dtype=torch.uint8, device=dev)      # scratch of this call alone
-    else:
+    ws = _scratch(dev, wsz.value)
+    if ws is None:
         d.plan = _PLAN["keep"]
         raise_for_status(L.axc_qconv2d_workspace_bytes(C.byref(d), C.byref(wsz)), "workspace size")
         ws = _workspace(dev, wsz.value, (f.data_ptr(), tuple(f.shape), id(tab), "q"))

@@ -70,9 +70,8 @@ def forward_sharded(x_slabs, filters, table, ranges, strides, padding, gather_to
         dev = x.device
         oshape = ops.conv2d_output_shape(x.shape, f.shape, strides, padding)
         y = torch.empty(oshape, dtype=torch.float32, device=dev)
-        if fast[i]:
-            ws = torch.empty(fast[i], dtype=torch.uint8, device=dev)
-        else:
+        ws = ops._scratch(dev, fast[i])
+        if ws is None:
             ws = torch.zeros(ops.workspace_bytes(x.shape, f.shape, strides, padding), dtype=torch.uint8, device=dev)
         xs, fs = x.contiguous(), f.contiguous()
         keep += [xs, fs, ws]
