@@ -283,11 +283,11 @@ static void append_rows(const axc_table *t, std::vector<uint16_t> *image)
 {
     int mode, centred, e_min;
     table_form(t, &mode, &centred, &e_min);
+    if (mode != kXtabFull && mode != kXtabByte) return;      // nothing reads rows of an exact table or of one without a form
     const size_t at = image->size();
-    image->resize(at + 257 * 256, 0);
+    image->resize(at + 257 * (mode == kXtabFull ? 256 : 128), 0);
     uint16_t *digits = image->data() + at;
     uint8_t *bytes = reinterpret_cast<uint8_t *>(digits);
-    if (mode != kXtabFull && mode != kXtabByte) return;
     for (int a = 0; a < 256; ++a) {
         const uint16_t *row = t->host.data() + a * 256;
         for (int b = 0; b < 256; ++b) {

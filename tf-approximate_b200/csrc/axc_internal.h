@@ -137,7 +137,7 @@ void count_launch(int n = 1);
     } while (0)
 
 // Device replica of a table (native [a][b] order, 65536 uint16), followed by its form for the expanded tables (table_form): one row
-// of 256 entries (two digits, or one byte) per weight b, entry a, and a row of zeros.
+// of 256 entries (two digits, or one byte) per weight b, entry a, and a row of zeros - where the form has such rows.
 const uint16_t *table_device_ptr(axc_table *t, int device, int *status);
 // The replica on `device` if it has been uploaded already, else NULL.  Never allocates.
 const uint16_t *table_device_ptr_if_resident(axc_table *t, int device);
