@@ -66,6 +66,10 @@ constexpr double kXtabMinLookups = 8e6;
 constexpr size_t kXtMax = 640u << 20;          // expanded tables in global memory
 constexpr int kModelSms = 148;                 // what the scratch size is computed for
 
+// `n` bytes at `p` lie in the scratch of the call (debug flavour, as the checks of axc_internal.h)
+#define AXC_SCRATCH_OK(P, p, n, site) \
+    AXC_GLOBAL_OK(reinterpret_cast<const unsigned char *>(p) - reinterpret_cast<const unsigned char *>((P).hdr), (P).scratch_bytes - (long long)(n) + 1, site)
+
 // ---- shared memory -----------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint4 lds128(unsigned addr)
 {
@@ -200,6 +204,7 @@ struct PrepParams {
     float *asum, *bsum;
     uint8_t *qf_debug;
     PlanHeader *hdr;
+    long long scratch_bytes;
     int blocks_sum, blocks_w, blocks_t;      // leading blocks; the rest are input tiles
     int TH, TW, tiles_y, tiles_x, RH, RW, pitch, vec;
 };
@@ -218,7 +223,22 @@ __device__ __forceinline__ unsigned row_address(int mode, unsigned row)
     return row < unsigned(kLowRows) ? kRowsLow + row * 512u : kRowsHigh + (row - kLowRows) * 512u;
 }
 
-__device__ __forceinline__ float filter_value(const float *f, const uint8_t *u8, size_t at) { return u8 ? float(__ldg(u8 + at)) : __ldg(f + at); }
+__device__ __forceinline__ float filter_value(const XGeom &g, const float *f, const uint8_t *u8, size_t at)
+{
+    if (!AXC_GLOBAL_OK((long long)at, (long long)g.K * g.Cout, 320u)) return 0.0f;
+    return u8 ? float(__ldg(u8 + at)) : __ldg(f + at);
+}
+
+__device__ __forceinline__ bool staged_ok(long long at, int count, unsigned site)      // floats of xprep_kernel's shared memory
+{
+#ifdef AXC_BOUNDS_CHECK
+    unsigned size;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(size));
+    return AXC_GLOBAL_OK(at, (long long)(size / 4) - count + 1, site);
+#else
+    return true;
+#endif
+}
 
 // K index of element i of chunk ch, or -1 where there is none
 __device__ __forceinline__ int k_of(const XGeom &g, int ch, int i)
@@ -244,7 +264,7 @@ __device__ void prep_filter_sums(const PrepParams &P, const DevQuant &q, int blo
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
             const int l = l0 + e * 8 + warp;
-            v[e] = (l < P.g.K && j < P.g.Cout) ? filter_value(P.filter, P.filter_u8, (size_t)l * P.g.Cout + j) : 0.0f;
+            v[e] = (l < P.g.K && j < P.g.Cout) ? filter_value(P.g, P.filter, P.filter_u8, (size_t)l * P.g.Cout + j) : 0.0f;
         }
     };
     fetch(0);
@@ -252,7 +272,7 @@ __device__ void prep_filter_sums(const PrepParams &P, const DevQuant &q, int blo
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
-            stage[(e * 8 + warp) * 32 + lane] = v[e];
+            if (staged_ok((e * 8 + warp) * 32 + lane, 1, 321u)) stage[(e * 8 + warp) * 32 + lane] = v[e];
             if (P.bcode && l0 + e * 8 + warp < P.g.K) codes += int(code_of(v[e], q.f_off, q.f_inv));
         }
         __syncthreads();
@@ -270,7 +290,7 @@ __device__ void prep_filter_sums(const PrepParams &P, const DevQuant &q, int blo
             for (; l < n; ++l) acc = __fadd_rn(acc, stage[l * 32 + lane]);
         }
     }
-    if (warp == 0 && j < P.g.Cout) P.bsum[j] = acc;
+    if (warp == 0 && j < P.g.Cout && AXC_SCRATCH_OK(P, P.bsum + j, 4, 322u)) P.bsum[j] = acc;
     if (P.bcode) {
         int *sums = reinterpret_cast<int *>(stage);
         __syncthreads();
@@ -278,7 +298,7 @@ __device__ void prep_filter_sums(const PrepParams &P, const DevQuant &q, int blo
         __syncthreads();
         if (warp == 0 && j < P.g.Cout) {
             for (int w = 1; w < 8; ++w) codes += sums[w * 32 + lane];
-            P.bcode[j] = codes;
+            if (AXC_SCRATCH_OK(P, P.bcode + j, 4, 323u)) P.bcode[j] = codes;
         }
     }
 }
@@ -316,15 +336,15 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
             const int j = nt * g.TNC + slot_channel(P.mode, slot), k = k_of(g, ch, i);
             unsigned row = kNull;
             if (k >= 0 && j < g.Cout) {
-                row = code_of(filter_value(P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
+                row = code_of(filter_value(g, P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
                 if (P.qf_debug) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(row);
             }
-            P.wrow[x] = uint16_t(row_address(P.mode, row) >> 4);
+            if (AXC_SCRATCH_OK(P, P.wrow + x, 2, 324u)) P.wrow[x] = uint16_t(row_address(P.mode, row) >> 4);
             if (P.mode != kXtabFull) {
                 // B operand half h, column n: channel (n>>1)*4 + 2h + (n&1); lane (n, t) holds elements 4t..4t+3
                 const int cj = slot_channel(P.mode, slot), t = i >> 2, h = (cj >> 1) & 1, n = (cj >> 2) * 2 + (cj & 1);
                 unsigned char *w = reinterpret_cast<unsigned char *>(P.wb + tc * 32 + n * 4 + t) + h * 4 + (i & 3);
-                *w = row == kNull ? 0 : (unsigned char)row;
+                if (AXC_SCRATCH_OK(P, w, 1, 325u)) *w = row == kNull ? 0 : (unsigned char)row;
             }
         }
         return;
@@ -338,6 +358,7 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
             const int w = x >> 8, a = (x & 255) ^ int(z);
             const int less = (P.mode == kXtabFull ? 128 * (a + w) * P.centred : a * w) + P.e_min;
             const int v = w < 256 ? int(__ldg(P.lut + a * 256 + w)) - less : 0;
+            if (!AXC_SCRATCH_OK(P, P.tt + x * (P.mode == kXtabFull ? 2 : 1), P.mode == kXtabFull ? 2 : 1, 326u)) continue;
             if (P.mode == kXtabFull) reinterpret_cast<uint16_t *>(P.tt)[x] = uint16_t(v % 255 + (v / 255) * 256);
             else P.tt[x] = (unsigned char)v;
         }
@@ -358,7 +379,8 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
     // centred tables: the sum of the codes of every staged pixel (z for one outside the image) behind the staged taps
     int *pix_codes = reinterpret_cast<int *>(prep_smem + P.RH * P.RW * P.pitch);
     if (P.acode && !g.im2col) {
-        for (int x = tid; x < P.RH * P.RW; x += 256) pix_codes[x] = 0;
+        for (int x = tid; x < P.RH * P.RW; x += 256)
+            if (staged_ok(P.RH * P.RW * P.pitch + x, 1, 327u)) pix_codes[x] = 0;
         __syncthreads();
     }
     if (P.vec) {
@@ -387,7 +409,8 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
                     at[u] = local[u] * P.pitch + c4 * 4;
                     if (unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W)) {
                         const int pix = (n * g.H + iy) * g.W + ix;
-                        if (P.input_u8) {
+                        if (!AXC_GLOBAL_OK((long long)pix * C4 + c4, (long long)planes * C4, 328u)) {
+                        } else if (P.input_u8) {
                             const uchar4 w = __ldg(reinterpret_cast<const uchar4 *>(P.input_u8 + (long long)pix * g.C) + c4);
                             v[u] = make_float4(float(int(w.x) - P.pad), float(int(w.y) - P.pad), float(int(w.z) - P.pad), float(int(w.w) - P.pad));
                         } else v[u] = __ldg(reinterpret_cast<const float4 *>(P.input + (long long)pix * g.C) + c4);
@@ -405,12 +428,12 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
             for (int u = 0; u < kBatch; ++u) {
                 v[u].x = max_keep_nan(v[u].x, P.in_floor); v[u].y = max_keep_nan(v[u].y, P.in_floor);
                 v[u].z = max_keep_nan(v[u].z, P.in_floor); v[u].w = max_keep_nan(v[u].w, P.in_floor);
-                if (at[u] >= 0) *reinterpret_cast<float4 *>(prep_smem + at[u]) = v[u];
+                if (at[u] >= 0 && staged_ok(at[u], 4, 329u)) *reinterpret_cast<float4 *>(prep_smem + at[u]) = v[u];
                 if (code_at[u] >= 0 || (P.acode && at[u] >= 0 && !g.im2col)) {
                     const unsigned w = code_of(v[u].x, q.in_off, q.in_inv) | code_of(v[u].y, q.in_off, q.in_inv) << 8 |
                                        code_of(v[u].z, q.in_off, q.in_inv) << 16 | code_of(v[u].w, q.in_off, q.in_inv) << 24;
-                    if (code_at[u] >= 0) reinterpret_cast<unsigned *>(P.codes)[(unsigned)code_at[u]] = w ^ zz;
-                    if (P.acode) atomicAdd(pix_codes + local[u], int(__dp4a(w, 0x01010101u, 0u)));
+                    if (code_at[u] >= 0 && AXC_SCRATCH_OK(P, P.codes + (size_t)(unsigned)code_at[u] * 4, 4, 330u)) reinterpret_cast<unsigned *>(P.codes)[(unsigned)code_at[u]] = w ^ zz;
+                    if (P.acode && staged_ok(P.RH * P.RW * P.pitch + local[u], 1, 331u)) atomicAdd(pix_codes + local[u], int(__dp4a(w, 0x01010101u, 0u)));
                 }
             }
         }
@@ -421,11 +444,11 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
             const int iy = iy0 + ry, ix = ix0 + rx;
             const bool inside = unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W);
             const long long pix = ((long long)n * g.H + iy) * g.W + ix;
-            float v = !inside ? 0.0f : P.input_u8 ? float(int(__ldg(P.input_u8 + pix * g.C + c)) - P.pad) : __ldg(P.input + pix * g.C + c);
+            float v = !inside || !AXC_GLOBAL_OK(pix * g.C + c, (long long)planes * g.C, 332u) ? 0.0f : P.input_u8 ? float(int(__ldg(P.input_u8 + pix * g.C + c)) - P.pad) : __ldg(P.input + pix * g.C + c);
             v = max_keep_nan(v, P.in_floor);
-            prep_smem[(ry * P.RW + rx) * P.pitch + c] = v;
-            if (P.acode && !g.im2col) atomicAdd(pix_codes + ry * P.RW + rx, int(code_of(v, q.in_off, q.in_inv)));
-            if (inside && ry < own_h && rx < own_w && !g.im2col)
+            if (staged_ok((ry * P.RW + rx) * P.pitch + c, 1, 333u)) prep_smem[(ry * P.RW + rx) * P.pitch + c] = v;
+            if (P.acode && !g.im2col && staged_ok(P.RH * P.RW * P.pitch + ry * P.RW + rx, 1, 334u)) atomicAdd(pix_codes + ry * P.RW + rx, int(code_of(v, q.in_off, q.in_inv)));
+            if (inside && ry < own_h && rx < own_w && !g.im2col && AXC_SCRATCH_OK(P, P.codes + ((long long)(c >> 4) * planes + pix) * 16 + (c & 15), 1, 335u))
                 P.codes[((long long)(c >> 4) * planes + pix) * 16 + (c & 15)] = (unsigned char)(code_of(v, q.in_off, q.in_inv) ^ z);
         }
     }
@@ -445,6 +468,7 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
             for (int ky = 0; ky < g.KH; ++ky)
                 for (int kx = 0; kx < g.KW; ++kx) {
                     const float *src = prep_smem + ((ly * g.sh + ky * g.dh) * P.RW + lx * g.sw + kx * g.dw) * P.pitch;
+                    if (!staged_ok(src - prep_smem, g.C, 336u)) continue;
                     if (P.vec) {
 #pragma unroll 4
                         for (int c = 0; c < g.C; c += 4) {
@@ -463,6 +487,7 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
             for (int ky = 0; ky < g.KH; ++ky)
                 for (int kx = 0; kx < g.KW; ++kx) {
                     const float *src = prep_smem + ((ly * g.sh + ky * g.dh) * P.RW + lx * g.sw + kx * g.dw) * P.pitch;
+                    if (!staged_ok(src - prep_smem, g.C, 337u)) continue;
                     for (int c = 0; c < g.C; ++c) {
                         const float v = src[c];
                         s = __fadd_rn(s, v);
@@ -472,7 +497,7 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
                         w[0] = __funnelshift_r(w[0], w[1], 8); w[1] = __funnelshift_r(w[1], w[2], 8);
                         w[2] = __funnelshift_r(w[2], w[3], 8); w[3] = (w[3] >> 8) | byte;
                         if (++i == 16) {
-                            *dst = make_uint4(w[0], w[1], w[2], w[3]);
+                            if (AXC_SCRATCH_OK(P, dst, 16, 338u)) *dst = make_uint4(w[0], w[1], w[2], w[3]);
                             dst += g.M;
                             i = 0;
                         }
@@ -483,11 +508,11 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
                     w[0] = __funnelshift_r(w[0], w[1], 8); w[1] = __funnelshift_r(w[1], w[2], 8);
                     w[2] = __funnelshift_r(w[2], w[3], 8); w[3] >>= 8;
                 }
-                *dst = make_uint4(w[0], w[1], w[2], w[3]);
+                if (AXC_SCRATCH_OK(P, dst, 16, 339u)) *dst = make_uint4(w[0], w[1], w[2], w[3]);
             }
         }
-        P.asum[m] = s;
-        if (P.acode) P.acode[m] = codes;
+        if (AXC_SCRATCH_OK(P, P.asum + m, 4, 340u)) P.asum[m] = s;
+        if (P.acode && AXC_SCRATCH_OK(P, P.acode + m, 4, 341u)) P.acode[m] = codes;
     }
 }
 
@@ -507,6 +532,7 @@ struct ExpandParams {
     uint2 *wb;
     uint8_t *qf_debug;
     PlanHeader *hdr;
+    long long scratch_bytes;
 };
 
 // xt[channel tile][chunk][row a][piece kk][16 bytes], kk = octet * 8 + k.  The table's rows (one per weight) lie in shared memory.
@@ -548,14 +574,16 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
             const int k = k_of(g, ch, elem), cj = slot_channel(MODE, slot), j = nt * TNC + cj;
             unsigned row = kNull;
             if (k >= 0 && j < g.Cout) {
-                row = code_of(filter_value(P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
+                row = code_of(filter_value(g, P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
                 if (P.qf_debug) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(row);
             }
-            asm volatile("st.shared.u16 [%0], %1;" ::"r"(lists + parity * (16u * TNC * 2u) + unsigned(kk * TNC + slot) * 2u), "h"((unsigned short)row) : "memory");
+            if (AXC_SHARED_OK(lists + parity * (16u * TNC * 2u) + unsigned(kk * TNC + slot) * 2u, 2u, lists, bar, 350u))
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(lists + parity * (16u * TNC * 2u) + unsigned(kk * TNC + slot) * 2u), "h"((unsigned short)row) : "memory");
             if (MODE != kXtabFull) {
                 // exact products, B operand half h, column n: channel (n>>1)*4 + 2h + (n&1); lane (n, t) holds elements 4t..4t+3
                 const int t = elem >> 2, h = (cj >> 1) & 1, n = (cj >> 2) * 2 + (cj & 1);
-                reinterpret_cast<unsigned char *>(P.wb + (size_t)tc * 32 + n * 4 + t)[h * 4 + (elem & 3)] = row == kNull ? 0 : (unsigned char)row;
+                unsigned char *w = reinterpret_cast<unsigned char *>(P.wb + (size_t)tc * 32 + n * 4 + t) + h * 4 + (elem & 3);
+                if (AXC_SCRATCH_OK(P, w, 1, 351u)) *w = row == kNull ? 0 : (unsigned char)row;
             }
         }
         __syncthreads();                                           // (the other list's readers are a chunk behind this barrier)
@@ -572,6 +600,7 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
                 for (int s = 0; s < 8; ++s) v[s4 * 8 + s] = lds32(tab + ((s & 1) ? l4[s >> 1] >> 16 : l4[s >> 1] & 0xFFFFu) * kRow + word * 4u);
             }
             uint4 *dst = reinterpret_cast<uint4 *>(P.xt + (size_t)tc * 65536u) + o * 8 + kidx;
+            if (!AXC_SCRATCH_OK(P, dst, 255 * 256 + 16, 352u)) continue;      // the rows a of this piece
             if (MODE == kXtabFull) {
                 const unsigned a = word * 2u;
                 dst[(a ^ z) * 16u] = make_uint4(prmt<0x5410>(v[0], v[1]), prmt<0x5410>(v[2], v[3]), prmt<0x5410>(v[4], v[5]), prmt<0x5410>(v[6], v[7]));
@@ -608,6 +637,7 @@ struct XParams {
     const unsigned char *xt;    // expanded tables [channel tile][chunk][256][2 octets][8][16], or NULL: built by the CTAs
     const float *asum, *bsum;
     const PlanHeader *hdr;
+    long long scratch_bytes;
     float *output;              // NULL: integer sums only
     int32_t *acc_out;
     int32_t *partial;           // K split over CTAs: integer sums are added here
@@ -772,7 +802,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
             if (b_unit >= units) return;
             build_unit();
         }
-        wq_next = __ldg(b_rows);
+        if (AXC_SCRATCH_OK(P, b_rows, 16, 312u)) wq_next = __ldg(b_rows);
         b_rows += 8 * HV;
         --b_left;
     };
@@ -825,6 +855,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
             x_left = c_end - c_begin;
             x_src = P.xt + ((size_t)nt * g.chunks + c_begin) * 65536u;
         }
+        if (!AXC_SCRATCH_OK(P, x_src, 65536, 311u)) { ok = false; return; }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tab_full + buf * 8), "r"(65536u) : "memory");
         bulk_copy(kTab * (1u + buf), x_src, 65536u, tab_full + buf * 8);
@@ -976,11 +1007,11 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
             for (int e = 0; e < 4; ++e) acc[i][e] = 0;
         const uint2 *wbp = P.wb + ((size_t)nt * g.chunks + c_begin) * 32 + lane;
         uint2 wb_next = make_uint2(0, 0);
-        if (MODE != kXtabFull) wb_next = __ldg(wbp);
+        if (MODE != kXtabFull && AXC_SCRATCH_OK(P, wbp, 8, 316u)) wb_next = __ldg(wbp);
         for (int c = c_begin; c < c_end; ++c, ++chunk) {
             const uint2 wb = wb_next;
             wbp += 32;
-            if (MODE != kXtabFull && c + 1 < c_end) wb_next = __ldg(wbp);
+            if (MODE != kXtabFull && c + 1 < c_end && AXC_SCRATCH_OK(P, wbp, 8, 317u)) wb_next = __ldg(wbp);
             if (PRE) {
                 const unsigned st = chunk & 1u;
                 mbar_wait(tab_full + st * 8, (chunk >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
@@ -1018,7 +1049,9 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         constexpr int EB = kAcc < 4 ? kAcc : 4;
         constexpr int kStep = MODE == kXtabFull ? 16 : 8;          // pixels from fragment to fragment
         const int first = warp * (NB * 8) + gr + (MODE == kXtabFull ? (t >> 1) * 8 : 0);
-        const int left = chan ? g.M - m0 - first : 0;              // > kStep * i: fragment i has a pixel
+        int left = chan ? g.M - m0 - first : 0;                    // > kStep * i: fragment i has a pixel
+        if (left > 0 && !P.partial && !AXC_SCRATCH_OK(P, P.asum + g.M - 1, 4, 318u)) left = 0;
+        if (left > 0 && P.acode && !AXC_SCRATCH_OK(P, P.acode + g.M - 1, 4, 319u)) left = 0;
         const long long at0 = (long long)(m0 + first) * g.Cout + j0;
         const int row = kStep * g.Cout;
         if (P.plain && whole && P.acc_out) {
@@ -1080,6 +1113,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
                 for (int e = 0; e < 4; ++e) {
                     if (j0 + e >= g.Cout) continue;
                     if (P.partial) {
+                        if (!AXC_SCRATCH_OK(P, P.partial + at + e, 4, 342u)) continue;
                         atomicAdd(P.partial + at + e, acc[i][e]);
                         continue;
                     }
@@ -1113,6 +1147,7 @@ __global__ void __launch_bounds__(256) xfinal_kernel(const XParams P)
     const long long total = (long long)P.g.M * P.g.Cout;
     for (long long x = (long long)blockIdx.x * 256 + threadIdx.x; x < total; x += (long long)gridDim.x * 256) {
         const int m = int(x / P.g.Cout), j = int(x - (long long)m * P.g.Cout);
+        if (!AXC_SCRATCH_OK(P, P.partial + x, 4, 360u) || !AXC_SCRATCH_OK(P, P.asum + m, 4, 361u)) continue;
         const int tot = P.partial[x] + P.k_e_min + (P.acode ? P.a_coef * __ldg(P.acode + m) + P.b_coef * __ldg(P.bcode + j) : 0);
         float y = dequantise(Q, tot, __ldg(P.asum + m), __fmul_rn(Q.m1, __ldg(P.bsum + j)));
         if (P.bias) y = __fadd_rn(y, __ldg(P.bias + j));
@@ -1357,6 +1392,7 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     A.asum = reinterpret_cast<float *>(scratch + L.asum); A.bsum = reinterpret_cast<float *>(scratch + L.bsum);
     A.qf_debug = dbg ? dbg->qfilter : nullptr;
     A.hdr = reinterpret_cast<PlanHeader *>(scratch);
+    A.scratch_bytes = P.scratch_bytes = (long long)L.total;
     A.TH = t.TH; A.TW = t.TW; A.RH = t.RH; A.RW = t.RW; A.pitch = t.pitch; A.vec = t.vec;
     A.tiles_y = (g.OH + t.TH - 1) / t.TH; A.tiles_x = (g.OW + t.TW - 1) / t.TW;
     A.blocks_sum = (g.Cout + 31) / 32;
@@ -1378,7 +1414,7 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     if (cf.pre) {
         ExpandParams E;
         E.g = x; E.filter = filter; E.filter_u8 = A.filter_u8; E.rows = reinterpret_cast<const unsigned char *>(lut_dev + 65536); E.ranges = ranges_dev; E.host_q = A.host_q;
-        E.xt = scratch + L.xt; E.wb = A.wb; E.qf_debug = A.qf_debug; E.hdr = A.hdr;
+        E.xt = scratch + L.xt; E.wb = A.wb; E.qf_debug = A.qf_debug; E.hdr = A.hdr; E.scratch_bytes = A.scratch_bytes;
         const int rc = mode == kXtabFull ? launch_expand<kXtabFull>(E, di, stream) : launch_expand<kXtabByte>(E, di, stream);
         if (rc) return rc;
     }
