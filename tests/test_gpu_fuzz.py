@@ -28,6 +28,7 @@ def _ranges(rng, x, f, loose):
 def test_dense_random_cases(built):
     import torch
     import tf_approximate_b200 as ax
+    from tf_approximate_b200 import ops
     rng = np.random.Generator(np.random.PCG64(7001 + SEED))
     tables = [cases.make_table(("noisy", 71)), cases.make_table(("truncated",)), cases.make_table(("exact",))]
     handles = [ax.Table(array=t) for t in tables]
@@ -64,6 +65,12 @@ def test_dense_random_cases(built):
         y, dbg = ax.approx_conv2d_with_min_max_vars(xd, fd, *mm, [1, sh, sw, 1], 8, handles[ti], pad,
                                                     dilations=[1, dh, dw, 1], debug=True, input_relu=input_relu, **opts)
         what = (it, n, h, w, c, kh, kw, co, sh, sw, dh, dw, pad, ti, mode, input_relu)
+        if dbg["plan"]["route"]["kernels"] == "expanded":       # the scheduled kernel as well: a workspace of the plan's size selects it
+            ws = torch.zeros(ops.workspace_bytes(x.shape, f.shape, [1, sh, sw, 1], pad, (1, dh, dw, 1)), dtype=torch.uint8, device="cuda")
+            y2, dbg2 = ax.approx_conv2d_with_min_max_vars(xd, fd, *mm, [1, sh, sw, 1], 8, handles[ti], pad, dilations=[1, dh, dw, 1],
+                                                          debug=True, input_relu=input_relu, workspace=ws)
+            assert dbg2["plan"]["route"]["kernels"] == "plan" and torch.equal(dbg2["acc"], dbg["acc"]), what
+            assert torch.equal(y2.view(torch.int32), y.view(torch.int32)), what
         if mode != 2:
             assert np.array_equal(dbg["acc"].cpu().numpy(), ref["acc"]), what
         assert np.array_equal(y.cpu().numpy().view(np.uint32), ref[key].view(np.uint32)), what

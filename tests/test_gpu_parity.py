@@ -35,15 +35,20 @@ def linf(a, ref):
     return float(np.abs(a - ref).max() / (m if m > 0 else 1.0))
 
 
-def run_dense(ax, lut, x, f, mm, stride, dil, pad, accumulate="exact"):
+def run_dense(ax, lut, x, f, mm, stride, dil, pad, accumulate="exact", scheduled=False):
     import torch
+    from tf_approximate_b200 import ops
     t = ax.Table(array=lut)
+    ws = None
+    if scheduled:          # a buffer of the plan's size belongs to the plan
+        ws = torch.zeros(ops.workspace_bytes(x.shape, f.shape, [1, stride[0], stride[1], 1], pad, (1, dil[0], dil[1], 1)), dtype=torch.uint8, device="cuda")
     y, dbg = ax.approx_conv2d_with_min_max_vars(torch.from_numpy(x).cuda(), torch.from_numpy(f).cuda(), *mm,
                                                 strides=[1, stride[0], stride[1], 1], num_bits=8, mul_map_file=t,
                                                 padding=pad, dilations=[1, dil[0], dil[1], 1], debug=True,
-                                                accumulate=accumulate)
+                                                accumulate=accumulate, workspace=ws)
     torch.cuda.synchronize()
     assert dbg["plan"]["status"] == 0
+    assert not scheduled or dbg["plan"]["route"]["kernels"] == "plan"
     return y.cpu().numpy(), {k: (v if k == "plan" else v.cpu().numpy()) for k, v in dbg.items()}
 
 
@@ -67,6 +72,9 @@ def check_dense(ax, lut, x, f, mm, stride=(1, 1), dil=(1, 1), pad="SAME"):
     if kh * kw * c <= 256:
         assert np.array_equal(y.view(np.uint32), ref["out_ref"].view(np.uint32))
         assert linf(y, ref["out_ref"]) < TOL_REF
+    if dbg["plan"]["route"]["kernels"] == "expanded":
+        ys, dbgs = run_dense(ax, lut, x, f, mm, stride, dil, pad, scheduled=True)
+        assert np.array_equal(dbgs["acc"], ref["acc"]) and np.array_equal(ys.view(np.uint32), ref["out_exact"].view(np.uint32))
     # the reference's own arithmetic (fp32 running total in K order): its bits, whatever K
     y_ro, dbg_ro = run_dense(ax, lut, x, f, mm, stride, dil, pad, accumulate="reference")
     assert np.array_equal(y_ro.view(np.uint32), ref["out_ref"].view(np.uint32))
@@ -197,8 +205,10 @@ def test_config_shapes_within_tolerance_of_reference_order(ax, tspec, shape):
     """Default (exact-sum) mode against the reference-order result on the configurations' shapes: within 1e-5,
     and the share of outputs on which the reference rounded is reported.  With the truncated table every entry
     is a multiple of 64, so the fp32 running total cannot round below K = 16 512 and accumulate="reference" is
-    served by the scheduled kernel too (its plan is present in the workspace afterwards)."""
+    served by the kernels of the exact sum too: the expanded tables, or with a plan's workspace the scheduled kernel (its
+    plan is present there afterwards)."""
     import torch
+    from tf_approximate_b200 import ops
     n, h, w, c, kh, kw, co, s = shape
     rng = np.random.Generator(np.random.PCG64(900 + c + co))
     x = np.maximum(rng.uniform(-1, 1, (n, h, w, c)), 0 if c > 64 else -1).astype(np.float32)   # deeper layers see ReLU outputs
@@ -211,11 +221,14 @@ def test_config_shapes_within_tolerance_of_reference_order(ax, tspec, shape):
     assert linf(y, ref["out_ref"]) < TOL_REF
     if tspec[0] == "truncated":
         assert share == 0.0
-        f2 = torch.from_numpy(f).cuda().clone()        # a filter storage of its own: a fresh workspace
-        y2, dbg2 = ax.approx_conv2d_with_min_max_vars(torch.from_numpy(x).cuda(), f2, *mm, [1, s, s, 1], 8,
-                                                      ax.Table(array=lut), "SAME", debug=True, accumulate="reference")
-        assert dbg2["plan"]["steps_per_mille"] >= 1000 and dbg2["plan"]["fallback"] == 0
-        assert np.array_equal(y2.cpu().numpy().view(np.uint32), ref["out_ref"].view(np.uint32))
+        ws = torch.zeros(ops.workspace_bytes(x.shape, f.shape, [1, s, s, 1], "SAME"), dtype=torch.uint8, device="cuda")
+        for workspace, kernels in ((None, "expanded"), (ws, "plan")):
+            y2, dbg2 = ax.approx_conv2d_with_min_max_vars(torch.from_numpy(x).cuda(), torch.from_numpy(f).cuda(), *mm, [1, s, s, 1], 8,
+                                                          ax.Table(array=lut), "SAME", debug=True, accumulate="reference", workspace=workspace)
+            assert dbg2["plan"]["route"]["kernels"] == kernels
+            assert dbg2["plan"]["rebuilt"] == (kernels == "plan") and dbg2["plan"]["fallback"] == 0
+            assert kernels == "expanded" or 1000 <= dbg2["plan"]["steps_per_mille"] < 2000
+            assert np.array_equal(y2.cpu().numpy().view(np.uint32), ref["out_ref"].view(np.uint32))
 
 
 def test_out_of_range_inputs_saturate(ax):
@@ -342,16 +355,19 @@ def test_first_use_of_a_table_on_a_non_blocking_stream(ax):
 
 
 def test_host_threads_call_concurrently(ax):
-    """Four host threads, each with its own table handle, stream and workspace, call the op at the same time (ctypes
+    """Eight host threads, each with its own table handle, stream and workspace, call the op at the same time (ctypes
     releases the interpreter lock during a call): every result equals the one computed alone."""
     import threading
     import torch
     rng = np.random.Generator(np.random.PCG64(44))
     jobs = []
-    for i in range(4):
-        x = torch.from_numpy(rng.uniform(-1, 1, (2, 14 + i, 14, 16)).astype(np.float32)).cuda()
-        f = torch.from_numpy(rng.normal(0, 0.1, (3, 3, 16, 32 * (i + 1))).astype(np.float32)).cuda()
-        lut = cases.make_table(("noisy", 600 + i))
+    for i in range(8):                      # four on the scheduled kernel, four on the expanded tables (every form of entry)
+        c = 16 if i < 4 else 64
+        x = torch.from_numpy(rng.uniform(-1, 1, (2, 14 + i, 14, c)).astype(np.float32)).cuda()
+        f = torch.from_numpy(rng.normal(0, 0.1, (3, 3, c, 32 * (i % 4 + 1) if i < 4 else 64)).astype(np.float32)).cuda()
+        lut = cases.make_table({5: ("truncated",), 6: ("exact",)}.get(i, ("noisy", 600 + i)))
+        _, dbg = ax.approx_conv2d_with_min_max_vars(x, f, -1.0, 1.0, -0.4, 0.4, [1, 1, 1, 1], 8, ax.Table(array=lut), "SAME", debug=True)
+        assert dbg["plan"]["route"]["kernels"] == ("expanded" if i >= 3 else "plan")
         want = ax.approx_conv2d_with_min_max_vars(x, f, -1.0, 1.0, -0.4, 0.4, [1, 1, 1, 1], 8, ax.Table(array=lut), "SAME")
         jobs.append((x, f, lut, want))
     torch.cuda.synchronize()

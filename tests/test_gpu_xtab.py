@@ -1,6 +1,7 @@
-"""GPU: the expanded-table kernels against the CPU checker, bit for bit, at the sizes where they can go wrong: edges of
-pixel tiles (256 to 3072 pixels), channel tiles (8 / 16), K chunks (16), codes in pixel order and as im2col rows, K split
-over CTAs, tables built by the CTAs and taken from global memory, and every form a table can be kept in."""
+"""GPU: the expanded-table kernels against the CPU checker, bit for bit, at the sizes where they can go wrong: channel tiles
+(8 / 16), K chunks (16), codes in pixel order and as im2col rows, K split over CTAs, tables built by the CTAs and taken from global
+memory, and every form a table can be kept in, with small pixel tiles (SHAPES); edges of the larger ones and CTAs that go from
+unit to unit (TILES)."""
 import numpy as np
 import pytest
 
@@ -11,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 def tables(ax):
     rng = np.random.Generator(np.random.PCG64(8))
-    return {"exact": ax.exact_table(), "byte": ax.truncated_table(), "digits": rng.integers(0, 65280, 65536).astype(np.uint16),
+    return {"exact": ax.exact_table(), "offset": (ax.exact_table() + 7).astype(np.uint16), "byte": ax.truncated_table(), "digits": rng.integers(0, 65280, 65536).astype(np.uint16),
             "centred": ax.noisy_table(3), "neither": rng.integers(0, 65536, 65536).astype(np.uint16)}
 
 
@@ -30,7 +31,7 @@ SHAPES = [
 ]
 
 
-@pytest.mark.parametrize("kind", ["exact", "byte", "digits", "centred", "neither"])
+@pytest.mark.parametrize("kind", ["exact", "offset", "byte", "digits", "centred", "neither"])
 @pytest.mark.parametrize("shape", SHAPES, ids=["-".join(str(v) for v in s) for s in SHAPES])
 def test_expanded_tables_match_the_checker(built, shape, kind):
     import torch
@@ -60,10 +61,60 @@ def test_expanded_tables_match_the_checker(built, shape, kind):
     bias, res = torch.randn(co, device="cuda", generator=g), torch.randn(want.shape, device="cuda", generator=g)
     fused = call(*mm, bias=bias, residual=res, relu=True)
     assert torch.equal(fused.view(torch.int32), torch.relu(want + bias + res).view(torch.int32))
-    # the plan-based kernels, which a workspace of their size selects (unless it has room for the expanded tables as well)
+    # the plan-based kernels, which a workspace of their size selects
     ws = torch.zeros(ops.workspace_bytes((n, h, w, c), (kh, kw, c, co), [1, s, s, 1], pad, (1, d, d, 1)), dtype=torch.uint8, device="cuda")
-    a, b = call(*mm, input_relu=True), call(*mm, input_relu=True, workspace=ws)
+    (a, da), (b, db) = call(*mm, input_relu=True, debug=True), call(*mm, input_relu=True, workspace=ws, debug=True)
     assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    assert da["plan"]["route"]["kernels"] == ("plan" if kind == "neither" else "expanded") and db["plan"]["route"]["kernels"] == "plan"
+
+
+# n, h, w, c, k, cout, form, pixels per tile, tables from global memory, K split; at least as many units as fill 148 CTAs more
+# than once, and a ragged last tile and channel tile
+TILES = [
+    (40, 97, 97, 20, 1, 8, "byte", 1024, True, False),
+    (12, 149, 149, 20, 1, 24, "byte", 2048, True, False),
+    (20, 97, 97, 32, 3, 8, "byte", 2048, True, True),
+    (40, 97, 97, 16, 1, 8, "byte", 1024, False, False),
+    (12, 149, 149, 16, 1, 24, "byte", 2048, False, False),
+    (12, 149, 149, 16, 1, 24, "exact", 2048, False, False),
+    (40, 97, 97, 64, 1, 13, "digits", 1024, True, False),
+    (12, 149, 149, 20, 1, 13, "digits", 2048, True, False),
+    (12, 149, 149, 20, 1, 13, "centred", 2048, True, False),
+    (12, 149, 149, 16, 1, 13, "digits", 2048, False, False),
+    (40, 97, 97, 16, 1, 13, "digits", 3072, True, False),
+    (40, 97, 97, 16, 1, 13, "centred", 3072, True, False),
+]
+
+
+@pytest.mark.parametrize("shape", TILES, ids=["-".join(str(v) for v in s) for s in TILES])
+def test_large_tiles_and_several_units_per_cta(built, shape):
+    import torch
+    import tf_approximate_b200 as ax
+    n, h, w, c, k, co, kind, tile, in_global, split = shape
+    lut = tables(ax)[kind]
+    t = ax.Table(array=lut)
+    rng = np.random.Generator(np.random.PCG64(sum(shape[:6])))
+    x = rng.uniform(-1, 1, (n, h, w, c)).astype(np.float32)
+    f = rng.normal(0, 0.1, (k, k, c, co)).astype(np.float32)
+    mm = (-0.7, 1.0, float(f.min()), float(f.max()))
+    d = O.desc(n, h, w, c, k, k, co)
+    ref = O.conv2d(d, lut, x, f, *mm, want=("out_exact", "acc"))
+    xd, fd = torch.from_numpy(x).cuda(), torch.from_numpy(f).cuda()
+    y, dbg = ax.approx_conv2d_with_min_max_vars(xd, fd, *mm, [1, 1, 1, 1], 8, t, "SAME", debug=True)
+    route = dbg["plan"]["route"]
+    assert dbg["plan"]["status"] == 0
+    assert (route["kernels"], route["tile"], route["tables_in_global_memory"], route["splits"] > 1) == ("expanded", tile, in_global, split)
+    units = -(-n * h * w // tile) * -(-co // (16 if kind in ("byte", "exact") else 8)) * route["splits"]
+    assert units > 148 and n * h * w % tile
+    assert np.array_equal(dbg["acc"].cpu().numpy(), ref["acc"])
+    want = torch.from_numpy(ref["out_exact"]).cuda()
+    assert torch.equal(y.view(torch.int32), want.view(torch.int32))
+    res = torch.flip(want, [0])
+    fused = ax.approx_conv2d_with_min_max_vars(xd, fd, *mm, [1, 1, 1, 1], 8, t, "SAME", residual=res, relu=True)
+    assert torch.equal(fused.view(torch.int32), torch.relu(want + res).view(torch.int32))
+    a, b = rng.integers(0, 256, x.shape).astype(np.uint8), rng.integers(0, 256, f.shape).astype(np.uint8)
+    q, _, _ = ax.ax_conv2d(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), -1.0, 2.0, -0.5, 0.5, [1, 1, 1, 1], "SAME", table=t, ax_tune=False)
+    assert np.array_equal(q.cpu().numpy(), O.qconv2d(d, lut, a, b, O.quantized_zero_point(-1.0, 2.0), O.quantized_zero_point(-0.5, 0.5)))
 
 
 def test_a_table_without_a_form_keeps_its_plan(built):
@@ -101,25 +152,32 @@ def test_unusual_values_and_addresses(built):
 
 Q_SHAPES = [  # n, h, w, c, k, cout, stride, padding, input range, filter range
     (2, 28, 28, 64, 3, 96, 1, "SAME", (-1.0, 2.0), (-0.5, 0.5)),
-    (3, 21, 23, 30, 3, 45, 2, "SAME", (0.5, 2.0), (-0.5, 0.25)),        # zero point of the input below 0: padded taps wrap
-    (1, 50, 50, 3, 5, 50, 1, "VALID", (0.0, 1.0), (0.0, 1.0)),          # im2col rows, no zero-point terms
+    (9, 21, 23, 30, 3, 45, 2, "SAME", (0.5, 2.0), (-0.5, 0.25)),        # zero point of the input below 0: padded taps wrap
+    (2, 50, 50, 3, 5, 50, 1, "VALID", (0.0, 1.0), (0.0, 1.0)),          # im2col rows, no zero-point terms
     (5, 50, 51, 32, 3, 64, 1, "SAME", (-3.0, -1.0), (-1.0, 3.0)),
 ]
 
 
-@pytest.mark.parametrize("kind", ["exact", "byte", "digits", "centred"])
+@pytest.mark.parametrize("kind", ["exact", "offset", "byte", "digits", "centred"])
 @pytest.mark.parametrize("shape", Q_SHAPES, ids=["-".join(str(v) for v in s[:8]) for s in Q_SHAPES])
 def test_quantised_operands(built, shape, kind):
     """uint8 operands on the expanded tables, the zero-point terms added at the end, against the checker's functor."""
+    import ctypes as C
     import torch
     import tf_approximate_b200 as ax
+    from tf_approximate_b200 import _lib
     n, h, w, c, k, co, s, pad, ri, rf = shape
     lut = tables(ax)[kind]
     rng = np.random.Generator(np.random.PCG64(77 + c))
     a = rng.integers(0, 256, (n, h, w, c)).astype(np.uint8)
     b = rng.integers(0, 256, (k, k, c, co)).astype(np.uint8)
     zi, zf = O.quantized_zero_point(*ri), O.quantized_zero_point(*rf)
+    t = ax.Table(array=lut)
+    size, out = C.c_size_t(), (C.c_int32 * 4)()
+    desc = _lib.ConvDesc(n, h, w, c, k, k, c, co, s, s, 1, 1, 0 if pad == "SAME" else 1, 0, 0, 1)
+    assert _lib.load().axc_qconv2d_fast_workspace_bytes(t.handle, C.byref(desc), C.byref(size)) == 0 and size.value > 0
+    assert _lib.load().axc_qconv2d_route(t.handle, C.byref(desc), size.value, out) == 0 and out[0] == 3
     ref = O.qconv2d(O.desc(n, h, w, c, k, k, co, (s, s), (1, 1), pad), lut, a, b, zi, zf)
-    y, _, _ = ax.ax_conv2d(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), *ri, *rf, [1, s, s, 1], pad, table=ax.Table(array=lut),
+    y, _, _ = ax.ax_conv2d(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), *ri, *rf, [1, s, s, 1], pad, table=t,
                            ax_tune=False)
     assert np.array_equal(y.cpu().numpy(), ref)
