@@ -148,7 +148,7 @@ def test_exact_table_matches_reference_test_table():
     assert np.array_equal(O.exact_table(), ax.exact_table())
 
 
-@pytest.mark.skipif(not os.path.isdir(REF_ROOT), reason="no reference checkout on this machine")
+@pytest.mark.skipif(not os.path.isdir(os.path.join(REF_ROOT, "tf2")), reason="no reference checkout on this machine")
 def test_table_loader_reads_reference_files(built):
     digests = json.load(open(os.path.join(GDIR, "tables.json")))
     for rel, info in digests.items():
