@@ -21,8 +21,9 @@
 //
 // Bound: the shared-memory pipe, 64 lookups (16-bit) or 128 lookups (8-bit) per clock and SM, less what the expansion costs:
 // 32 KiB read and 32 KiB written per 8 K elements and channel group, 512 clocks against one clock per pixel of the tile for the
-// lookups - hence tiles of up to 2048 pixels.  Measured on a B200: LDS.128 alone 4.02 clocks per warp instruction, LDS.128 + MMA
-// 4.05 (the MMA pipe is half idle), against 4.50 with eight dp2a in the MMA's place.  A 16-bit lookup per lane and
+// lookups - hence tiles of up to 2048 pixels, 3072 with two-digit entries and tables from global memory.  Measured on a B200:
+// LDS.128 alone 4.02 clocks per warp instruction, LDS.128 + MMA 4.05 (the MMA pipe is half idle), against 4.50 with eight dp2a
+// in the MMA's place.  A 16-bit lookup per lane and
 // instruction (axc_sched.cu) cannot pass 32 per clock.
 //
 //   xprep_kernel   one pass over the input: 8-bit codes in pixel order (or the im2col rows where the channel count would
@@ -62,7 +63,7 @@ constexpr int kNull = 256;                     // table row of a weight that doe
 static_assert(kRowsLow + kLowRows * 512u == kTab && kRowsHigh + (257u - kLowRows) * 512u <= kWindowEnd, "shared window");
 constexpr int kWaitPolls = 1 << 20;
 constexpr size_t kPartialMax = 64u << 20;      // integer sums of a call whose K is split over CTAs
-constexpr double kXtabMinLookups = 8e6;
+constexpr double kXtabMinLookups = 8e6;        // (xtab_scratch_bytes)
 constexpr size_t kXtMax = 640u << 20;          // expanded tables in global memory
 constexpr int kModelSms = 148;                 // what the scratch size is computed for
 
@@ -128,12 +129,15 @@ __device__ int g_wait_polls[2] = {kWaitPolls, kWaitPolls};
 // whatever the tables hold), waits for its own copies in flight and leaves 3 in the header's status.
 __device__ __forceinline__ void mbar_wait(unsigned bar, unsigned parity, bool &ok, int polls)
 {
+#ifdef AXC_BOUNDS_CHECK
+    if (polls <= 0) ok = false;
+#endif
     for (int it = 0; ok; ++it) {
-        if (it >= polls) { ok = false; return; }
         unsigned done;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
         if (done) return;
+        if (it >= polls) ok = false;
     }
 }
 // The end of a kernel that gave up: the phase that a copy in flight completes.
@@ -679,14 +683,14 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
     unsigned dyn_size;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_size));
     const unsigned bars = (dyn0 + 15u) & ~15u;
-    const unsigned tab_full = bars, tab_empty = bars + 16u, rows_full = bars + 32u, copies = bars + 40u;
+    const unsigned tab_full = bars, tab_empty = bars + 16u, rows_full = bars + 32u, asked = bars + 40u;
     pdl_wait();
-    if (copies + 4u > kCodes || dyn0 + dyn_size < kWindowEnd) {
+    if (asked + 4u > kCodes || dyn0 + dyn_size < kWindowEnd) {
         if (tid == 0) atomicExch(const_cast<int *>(&P.hdr->status), 2);      // (xprep_kernel, which clears it, is complete)
         return;
     }
     if (tid == 0) {
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(copies), "r"(0u) : "memory");
+        if (PRE) asm volatile("st.shared.u32 [%0], %1;" ::"r"(asked), "r"(0xFFFFFFFFu) : "memory");
         for (int s = 0; s < 2; ++s) { mbar_init(tab_full + s * 8, PRE ? 1 : kWarps); mbar_init(tab_empty + s * 8, kWarps); }
         mbar_init(rows_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -846,7 +850,6 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
     int x_left = 0;
     const unsigned char *x_src = nullptr;
     auto copy_table = [&](unsigned buf) {                          // the next chunk's table into buffer `buf`
-        if (!ok) return;                                           // the buffer's last copy may still be in flight
         if (x_left == 0) {
             if (x_src) x_unit += gridDim.x;
             if (x_unit >= units) return;
@@ -859,7 +862,6 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tab_full + buf * 8), "r"(65536u) : "memory");
         bulk_copy(kTab * (1u + buf), x_src, 65536u, tab_full + buf * 8);
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(copies), "r"(lds32(copies) + 1u) : "memory");
         x_src += 65536;
         --x_left;
     };
@@ -936,7 +938,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
             if (PRE && h == 0 && n == 1 && tid == 0 && oct > 0) {
                 // the other buffer's readers finished the chunk before this one: ask for the chunk after this one
                 mbar_wait(tab_empty + (st ^ 1u) * 8, ((oct - 1) >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
-                copy_table(st ^ 1u);
+                if (ok) copy_table(st ^ 1u);
+                else asm volatile("st.shared.u32 [%0], %1;" ::"r"(asked), "r"(min(lds32(asked), oct + 1u)) : "memory");   // the buffer's last copy may be in flight
             }
             if (kBuild && more) {
 #pragma unroll
@@ -1132,7 +1135,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         // thread 0 issued all bulk copies and, had every wait of its own come true, would have seen each of them arrive
         if (tid == 0) {
             if (kBuild) mbar_drain(rows_full, 0u);
-            const unsigned n = PRE ? lds32(copies) : 0u;
+            // tables asked for: all of this CTA's chunks, or as many as before the first wait that gave up
+            const unsigned n = PRE ? min(chunk, lds32(asked)) : 0u;
             if (n > 1) mbar_drain(tab_full + (n & 1u) * 8, ((n - 2) >> 1) & 1u);
             if (n > 0) mbar_drain(tab_full + ((n - 1) & 1u) * 8, ((n - 1) >> 1) & 1u);
         }
@@ -1239,6 +1243,13 @@ size_t xt_size(const XGeom &x, int mode) { return size_t((x.Cout + (mode == kXta
 // Pixels per tile, splits of K, and where the expanded tables are made.  In clocks per octet: lookups and codes 1.09 per pixel,
 // about 130 for the waits around a table, 720 for building one (512 of them on the shared-memory pipe); a start and an end that
 // do not shrink with the tile; tables from global memory cost their writes (2.3 KiB per clock over the chip) and a launch.
+// Against every other tile, split and place forced (one B200, us per call, chosen / best of the others / worst):
+//   3x3 512 -> 512 at 7x7, 1 image, one byte          186 (256 pixels, K in 9) / 194 (K in 13) / 1306
+//   3x3 256 -> 256 at 14x14, 8 images, one byte       140 (2048, K in 9) / 151 (1024) / 664
+//   3x3 256 -> 256 at 14x14, 128 images, one byte     786 (1024, global) / 976 (2048, global) / 2362
+//   1x1 64 -> 256 at 56x56, 64 images, one byte       249 (2048, global) / 249 (1024, global) / 680
+//   3x3 64 -> 96 at 28x28, 64 images, two digits      259 (1024, global) / 331 (2048, global) / 836
+//   3x3 64 -> 64 at 56x56, 64 images, two digits      679 (1024, global) / 660 (2048, global) / 2232
 Config choose_config(int mode, const XGeom &x, int sms, bool may_split, size_t xt_bytes)
 {
     const int tiles_n = (x.Cout + (mode == kXtabFull ? 7 : 15)) / (mode == kXtabFull ? 8 : 16);
@@ -1345,8 +1356,10 @@ int launch_expand(const ExpandParams &E, const DeviceInfo &di, cudaStream_t stre
 size_t xtab_scratch_bytes(const Geom &g, int mode)
 {
     if (mode == kXtabNone) return 0;
-    // Few lookups: the latency of preparation plus convolution is longer than the plan-based kernels' single pass over a
-    // filter that is already laid out.
+    // Calls with fewer lookups stay on the plan-based kernels.  The line is a cautious one, not the crossing: measured with it at 0
+    // (us per call, a filter whose plan is kept / expanded tables; CUDA-graph replay in brackets), the expanded tables are faster at
+    // every size tried - 50 / 31 (41 / 14) at 3.0e5 lookups, 69 / 31 (59 / 16) at 1.8e6, 40 / 26 (31 / 18) at 6.4e6,
+    // 104 / 31 (94 / 25) at 1.5e7 - and a new filter's plan costs 1.2 to 22 ms on top.
     if ((double)g.M * g.K * g.Cout < kXtabMinLookups) return 0;
     XGeom x;
     PrepTile t;
