@@ -166,8 +166,11 @@ def test_a_kept_plan_survives_every_batch_size(built):
         for n in (8, 64, 128, 8):
             x = torch.rand((n, 7, 7, 128), device="cuda", generator=g) * 2 - 1
             y, dbg = ax.approx_conv2d_with_min_max_vars(x, f, -1.0, 1.0, -0.2, 0.2, one, 8, t, "SAME", workspace=ws, debug=True)
+            assert dbg["plan"]["status"] == 0
             if n == 128:
                 assert dbg["plan"]["route"]["kernels"] == last
+            if dbg["plan"]["route"]["kernels"] == "expanded":
+                assert dbg["plan"]["steps_per_mille"] == 1000 and dbg["plan"]["rebuilt"] == 0
             if dbg["plan"]["route"]["kernels"] == "plan":
                 rebuilt.append(dbg["plan"]["rebuilt"])
             want = ax.approx_conv2d_with_min_max_vars(x, f, -1.0, 1.0, -0.2, 0.2, one, 8, t, "SAME")
