@@ -27,7 +27,20 @@ import numpy as np  # noqa: E402
 
 SM_COUNT = 148
 SMEM_BYTES_PER_CLK_PER_SM = 128   # shared-memory bandwidth: what bounds the table lookups
-NCU_DRAM_OVER_ALGORITHMIC = (205.0 + 162.1) / 411.2
+
+
+def call_bytes(spec, in_hw, batch, group):
+    """Bytes that a dense call on the expanded tables moves between its kernels and memory, from their layout: the fp32 tensors
+    once; the 8-bit codes, the patch sums and - with `group` channels each, 0: not in memory - the expanded tables written by one kernel and
+    read once by the next.  (Further reads of a table by other pixel tiles are expected to hit L2.)"""
+    from tf_approximate_b200 import workloads as W
+    o = W.out_hw(in_hw, spec.stride)
+    pixels, taps, pieces = batch * o * o, spec.k * spec.k, -(-spec.cin // 16)
+    rows = -(-taps * spec.cin // 16)
+    im2col = taps * pieces * 8 > rows * 9
+    codes = 16 * (pixels * rows if im2col else batch * in_hw * in_hw * pieces)
+    tables = 65536 * (rows if im2col else taps * pieces) * -(-spec.cout // group) if group else 0
+    return W.conv_io_bytes(spec, in_hw, batch) + 2 * (codes + 4 * pixels + tables)
 
 
 # name -> (description for `config.workload`, default batch per GPU, input description, configuration number)
@@ -377,10 +390,13 @@ def run_gpu(args):
     except Exception:
         pass
     hbm_peak = float(peaks.get("hbm_gbs", 6650.0))
-    # DRAM bytes per launch: ncu on the single 3x3 layer N=256, 56x56x64->64 read 205.0 MB and wrote 162.1 MB
-    # against 411.2 MB algorithmic; the whole step is too large to capture, so the measured ratio is applied to
-    # the average algorithmic bytes of a launch here.
-    traffic = NCU_DRAM_OVER_ALGORITHMIC * io_bytes / dense_launches
+    # bytes per call, computed from the layout of the kernels' data (the whole step is too large to capture)
+    traffic = 0.0
+    for i, (s, h) in enumerate(net.convs):
+        if not s.depthwise:
+            table = runner.tables[i % len(runner.tables)]
+            r = ax.ops.dense_route((batch, h, h, s.cin), (s.k, s.k, s.cin, s.cout), (1, s.stride, s.stride, 1), "SAME", table)
+            traffic += call_bytes(s, h, batch, (16 if entry_bytes == 1 else 8) if r["tables_in_global_memory"] else 0) / dense_launches
     slowest = sorted(per_layer.items(), key=lambda kv: -kv[1])[:3]
     roofline = {
         "kernel": "xtab_kernel (table convolution, %d convolution calls per step)" % dense_launches,
@@ -394,7 +410,7 @@ def run_gpu(args):
                                "axc_measure_lookup_peak (512 threads per SM, 16 independent loads per thread and "
                                "iteration), x %d entries x 148 SMs x the sampled clock" % (measured_per_clk / 32, lookups_per_clk),
         "units_per_launch": dense_macs / dense_launches, "ms_per_launch": dense_ms / dense_launches,
-        "traffic": traffic, "traffic_unit": "bytes per launch (scaled from an ncu capture of one layer)",
+        "traffic": traffic, "traffic_unit": "bytes per convolution call, computed from the data layout of its kernels (not measured)",
         "hbm": {"algorithmic_bytes_per_step": io_bytes, "achieved_gbs": io_bytes / (dense_ms * 1e-3) / 1e9,
                 "peak_gbs": hbm_peak, "frac": io_bytes / (dense_ms * 1e-3) / 1e9 / hbm_peak,
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback"},

@@ -202,6 +202,19 @@ def _route(out4):
             "tables_in_global_memory": bool(out4[3])}
 
 
+def dense_route(input_shape, filter_shape, strides, padding, table, dilations=(1, 1, 1, 1), workspace_bytes=None):
+    """Which kernels serve a dense call (axc_conv2d_route): a call without `workspace=`, or with one of that many bytes."""
+    d = _desc(input_shape, filter_shape, strides, padding, "NHWC", list(dilations), [], plan="keep" if workspace_bytes is not None else "none")
+    L, size, out = _lib.load(), C.c_size_t(workspace_bytes or 0), (C.c_int32 * 4)()
+    if workspace_bytes is None:
+        raise_for_status(L.axc_conv2d_fast_workspace_bytes(table.handle, C.byref(d), C.byref(size)), "workspace size")
+        if size.value == 0:
+            d.plan = _PLAN["keep"]
+            raise_for_status(L.axc_conv2d_workspace_bytes(C.byref(d), C.byref(size)), "workspace size")
+    raise_for_status(L.axc_conv2d_route(table.handle, C.byref(d), size.value, out), "route")
+    return _route(out)
+
+
 def _scratch(dev, nbytes):
     """Scratch of one call on the expanded tables, or None where the device has not that much memory left (up to hundreds of
     MB; the other kernels need a plan's workspace only).  torch's allocator hands it to later work of the same stream only."""
