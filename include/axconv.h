@@ -48,8 +48,8 @@ enum { AXC_FORMAT_NHWC = 0, AXC_FORMAT_NCHW = 1 };
  *   total (tf2/src/approx_nn_conv_kernels.cpp:245-246), which rounds once a partial sum passes 2^24.  Output
  *   bits equal the reference's CPU kernel for every K.  Where the table and K prove that no partial sum can
  *   round (K * largest entry <= 2^24 * the power of two dividing every entry) the fast integer kernel serves
- *   the call, since both give the same bits; otherwise a kernel that walks K in order does (about half the
- *   speed).  Depthwise calls ignore the field (K = kh*kw never rounds). */
+ *   the call, since both give the same bits; otherwise a kernel that walks K in order does (a quarter
+ *   to half of the speed).  Depthwise calls ignore the field (K = kh*kw never rounds). */
 enum { AXC_ACCUM_EXACT_I32 = 0, AXC_ACCUM_REFERENCE_F32 = 1 };
 /* Whether the dense op prepares a per-filter lookup plan (kept in the workspace, built in 3-90 ms, reused while the
  * filter is unchanged) or serves the call without one.
@@ -173,8 +173,8 @@ int axc_conv2d_forward(axc_table *table, const axc_conv_desc *desc,
  * the ReLU of the layer that PRODUCED this call's input.
  *   output side:  y = conv;  if (bias) y += bias[channel];  if (residual) y += residual[same index];
  *                 if (relu) y = max(y, 0)   - each a separately rounded fp32 operation, i.e. the bits of the same steps
- *                 done by separate kernels.  The dense op runs them as one extra pass over the output (inside the lookup
- *                 kernels even two instructions per output cost more than that pass); the depthwise kernels in place.
+ *                 done by separate kernels.  The expanded-table and the depthwise kernels apply them in place, the other
+ *                 dense kernels as one extra pass over the output (there even two instructions per output cost more).
  *   input side:   input_relu != 0: every input element counts as max(x, 0) - applied by the kernels' loaders to the raw
  *                 value, before quantisation and patch sum, at no cost to the lookups.  A chain conv -> ReLU -> conv
  *                 can thus leave the ReLU to the second convolution and never write the activated tensor.

@@ -125,8 +125,8 @@ class FakeApproxConv2D(torch.nn.Module):
         return self._ranges, self._workspace
 
     def plan_info(self):
-        """{rebuilt in the last call, fallback, status, steps per mille} of the lookup plan in the layer's workspace
-        (blocks until the current stream is idle)."""
+        """{rebuilt, fallback, status, steps per mille} of the lookup plan in the layer's workspace, as the last call that used it
+        left them (blocks until the current stream is idle); None where no call has: calls on the expanded tables keep none."""
         import ctypes as C
         from . import _lib
         if self._workspace is None:
