@@ -73,6 +73,7 @@ __global__ void dw_filter_prep_kernel(const float *__restrict__ filter, int KHW,
                                       uint32_t *__restrict__ prog, uint32_t *__restrict__ prog_packed,
                                       float *__restrict__ bsum, uint8_t *__restrict__ qfilter, int *status)
 {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int oc = blockIdx.x * blockDim.x + threadIdx.x;
     if (oc == 0) *status = 0;
     if (oc >= OC) return;
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) depthwise_3x3_kernel(const DwPa
 // whole LDS.32 are conflict-free - 5 wavefronts per 9 table MACs instead of 29.
 //
 // Work: the CTA owns a contiguous range of (channel group, image, band of R output rows) units; it rebuilds the
-// table when the range crosses into the next group.  A warp walks a band from left to right, lane = channel: per
+// table when the range crosses into the next group.  A warp walks its share of the bands' columns from left to right, lane = channel: per
 // input column it loads the (R-1)*S+3 rows of the column (one 128-byte line each), quantises, looks up and adds
 // the products into the accumulators of the (at most) three output columns in flight; a finished output column
 // gets its patch sum - the raw taps added in (ky, kx) order like the reference's im2col
@@ -445,6 +446,7 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
     const unsigned stages0 = tab4 + kTab4Bytes;                                        // [warp][stage][row][channel]
     const unsigned bars0 = stages0 + (TMA ? unsigned(kTabWarps * STAGES) * stage_bytes : 0u);   // [warp][stage] mbarriers
     if (bars0 + (TMA ? unsigned(kTabWarps * STAGES) * 8u : 0u) > dyn0 + dyn_size) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         if (threadIdx.x == 0) atomicExch(P.status, 1);
         return;
     }
@@ -478,6 +480,7 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
     for (int g = slot; g < P.groups; g += wave) {
         __syncthreads();                                    // every warp is done with the previous group's table
         dw_build_table<NT>(P, g, tab16, tab4, tid);
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // the filter sums and a status that nothing sets back (the table needs neither)
         __syncthreads();
 
         const int oc = g * 32 + lane;
@@ -486,7 +489,15 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
         const float t2 = oc_ok ? __fmul_rn(P.m1, __ldg(P.bsum + oc)) : 0.0f;
         const float bias_j = (oc_ok && P.ep.bias) ? __ldg(P.ep.bias + oc) : 0.0f;
 
-        for (int w = w_begin + warp; w < w_end; w += kTabWarps) {
+        // Each warp takes an even share of the output columns of all bands, wherever that begins and ends: two (stride 2: one)
+        // input columns more per piece.  Whole bands in turn left a quarter of the warps idle in the last round
+        // (56x56x144, 128 images: 1024 bands in 29 sets of 16 warps are 2.2 rounds, three taken; 174 us, now 150 with the launch below).
+        const long long columns = (long long)(w_end - w_begin) * P.OW;
+        const long long last = columns * (warp + 1) / kTabWarps;
+        for (long long next = columns * warp / kTabWarps; next < last;) {
+            const int band = int(next / P.OW), x0 = int(next - (long long)band * P.OW), w = w_begin + band;
+            const int cols = int(last - next < P.OW - x0 ? last - next : P.OW - x0);          // output columns x0 .. x0 + cols - 1
+            next += cols;
             const int n = w / P.bands;
             const int oy0 = (w - n * P.bands) * R;
             const int rows_here = oc_ok ? (P.OH - oy0 < R ? P.OH - oy0 : R) : 0;      // rows this lane stores
@@ -494,10 +505,11 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
             // input rows lo <= i < hi of the band lie inside the image (lo is 0 or 1)
             const int lo = iy0 < 0 ? -iy0 : 0;
             const int hi = P.H - iy0 < IR ? P.H - iy0 : IR;
-            // byte pointers: input element (n, iy0, image column -pw, cin); output element (n, oy0, 0, oc)
-            const char *in0 = reinterpret_cast<const char *>(P.input + ((long long)n * P.H + iy0) * (long long)(P.W * P.C) -
-                                                             (long long)P.pw * P.C + cin);
-            const long long o0 = ((long long)n * P.OH + oy0) * (long long)(P.OW * P.OC) + (oc_ok ? oc : 0);
+            const int ix0 = x0 * S - P.pw;                                 // image column of input column 0 of the piece
+            // byte pointers: input element (n, iy0, image column ix0, cin); output element (n, oy0, x0, oc)
+            const char *in0 = reinterpret_cast<const char *>(P.input + ((long long)n * P.H + iy0) * (long long)(P.W * P.C) +
+                                                             (long long)ix0 * P.C + cin);
+            const long long o0 = ((long long)n * P.OH + oy0) * (long long)(P.OW * P.OC) + (long long)x0 * P.OC + (oc_ok ? oc : 0);
             const char *out0 = reinterpret_cast<const char *>(P.output + o0);
             const char *acc0 = DBG ? reinterpret_cast<const char *>(P.acc_out + o0) : nullptr;
             const char *res0 = P.ep.residual ? reinterpret_cast<const char *>(P.ep.residual + o0) : nullptr;
@@ -506,7 +518,7 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
             float xf[IR][3];      // raw taps of the columns in flight: S == 1 ring slot = column % 3; S == 2: 0 / 1 = even
                                   // columns (m % 2), 2 = odd column
             float nx[IR];         // raw taps of the column being fetched (plain loads only)
-            const int ncols = S == 1 ? P.OW + 2 : 2 * P.OW + 1;                   // input columns of the band
+            const int ncols = S == 1 ? cols + 2 : 2 * cols + 1;                   // input columns of the piece
             const unsigned lane_off = unsigned(lane) * 4u;
 
             // TMA: column `c` into stage `st`, issued by lane 0 after the whole warp has consumed the stage
@@ -515,8 +527,8 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
                 if (lane == 0 && c < ncols) {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     dw_tma_column(my_stage0 + unsigned(st) * stage_bytes, tmap, my_bar0 + unsigned(st) * 8u, box_bytes, g * 32,
-                                  c - P.pw, iy0, n);
-                    if (c + kTmaL2Ahead < ncols) dw_tma_prefetch_l2(tmap, g * 32, c + kTmaL2Ahead - P.pw, iy0, n);
+                                  c + ix0, iy0, n);
+                    if (c + kTmaL2Ahead < ncols) dw_tma_prefetch_l2(tmap, g * 32, c + kTmaL2Ahead + ix0, iy0, n);
                 }
             };
             // TMA: raw taps of the column in stage `st` into xf slot `slot`
@@ -539,9 +551,9 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
                 }
             };
 
-            // raw taps of input column `c` (relative: image column c - pw); zeros outside the image
+            // raw taps of input column `c` (relative: image column c + ix0); zeros outside the image
             auto fetch = [&](int c) {
-                if (unsigned(c - P.pw) < unsigned(P.W)) {          // the same for all lanes
+                if (unsigned(c + ix0) < unsigned(P.W)) {          // the same for all lanes
                     const char *colp = dw_ptr_mad(in0, unsigned(c), pix_bytes);
 #pragma unroll
                     for (int i = 0; i < IR; ++i) {
@@ -549,7 +561,7 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
                         if (i >= lo && i < hi) x = max_keep_nan(__ldg(reinterpret_cast<const float *>(dw_ptr_mad(colp, unsigned(i), row_bytes))), in_floor);
                         nx[i] = x;
                     }
-                    if (PF > 0 && unsigned(c + PF - P.pw) < unsigned(P.W)) {
+                    if (PF > 0 && unsigned(c + PF + ix0) < unsigned(P.W)) {
                         const char *pfp = colp + PF * pix_bytes;
 #pragma unroll
                         for (int i = 0; i < IR; ++i)
@@ -560,7 +572,7 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
                     for (int i = 0; i < IR; ++i) nx[i] = 0.0f;
                 }
             };
-            // patch sum, dequantisation and store of output column ox, rows 0..R-1: raw columns in xf slots
+            // patch sum, dequantisation and store of the piece's output column ox, rows 0..R-1: raw columns in xf slots
             // (k0, k1, k2) for kx = 0, 1, 2, integer sums in slot sa
             auto emit = [&](int ox, auto k0c, auto k1c, auto k2c, auto sac) {
                 constexpr int k0 = decltype(k0c)::value, k1 = decltype(k1c)::value, k2 = decltype(k2c)::value;
@@ -650,7 +662,7 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
                 } else {
                     fetch(0);
                 }
-                const int c_end = P.OW + 2;
+                const int c_end = cols + 2;
                 for (int c = 0; c < c_end; c += 3) {
                     column(c, I0{});
                     if (c + 1 < c_end) column(c + 1, I1{});
@@ -730,12 +742,12 @@ __device__ __forceinline__ void depthwise_3x3_tab_body(const DwParams &P, const 
                 } else {
                     fetch(0);
                 }
-                for (int m = 0; m <= P.OW; m += 2) {
+                for (int m = 0; m <= cols; m += 2) {
                     even_column(m, I0{});
-                    if (m < P.OW) odd_column(m, I0{});
-                    if (m + 1 <= P.OW) {
+                    if (m < cols) odd_column(m, I0{});
+                    if (m + 1 <= cols) {
                         even_column(m + 1, I1{});
-                        if (m + 1 < P.OW) odd_column(m + 1, I1{});
+                        if (m + 1 < cols) odd_column(m + 1, I1{});
                     }
                 }
             }
@@ -791,18 +803,25 @@ int launch_dw_tab_variant(DwParams P, const DeviceInfo &di, cudaStream_t stream)
     if (P.sets > P.units_per_group) P.sets = P.units_per_group;
     // Input columns by TMA where the tensor allows it (at least 32 channels, and a channel multiplier of 1, so that
     // a lane's input channel is its output channel); plain loads otherwise.
+    // The kernel may start while the filter's preparation runs: it waits for that once its first table is built.
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(P.wave * P.sets)); cfg.blockDim = dim3(NT); cfg.stream = stream;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
     CUtensorMap tmap;
     const unsigned tma_smem = kTabSmem + unsigned(NT / 32 * STAGES) * (unsigned(IR) * 128u + 8u);
     if (P.mult == 1 && P.C >= 32 && tma_smem <= unsigned(di.max_smem_optin) && dw_make_tensor_map(P, IR, &tmap)) {
         AXC_CUDA(cudaFuncSetAttribute(depthwise_3x3_tma_kernel<S, R, NT, DBG>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tma_smem)));
-        depthwise_3x3_tma_kernel<S, R, NT, DBG><<<unsigned(P.wave * P.sets), NT, tma_smem, stream>>>(P, tmap);
-        AXC_CUDA(cudaGetLastError());
+        cfg.dynamicSmemBytes = tma_smem;
+        AXC_CUDA(cudaLaunchKernelEx(&cfg, depthwise_3x3_tma_kernel<S, R, NT, DBG>, P, tmap));
         count_launch();
         return AXC_OK;
     }
     AXC_CUDA(cudaFuncSetAttribute(depthwise_3x3_tab_kernel<S, R, NT, DBG>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTabSmem)));
-    depthwise_3x3_tab_kernel<S, R, NT, DBG><<<unsigned(P.wave * P.sets), NT, kTabSmem, stream>>>(P);
-    AXC_CUDA(cudaGetLastError());
+    cfg.dynamicSmemBytes = kTabSmem;
+    AXC_CUDA(cudaLaunchKernelEx(&cfg, depthwise_3x3_tab_kernel<S, R, NT, DBG>, P));
     count_launch();
     return AXC_OK;
 }
