@@ -327,6 +327,10 @@ int axc_tensor_range(const float *x, size_t count, float *range2, int device, vo
  * FakeQuantWithMinMaxVars with num_bits = 8, with the range read from device memory (range2 = {min, max}); the
  * nudging is the op's own (tf2/src/approx_ops_types.h:29-49), operation by operation.  out may equal x. */
 int axc_fake_quant(const float *x, size_t count, const float *range2, float *out, int device, void *stream);
+/* out[c] = sum over r of x[r * cols + c] (fp32, device; no chain of additions longer than rows / 2368 + 60): the gradient of the
+ * wrapper's bias (:258-259).  scratch: AXC_COLUMN_SUM_ROWS * cols floats, nothing kept. */
+enum { AXC_COLUMN_SUM_ROWS = 296 };
+int axc_column_sums(const float *x, size_t rows, int cols, float *scratch, float *out, int device, void *stream);
 
 /* ---- quantisation parameters: Nudge + UpdateVarQuantProps
  *      (tf2/src/approx_ops_types.h:29-49, 135-152).  out3 = {scale, 1/scale, nudged_min}. */

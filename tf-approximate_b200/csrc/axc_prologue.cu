@@ -156,6 +156,95 @@ extern "C" int axc_fake_quant(const float *x, size_t count, const float *range2,
 }
 
 // ------------------------------------------------------------------------------------------------
+// Sums of a matrix's columns: the gradient of a bias.  Bound by reading the matrix once.  Lanes take neighbouring columns, warps and
+// blocks share the rows evenly, so that no sum is a chain of more than rows / (8 blocks) additions; a second kernel adds the
+// blocks' sums, a block per 32 columns.  25088 x 128: 4.6 us, of which the second kernel 2 (a library reduction over the same rows: 39).
+// ------------------------------------------------------------------------------------------------
+namespace axc {
+namespace {
+
+constexpr int kColumnBlocks = 296;             // AXC_COLUMN_SUM_ROWS of the header
+
+template <int V>
+__global__ void __launch_bounds__(256) column_sums_kernel(const float *__restrict__ x, long long rows, int cols, float *__restrict__ part)
+{
+    __shared__ float sums[8][32 * V];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long begin = rows * blockIdx.x / gridDim.x, end = rows * (blockIdx.x + 1) / gridDim.x;
+    for (int c0 = 0; c0 < cols; c0 += 32 * V) {
+        const int c = c0 + lane * V;
+        float a[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) a[e] = 0.0f;
+        if (c < cols) {
+#pragma unroll 4
+            for (long long r = begin + warp; r < end; r += 8) {
+                if (V == 4) {
+                    const float4 v = __ldg(reinterpret_cast<const float4 *>(x + r * cols + c));
+                    a[0] += v.x; a[1 % V] += v.y; a[2 % V] += v.z; a[3 % V] += v.w;
+                } else a[0] += __ldg(x + r * cols + c);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < V; ++e) sums[warp][lane * V + e] = a[e];
+        __syncthreads();
+        for (int i = threadIdx.x; i < 32 * V && c0 + i < cols; i += 256) {
+            float s = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) s += sums[w][i];
+            part[(long long)blockIdx.x * cols + c0 + i] = s;
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(256) column_total_kernel(const float *__restrict__ part, int count, int cols, float *__restrict__ out)
+{
+    __shared__ float sums[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+    float a = 0.0f;
+    if (c < cols)
+#pragma unroll 8
+        for (int r = warp; r < count; r += 8) a += __ldg(part + (long long)r * cols + c);
+    sums[warp][lane] = a;
+    __syncthreads();
+    if (warp == 0 && c < cols) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) a += sums[w][lane];
+        out[c] = a;
+    }
+}
+
+}  // namespace
+}  // namespace axc
+
+extern "C" int axc_column_sums(const float *x, size_t rows, int cols, float *scratch, float *out, int device, void *stream)
+{
+    using namespace axc;
+    if (cols < 0 || rows > (size_t(1) << 40)) return AXC_INVALID_ARGUMENT;
+    if (cols == 0) return AXC_OK;
+    if (!out || (rows > 0 && (!x || !scratch))) return AXC_INVALID_ARGUMENT;
+    DeviceInfo di;
+    int rc = device_info(device, &di);
+    if (rc) return rc;
+    int prev = 0;
+    rc = with_device(device, &prev);
+    if (rc) return rc;
+    cudaStream_t s = cudaStream_t(stream);
+    const unsigned blocks = unsigned((rows + 7) / 8 < size_t(kColumnBlocks) ? (rows + 7) / 8 : size_t(kColumnBlocks));
+    if (blocks > 0) {
+        if (cols % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) column_sums_kernel<4><<<blocks, 256, 0, s>>>(x, (long long)rows, cols, scratch);
+        else column_sums_kernel<1><<<blocks, 256, 0, s>>>(x, (long long)rows, cols, scratch);
+        count_launch();
+    }
+    column_total_kernel<<<unsigned((cols + 31) / 32), 256, 0, s>>>(scratch, int(blocks), cols, out);
+    count_launch();
+    const cudaError_t e = cudaGetLastError();
+    if (prev != device) cudaSetDevice(prev);
+    return e == cudaSuccess ? AXC_OK : cuda_failed(e);
+}
+
+// ------------------------------------------------------------------------------------------------
 // Max pooling, NHWC, SAME padding: one thread per output pixel and group of four channels (or one channel when the
 // channel count or the pointers do not allow 16-byte accesses).
 // ------------------------------------------------------------------------------------------------

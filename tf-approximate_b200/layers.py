@@ -60,32 +60,43 @@ class _FakeQuantFn(torch.autograd.Function):
 
 class _ApproxConvFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w, ranges, strides, padding, mul_map_file, num_bits, dilations, plan, workspace):
+    def forward(ctx, x, w, bias, ranges, strides, padding, mul_map_file, num_bits, dilations, plan, workspace):
         ctx.save_for_backward(x, w)
         ctx.cfg = (strides, padding, dilations)
         return approx_conv2d_with_min_max_vars(x, w, None, None, None, None, strides=strides, num_bits=num_bits,
                                                mul_map_file=mul_map_file, padding=padding, dilations=dilations,
-                                               plan=plan, workspace=workspace, ranges=ranges)
+                                               plan=plan, workspace=workspace, ranges=ranges, bias=bias)
 
     @staticmethod
     def backward(ctx, grad):
         x, w = ctx.saved_tensors
         strides, padding, dilations = ctx.cfg
-        with torch.enable_grad():
-            xc = x.detach().permute(0, 3, 1, 2).requires_grad_(True)
-            wc = w.detach().permute(3, 2, 0, 1).requires_grad_(True)
-            kh, kw = w.shape[0], w.shape[1]
-            sh, sw, dh, dw = strides[1], strides[2], dilations[1], dilations[2]
-            if padding == "SAME":
-                oh, ow = -(-x.shape[1] // sh), -(-x.shape[2] // sw)
-                ph = max((oh - 1) * sh + (kh - 1) * dh + 1 - x.shape[1], 0)
-                pw = max((ow - 1) * sw + (kw - 1) * dw + 1 - x.shape[2], 0)
-                xp = torch.nn.functional.pad(xc, (pw // 2, pw - pw // 2, ph // 2, ph - ph // 2))
-            else:
-                xp = xc
-            y = torch.nn.functional.conv2d(xp, wc, stride=(sh, sw), dilation=(dh, dw))
-            gx, gw = torch.autograd.grad(y, (xc, wc), grad.permute(0, 3, 1, 2))
-        return gx.permute(0, 2, 3, 1), gw.permute(2, 3, 1, 0), None, None, None, None, None, None, None, None
+        kh, kw = w.shape[0], w.shape[1]
+        sh, sw, dh, dw = strides[1], strides[2], dilations[1], dilations[2]
+        ph = pw = 0
+        if padding == "SAME":
+            oh, ow = -(-x.shape[1] // sh), -(-x.shape[2] // sw)
+            ph = max((oh - 1) * sh + (kh - 1) * dh + 1 - x.shape[1], 0)
+            pw = max((ow - 1) * sw + (kw - 1) * dw + 1 - x.shape[2], 0)
+        need_x, need_w, need_b = ctx.needs_input_grad[:3]
+        gx = gw = None
+        with torch.no_grad():
+            if need_x or need_w:
+                # the exact convolution's two gradients, asked for as such: no forward convolution to differentiate, and a padded
+                # copy only where the padding is not the same on both sides
+                xc, even = x.permute(0, 3, 1, 2), ph % 2 == 0 and pw % 2 == 0
+                if not even:
+                    xc = torch.nn.functional.pad(xc, (pw // 2, pw - pw // 2, ph // 2, ph - ph // 2))
+                gx, gw, _ = torch.ops.aten.convolution_backward(
+                    grad.permute(0, 3, 1, 2), xc, w.permute(3, 2, 0, 1), None, (sh, sw), (ph // 2, pw // 2) if even else (0, 0), (dh, dw),
+                    False, (0, 0), 1, (need_x, need_w, False))
+                if need_x:
+                    gx = gx if even else gx[:, :, ph // 2:ph // 2 + x.shape[1], pw // 2:pw // 2 + x.shape[2]]
+                    gx = gx.permute(0, 2, 3, 1)
+                if need_w:
+                    gw = gw.permute(2, 3, 1, 0)
+            gb = ops.column_sums(grad) if need_b else None
+        return gx, gw, gb, None, None, None, None, None, None, None, None
 
 
 class FakeApproxConv2D(torch.nn.Module):
@@ -152,9 +163,11 @@ class FakeApproxConv2D(torch.nn.Module):
         q_k = _FakeQuantFn.apply(self.kernel, ranges[2:4])
         # while the weights are being trained they change every step: no lookup plan then (nothing to rebuild)
         plan = "none" if (self.training and self.kernel.requires_grad) else "keep"
-        y = _ApproxConvFn.apply(q_in, q_k, ranges, strides4, self.padding, table, self.num_bits, dilations4,
+        # the op adds a bias that it can take in the same pass
+        fused = self.bias if self.bias is not None and self.bias.dtype == torch.float32 and self.bias.device == inputs.device and self.bias.dim() == 1 else None
+        y = _ApproxConvFn.apply(q_in, q_k, fused, ranges, strides4, self.padding, table, self.num_bits, dilations4,
                                 plan, workspace)
-        if self.bias is not None:
+        if self.bias is not None and fused is None:
             y = y + self.bias
         if self.activation is not None:
             y = self.activation(y)

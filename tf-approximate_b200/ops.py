@@ -19,6 +19,7 @@ _PADDING = {"SAME": 0, "VALID": 1, "EXPLICIT": 2}
 _FORMAT = {"NHWC": 0, "NCHW": 1}
 _ACCUMULATE = {"exact": 0, "reference": 1}
 _PLAN = {"keep": 0, "none": 1}
+_COLUMN_SUM_ROWS = 296       # AXC_COLUMN_SUM_ROWS
 
 
 class Table:
@@ -493,6 +494,19 @@ def fake_quant_device_range(x, range2, out=None):
     st = _lib.load().axc_fake_quant(x.data_ptr(), x.numel(), range2.data_ptr(), out.data_ptr(), dev_index,
                                     C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream))
     raise_for_status(st, "fake quant", _cuda_detail() if st == 100 else "")
+    return out
+
+
+def column_sums(x):
+    """Sums over all but the last dimension of a fp32 CUDA tensor: the gradient of a bias."""
+    if not x.is_cuda or x.dtype != torch.float32 or x.dim() == 0:
+        raise InvalidArgumentError("column_sums expects a fp32 CUDA tensor")
+    x = x.contiguous()
+    cols = x.shape[-1]
+    out, scratch = torch.empty(cols, dtype=torch.float32, device=x.device), torch.empty(_COLUMN_SUM_ROWS * cols, dtype=torch.float32, device=x.device)
+    st = _lib.load().axc_column_sums(x.data_ptr(), x.numel() // cols if cols else 0, cols, scratch.data_ptr(), out.data_ptr(), _device_index(x.device),
+                                     C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream))
+    raise_for_status(st, "column sums", _cuda_detail() if st == 100 else "")
     return out
 
 
