@@ -179,6 +179,16 @@ __device__ __forceinline__ unsigned code_of(float x, float off, float inv)
     return __float_as_uint(__fadd_rd(fminf(fmaxf(v, 0.0f), 255.0f), 8388608.0f)) & 0xFFu;
 }
 
+// The codes of four neighbouring values as a word.
+__device__ __forceinline__ unsigned codes_of(const float4 &x, float off, float inv)
+{
+    auto biased = [&](float y) {
+        const float v = __fadd_rn(__fmul_rn(__fsub_rn(y, off), inv), 0.5f);
+        return __float_as_uint(__fadd_rd(fminf(fmaxf(v, 0.0f), 255.0f), 8388608.0f));
+    };
+    return prmt<0x5410>(prmt<0x0040>(biased(x.x), biased(x.y)), prmt<0x0040>(biased(x.z), biased(x.w)));
+}
+
 // ------------------------------------------------------------------------------------------------------------------
 // preparation
 // ------------------------------------------------------------------------------------------------------------------
@@ -190,6 +200,8 @@ struct XGeom {
     int TNC;            // channels per tile: 8 (16-bit entries) or 16
     int tiles_n;
 };
+
+constexpr int kPrepThreads = 512;
 
 struct PrepParams {
     XGeom g;
@@ -209,8 +221,10 @@ struct PrepParams {
     uint8_t *qf_debug;
     PlanHeader *hdr;
     long long scratch_bytes;
-    int blocks_sum, blocks_w, blocks_t;      // leading blocks; the rest are input tiles
+    int blocks_sum, blocks_w, blocks_t;      // first blocks, last but one and last; the rest are input tiles
     int TH, TW, tiles_y, tiles_x, RH, RW, pitch, vec;
+    int sums;                                 // patch and filter sums are asked for (a quantised call has none)
+    int bytes_at, bytes_pitch;                // im2col: codes of the staged taps behind the taps, bytes per region row
 };
 
 // channel of slot s in a piece: the order in which a lane's accumulators hold four neighbouring channels
@@ -227,10 +241,13 @@ __device__ __forceinline__ unsigned row_address(int mode, unsigned row)
     return row < unsigned(kLowRows) ? kRowsLow + row * 512u : kRowsHigh + (row - kLowRows) * 512u;
 }
 
+// (The operands' type is a template parameter of the preparation: a branch on it between loads has each of them waited for before
+// the next is issued - 53 us instead of 13 for the sums of a filter with K = 4608.)
+template <bool U8>
 __device__ __forceinline__ float filter_value(const XGeom &g, const float *f, const uint8_t *u8, size_t at)
 {
     if (!AXC_GLOBAL_OK((long long)at, (long long)g.K * g.Cout, 320u)) return 0.0f;
-    return u8 ? float(__ldg(u8 + at)) : __ldg(f + at);
+    return U8 ? float(__ldg(u8 + at)) : __ldg(f + at);
 }
 
 __device__ __forceinline__ bool staged_ok(long long at, int count, unsigned site)      // floats of xprep_kernel's shared memory
@@ -255,59 +272,107 @@ __device__ __forceinline__ int k_of(const XGeom &g, int ch, int i)
     return c < g.C ? tap * g.C + c : -1;
 }
 
-// Filter sums in l order (tf2/src/approx_nn_conv_kernels.cpp:187-197), 32 channels per block: the whole block stages 256
-// rows at a time, one warp adds (a chain of K additions per channel; the staging hides the memory latency behind it).
+// Filter sums in l order (tf2/src/approx_nn_conv_kernels.cpp:187-197), 32 channels per block.  Bound by the order: a chain of K
+// additions per channel, 4 clocks each.  One warp adds, a lane per channel, and does nothing else: eight others have the rows
+// brought into a ring of six stages of 64 (cp.async).  The whole preparation of 3x3 512 -> 512 at 7x7, one image: 28 us; with the rows
+// staged through registers by the whole block, 256 at a time between barriers, 40; asked for by the adding warp itself 104; by a
+// bulk copy per row 143.  The sums of the codes, where they are asked for, are the other warps'.
+constexpr int kSumRows = 64, kSumStages = 6, kSumLoaders = 256;
+constexpr size_t kSumSmem = size_t(kSumRows) * kSumStages * 128 + 128 + 128;      // the ring, code sums, barriers
+
+template <bool U8>
 __device__ void prep_filter_sums(const PrepParams &P, const DevQuant &q, int block, float *stage)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int j = block * 32 + lane;
-    float acc = 0.0f;
-    int codes = 0;
-    float v[32];
-    auto fetch = [&](int l0) {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-            const int l = l0 + e * 8 + warp;
-            v[e] = (l < P.g.K && j < P.g.Cout) ? filter_value(P.g, P.filter, P.filter_u8, (size_t)l * P.g.Cout + j) : 0.0f;
-        }
-    };
-    fetch(0);
-    for (int l0 = 0; l0 < P.g.K; l0 += 256) {
-        __syncthreads();
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-            if (staged_ok((e * 8 + warp) * 32 + lane, 1, 321u)) stage[(e * 8 + warp) * 32 + lane] = v[e];
-            if (P.bcode && l0 + e * 8 + warp < P.g.K) codes += int(code_of(v[e], q.f_off, q.f_inv));
+    const int j = block * 32 + lane, K = P.g.K, Cout = P.g.Cout;
+    const bool have = j < Cout;
+    const unsigned ring = (unsigned)__cvta_generic_to_shared(stage), full = ring + kSumRows * kSumStages * 128u + 128u, empty = full + 8u * kSumStages;
+    if (P.sums) {
+        if (threadIdx.x == 0) {
+            for (int s = 0; s < kSumStages; ++s) { mbar_init(full + 8u * s, kSumLoaders); mbar_init(empty + 8u * s, 1); }
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         __syncthreads();
-        if (l0 + 256 < P.g.K) fetch(l0 + 256);
-        if (warp == 0) {
-            const int n = min(256, P.g.K - l0);
-            int l = 0;
-            for (; l + 16 <= n; l += 16) {
-                float u[16];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) u[e] = stage[(l + e) * 32 + lane];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) acc = __fadd_rn(acc, u[e]);
-            }
-            for (; l < n; ++l) acc = __fadd_rn(acc, stage[l * 32 + lane]);
-        }
     }
-    if (warp == 0 && j < P.g.Cout && AXC_SCRATCH_OK(P, P.bsum + j, 4, 322u)) P.bsum[j] = acc;
-    if (P.bcode) {
-        int *sums = reinterpret_cast<int *>(stage);
-        __syncthreads();
-        sums[warp * 32 + lane] = codes;
-        __syncthreads();
-        if (warp == 0 && j < P.g.Cout) {
-            for (int w = 1; w < 8; ++w) codes += sums[w * 32 + lane];
-            if (AXC_SCRATCH_OK(P, P.bcode + j, 4, 323u)) P.bcode[j] = codes;
+    bool ok = true;
+    const int stages = (K + kSumRows - 1) / kSumRows;
+    if (P.sums && warp == 0) {
+        float acc = 0.0f;
+        for (int i = 0; i < stages; ++i) {
+            const int at = i % kSumStages, n = min(kSumRows, K - i * kSumRows);
+            mbar_wait(full + 8u * at, (i / kSumStages) & 1, ok, kWaitPolls);
+            const float *src = stage + at * (kSumRows * 32) + lane;
+            float u[2][16];
+            auto rows16 = [&](int l, float (&to)[16]) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) to[e] = src[(l + e) * 32];
+            };
+            auto add16 = [&](const float (&a)[16]) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) acc = __fadd_rn(acc, a[e]);
+            };
+            if (n == kSumRows) {                                   // the next 16 rows are read while the last 16 are added
+                rows16(0, u[0]); rows16(16, u[1]);
+                add16(u[0]); rows16(32, u[0]);
+                add16(u[1]); rows16(48, u[1]);
+                add16(u[0]); add16(u[1]);
+            } else
+                for (int l = 0; l < n; ++l) acc = __fadd_rn(acc, src[l * 32]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + 8u * at);
         }
+        if (have && AXC_SCRATCH_OK(P, P.bsum + j, 4, 322u)) P.bsum[j] = acc;
+    } else if (P.sums && warp <= kSumLoaders / 32) {
+        const int who = int(threadIdx.x) - 32, wide = (Cout & 3) == 0 && (reinterpret_cast<uintptr_t>(P.filter) & 15u) == 0 ? 1 : 0;
+        for (int i = 0; i < stages; ++i) {
+            const int at = i % kSumStages, l0 = i * kSumRows;
+            if (i >= kSumStages) mbar_wait(empty + 8u * at, (i / kSumStages - 1) & 1, ok, kWaitPolls);
+            if (!ok) break;
+            const unsigned to = ring + unsigned(at) * (kSumRows * 128u);
+            if (wide) {                                            // 16 bytes at a time, 8 pieces to a row
+#pragma unroll
+                for (int e = 0; e < kSumRows * 8 / kSumLoaders; ++e) {
+                    const int x = e * kSumLoaders + who, l = l0 + (x >> 3), c = block * 32 + (x & 7) * 4;
+                    if (l < K && c < Cout && AXC_GLOBAL_OK((long long)l * Cout + c + 3, (long long)K * Cout, 320u)) cp_async16(to + unsigned(x) * 16u, P.filter + (size_t)l * Cout + c, 16u);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < kSumRows * 32 / kSumLoaders; ++e) {
+                    const int x = e * kSumLoaders + who, l = l0 + (x >> 5), c = block * 32 + (x & 31);
+                    if (l < K && c < Cout && AXC_GLOBAL_OK((long long)l * Cout + c, (long long)K * Cout, 319u))
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to + unsigned(x) * 4u), "l"(P.filter + (size_t)l * Cout + c) : "memory");
+                }
+            }
+            // the barrier hears of it when this thread's copies have arrived
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full + 8u * at) : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    if (!ok) atomicExch(&P.hdr->status, 3);
+    if (P.bcode) {
+        // the warps after the loaders share the rows
+        int *sums = reinterpret_cast<int *>(stage) + kSumRows * kSumStages * 32;
+        constexpr int kFirst = kSumLoaders / 32 + 1, kStep = kPrepThreads / 32 - kFirst;
+        if (warp == kFirst) sums[lane] = 0;
+        __syncthreads();
+        int codes = 0;
+        if (warp >= kFirst)
+            for (int l0 = warp - kFirst; l0 < K; l0 += 8 * kStep) {
+                float v[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = have && l0 + e * kStep < K ? filter_value<U8>(P.g, P.filter, P.filter_u8, (size_t)(l0 + e * kStep) * Cout + j) : 0.0f;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) codes += have && l0 + e * kStep < K ? int(code_of(v[e], q.f_off, q.f_inv)) : 0;
+            }
+        if (warp >= kFirst) atomicAdd(sums + lane, codes);
+        __syncthreads();
+        if (warp == kFirst && have && AXC_SCRATCH_OK(P, P.bcode + j, 4, 323u)) P.bcode[j] = sums[lane];
     }
 }
 
-__global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
+template <bool U8>
+__global__ void __launch_bounds__(kPrepThreads, 2) xprep_kernel(const PrepParams P)
 {
     extern __shared__ __align__(16) float prep_smem[];
     pdl_trigger();
@@ -322,43 +387,64 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
         P.hdr->dirty = 0; P.hdr->fallback = 0; P.hdr->status = 0;
     }
     if (b < P.blocks_sum) {
-        prep_filter_sums(P, q, b, prep_smem);
+        prep_filter_sums<U8>(P, q, b, prep_smem);
         return;
     }
+    // sums of filter and patches first: their chains of additions are the longest work of a block
     b -= P.blocks_sum;
-    if (b < P.blocks_w) {
-        // wrow[tile][chunk][octet][k][slot]: where the table row of the slot's weight lies, in 16-byte units; wb[tile][chunk][lane]: the weight
-        // codes as B operand of the exact products
-        const int per_chunk = 16 * g.TNC;
-        const long long total = (long long)g.tiles_n * g.chunks * per_chunk;
-        for (long long x = (long long)b * 256 + tid; x < total; x += (long long)P.blocks_w * 256) {
-            const long long tc = x / per_chunk;
-            const int r = int(x - tc * per_chunk);
+    const int tiles = int(gridDim.x) - P.blocks_sum - P.blocks_w - P.blocks_t;
+    const unsigned z = code_of(0.0f, q.in_off, q.in_inv);        // code of a tap outside the image; codes are stored xor z
+    if (b >= tiles && b < tiles + P.blocks_w) {
+        b -= tiles;
+        // wrow[tile][chunk][octet][k][slot]: where the table row of the slot's weight lies, in 16-byte units; wb[tile][chunk][lane]:
+        // the weight codes as B operand of the exact products.  A warp takes a chunk at a time, eight weights (four of two-digit
+        // entries) per lane: all loads of a chunk are in flight together and nothing is divided per weight.
+        const int lane = tid & 31;
+        const long long total = (long long)g.tiles_n * g.chunks;
+        for (long long tc = (long long)b * (kPrepThreads / 32) + (tid >> 5); tc < total; tc += (long long)P.blocks_w * (kPrepThreads / 32)) {
             const int nt = int(tc / g.chunks), ch = int(tc - (long long)nt * g.chunks);
-            const int slot = r % g.TNC, kk = r / g.TNC;                          // kk = octet * 8 + t + 4p
-            const int i = ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);     // element 4t + 2*octet + p
-            const int j = nt * g.TNC + slot_channel(P.mode, slot), k = k_of(g, ch, i);
-            unsigned row = kNull;
-            if (k >= 0 && j < g.Cout) {
-                row = code_of(filter_value(g, P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
-                if (P.qf_debug) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(row);
+            const int slot = lane & (g.TNC - 1), cj = slot_channel(P.mode, slot), j = nt * g.TNC + cj;
+            const bool full = P.mode == kXtabFull;
+            float v[8];
+            int k[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int kk = full ? e * 4 + (lane >> 3) : (lane >> 4) * 8 + e;     // octet * 8 + t + 4p
+                const int i = ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);   // element 4t + 2*octet + p
+                k[e] = (!full || e < 4) && j < g.Cout ? k_of(g, ch, i) : -1;
+                v[e] = k[e] >= 0 ? filter_value<U8>(g, P.filter, P.filter_u8, (size_t)k[e] * g.Cout + j) : 0.0f;
             }
-            if (AXC_SCRATCH_OK(P, P.wrow + x, 2, 324u)) P.wrow[x] = uint16_t(row_address(P.mode, row) >> 4);
-            if (P.mode != kXtabFull) {
-                // B operand half h, column n: channel (n>>1)*4 + 2h + (n&1); lane (n, t) holds elements 4t..4t+3
-                const int cj = slot_channel(P.mode, slot), t = i >> 2, h = (cj >> 1) & 1, n = (cj >> 2) * 2 + (cj & 1);
-                unsigned char *w = reinterpret_cast<unsigned char *>(P.wb + tc * 32 + n * 4 + t) + h * 4 + (i & 3);
-                if (AXC_SCRATCH_OK(P, w, 1, 325u)) *w = row == kNull ? 0 : (unsigned char)row;
+            unsigned row[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                if (full && e >= 4) break;
+                row[e] = kNull;
+                if (k[e] >= 0) {
+                    row[e] = code_of(v[e], q.f_off, q.f_inv);
+                    if (P.qf_debug) P.qf_debug[(size_t)k[e] * g.Cout + j] = uint8_t(row[e]);
+                }
+                const int kk = full ? e * 4 + (lane >> 3) : (lane >> 4) * 8 + e;
+                uint16_t *w = P.wrow + tc * (16 * g.TNC) + kk * g.TNC + slot;
+                if (P.mode != kXtabExact && AXC_SCRATCH_OK(P, w, 2, 324u)) *w = uint16_t(row_address(P.mode, row[e]) >> 4);
+            }
+            if (!full) {
+                // B operand half h, column n: channel (n>>1)*4 + 2h + (n&1); lane (n, t) holds elements 4t..4t+3, of which this
+                // lane has 2*octet and the one after it
+                const int h = (cj >> 1) & 1, n = (cj >> 2) * 2 + (cj & 1);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    unsigned char *w = reinterpret_cast<unsigned char *>(P.wb + tc * 32 + n * 4 + t) + h * 4 + 2 * (lane >> 4);
+                    if (AXC_SCRATCH_OK(P, w, 2, 325u)) *reinterpret_cast<uint16_t *>(w) = uint16_t((row[t] & 0xFFu) | (row[4 + t] & 0xFFu) << 8);   // kNull: 0
+                }
             }
         }
         return;
     }
-    b -= P.blocks_w;
-    const unsigned z = code_of(0.0f, q.in_off, q.in_inv);        // code of a tap outside the image; codes are stored xor z
-    if (b < P.blocks_t) {
+    if (b >= tiles) {
+        b -= tiles + P.blocks_w;
         // transposed table: row = weight, column = stored code; row 256 = zeros
         const int total = 257 * 256;
-        for (int x = b * 256 + tid; x < total; x += P.blocks_t * 256) {
+        for (int x = b * kPrepThreads + tid; x < total; x += P.blocks_t * kPrepThreads) {
             const int w = x >> 8, a = (x & 255) ^ int(z);
             const int less = (P.mode == kXtabFull ? 128 * (a + w) * P.centred : a * w) + P.e_min;
             const int v = w < 256 ? int(__ldg(P.lut + a * 256 + w)) - less : 0;
@@ -368,9 +454,10 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
         }
         return;
     }
-    b -= P.blocks_t;
 
     // ---- an input tile: TH x TW output pixels of one image, the taps they read staged in shared memory ----------------
+    // Bound by memory where K is short, by the additions' order where it is long: a pixel's sum is a chain of K dependent
+    // additions (4 clocks each), so the host takes tiles that put as many pixels as possible on the chip at once (prep_tile).
     const int tx = b % P.tiles_x, rest = b / P.tiles_x;
     const int ty = rest % P.tiles_y, n = rest / P.tiles_y;
     const int oy0 = ty * P.TH, ox0 = tx * P.TW;
@@ -379,143 +466,246 @@ __global__ void __launch_bounds__(256) xprep_kernel(const PrepParams P)
     const int own_h = ty + 1 < P.tiles_y ? P.TH * g.sh : P.RH, own_w = tx + 1 < P.tiles_x ? P.TW * g.sw : P.RW;
     const unsigned zz = z * 0x01010101u;
     // codes[piece][pixel][16]: the pieces of neighbouring pixels lie side by side, so that the producers read whole lines
-    const int planes = g.N * g.H * g.W;
-    // centred tables: the sum of the codes of every staged pixel (z for one outside the image) behind the staged taps
-    int *pix_codes = reinterpret_cast<int *>(prep_smem + P.RH * P.RW * P.pitch);
-    if (P.acode && !g.im2col) {
-        for (int x = tid; x < P.RH * P.RW; x += 256)
-            if (staged_ok(P.RH * P.RW * P.pitch + x, 1, 327u)) pix_codes[x] = 0;
-        __syncthreads();
-    }
+    const int planes = g.N * g.H * g.W, region = P.RH * P.RW;
+    // the sum of the codes of every staged pixel (z for one outside the image) behind the staged taps, where it is asked for
+    int *pix_codes = reinterpret_cast<int *>(prep_smem + region * P.pitch);
+    unsigned char *const code_bytes = reinterpret_cast<unsigned char *>(prep_smem) + P.bytes_at;
     if (P.vec) {
+        // Eight lanes read 128 bytes of a pixel, a warp four pixels: whole sectors in, and 64-byte runs of codes out.  A thread keeps
+        // where its pixel's piece comes from and goes to, and steps along the channels (140 instructions per piece otherwise, twice
+        // what is left; the loop is bound by them).
         const int C4 = g.C >> 2;
         int lp = 1;
-        while (lp < C4 && lp < 32) lp <<= 1;                      // lanes per pixel
-        const int px_step = 256 / lp, c_lane = tid & (lp - 1);
+        while (lp < C4 && lp < 8) lp <<= 1;                       // lanes per pixel
+        const int px_step = kPrepThreads / lp, c_lane = tid & (lp - 1), c_blocks = (C4 + lp - 1) / lp, code_step = lp * planes;
         const int p = tid / lp;
-        int ry = p / P.RW, rx = p - ry * P.RW, c4 = c_lane;
+        int ry = p / P.RW, rx = p - ry * P.RW, cb = 0;
         const int step_y = px_step / P.RW, step_x = px_step - step_y * P.RW;
-        // eight pieces are requested before the first is used: the tile's load is a chain of memory latencies otherwise
-        // (cfg 56x56x64, 64 images: 63 us with one in flight)
-        constexpr int kBatch = 8;
-        while (ry < P.RH) {
+        int from = -1, at = -1, code_to = -1;                     // float4 of the input, float of the stage, word of the codes; -1: none
+        auto pixel = [&]() {
+            from = at = code_to = -1;
+            if (ry >= P.RH || c_lane >= C4) return;
+            const int iy = iy0 + ry, ix = ix0 + rx;
+            at = (ry * P.RW + rx) * P.pitch + c_lane * 4;
+            if (unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W)) {
+                const int pix = (n * g.H + iy) * g.W + ix;
+                from = pix * C4 + c_lane;
+                if (ry < own_h && rx < own_w) code_to = ((c_lane >> 2) * planes + pix) * 4 + (c_lane & 3);
+            }
+        };
+        pixel();
+        constexpr int kBatch = 4;                                 // loads of a thread in flight
+        int sum = 0, cb_done = 0, done = p;                       // code sum of the pixel being finished
+        for (int left = (region + px_step - 1) / px_step * c_blocks; left > 0; left -= kBatch) {
             float4 v[kBatch];
-            int at[kBatch];                                       // float offset in the staged region, -1: nothing
-            int code_at[kBatch];                                  // word offset of the codes, -1: not this tile's
-            int local[kBatch];                                    // pixel of the region
+            int to[kBatch], code_at[kBatch];
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
                 v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                at[u] = -1; code_at[u] = -1; local[u] = 0;
-                if (ry < P.RH && c4 < C4) {
-                    const int iy = iy0 + ry, ix = ix0 + rx;
-                    local[u] = ry * P.RW + rx;
-                    at[u] = local[u] * P.pitch + c4 * 4;
-                    if (unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W)) {
-                        const int pix = (n * g.H + iy) * g.W + ix;
-                        if (!AXC_GLOBAL_OK((long long)pix * C4 + c4, (long long)planes * C4, 328u)) {
-                        } else if (P.input_u8) {
-                            const uchar4 w = __ldg(reinterpret_cast<const uchar4 *>(P.input_u8 + (long long)pix * g.C) + c4);
-                            v[u] = make_float4(float(int(w.x) - P.pad), float(int(w.y) - P.pad), float(int(w.z) - P.pad), float(int(w.w) - P.pad));
-                        } else v[u] = __ldg(reinterpret_cast<const float4 *>(P.input + (long long)pix * g.C) + c4);
-                        if (ry < own_h && rx < own_w && !g.im2col) code_at[u] = ((c4 >> 2) * planes + pix) * 4 + (c4 & 3);
-                    }
+                const bool in_c = cb * lp + c_lane < C4;
+                to[u] = in_c ? at : -1;
+                code_at[u] = in_c ? code_to : -1;
+                if (from >= 0 && in_c && AXC_GLOBAL_OK((long long)from, (long long)planes * C4, 328u)) {
+                    if (U8) {
+                        const uchar4 w = __ldg(reinterpret_cast<const uchar4 *>(P.input_u8) + from);
+                        v[u] = make_float4(float(int(w.x) - P.pad), float(int(w.y) - P.pad), float(int(w.z) - P.pad), float(int(w.w) - P.pad));
+                    } else v[u] = __ldg(reinterpret_cast<const float4 *>(P.input) + from);
                 }
-                c4 += lp;
-                if (c4 >= C4) {
-                    c4 = c_lane;
+                if (++cb == c_blocks) {
+                    cb = 0;
                     rx += step_x; ry += step_y;
                     if (rx >= P.RW) { rx -= P.RW; ++ry; }
+                    pixel();
+                } else {
+                    if (from >= 0) from += lp;
+                    if (code_to >= 0) code_to += code_step;
+                    if (at >= 0) at += lp * 4;
                 }
             }
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
                 v[u].x = max_keep_nan(v[u].x, P.in_floor); v[u].y = max_keep_nan(v[u].y, P.in_floor);
                 v[u].z = max_keep_nan(v[u].z, P.in_floor); v[u].w = max_keep_nan(v[u].w, P.in_floor);
-                if (at[u] >= 0 && staged_ok(at[u], 4, 329u)) *reinterpret_cast<float4 *>(prep_smem + at[u]) = v[u];
-                if (code_at[u] >= 0 || (P.acode && at[u] >= 0 && !g.im2col)) {
-                    const unsigned w = code_of(v[u].x, q.in_off, q.in_inv) | code_of(v[u].y, q.in_off, q.in_inv) << 8 |
-                                       code_of(v[u].z, q.in_off, q.in_inv) << 16 | code_of(v[u].w, q.in_off, q.in_inv) << 24;
+                if (P.sums && to[u] >= 0 && staged_ok(to[u], 4, 329u)) *reinterpret_cast<float4 *>(prep_smem + to[u]) = v[u];
+                if (code_at[u] >= 0 || P.acode) {
+                    const unsigned w = codes_of(v[u], q.in_off, q.in_inv);
                     if (code_at[u] >= 0 && AXC_SCRATCH_OK(P, P.codes + (size_t)(unsigned)code_at[u] * 4, 4, 330u)) reinterpret_cast<unsigned *>(P.codes)[(unsigned)code_at[u]] = w ^ zz;
-                    if (P.acode && staged_ok(P.RH * P.RW * P.pitch + local[u], 1, 331u)) atomicAdd(pix_codes + local[u], int(__dp4a(w, 0x01010101u, 0u)));
+                    if (P.acode) {                                // (the same for all threads)
+                        if (to[u] >= 0) sum = int(__dp4a(w, 0x01010101u, unsigned(sum)));
+                        if (++cb_done == c_blocks) {
+                            for (int d = lp >> 1; d > 0; d >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
+                            if (c_lane == 0 && done < region && staged_ok(region * P.pitch + done, 1, 331u)) pix_codes[done] = sum;
+                            sum = cb_done = 0;
+                            done += px_step;
+                        }
+                    }
                 }
             }
         }
     } else {
-        const int row = P.RW * g.C;
-        for (int x = tid; x < P.RH * row; x += 256) {
-            const int ry = x / row, e = x - ry * row, rx = e / g.C, c = e - rx * g.C;
-            const int iy = iy0 + ry, ix = ix0 + rx;
-            const bool inside = unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W);
-            const long long pix = ((long long)n * g.H + iy) * g.W + ix;
-            float v = !inside || !AXC_GLOBAL_OK(pix * g.C + c, (long long)planes * g.C, 332u) ? 0.0f : P.input_u8 ? float(int(__ldg(P.input_u8 + pix * g.C + c)) - P.pad) : __ldg(P.input + pix * g.C + c);
-            v = max_keep_nan(v, P.in_floor);
-            if (staged_ok((ry * P.RW + rx) * P.pitch + c, 1, 333u)) prep_smem[(ry * P.RW + rx) * P.pitch + c] = v;
-            if (P.acode && !g.im2col && staged_ok(P.RH * P.RW * P.pitch + ry * P.RW + rx, 1, 334u)) atomicAdd(pix_codes + ry * P.RW + rx, int(code_of(v, q.in_off, q.in_inv)));
-            if (inside && ry < own_h && rx < own_w && !g.im2col && AXC_SCRATCH_OK(P, P.codes + ((long long)(c >> 4) * planes + pix) * 16 + (c & 15), 1, 335u))
-                P.codes[((long long)(c >> 4) * planes + pix) * 16 + (c & 15)] = (unsigned char)(code_of(v, q.in_off, q.in_inv) ^ z);
+        // The taps of a region row lie side by side in memory: a warp takes 256 of them at a time, eight loads in flight per lane.
+        if (P.acode && !g.im2col) {
+            for (int x = tid; x < region; x += kPrepThreads)
+                if (staged_ok(region * P.pitch + x, 1, 327u)) pix_codes[x] = 0;
+        }
+        const int row = P.RW * g.C, parts = (row + 255) >> 8, lane = tid & 31;
+        const int x_lo = ix0 * g.C, x_end = g.W * g.C;
+        const unsigned per_c = g.C > 1 ? 0xFFFFFFFFu / unsigned(g.C) + 1u : 0u;       // e / C for e * C < 2^32
+        for (int task = tid >> 5; task < P.RH * parts; task += kPrepThreads / 32) {
+            const int ry = task / parts, e0 = (task - ry * parts) * 256 + lane, iy = iy0 + ry;
+            const bool row_in = unsigned(iy) < unsigned(g.H);
+            const long long base = ((long long)n * g.H + iy) * x_end + x_lo;
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int e = e0 + u * 32;
+                const bool in = row_in && e < row && unsigned(x_lo + e) < unsigned(x_end) && AXC_GLOBAL_OK(base + e, (long long)planes * g.C, 332u);
+                v[u] = !in ? 0.0f : U8 ? float(int(__ldg(P.input_u8 + base + e)) - P.pad) : __ldg(P.input + base + e);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int e = e0 + u * 32;
+                if (e >= row) break;
+                v[u] = max_keep_nan(v[u], P.in_floor);
+                const int at = ry * P.RW * P.pitch + e + (P.pitch != g.C ? int(__umulhi(unsigned(e), per_c)) : 0);
+                if (staged_ok(at, 1, 333u)) prep_smem[at] = v[u];
+                if (g.im2col && staged_ok(P.bytes_at / 4 + (ry * P.bytes_pitch + e) / 4, 1, 334u)) code_bytes[ry * P.bytes_pitch + e] = (unsigned char)code_of(v[u], q.in_off, q.in_inv);
+            }
+        }
+        if (!g.im2col) {
+            // codes: a piece of a pixel per thread, neighbouring pixels side by side
+            __syncthreads();
+            for (int x = tid; x < region * g.CC; x += kPrepThreads) {
+                const int piece = x / region, local = x - piece * region, ry = local / P.RW, rx = local - ry * P.RW;
+                const int iy = iy0 + ry, ix = ix0 + rx;
+                const bool mine = unsigned(iy) < unsigned(g.H) && unsigned(ix) < unsigned(g.W) && ry < own_h && rx < own_w;
+                if (!mine && !P.acode) continue;
+                const float *src = prep_smem + local * P.pitch + piece * 16;
+                const int count = min(16, g.C - piece * 16);
+                if (!staged_ok(src - prep_smem, count, 335u)) continue;
+                unsigned w[4] = {0, 0, 0, 0};
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                    if (e < count) w[e >> 2] |= code_of(src[e], q.in_off, q.in_inv) << (8 * (e & 3));
+                if (P.acode && staged_ok(region * P.pitch + local, 1, 342u))
+                    atomicAdd(pix_codes + local, int(__dp4a(w[0], 0x01010101u, __dp4a(w[1], 0x01010101u, __dp4a(w[2], 0x01010101u, __dp4a(w[3], 0x01010101u, 0u))))));
+                uint4 *dst = reinterpret_cast<uint4 *>(P.codes) + ((size_t)piece * planes + ((size_t)n * g.H + iy) * g.W + ix);
+                if (mine && AXC_SCRATCH_OK(P, dst, 16, 343u)) *dst = make_uint4(w[0] ^ zz, w[1] ^ zz, w[2] ^ zz, w[3] ^ zz);
+            }
         }
     }
     __syncthreads();
     // patch sums (tf2/src/approx_nn_conv_kernels.cpp:272-295): the raw taps in K order, one thread per output pixel
-    for (int o = tid; o < P.TH * P.TW; o += 256) {
+    const int run = g.dw == 1 ? g.KW * g.C : g.C, runs_x = g.dw == 1 ? 1 : g.KW;      // taps that lie side by side (no padding between pixels)
+    for (int o = tid; o < P.TH * P.TW; o += kPrepThreads) {
         const int ly = o / P.TW, lx = o - ly * P.TW;
         const int oy = oy0 + ly, ox = ox0 + lx;
         if (oy >= g.OH || ox >= g.OW) continue;
         const long long m = ((long long)n * g.OH + oy) * g.OW + ox;
+        const int first = ly * g.sh * P.RW + lx * g.sw;            // region pixel of the first tap
         float s = 0.0f;
         int codes = 0;
-        if (!g.im2col) {
-            if (P.acode)
-                for (int ky = 0; ky < g.KH; ++ky)
-                    for (int kx = 0; kx < g.KW; ++kx) codes += pix_codes[(ly * g.sh + ky * g.dh) * P.RW + lx * g.sw + kx * g.dw];
+        if (!g.im2col && P.acode)
             for (int ky = 0; ky < g.KH; ++ky)
-                for (int kx = 0; kx < g.KW; ++kx) {
-                    const float *src = prep_smem + ((ly * g.sh + ky * g.dh) * P.RW + lx * g.sw + kx * g.dw) * P.pitch;
-                    if (!staged_ok(src - prep_smem, g.C, 336u)) continue;
-                    if (P.vec) {
-#pragma unroll 4
-                        for (int c = 0; c < g.C; c += 4) {
-                            const float4 v = *reinterpret_cast<const float4 *>(src + c);
-                            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
-                        }
-                    } else {
-#pragma unroll 4
-                        for (int c = 0; c < g.C; ++c) s = __fadd_rn(s, src[c]);
-                    }
+                for (int kx = 0; kx < g.KW; ++kx) codes += pix_codes[first + ky * g.dh * P.RW + kx * g.dw];
+        if (P.sums && P.vec && (g.C & 15) == 0) {
+            // 16 channels at a time over all taps, the next ones on their way while the last ones are added
+            const int steps = g.KH * g.KW * (g.C >> 4);
+            const float *src = prep_smem + first * P.pitch;
+            int c = 0, kx = 0;
+            float4 v[2][4];
+            auto take = [&](float4 (&to)[4]) {
+                if (!staged_ok(src - prep_smem, 16, 336u)) return;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) to[e] = reinterpret_cast<const float4 *>(src)[e];
+                src += 16; c += 16;
+                if (c == g.C) {
+                    c = 0;
+                    src += g.dw * P.pitch - g.C;
+                    if (++kx == g.KW) { kx = 0; src += (g.dh * P.RW - g.KW * g.dw) * P.pitch; }
                 }
-        } else {
-            unsigned w[4] = {0, 0, 0, 0};
-            int i = 0;
-            uint4 *dst = reinterpret_cast<uint4 *>(P.codes) + m;
-            for (int ky = 0; ky < g.KH; ++ky)
-                for (int kx = 0; kx < g.KW; ++kx) {
-                    const float *src = prep_smem + ((ly * g.sh + ky * g.dh) * P.RW + lx * g.sw + kx * g.dw) * P.pitch;
-                    if (!staged_ok(src - prep_smem, g.C, 337u)) continue;
-                    for (int c = 0; c < g.C; ++c) {
-                        const float v = src[c];
-                        s = __fadd_rn(s, v);
-                        const unsigned code = code_of(v, q.in_off, q.in_inv), byte = (code ^ z) << 24;
-                        codes += int(code);
-                        // four words shift along: the newest byte enters at the top of w[3]
-                        w[0] = __funnelshift_r(w[0], w[1], 8); w[1] = __funnelshift_r(w[1], w[2], 8);
-                        w[2] = __funnelshift_r(w[2], w[3], 8); w[3] = (w[3] >> 8) | byte;
-                        if (++i == 16) {
-                            if (AXC_SCRATCH_OK(P, dst, 16, 338u)) *dst = make_uint4(w[0], w[1], w[2], w[3]);
-                            dst += g.M;
-                            i = 0;
-                        }
-                    }
-                }
-            if (i > 0) {
-                for (; i < 16; ++i) {
-                    w[0] = __funnelshift_r(w[0], w[1], 8); w[1] = __funnelshift_r(w[1], w[2], 8);
-                    w[2] = __funnelshift_r(w[2], w[3], 8); w[3] >>= 8;
-                }
-                if (AXC_SCRATCH_OK(P, dst, 16, 339u)) *dst = make_uint4(w[0], w[1], w[2], w[3]);
+            };
+            auto add = [&](const float4 (&a)[4]) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, a[e].x), a[e].y), a[e].z), a[e].w);
+            };
+            take(v[0]);
+            int i = 1;
+            for (; i + 1 < steps; i += 2) {
+                take(v[1]);
+                add(v[0]);
+                take(v[0]);
+                add(v[1]);
             }
+            if (i < steps) {
+                take(v[1]);
+                add(v[0]);
+                add(v[1]);
+            } else add(v[0]);
+        } else if (P.sums && P.vec) {
+            for (int ky = 0; ky < g.KH; ++ky)
+                for (int kx = 0; kx < g.KW; ++kx) {
+                    const float *src = prep_smem + (first + ky * g.dh * P.RW + kx * g.dw) * P.pitch;
+                    if (!staged_ok(src - prep_smem, g.C, 337u)) continue;
+#pragma unroll 4
+                    for (int c = 0; c < g.C; c += 4) {
+                        const float4 v = *reinterpret_cast<const float4 *>(src + c);
+                        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
+                    }
+                }
+        } else if (P.sums) {
+            const bool joined = P.pitch == g.C;                   // a run crosses pixels only where they lie side by side
+            const int len = joined ? run : g.C, xs = joined ? runs_x : g.KW;
+            for (int ky = 0; ky < g.KH; ++ky)
+                for (int kx = 0; kx < xs; ++kx) {
+                    const float *src = prep_smem + (first + ky * g.dh * P.RW + kx * g.dw) * P.pitch;
+                    if (!staged_ok(src - prep_smem, len, 338u)) continue;
+#pragma unroll 8
+                    for (int c = 0; c < len; ++c) s = __fadd_rn(s, src[c]);
+                }
         }
-        if (AXC_SCRATCH_OK(P, P.asum + m, 4, 340u)) P.asum[m] = s;
+        if (g.im2col) {
+            // im2col rows of codes off the runs of taps that lie side by side in a region row, a word at a time: one aligned word read,
+            // one shift to the run's start, one to the place in the row (every word put together byte by byte: 25 instructions)
+            uint4 *dst = reinterpret_cast<uint4 *>(P.codes) + m;
+            const unsigned src0 = unsigned(P.bytes_at) + unsigned(ly * g.sh * P.bytes_pitch + lx * g.sw * g.C);
+            const unsigned *words = reinterpret_cast<const unsigned *>(prep_smem);
+            unsigned w[4] = {0, 0, 0, 0}, pending = 0;            // the last four words, and the bytes after them
+            int count = 0, bits = 0;
+            auto put = [&](unsigned v) {
+                w[0] = w[1]; w[1] = w[2]; w[2] = w[3]; w[3] = v;
+                if ((++count & 3) != 0) return;
+                codes += int(__dp4a(w[0], 0x01010101u, __dp4a(w[1], 0x01010101u, __dp4a(w[2], 0x01010101u, __dp4a(w[3], 0x01010101u, 0u)))));
+                if (AXC_SCRATCH_OK(P, dst, 16, 344u)) *dst = make_uint4(w[0] ^ zz, w[1] ^ zz, w[2] ^ zz, w[3] ^ zz);
+                dst += g.M;
+            };
+            for (int ky = 0; ky < g.KH; ++ky)
+                for (int kx = 0; kx < runs_x; ++kx) {
+                    const unsigned at = src0 + unsigned(ky * g.dh * P.bytes_pitch + kx * g.dw * g.C), shift = (at & 3u) * 8u;
+                    if (!staged_ok(at >> 2, (run + 7) / 4, 339u)) continue;
+                    const unsigned *src = words + (at >> 2);
+                    unsigned lo = *src++;
+                    for (int i = run >> 2; i > 0; --i) {
+                        const unsigned hi = *src++, v = __funnelshift_r(lo, hi, shift);
+                        lo = hi;
+                        put(pending | v << bits);
+                        pending = __funnelshift_rc(v, 0u, 32u - unsigned(bits));       // (a shift by 32 leaves nothing)
+                    }
+                    const int rest = (run & 3) * 8;
+                    if (rest > 0) {
+                        const unsigned v = __funnelshift_r(lo, *src, shift) & ((1u << rest) - 1u);
+                        pending |= v << bits;
+                        if ((bits += rest) >= 32) {
+                            bits -= 32;
+                            put(pending);
+                            pending = __funnelshift_rc(v, 0u, unsigned(rest - bits));
+                        }
+                    }
+                }
+            if (bits > 0) put(pending);
+            while (count & 3) put(0u);
+        }
+        if (P.sums && AXC_SCRATCH_OK(P, P.asum + m, 4, 340u)) P.asum[m] = s;
         if (P.acode && AXC_SCRATCH_OK(P, P.acode + m, 4, 341u)) P.acode[m] = codes;
     }
 }
@@ -578,7 +768,7 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
             const int k = k_of(g, ch, elem), cj = slot_channel(MODE, slot), j = nt * TNC + cj;
             unsigned row = kNull;
             if (k >= 0 && j < g.Cout) {
-                row = code_of(filter_value(g, P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
+                row = code_of(P.filter_u8 ? filter_value<true>(g, P.filter, P.filter_u8, (size_t)k * g.Cout + j) : filter_value<false>(g, P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
                 if (P.qf_debug) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(row);
             }
             if (AXC_SHARED_OK(lists + parity * (16u * TNC * 2u) + unsigned(kk * TNC + slot) * 2u, 2u, lists, bar, 350u))
@@ -1170,36 +1360,59 @@ struct XLayout {
     size_t tt, wrow, wb, asum, bsum, acode, bcode, partial, codes, xt, xt_bytes, total;
 };
 
-constexpr size_t kPrepSmem = 72 * 1024;        // three preparation tiles per SM
 constexpr size_t kPrepSmemMax = 220 * 1024;
 
 struct PrepTile {
-    int TH, TW, RH, RW, pitch, vec;
+    int TH, TW, RH, RW, pitch, vec, bytes_at, bytes_pitch;
     size_t smem;
 };
 
-// Output pixels per preparation tile: at most 256 (one per thread), as wide as an output row allows, within the shared
-// memory of three CTAs per SM where that is possible.
-bool prep_tile(const Geom &g, int vec, bool im2col, PrepTile *out)
+// Output pixels per preparation tile: at most one per thread, whatever is quickest by the clocks of a round: as many CTAs as shared
+// memory and registers (two) allow, each loading its region (20 bytes per clock and SM, a batch of loads 700, a piece 100) and then
+// adding K taps per pixel in a chain (4.5 clocks each, 32 taps per clock and SM at most).  Tiles of at most 72 KiB, as many as
+// fill it, left 14 of 256 threads adding at 14x14x256.  out == NULL: only whether there is such a tile.
+bool prep_tile(const Geom &g, int vec, bool im2col, bool sums, PrepTile *out)
 {
-    PrepTile t;
+    PrepTile t = {};
     t.vec = vec;
     // an odd number of 16-byte pieces (floats) per pixel keeps the lanes of the patch sums on different banks
-    if (vec) t.pitch = ((g.C >> 2) | 1) * 4;
+    if (vec) t.pitch = sums ? ((g.C >> 2) | 1) * 4 : 0;
     else t.pitch = im2col ? g.C : g.C | 1;
-    auto smem = [&](int th, int tw) {
-        const size_t rh = size_t(th - 1) * g.sh + size_t(g.KH - 1) * g.dh + 1, rw = size_t(tw - 1) * g.sw + size_t(g.KW - 1) * g.dw + 1;
-        return rh * rw * (t.pitch + 1) * 4;
-    };
-    t.TW = g.OW < 64 ? g.OW : 64;
-    while (t.TW > 1 && smem(1, t.TW) > kPrepSmem) t.TW = (t.TW + 1) / 2;
-    if (smem(1, t.TW) > kPrepSmemMax) return false;
-    t.TH = 1;
-    while (t.TH < g.OH && (t.TH + 1) * t.TW <= 256 && smem(t.TH + 1, t.TW) <= kPrepSmem) ++t.TH;
-    t.RH = (t.TH - 1) * g.sh + (g.KH - 1) * g.dh + 1;
-    t.RW = (t.TW - 1) * g.sw + (g.KW - 1) * g.dw + 1;
-    t.smem = smem(t.TH, t.TW);
-    if (t.smem < 32768) t.smem = 32768;        // the staging of the filter sums
+    auto region_h = [&](int th) { return size_t(th - 1) * g.sh + size_t(g.KH - 1) * g.dh + 1; };
+    auto region_w = [&](int tw) { return size_t(tw - 1) * g.sw + size_t(g.KW - 1) * g.dw + 1; };
+    // per pixel: the staged taps, then its code sum or (im2col) its codes
+    auto smem = [&](size_t rh, size_t rw) { return (rh * rw * (size_t(t.pitch) * 4 + (im2col ? size_t(g.C) : 4)) + 8 + 15) & ~size_t(15); };
+    if (smem(region_h(1), region_w(1)) > kPrepSmemMax) return false;
+    if (!out) return true;
+    double best = 1e300;
+    for (int parts = 1, last = 0; !last; parts = parts < 4 ? parts + 1 : parts * 2) {
+        last = parts >= g.OW;
+        const int tw = last ? 1 : (g.OW + parts - 1) / parts;
+        if (tw > kPrepThreads) continue;
+        const size_t rw = region_w(tw);
+        for (int th = 1; th <= g.OH && th * tw <= kPrepThreads; th += th < 8 ? 1 : 2) {
+            const size_t rh = region_h(th), bytes = smem(rh, rw);
+            if (bytes > kPrepSmemMax) break;
+            const size_t block = (bytes < kSumSmem ? kSumSmem : bytes) + 1024;
+            const int ctas = block * 2 <= 228 * 1024 ? 2 : 1;
+            const long long tiles = (long long)g.N * ((g.OH + th - 1) / th) * ((g.OW + tw - 1) / tw), slots = kModelSms * ctas;
+            const long long taps = (long long)rh * (long long)rw * g.C, per_batch = kPrepThreads * (vec ? 16 : 8);
+            const double rounds = double((tiles + slots - 1) / slots);
+            const double chain = sums ? 4.5 * g.K : 0.0, adds = sums ? double((th * tw + 31) / 32) * g.K : 0.0;
+            const double load = double(taps) * 4.0 / 20.0;
+            const double latency = 1000.0 + 700.0 * double((taps + per_batch - 1) / per_batch) + (vec ? 25.0 : 30.0) * double(taps / kPrepThreads);
+            const double one = latency + chain, all = double(tiles) / kModelSms * (load + adds);
+            const double cost = rounds * one > all ? rounds * one + 0.3 * all : all + 0.3 * rounds * one;
+            if (cost < best) {
+                best = cost;
+                t.TH = th; t.TW = tw; t.RH = int(rh); t.RW = int(rw);
+            }
+        }
+    }
+    t.smem = smem(size_t(t.RH), size_t(t.RW));
+    t.bytes_at = t.RH * t.RW * t.pitch * 4;
+    t.bytes_pitch = t.RW * g.C;
+    if (t.smem < kSumSmem) t.smem = kSumSmem;
     *out = t;
     return true;
 }
@@ -1362,8 +1575,7 @@ size_t xtab_scratch_bytes(const Geom &g, int mode)
     // 104 / 31 (94 / 25) at 1.5e7 - and a new filter's plan costs 1.2 to 22 ms on top.
     if ((double)g.M * g.K * g.Cout < kXtabMinLookups) return 0;
     XGeom x;
-    PrepTile t;
-    if (!xgeom(g, &x) || !prep_tile(g, g.C % 4 == 0, x.im2col != 0, &t) || !prep_tile(g, 0, x.im2col != 0, &t)) return 0;
+    if (!xgeom(g, &x) || !prep_tile(g, g.C % 4 == 0 && !x.im2col, x.im2col != 0, true, nullptr) || !prep_tile(g, 0, x.im2col != 0, true, nullptr)) return 0;
     return xlayout(g, x, mode).total;
 }
 
@@ -1388,9 +1600,10 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     const XLayout L = xlayout(g, x, mode);
     const size_t partial_bytes = size_t(g.M) * g.Cout * 4;
     const Config cf = choose_config(mode, x, di.sm_count, partial_bytes <= kPartialMax, L.xt_bytes);
-    const int vec = (g.C % 4 == 0 && (u8 ? (reinterpret_cast<uintptr_t>(u8->input) & 3u) : (reinterpret_cast<uintptr_t>(input) & 15u)) == 0) ? 1 : 0;
+    const int vec = (g.C % 4 == 0 && !x.im2col && (u8 ? (reinterpret_cast<uintptr_t>(u8->input) & 3u) : (reinterpret_cast<uintptr_t>(input) & 15u)) == 0) ? 1 : 0;
     PrepTile t;
-    if (!prep_tile(g, vec, x.im2col != 0, &t)) return AXC_INTERNAL;
+    A.sums = u8 ? 0 : 1;
+    if (!prep_tile(g, vec, x.im2col != 0, A.sums != 0, &t)) return AXC_INTERNAL;
     A.input_u8 = u8 ? u8->input : nullptr; A.filter_u8 = u8 ? u8->filter : nullptr; A.pad = u8 ? u8->input_offset & 255 : 0;
     A.input = input; A.filter = filter; A.lut = lut_dev; A.ranges = ranges_dev; A.host_q = host_dev_quant(q, g.K);
     A.in_floor = g.ep.input_relu ? 0.0f : -INFINITY;
@@ -1406,12 +1619,12 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     A.qf_debug = dbg ? dbg->qfilter : nullptr;
     A.hdr = reinterpret_cast<PlanHeader *>(scratch);
     A.scratch_bytes = P.scratch_bytes = (long long)L.total;
-    A.TH = t.TH; A.TW = t.TW; A.RH = t.RH; A.RW = t.RW; A.pitch = t.pitch; A.vec = t.vec;
+    A.TH = t.TH; A.TW = t.TW; A.RH = t.RH; A.RW = t.RW; A.pitch = t.pitch; A.vec = t.vec; A.bytes_at = t.bytes_at; A.bytes_pitch = t.bytes_pitch;
     A.tiles_y = (g.OH + t.TH - 1) / t.TH; A.tiles_x = (g.OW + t.TW - 1) / t.TW;
-    A.blocks_sum = (g.Cout + 31) / 32;
-    const long long w_items = (long long)x.tiles_n * x.chunks * 16 * x.TNC;
-    A.blocks_w = cf.pre ? 0 : int(w_items / 1024 + 1 < 592 ? w_items / 1024 + 1 : 592);
-    A.blocks_t = cf.pre ? 0 : 32;
+    A.blocks_sum = A.sums || A.bcode ? (g.Cout + 31) / 32 : 0;
+    const long long w_warps = (long long)x.tiles_n * x.chunks;
+    A.blocks_w = cf.pre ? 0 : int((w_warps + 15) / 16 < 296 ? (w_warps + 15) / 16 : 296);
+    A.blocks_t = cf.pre || mode == kXtabExact ? 0 : 32;
     const long long blocks = (long long)A.blocks_sum + A.blocks_w + A.blocks_t + (long long)g.N * A.tiles_y * A.tiles_x;
     if (blocks >= (1ll << 31)) return AXC_INTERNAL;
     P.partial = nullptr;
@@ -1419,8 +1632,9 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
         P.partial = reinterpret_cast<int32_t *>(scratch + L.partial);
         AXC_CUDA(cudaMemsetAsync(P.partial, 0, partial_bytes, stream));
     }
-    AXC_CUDA(cudaFuncSetAttribute(xprep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPrepSmemMax)));
-    xprep_kernel<<<unsigned(blocks), 256, t.smem, stream>>>(A);
+    const auto prep = u8 ? xprep_kernel<true> : xprep_kernel<false>;
+    AXC_CUDA(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPrepSmemMax)));
+    prep<<<unsigned(blocks), kPrepThreads, t.smem, stream>>>(A);
     AXC_CUDA(cudaGetLastError());
     count_launch();
 
