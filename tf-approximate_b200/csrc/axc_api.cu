@@ -97,7 +97,8 @@ size_t expanded_scratch_bytes(const axc_table *table, const Geom &g)
     if (dense_variant() != 0) return 0;
     int mode = kXtabAny, centred, e_min;
     if (table) {
-        if (sums_in_reference_order(table, g)) return 0;
+        // (a sum that is only too large for an int32 has no scratch: the quantised entry point asks here too, and refuses it)
+        if (sums_in_reference_order(table, g)) return g.accum == AXC_ACCUM_REFERENCE_F32 ? xtab_scratch_bytes(g, kXtabRef) : 0;
         table_form(table, &mode, &centred, &e_min);
     }
     return xtab_scratch_bytes(g, mode);
@@ -126,8 +127,9 @@ int describe_route(const axc_table *table, const Geom &g, size_t bytes, size_t g
     out4[1] = out4[2] = out4[3] = 0;
     const Route r = choose_route(table, g, bytes, general);
     if (g.M * g.Cout == 0 || !r.enough) return AXC_OK;
-    if (!r.expanded) {
-        out4[0] = plan_serves(g, sums_in_reference_order(table, g)) ? AXC_ROUTE_PLAN : AXC_ROUTE_COMMON_K;
+    const bool ref_order = sums_in_reference_order(table, g);
+    if (!r.expanded || ref_order) {
+        out4[0] = plan_serves(g, ref_order) ? AXC_ROUTE_PLAN : AXC_ROUTE_COMMON_K;
         return AXC_OK;
     }
     int mode, centred, e_min;

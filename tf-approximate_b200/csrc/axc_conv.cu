@@ -605,6 +605,7 @@ int launch_dense(const uint16_t *lut_dev, const axc_table *table, const Geom &g,
     if (expanded) {
         int mode, centred, e_min;
         table_form(table, &mode, &centred, &e_min);
+        if (ref_order) { mode = kXtabRef; centred = e_min = 0; }
         if (dbg && dbg->qinput) {
             rc = launch_quant(q, ranges_dev, g.K, static_cast<unsigned char *>(workspace), stream);
             if (rc == AXC_OK)

@@ -227,17 +227,19 @@ struct PrepParams {
     int bytes_at, bytes_pitch;                // im2col: codes of the staged taps behind the taps, bytes per region row
 };
 
+__host__ __device__ __forceinline__ bool two_bytes(int mode) { return mode == kXtabFull || mode == kXtabRef; }
+
 // channel of slot s in a piece: the order in which a lane's accumulators hold four neighbouring channels
 __device__ __forceinline__ int slot_channel(int mode, int s)
 {
-    if (mode == kXtabFull) return s;
+    if (two_bytes(mode)) return s;
     return ((s >> 3) << 3) + ((s >> 1) & 1) * 4 + ((s >> 2) & 1) * 2 + (s & 1);     // 0 1 4 5 2 3 6 7 8 9 12 13 10 11 14 15
 }
 
 // shared-memory address of a row of the transposed table
 __device__ __forceinline__ unsigned row_address(int mode, unsigned row)
 {
-    if (mode != kXtabFull) return kRowsHigh + row * 256u;
+    if (!two_bytes(mode)) return kRowsHigh + row * 256u;
     return row < unsigned(kLowRows) ? kRowsLow + row * 512u : kRowsHigh + (row - kLowRows) * 512u;
 }
 
@@ -404,13 +406,13 @@ __global__ void __launch_bounds__(kPrepThreads, 2) xprep_kernel(const PrepParams
         for (long long tc = (long long)b * (kPrepThreads / 32) + (tid >> 5); tc < total; tc += (long long)P.blocks_w * (kPrepThreads / 32)) {
             const int nt = int(tc / g.chunks), ch = int(tc - (long long)nt * g.chunks);
             const int slot = lane & (g.TNC - 1), cj = slot_channel(P.mode, slot), j = nt * g.TNC + cj;
-            const bool full = P.mode == kXtabFull;
+            const bool full = two_bytes(P.mode);
             float v[8];
             int k[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const int kk = full ? e * 4 + (lane >> 3) : (lane >> 4) * 8 + e;     // octet * 8 + t + 4p
-                const int i = ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);   // element 4t + 2*octet + p
+                const int i = P.mode == kXtabRef ? kk : ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);   // element 4t + 2*octet + p
                 k[e] = (!full || e < 4) && j < g.Cout ? k_of(g, ch, i) : -1;
                 v[e] = k[e] >= 0 ? filter_value<U8>(g, P.filter, P.filter_u8, (size_t)k[e] * g.Cout + j) : 0.0f;
             }
@@ -448,7 +450,9 @@ __global__ void __launch_bounds__(kPrepThreads, 2) xprep_kernel(const PrepParams
             const int w = x >> 8, a = (x & 255) ^ int(z);
             const int less = (P.mode == kXtabFull ? 128 * (a + w) * P.centred : a * w) + P.e_min;
             const int v = w < 256 ? int(__ldg(P.lut + a * 256 + w)) - less : 0;
-            if (!AXC_SCRATCH_OK(P, P.tt + x * (P.mode == kXtabFull ? 2 : 1), P.mode == kXtabFull ? 2 : 1, 326u)) continue;
+            if (!AXC_SCRATCH_OK(P, P.tt + x * (two_bytes(P.mode) ? 2 : 1), two_bytes(P.mode) ? 2 : 1, 326u)) continue;
+            if (P.mode == kXtabRef) reinterpret_cast<uint16_t *>(P.tt)[x] = w < 256 ? __ldg(P.lut + a * 256 + w) : 0;
+            else
             if (P.mode == kXtabFull) reinterpret_cast<uint16_t *>(P.tt)[x] = uint16_t(v % 255 + (v / 255) * 256);
             else P.tt[x] = (unsigned char)v;
         }
@@ -1334,6 +1338,23 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
     }
 }
 
+// launch of a kernel that calls pdl_wait() before it touches what earlier kernels of the stream leave
+template <typename Kernel, typename Params>
+int launch_dependent(Kernel kernel, unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const Params &P)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    AXC_CUDA(cudaLaunchKernelEx(&cfg, kernel, P));
+    count_launch();
+    return AXC_OK;
+}
+
+#include "axc_xref.cuh"
+
 // The dequantisation of a call whose K was split over CTAs.
 __global__ void __launch_bounds__(256) xfinal_kernel(const XParams P)
 {
@@ -1501,7 +1522,7 @@ XLayout xlayout(const Geom &g, const XGeom &x, int mode)
     L.bsum = off;    off += r256(size_t(g.Cout) * 4);
     L.acode = off;   off += r256(size_t(g.M) * 4);
     L.bcode = off;   off += r256(size_t(g.Cout) * 4);
-    L.partial = off; off += r256(size_t(g.M) * g.Cout * 4 <= kPartialMax ? size_t(g.M) * g.Cout * 4 : 0);
+    L.partial = off; off += r256(size_t(g.M) * g.Cout * 4 <= kPartialMax && mode != kXtabRef ? size_t(g.M) * g.Cout * 4 : 0);
     L.codes = off;   off += r256((x.im2col ? size_t(g.M) : size_t(g.N) * g.H * g.W) * x.CC * 16);
     // room for the expanded tables where a call would have them made in global memory
     L.xt = off;
@@ -1513,21 +1534,6 @@ XLayout xlayout(const Geom &g, const XGeom &x, int mode)
     off += L.xt_bytes;
     L.total = off;
     return L;
-}
-
-// launch of a kernel that calls pdl_wait() before it touches what earlier kernels of the stream leave
-template <typename Kernel, typename Params>
-int launch_dependent(Kernel kernel, unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const Params &P)
-{
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cfg.attrs = &attr; cfg.numAttrs = 1;
-    AXC_CUDA(cudaLaunchKernelEx(&cfg, kernel, P));
-    count_launch();
-    return AXC_OK;
 }
 
 template <int MODE, int NB, bool PRE>
@@ -1595,11 +1601,11 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     XParams P;
     if (!xgeom(g, &A.g)) return AXC_INTERNAL;
     XGeom &x = A.g;
-    x.TNC = mode == kXtabFull ? 8 : 16;
+    x.TNC = two_bytes(mode) ? 8 : 16;
     x.tiles_n = (g.Cout + x.TNC - 1) / x.TNC;
     const XLayout L = xlayout(g, x, mode);
     const size_t partial_bytes = size_t(g.M) * g.Cout * 4;
-    const Config cf = choose_config(mode, x, di.sm_count, partial_bytes <= kPartialMax, L.xt_bytes);
+    const Config cf = mode == kXtabRef ? Config{0, 1, x.chunks, false} : choose_config(mode, x, di.sm_count, partial_bytes <= kPartialMax, L.xt_bytes);
     const int vec = (g.C % 4 == 0 && !x.im2col && (u8 ? (reinterpret_cast<uintptr_t>(u8->input) & 3u) : (reinterpret_cast<uintptr_t>(input) & 15u)) == 0) ? 1 : 0;
     PrepTile t;
     A.sums = u8 ? 0 : 1;
@@ -1653,6 +1659,7 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     P.acode = A.acode; P.bcode = A.bcode;
     P.bias = g.ep.bias; P.residual = g.ep.residual; P.out_floor = g.ep.relu ? 0.0f : -INFINITY;
     P.k_e_min = int(unsigned(g.K) * (unsigned(e_min) + (u8 ? unsigned(u8->input_offset) * unsigned(u8->filter_offset) : 0u)));
+    if (mode == kXtabRef) return launch_ref(P, di, stream);
     P.splits = cf.splits; P.chunks_per_split = cf.chunks_per_split;
     P.units = ((long long)x.M + kWarps * 8 * cf.nb - 1) / (kWarps * 8 * cf.nb) * x.tiles_n * cf.splits;
     if (P.units >= (1ll << 31)) return AXC_INTERNAL;
