@@ -18,6 +18,7 @@ struct axc_table {
     int common_tz;               // trailing zero bits shared by all entries (16 for an all-zero table)
     int e_min, e_max;            // smallest and largest distance of an entry from the exact product
     int c_min, c_max;            // and of an entry from 128 (a + b)
+    bool e_period64;             // the distance from the exact product is the same for a and a + 64
     std::vector<uint16_t> host;  // 65536 entries, index (a << 8) | b
     std::mutex mu;
     std::vector<uint16_t *> dev;  // per-device replica, lazily created
@@ -51,6 +52,9 @@ void stamp(axc_table *t)
         t->c_min = c < t->c_min ? c : t->c_min;
         t->c_max = c > t->c_max ? c : t->c_max;
     }
+    t->e_period64 = true;
+    for (int i = 64 * 256; i < 65536 && t->e_period64; ++i)
+        t->e_period64 = int(t->host[size_t(i)]) - (i >> 8) * (i & 255) == int(t->host[size_t(i - 64 * 256)]) - ((i >> 8) - 64) * (i & 255);
 }
 
 void table_form(const axc_table *t, int *mode, int *centred, int *e_min)
@@ -60,7 +64,7 @@ void table_form(const axc_table *t, int *mode, int *centred, int *e_min)
     *centred = 0;
     *e_min = 0;
     if (span <= 255) {
-        *mode = span == 0 ? kXtabExact : kXtabByte;
+        *mode = span == 0 ? kXtabExact : t->e_period64 ? kXtabByte64 : kXtabByte;
         *e_min = t->e_min;
     } else if (int(t->max_entry) <= kTwoDigits) {
         *mode = kXtabFull;
@@ -285,16 +289,17 @@ static void append_rows(const axc_table *t, std::vector<uint16_t> *image)
 {
     int mode, centred, e_min;
     table_form(t, &mode, &centred, &e_min);
-    if (mode != kXtabFull && mode != kXtabByte) return;      // nothing reads rows of an exact table or of one without a form
+    if (mode != kXtabFull && mode != kXtabByte && mode != kXtabByte64) return;      // nothing reads rows of an exact table or of one without a form
     const size_t at = image->size();
-    image->resize(at + 257 * (mode == kXtabFull ? 256 : 128), 0);
+    const int bytes_per_row = mode == kXtabFull ? 512 : mode == kXtabByte ? 256 : 128;      // (kXtabByte64: its 64 entries twice)
+    image->resize(at + size_t(257 * bytes_per_row / 2), 0);
     uint16_t *digits = image->data() + at;
     uint8_t *bytes = reinterpret_cast<uint8_t *>(digits);
     for (int a = 0; a < 256; ++a) {
         const uint16_t *row = t->host.data() + a * 256;
         for (int b = 0; b < 256; ++b) {
-            const unsigned d = unsigned(int(row[b]) - (mode == kXtabByte ? a * b : centred * 128 * (a + b)) - e_min);
-            if (mode == kXtabByte) bytes[b * 256 + a] = uint8_t(d);
+            const unsigned d = unsigned(int(row[b]) - (mode != kXtabFull ? a * b : centred * 128 * (a + b)) - e_min);
+            if (mode != kXtabFull) bytes[b * bytes_per_row + a % bytes_per_row] = uint8_t(d);
             else digits[b * 256 + a] = uint16_t(d + d / 255u);     // (d mod 255) + 256 (d div 255)
         }
     }

@@ -57,6 +57,8 @@ constexpr unsigned kRowsLow = 35840u;
 constexpr unsigned kTab = 65536u;
 constexpr unsigned kRowsHigh = 131072u;
 constexpr unsigned kWindowEnd = 233472u;
+constexpr unsigned kRowsSmall = 19456u;        // rows that repeat every 64 activations: the transposed table
+constexpr unsigned kWindowHalf = 98304u;       // and where the window ends, two CTAs to an SM
 constexpr int kLowRows = 58;
 constexpr int kWarps = 8;
 constexpr int kNull = 256;                     // table row of a weight that does not exist: all zeros
@@ -147,7 +149,7 @@ __device__ __forceinline__ void mbar_drain(unsigned bar, unsigned parity)
     mbar_wait(bar, parity, ok, kWaitPolls);
 }
 
-// Programmatic dependent launch: the three kernels of a call are launched so that each may start while the one before it
+// Programmatic dependent launch: the kernels of a call after the first are launched so that each may start while the one before it
 // runs.  pdl_trigger: the next kernel may be brought in; pdl_wait: everything before this kernel is complete and visible.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -214,6 +216,8 @@ struct PrepParams {
     float in_floor;
     int mode, centred, e_min;
     int *acode, *bcode;         // sums of activation / weight codes where the end of the call needs them, else NULL
+    uint4 *zeros;               // integer sums of a call whose K is split, to be set to zero: 16-byte pieces of them, or NULL
+    long long zero_pieces;
     unsigned char *codes, *tt;
     uint16_t *wrow;
     uint2 *wb;
@@ -239,6 +243,7 @@ __device__ __forceinline__ int slot_channel(int mode, int s)
 // shared-memory address of a row of the transposed table
 __device__ __forceinline__ unsigned row_address(int mode, unsigned row)
 {
+    if (mode == kXtabByte64) return kRowsSmall + row * 128u;
     if (!two_bytes(mode)) return kRowsHigh + row * 256u;
     return row < unsigned(kLowRows) ? kRowsLow + row * 512u : kRowsHigh + (row - kLowRows) * 512u;
 }
@@ -380,6 +385,9 @@ __global__ void __launch_bounds__(kPrepThreads, 2) xprep_kernel(const PrepParams
     pdl_trigger();
     const XGeom &g = P.g;
     const int tid = threadIdx.x;
+    if (P.zeros)
+        for (long long x = (long long)blockIdx.x * kPrepThreads + tid; x < P.zero_pieces; x += (long long)gridDim.x * kPrepThreads)
+            if (AXC_SCRATCH_OK(P, P.zeros + x, 16, 345u)) P.zeros[x] = make_uint4(0, 0, 0, 0);
     const DevQuant q = P.ranges ? dev_quant_from_ranges(P.ranges, g.K) : P.host_q;
     int b = int(blockIdx.x);
     if (b == 0 && tid == 0) {
@@ -445,9 +453,10 @@ __global__ void __launch_bounds__(kPrepThreads, 2) xprep_kernel(const PrepParams
     if (b >= tiles) {
         b -= tiles + P.blocks_w;
         // transposed table: row = weight, column = stored code; row 256 = zeros
-        const int total = 257 * 256;
+        const int row_shift = P.mode == kXtabByte64 ? 7 : 8;       // (64 entries, twice)
+        const int total = 257 << row_shift;
         for (int x = b * kPrepThreads + tid; x < total; x += P.blocks_t * kPrepThreads) {
-            const int w = x >> 8, a = (x & 255) ^ int(z);
+            const int w = x >> row_shift, a = (x & ((1 << row_shift) - 1)) ^ int(z);
             const int less = (P.mode == kXtabFull ? 128 * (a + w) * P.centred : a * w) + P.e_min;
             const int v = w < 256 ? int(__ldg(P.lut + a * 256 + w)) - less : 0;
             if (!AXC_SCRATCH_OK(P, P.tt + x * (two_bytes(P.mode) ? 2 : 1), two_bytes(P.mode) ? 2 : 1, 326u)) continue;
@@ -733,7 +742,7 @@ struct ExpandParams {
     long long scratch_bytes;
 };
 
-// xt[channel tile][chunk][row a][piece kk][16 bytes], kk = octet * 8 + k.  The table's rows (one per weight) lie in shared memory.
+// xt[channel tile][chunk][row a][piece kk][16 bytes], kk = octet * 8 + k; 64 rows where they repeat, else 256.  The table's rows (one per weight) lie in shared memory.
 // A lane reads the same word (two or four a) of the rows of its piece's 8 or 16 weights, transposes in registers and writes
 // whole pieces; the 32 lanes (8 k x 4 words) read 32 different banks whatever the weights are, and write 128-byte runs.
 // Bound by the writes, 64 KiB per chunk (gathering entry by entry with random banks took 12 700 clocks per chunk, this 1500).
@@ -741,8 +750,9 @@ template <int MODE>
 __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const ExpandParams P)
 {
     constexpr int TNC = MODE == kXtabFull ? 8 : 16;
-    constexpr unsigned kRow = MODE == kXtabFull ? 512u : 256u;     // bytes of a table row
-    constexpr int kRounds = MODE == kXtabFull ? 64 : 32;           // warp rounds per chunk
+    constexpr unsigned kRow = MODE == kXtabFull ? 512u : MODE == kXtabByte ? 256u : 128u;     // bytes of a table row
+    constexpr int kRounds = MODE == kXtabFull ? 64 : MODE == kXtabByte ? 32 : 8;               // warp rounds per chunk
+    constexpr unsigned kRowsA = MODE == kXtabByte64 ? 64u : 256u;                              // rows of the expanded table
     extern __shared__ __align__(16) unsigned char expand_smem[];
     const XGeom &g = P.g;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -757,7 +767,7 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
     }
     __syncthreads();
     const DevQuant q = P.ranges ? dev_quant_from_ranges(P.ranges, g.K) : P.host_q;
-    const unsigned z = code_of(0.0f, q.in_off, q.in_inv);
+    const unsigned z = code_of(0.0f, q.in_off, q.in_inv) & (kRowsA - 1u);
     bool ok = true;
     mbar_wait(bar, 0u, ok, AXC_WAIT_POLLS(0));
     // thread (kk, slot) of the first 16*TNC prepares the list of table rows of a chunk
@@ -797,8 +807,8 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
 #pragma unroll
                 for (int s = 0; s < 8; ++s) v[s4 * 8 + s] = lds32(tab + ((s & 1) ? l4[s >> 1] >> 16 : l4[s >> 1] & 0xFFFFu) * kRow + word * 4u);
             }
-            uint4 *dst = reinterpret_cast<uint4 *>(P.xt + (size_t)tc * 65536u) + o * 8 + kidx;
-            if (!AXC_SCRATCH_OK(P, dst, 255 * 256 + 16, 352u)) continue;      // the rows a of this piece
+            uint4 *dst = reinterpret_cast<uint4 *>(P.xt + (size_t)tc * (kRowsA * 256u)) + o * 8 + kidx;
+            if (!AXC_SCRATCH_OK(P, dst, (kRowsA - 1u) * 256 + 16, 352u)) continue;      // the rows a of this piece
             if (MODE == kXtabFull) {
                 const unsigned a = word * 2u;
                 dst[(a ^ z) * 16u] = make_uint4(prmt<0x5410>(v[0], v[1]), prmt<0x5410>(v[2], v[3]), prmt<0x5410>(v[4], v[5]), prmt<0x5410>(v[6], v[7]));
@@ -813,7 +823,7 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
                     w4[2][w] = prmt<0x5410>(t2, t3); w4[3][w] = prmt<0x7632>(t2, t3);
                 }
 #pragma unroll
-                for (unsigned i = 0; i < 4; ++i) dst[((word * 4u + i) ^ z) * 16u] = make_uint4(w4[i][0], w4[i][1], w4[i][2], w4[i][TNC / 4 - 1]);
+                for (unsigned i = 0; i < 4; ++i) dst[(((word * 4u + i) & (kRowsA - 1u)) ^ z) * 16u] = make_uint4(w4[i][0], w4[i][1], w4[i][2], w4[i][TNC / 4 - 1]);
             }
         }
     }
@@ -864,12 +874,20 @@ __device__ __forceinline__ float dequantise(const DevQuant &Q, int total, float 
 // block pairs are in flight while the MMAs of the last two run.
 // PRE: the expanded tables come from global memory (xexpand_kernel) by bulk copies, 64 KiB per 16 elements of K, which cost the
 // shared-memory pipe next to nothing (measured: 2 to 4 % beside a stream of LDS.128 + MMA); otherwise they are built here.
+// W: warps.  Where the rows repeat, an expanded table is a quarter as large and half of a tile and its tables fit half of an SM: two
+// CTAs of four warps then, and one looks up while the other waits, starts or ends a tile.
+template <int MODE>
+constexpr int kWarpsOf = MODE == kXtabByte64 ? 4 : kWarps;
+
 template <int MODE, int NB, bool PRE>
-__global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
+__global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 : 1) xtab_kernel(const XParams P)
 {
-    constexpr int kPix = kWarps * 8 * NB;
+    constexpr int W = kWarpsOf<MODE>;
+    constexpr int kPix = W * 8 * NB;
     constexpr int TNC = MODE == kXtabFull ? 8 : 16, HV = TNC / 8;
     constexpr bool kTables = MODE != kXtabExact, kBuild = kTables && !PRE;
+    constexpr bool kSmall = MODE == kXtabByte64, kBytes = kSmall || MODE == kXtabByte;
+    constexpr unsigned kChunkTable = kSmall ? 16384u : 65536u;     // expanded table of 16 elements of K
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const XGeom &g = P.g;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -877,24 +895,25 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
     unsigned dyn_size;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_size));
     const unsigned bars = (dyn0 + 15u) & ~15u;
-    const unsigned tab_full = bars, tab_empty = bars + 16u, rows_full = bars + 32u, asked = bars + 40u;
+    const unsigned tab_full = bars, tab_empty = bars + 32u, rows_full = bars + 64u, asked = bars + 72u;
+    pdl_trigger();
     pdl_wait();
-    if (asked + 4u > kCodes || dyn0 + dyn_size < kWindowEnd) {
+    if (asked + 4u > kCodes || dyn0 + dyn_size < (kSmall ? kWindowHalf : kWindowEnd)) {
         if (tid == 0) atomicExch(const_cast<int *>(&P.hdr->status), 2);      // (xprep_kernel, which clears it, is complete)
         return;
     }
     if (tid == 0) {
         if (PRE) asm volatile("st.shared.u32 [%0], %1;" ::"r"(asked), "r"(0xFFFFFFFFu) : "memory");
-        for (int s = 0; s < 2; ++s) { mbar_init(tab_full + s * 8, PRE ? 1 : kWarps); mbar_init(tab_empty + s * 8, kWarps); }
+        for (int s = 0; s < 2; ++s) { mbar_init(tab_full + s * 8, PRE ? 1 : W); mbar_init(tab_empty + s * 8, W); }
         mbar_init(rows_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (kBuild) {
             // the transposed table stays for the CTA's lifetime
-            constexpr unsigned low = MODE == kXtabFull ? kLowRows * 512u : 0u, high = MODE == kXtabFull ? (257u - kLowRows) * 512u : 257u * 256u;
+            constexpr unsigned low = MODE == kXtabFull ? kLowRows * 512u : 0u, high = MODE == kXtabFull ? (257u - kLowRows) * 512u : 257u * (kSmall ? 128u : 256u);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(rows_full), "r"(low + high) : "memory");
             if (low > 0) bulk_copy(kRowsLow, P.tt, low, rows_full);
-            bulk_copy(kRowsHigh, P.tt + low, high, rows_full);
+            bulk_copy(kSmall ? kRowsSmall : kRowsHigh, P.tt + low, high, rows_full);
         }
     }
     __syncthreads();
@@ -981,7 +1000,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
     // entries, whose 16 channels are shared by two lanes) and writes the expanded rows of those a.  The 32 lanes read 32
     // different banks, whatever the weights, and write different bank groups.
     const int kidx = lane & 7, sub = lane >> 3;
-    const int hf = MODE == kXtabByte ? sub & 1 : 0;
+    const int hf = kBytes ? sub & 1 : 0;
     unsigned raw[8];
     unsigned b_unit = blockIdx.x;
     int b_left = 0;                                                // octets left to build in b_unit
@@ -1006,7 +1025,10 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
     };
     // Words of a row that the lane works on: 32 r + (4 (warp + kidx) + sub) mod 32 in round r (8-bit entries: 32 (r / 2) + .. with
     // the two lanes that share a piece's channels swapped in odd rounds), so that a round is a constant offset.
-    const unsigned word0 = (4u * (unsigned(warp) + unsigned(kidx)) + unsigned(sub)) & 31u, word1 = word0 ^ 1u;
+    // Rows that repeat have 16 words, kept twice: two rounds of the four warps cover them, the lanes of the second copy with the low
+    // bit swapped so that both channel halves meet all of them.
+    const unsigned turn = (unsigned(warp) + unsigned(kidx)) & 7u;
+    const unsigned word0 = 4u * turn + (kSmall ? unsigned(sub) ^ (turn >> 2) : unsigned(sub)), word1 = word0 ^ 1u;
     unsigned row_at[8];
     auto build_rows = [&]() {
         const unsigned w4[4] = {wq.x, wq.y, wq.z, wq.w};
@@ -1014,14 +1036,15 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         for (int s = 0; s < 8; ++s) row_at[s] = ((s & 1) ? w4[s >> 1] >> 16 : w4[s >> 1] & 0xFFFFu) * 16u + word0 * 4u;
     };
     auto build_load = [&](int r) {
-        const unsigned odd = MODE == kXtabByte && (r & 1) ? word1 * 4u - word0 * 4u : 0u;
+        const unsigned odd = kSmall && r == 1 ? (word0 ^ 17u) * 4u - word0 * 4u : kBytes && (r & 1) ? word1 * 4u - word0 * 4u : 0u;
 #pragma unroll
-        for (int s = 0; s < 8; ++s) raw[s] = lds32(row_at[s] + odd + (MODE == kXtabByte ? unsigned(r >> 1) : unsigned(r)) * 128u);
+        for (int s = 0; s < 8; ++s) raw[s] = lds32(row_at[s] + odd + (kBytes ? unsigned(r >> 1) : unsigned(r)) * 128u);
     };
     auto build_store = [&](int r, unsigned st) {
-        const unsigned word = MODE == kXtabByte && (r & 1) ? word1 : word0;
-        const unsigned dst = kTab + st * 128u + unsigned(kidx) * 16u + unsigned(hf) * 8u +
-                             (MODE == kXtabFull ? word * 512u + unsigned(r) * 16384u : word * 1024u + unsigned(r >> 1) * 32768u);
+        // (rows that repeat: st = the octet's place among the 4 of two chunks, two to a row of 256 bytes)
+        const unsigned word = kSmall ? (word0 ^ unsigned(r)) & 15u : kBytes && (r & 1) ? word1 : word0;
+        const unsigned dst = kTab + (kSmall ? (st >> 1) * kChunkTable + (st & 1u) * 128u : st * 128u) + unsigned(kidx) * 16u + unsigned(hf) * 8u +
+                             (MODE == kXtabFull ? word * 512u + unsigned(r) * 16384u : word * 1024u + (kSmall ? 0u : unsigned(r >> 1) * 32768u));
         if (MODE == kXtabFull) {
             sts128(dst, make_uint4(prmt<0x5410>(raw[0], raw[1]), prmt<0x5410>(raw[2], raw[3]), prmt<0x5410>(raw[4], raw[5]), prmt<0x5410>(raw[6], raw[7])));
             sts128(dst + 256u, make_uint4(prmt<0x7632>(raw[0], raw[1]), prmt<0x7632>(raw[2], raw[3]), prmt<0x7632>(raw[4], raw[5]), prmt<0x7632>(raw[6], raw[7])));
@@ -1050,13 +1073,13 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
             int nt, m0, c_begin, c_end;
             coords(x_unit, nt, m0, c_begin, c_end);
             x_left = c_end - c_begin;
-            x_src = P.xt + ((size_t)nt * g.chunks + c_begin) * 65536u;
+            x_src = P.xt + ((size_t)nt * g.chunks + c_begin) * kChunkTable;
         }
-        if (!AXC_SCRATCH_OK(P, x_src, 65536, 311u)) { ok = false; return; }
+        if (!AXC_SCRATCH_OK(P, x_src, kChunkTable, 311u)) { ok = false; return; }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tab_full + buf * 8), "r"(65536u) : "memory");
-        bulk_copy(kTab * (1u + buf), x_src, 65536u, tab_full + buf * 8);
-        x_src += 65536;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tab_full + buf * 8), "r"(kChunkTable) : "memory");
+        bulk_copy(kSmall ? kTab + buf * kChunkTable : kTab * (1u + buf), x_src, kChunkTable, tab_full + buf * 8);
+        x_src += kChunkTable;
         --x_left;
     };
 
@@ -1094,6 +1117,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         const unsigned q = cw[i] ^ zz;
         mma_k32(acc[i * HV / 2], q, 0u, 0u, q, wb.x, wb.y);
     };
+    unsigned ring = 0;                                             // rows that repeat: place of the chunk's table, in the upper bits of every code byte
+    auto row_of = [&](unsigned codes) { return kSmall ? (codes & 0x3F3F3F3Fu) | ring : codes; };
     auto octet = [&](int h, unsigned toff, unsigned st, unsigned oct, bool more, uint2 wb) {
         const unsigned l0 = lane_k0 + toff, l1 = lane_k1 + toff;
         // address = {low byte of l, code byte, upper half of l}
@@ -1102,7 +1127,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         auto request = [&](int n, uint4 (&v)[4]) {
             const int i = (n >> 1) * 2;                            // pairs i, i + 1
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = lds128((n & 1) ? prmt_r(l1, cw[2 * i + e], s1) : prmt_r(l0, cw[2 * i + e], s0));
+            for (int e = 0; e < 4; ++e) v[e] = lds128((n & 1) ? prmt_r(l1, row_of(cw[2 * i + e]), s1) : prmt_r(l0, row_of(cw[2 * i + e]), s0));
         };
         request(0, x[0]);
         if (h == 0) fetch_begin();
@@ -1135,7 +1160,20 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
                 if (ok) copy_table(st ^ 1u);
                 else asm volatile("st.shared.u32 [%0], %1;" ::"r"(asked), "r"(min(lds32(asked), oct + 1u)) : "memory");   // the buffer's last copy may be in flight
             }
-            if (kBuild && more) {
+            if (kBuild && kSmall && more) {                            // oct: chunk; octet h of the next one, in two rounds
+                if (n == 0) {
+                    build_next();
+                    // the place's last readers worked on the chunk before this one
+                    if (h == 0 && oct > 0) mbar_wait(tab_empty + ((oct + 1u) & 1u) * 8, ((oct - 1u) >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
+                    build_rows();
+                    build_load(0);
+                }
+                if (n == (kSteps < 4 ? 1 : 2)) {
+                    build_store(0, ((oct + 1u) & 1u) * 2u + unsigned(h));
+                    build_load(1);
+                }
+                if (n == kSteps - 1) build_store(1, ((oct + 1u) & 1u) * 2u + unsigned(h));
+            } else if (kBuild && more) {
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     if (n == r * kSteps / 4) {
@@ -1153,8 +1191,13 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         }
         __syncwarp();                                              // also: every lane has the codes before the next are asked for
         if (lane == 0) {
-            if (kBuild && more) mbar_arrive(tab_full + (st ^ 1u) * 8);
-            if (kBuild || h == 1) mbar_arrive(tab_empty + st * 8);
+            if (kBuild && kSmall) {
+                if (h == 1 && more) mbar_arrive(tab_full + ((oct + 1u) & 1u) * 8);
+                if (h == 1) mbar_arrive(tab_empty + (oct & 1u) * 8);
+            } else {
+                if (kBuild && more) mbar_arrive(tab_full + (st ^ 1u) * 8);
+                if (kBuild || h == 1) mbar_arrive(tab_empty + st * 8);
+            }
         }
     };
 
@@ -1178,13 +1221,25 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         if (kBuild) {
             build_unit();
             build_next();
-            build_next();
             mbar_wait(rows_full, 0u, ok, AXC_WAIT_POLLS(1));
-            build_rows();
+            if (kSmall) {
+                for (unsigned o = 0; o < 2u; ++o) {                       // a chunk
+                    build_next();
+                    build_rows();
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                build_load(r);
-                build_store(r, 0u);
+                    for (int r = 0; r < 2; ++r) {
+                        build_load(r);
+                        build_store(r, o);
+                    }
+                }
+            } else {
+                build_next();
+                build_rows();
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    build_load(r);
+                    build_store(r, 0u);
+                }
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -1211,9 +1266,15 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
             if (MODE != kXtabFull && c + 1 < c_end && AXC_SCRATCH_OK(P, wbp, 8, 317u)) wb_next = __ldg(wbp);
             if (PRE) {
                 const unsigned st = chunk & 1u;
+                ring = st * 0x40404040u;
                 mbar_wait(tab_full + st * 8, (chunk >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
 #pragma unroll
-                for (int h = 0; h < 2; ++h) octet(h, st * kTab + unsigned(h) * 128u, st, chunk, true, wb);
+                for (int h = 0; h < 2; ++h) octet(h, (kSmall ? 0u : st * kTab) + unsigned(h) * 128u, st, chunk, true, wb);
+            } else if (kTables && kSmall) {
+                ring = (chunk & 1u) * 0x40404040u;
+                mbar_wait(tab_full + (chunk & 1u) * 8, (chunk >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
+#pragma unroll
+                for (int h = 0; h < 2; ++h) octet(h, unsigned(h) * 128u, 0u, chunk, 2u * chunk + 2u < oct_total, wb);
             } else if (kTables) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h, ++oct) {
@@ -1251,7 +1312,16 @@ __global__ void __launch_bounds__(kWarps * 32, 1) xtab_kernel(const XParams P)
         if (left > 0 && P.acode && !AXC_SCRATCH_OK(P, P.acode + g.M - 1, 4, 319u)) left = 0;
         const long long at0 = (long long)(m0 + first) * g.Cout + j0;
         const int row = kStep * g.Cout;
-        if (P.plain && whole && P.acc_out) {
+        if (P.partial && whole) {
+            // K split over CTAs: nothing but the additions, in as few instructions as the other cases below
+            int32_t *sums = P.partial + at0;
+#pragma unroll
+            for (int i = 0; i < kAcc; ++i) {
+                if (i * kStep >= left || !AXC_SCRATCH_OK(P, sums + i * row, 16, 342u)) continue;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) atomicAdd(sums + i * row + e, acc[i][e]);
+            }
+        } else if (P.plain && whole && P.acc_out) {
             int32_t *ints = P.acc_out + at0;
 #pragma unroll
             for (int i = 0; i < kAcc; ++i) {
@@ -1358,17 +1428,40 @@ int launch_dependent(Kernel kernel, unsigned grid, unsigned threads, size_t smem
 // The dequantisation of a call whose K was split over CTAs.
 __global__ void __launch_bounds__(256) xfinal_kernel(const XParams P)
 {
+    pdl_trigger();
+    pdl_wait();
     const DevQuant Q = *reinterpret_cast<const DevQuant *>(reinterpret_cast<const unsigned char *>(P.hdr) + kDevQuantOffset);
-    const long long total = (long long)P.g.M * P.g.Cout;
-    for (long long x = (long long)blockIdx.x * 256 + threadIdx.x; x < total; x += (long long)gridDim.x * 256) {
-        const int m = int(x / P.g.Cout), j = int(x - (long long)m * P.g.Cout);
-        if (!AXC_SCRATCH_OK(P, P.partial + x, 4, 360u) || !AXC_SCRATCH_OK(P, P.asum + m, 4, 361u)) continue;
-        const int tot = P.partial[x] + P.k_e_min + (P.acode ? P.a_coef * __ldg(P.acode + m) + P.b_coef * __ldg(P.bcode + j) : 0);
-        float y = dequantise(Q, tot, __ldg(P.asum + m), __fmul_rn(Q.m1, __ldg(P.bsum + j)));
+    // (at most 2^24 sums: kPartialMax)
+    const unsigned total = unsigned(P.g.M) * unsigned(P.g.Cout), Cout = unsigned(P.g.Cout);
+    auto one = [&](unsigned x, unsigned m, unsigned j, int sum, float a_sum, int a_code, float res) {
+        const int tot = sum + P.k_e_min + a_code + (P.bcode ? P.b_coef * __ldg(P.bcode + j) : 0);
+        float y = dequantise(Q, tot, a_sum, __fmul_rn(Q.m1, __ldg(P.bsum + j)));
         if (P.bias) y = __fadd_rn(y, __ldg(P.bias + j));
-        if (P.residual) y = __fadd_rn(y, __ldg(P.residual + x));
-        if (P.output) P.output[x] = max_keep_nan(y, P.out_floor);
+        if (P.residual) y = __fadd_rn(y, res);
         if (P.acc_out) P.acc_out[x] = tot;
+        return max_keep_nan(y, P.out_floor);
+    };
+    const unsigned step = gridDim.x * 256u, first = blockIdx.x * 256u + threadIdx.x;
+    if (Cout % 4 == 0 && ((reinterpret_cast<uintptr_t>(P.output) | reinterpret_cast<uintptr_t>(P.residual)) & 15u) == 0) {
+        for (unsigned v = first; v < total / 4; v += step) {
+            const unsigned x = v * 4, m = x / Cout, j = x - m * Cout;
+            if (!AXC_SCRATCH_OK(P, P.partial + x, 16, 360u) || !AXC_SCRATCH_OK(P, P.asum + m, 4, 361u)) continue;
+            const int4 sum = *reinterpret_cast<const int4 *>(P.partial + x);
+            const float a_sum = __ldg(P.asum + m);
+            const int a_code = P.acode ? P.a_coef * __ldg(P.acode + m) : 0;
+            const float4 res = P.residual ? __ldg(reinterpret_cast<const float4 *>(P.residual + x)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 y;
+            y.x = one(x, m, j, sum.x, a_sum, a_code, res.x); y.y = one(x + 1, m, j + 1, sum.y, a_sum, a_code, res.y);
+            y.z = one(x + 2, m, j + 2, sum.z, a_sum, a_code, res.z); y.w = one(x + 3, m, j + 3, sum.w, a_sum, a_code, res.w);
+            if (P.output) *reinterpret_cast<float4 *>(P.output + x) = y;
+        }
+        return;
+    }
+    for (unsigned x = first; x < total; x += step) {
+        const unsigned m = x / Cout, j = x - m * Cout;
+        if (!AXC_SCRATCH_OK(P, P.partial + x, 4, 360u) || !AXC_SCRATCH_OK(P, P.asum + m, 4, 361u)) continue;
+        const float y = one(x, m, j, P.partial[x], __ldg(P.asum + m), P.acode ? P.a_coef * __ldg(P.acode + m) : 0, P.residual ? __ldg(P.residual + x) : 0.0f);
+        if (P.output) P.output[x] = y;
     }
 }
 
@@ -1472,7 +1565,7 @@ struct Config {
     bool pre;
 };
 
-size_t xt_size(const XGeom &x, int mode) { return size_t((x.Cout + (mode == kXtabFull ? 7 : 15)) / (mode == kXtabFull ? 8 : 16)) * x.chunks * 65536u; }
+size_t xt_size(const XGeom &x, int mode) { return size_t((x.Cout + (mode == kXtabFull ? 7 : 15)) / (mode == kXtabFull ? 8 : 16)) * x.chunks * (mode == kXtabByte64 ? 16384u : 65536u); }
 
 // Pixels per tile, splits of K, and where the expanded tables are made.  In clocks per octet: lookups and codes 1.09 per pixel,
 // about 130 for the waits around a table, 720 for building one (512 of them on the shared-memory pipe); a start and an end that
@@ -1491,18 +1584,18 @@ Config choose_config(int mode, const XGeom &x, int sms, bool may_split, size_t x
     double best_cost = 1e300;
     for (int pre = 0; pre < 2; ++pre) {
         if (pre && (mode == kXtabExact || xt_size(x, mode) > xt_bytes)) continue;
-        for (int nb = mode == kXtabFull && pre ? 48 : 32; nb >= (pre ? 16 : 4); nb = nb == 48 ? 32 : nb >> 1) {
+        for (int nb = mode == kXtabFull && pre ? 48 : 32; nb >= (!pre ? 4 : mode == kXtabByte64 ? 8 : 16); nb = nb == 48 ? 32 : nb >> 1) {
             const int pix = kWarps * 8 * nb;
             const long long tiles = ((long long)x.M + pix - 1) / pix * tiles_n;
-            const double octet = mode == kXtabExact ? 0.30 * pix + 100.0 : 1.09 * pix + (pre ? 130.0 : 850.0);
+            const double octet = mode == kXtabExact ? 0.30 * pix + 100.0 : 1.09 * pix + (pre ? 130.0 : mode == kXtabByte64 ? 400.0 : 850.0);
             for (int r = 0; r <= 4; ++r) {                         // no split, or as many as fill one to four rounds
                 if (r > 0 && (!may_split || tiles >= sms)) break;
                 const int sp = r == 0 ? 1 : int(r * (long long)sms / tiles < x.chunks ? r * (long long)sms / tiles : x.chunks);
                 const int cps = (x.chunks + sp - 1) / sp;
                 const int spe = (x.chunks + cps - 1) / cps;
                 const long long rounds = (tiles * spe + sms - 1) / sms;
-                double cost = double(rounds) * (2.0 * cps * octet + 2000.0 + 3.0 * pix * (spe > 1 ? 2.0 : 1.0)) + (spe > 1 ? 6000.0 : 0.0);
-                cost += pre ? double(xt_size(x, mode)) / 2300.0 + 8000.0 : 3000.0;
+                double cost = double(rounds) * (2.0 * cps * octet + 2000.0 + 3.0 * pix) + (spe > 1 ? 6000.0 : 0.0);
+                cost += pre ? double(xt_size(x, mode)) / 2300.0 + (mode == kXtabByte64 ? 4700.0 : 8000.0) : 3000.0;
                 if (cost < best_cost) { best_cost = cost; best = {nb, spe, cps, pre != 0}; }
             }
         }
@@ -1527,7 +1620,7 @@ XLayout xlayout(const Geom &g, const XGeom &x, int mode)
     // room for the expanded tables where a call would have them made in global memory
     L.xt = off;
     L.xt_bytes = 0;
-    for (int m : {int(kXtabByte), int(kXtabFull)}) {
+    for (int m : {int(kXtabByte), int(kXtabByte64), int(kXtabFull)}) {
         const size_t bytes = xt_size(x, m);
         if ((mode == m || mode == kXtabAny) && bytes <= kXtMax && bytes > L.xt_bytes && choose_config(m, x, kModelSms, size_t(g.M) * g.Cout * 4 <= kPartialMax, bytes).pre) L.xt_bytes = bytes;
     }
@@ -1539,9 +1632,11 @@ XLayout xlayout(const Geom &g, const XGeom &x, int mode)
 template <int MODE, int NB, bool PRE>
 int launch_variant(const XParams &P, const DeviceInfo &di, cudaStream_t stream)
 {
-    AXC_CUDA(cudaFuncSetAttribute(xtab_kernel<MODE, NB, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin));
-    const long long grid = P.units < di.sm_count ? P.units : di.sm_count;
-    return launch_dependent(xtab_kernel<MODE, NB, PRE>, unsigned(grid), kWarps * 32, size_t(di.max_smem_optin), stream, P);
+    constexpr bool kHalf = MODE == kXtabByte64;                    // two CTAs to an SM, each a half of the tiles
+    const int smem = kHalf ? int(kWindowHalf - di.smem_base) : di.max_smem_optin, slots = kHalf ? 2 * di.sm_count : di.sm_count;
+    AXC_CUDA(cudaFuncSetAttribute(xtab_kernel<MODE, NB, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const long long grid = P.units < slots ? P.units : slots;
+    return launch_dependent(xtab_kernel<MODE, NB, PRE>, unsigned(grid), kWarpsOf<MODE> * 32, size_t(smem), stream, P);
 }
 
 template <int MODE>
@@ -1550,6 +1645,7 @@ int launch_mode(const Config &cf, const XParams &P, const DeviceInfo &di, cudaSt
     constexpr bool kPre = MODE != kXtabExact;
     if (cf.pre) {
         if (cf.nb == 48) return launch_variant<MODE, MODE == kXtabFull ? 48 : 32, kPre>(P, di, stream);
+        if (cf.nb == 8) return launch_variant<MODE, MODE == kXtabByte64 ? 8 : 16, kPre>(P, di, stream);
         return cf.nb == 32 ? launch_variant<MODE, 32, kPre>(P, di, stream) : launch_variant<MODE, 16, kPre>(P, di, stream);
     }
     switch (cf.nb) {
@@ -1563,7 +1659,7 @@ int launch_mode(const Config &cf, const XParams &P, const DeviceInfo &di, cudaSt
 template <int MODE>
 int launch_expand(const ExpandParams &E, const DeviceInfo &di, cudaStream_t stream)
 {
-    constexpr size_t smem = MODE == kXtabFull ? 257 * 512 + 2 * 16 * 8 * 2 + 16 : 257 * 256 + 2 * 16 * 16 * 2 + 16;
+    constexpr size_t smem = MODE == kXtabFull ? 257 * 512 + 2 * 16 * 8 * 2 + 16 : 257 * (MODE == kXtabByte ? 256 : 128) + 2 * 16 * 16 * 2 + 16;
     constexpr int per_sm = 1;
     AXC_CUDA(cudaFuncSetAttribute(xexpand_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const int total = E.g.tiles_n * E.g.chunks, grid = total < di.sm_count * per_sm ? total : di.sm_count * per_sm;
@@ -1634,9 +1730,11 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     const long long blocks = (long long)A.blocks_sum + A.blocks_w + A.blocks_t + (long long)g.N * A.tiles_y * A.tiles_x;
     if (blocks >= (1ll << 31)) return AXC_INTERNAL;
     P.partial = nullptr;
+    A.zeros = nullptr; A.zero_pieces = 0;
     if (cf.splits > 1) {
         P.partial = reinterpret_cast<int32_t *>(scratch + L.partial);
-        AXC_CUDA(cudaMemsetAsync(P.partial, 0, partial_bytes, stream));
+        A.zeros = reinterpret_cast<uint4 *>(P.partial);
+        A.zero_pieces = (long long)((partial_bytes + 15) / 16);    // (the region is rounded up to 256 bytes)
     }
     const auto prep = u8 ? xprep_kernel<true> : xprep_kernel<false>;
     AXC_CUDA(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPrepSmemMax)));
@@ -1648,7 +1746,7 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
         ExpandParams E;
         E.g = x; E.filter = filter; E.filter_u8 = A.filter_u8; E.rows = reinterpret_cast<const unsigned char *>(lut_dev + 65536); E.ranges = ranges_dev; E.host_q = A.host_q;
         E.xt = scratch + L.xt; E.wb = A.wb; E.qf_debug = A.qf_debug; E.hdr = A.hdr; E.scratch_bytes = A.scratch_bytes;
-        const int rc = mode == kXtabFull ? launch_expand<kXtabFull>(E, di, stream) : launch_expand<kXtabByte>(E, di, stream);
+        const int rc = mode == kXtabFull ? launch_expand<kXtabFull>(E, di, stream) : mode == kXtabByte ? launch_expand<kXtabByte>(E, di, stream) : launch_expand<kXtabByte64>(E, di, stream);
         if (rc) return rc;
     }
 
@@ -1661,18 +1759,18 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     P.k_e_min = int(unsigned(g.K) * (unsigned(e_min) + (u8 ? unsigned(u8->input_offset) * unsigned(u8->filter_offset) : 0u)));
     if (mode == kXtabRef) return launch_ref(P, di, stream);
     P.splits = cf.splits; P.chunks_per_split = cf.chunks_per_split;
-    P.units = ((long long)x.M + kWarps * 8 * cf.nb - 1) / (kWarps * 8 * cf.nb) * x.tiles_n * cf.splits;
+    const int tile = (mode == kXtabByte64 ? kWarpsOf<kXtabByte64> : kWarps) * 8 * cf.nb;
+    P.units = ((long long)x.M + tile - 1) / tile * x.tiles_n * cf.splits;
     if (P.units >= (1ll << 31)) return AXC_INTERNAL;
     P.plain = ((output != nullptr) != (P.acc_out != nullptr) && !P.partial &&
                ((reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(P.acc_out) | reinterpret_cast<uintptr_t>(g.ep.residual)) & 15u) == 0) ? 1 : 0;
     int rc = mode == kXtabFull ? launch_mode<kXtabFull>(cf, P, di, stream)
-             : mode == kXtabByte ? launch_mode<kXtabByte>(cf, P, di, stream) : launch_mode<kXtabExact>(cf, P, di, stream);
+             : mode == kXtabByte ? launch_mode<kXtabByte>(cf, P, di, stream)
+             : mode == kXtabByte64 ? launch_mode<kXtabByte64>(cf, P, di, stream) : launch_mode<kXtabExact>(cf, P, di, stream);
     if (rc) return rc;
     if (cf.splits > 1) {
-        const long long n = (g.M * g.Cout + 255) / 256;
-        xfinal_kernel<<<unsigned(n < 1184 ? n : 1184), 256, 0, stream>>>(P);
-        AXC_CUDA(cudaGetLastError());
-        count_launch();
+        const long long n = (g.M * g.Cout + (g.Cout % 4 == 0 ? 1023 : 255)) / (g.Cout % 4 == 0 ? 1024 : 256);
+        return launch_dependent(xfinal_kernel, unsigned(n < 1184 ? n : 1184), 256, 0, stream, P);
     }
     return AXC_OK;
 }

@@ -8,9 +8,9 @@
 
 namespace axc {
 
-// What an expanded entry holds (table_form): two digits to the base 255, one byte, or nothing (only the exact products).  kXtabRef:
-// the entry itself, for the fp32 running total in K order.
-enum XtabMode { kXtabRef = 17, kXtabFull = 16, kXtabByte = 8, kXtabExact = 0, kXtabNone = -1, kXtabAny = -2 };
+// What an expanded entry holds (table_form): two digits to the base 255, one byte, or nothing (only the exact products).  kXtabByte64: one byte, and the
+// rows repeat every 64 activations.  kXtabRef: the entry itself, for the fp32 running total in K order.
+enum XtabMode { kXtabRef = 17, kXtabFull = 16, kXtabByte = 8, kXtabByte64 = 9, kXtabExact = 0, kXtabNone = -1, kXtabAny = -2 };
 
 // The fixed shared-window addresses of the dense kernels fit this device.
 inline bool window_ok(const DeviceInfo &di) { return di.max_smem_optin >= 232448 && di.smem_base <= 2048u && di.smem_end >= 233472u; }
