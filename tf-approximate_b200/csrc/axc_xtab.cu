@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
     extern __shared__ __align__(16) unsigned char expand_smem[];
     const XGeom &g = P.g;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const unsigned tab = (unsigned)__cvta_generic_to_shared(expand_smem), lists = tab + 257u * kRow, bar = lists + 2u * 16u * TNC * 2u;
+    const unsigned tab = (unsigned)__cvta_generic_to_shared(expand_smem), lists = tab + 257u * kRow, bar = lists + (MODE == kXtabByte64 ? 4u : 2u) * 16u * TNC * 2u;
     pdl_trigger();
     if (tid == 0) {
         mbar_init(bar, 1);
@@ -771,13 +771,16 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
     bool ok = true;
     mbar_wait(bar, 0u, ok, AXC_WAIT_POLLS(0));
     // thread (kk, slot) of the first 16*TNC prepares the list of table rows of a chunk
-    const int kk = tid / TNC, slot = tid % TNC;
+    const int kk = tid / TNC % 16, slot = tid % TNC;
     const int elem = ((kk & 3) << 2) + ((kk >> 3) << 1) + ((kk >> 2) & 1);           // element 4t + 2*octet + p
     const int total = g.tiles_n * g.chunks;
     const int kidx = lane & 7, sub = lane >> 3;
     unsigned parity = 0;
-    for (int tc = int(blockIdx.x); tc < total; tc += int(gridDim.x), parity ^= 1u) {
-        if (tid < 16 * TNC) {
+    constexpr int kTurn = MODE == kXtabByte64 ? 2 : 1;             // chunks at a time (256 rows: one occupies all warps)
+    const unsigned my_lists = lists + unsigned(tid / (16 * TNC)) * (16u * TNC * 2u);
+    for (int tc0 = int(blockIdx.x) * kTurn; tc0 < total; tc0 += int(gridDim.x) * kTurn, parity ^= 1u) {
+        const int tc = tc0 + tid / (16 * TNC);
+        if (tid < 16 * TNC * kTurn && tc < total) {
             const int nt = tc / g.chunks, ch = tc - nt * g.chunks;
             const int k = k_of(g, ch, elem), cj = slot_channel(MODE, slot), j = nt * TNC + cj;
             unsigned row = kNull;
@@ -785,8 +788,8 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
                 row = code_of(P.filter_u8 ? filter_value<true>(g, P.filter, P.filter_u8, (size_t)k * g.Cout + j) : filter_value<false>(g, P.filter, P.filter_u8, (size_t)k * g.Cout + j), q.f_off, q.f_inv);
                 if (P.qf_debug) P.qf_debug[(size_t)k * g.Cout + j] = uint8_t(row);
             }
-            if (AXC_SHARED_OK(lists + parity * (16u * TNC * 2u) + unsigned(kk * TNC + slot) * 2u, 2u, lists, bar, 350u))
-                asm volatile("st.shared.u16 [%0], %1;" ::"r"(lists + parity * (16u * TNC * 2u) + unsigned(kk * TNC + slot) * 2u), "h"((unsigned short)row) : "memory");
+            if (AXC_SHARED_OK(my_lists + parity * (16u * TNC * 2u * kTurn) + unsigned(kk * TNC + slot) * 2u, 2u, lists, bar, 350u))
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(my_lists + parity * (16u * TNC * 2u * kTurn) + unsigned(kk * TNC + slot) * 2u), "h"((unsigned short)row) : "memory");
             if (MODE != kXtabFull) {
                 // exact products, B operand half h, column n: channel (n>>1)*4 + 2h + (n&1); lane (n, t) holds elements 4t..4t+3
                 const int t = elem >> 2, h = (cj >> 1) & 1, n = (cj >> 2) * 2 + (cj & 1);
@@ -795,10 +798,12 @@ __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const Expand
             }
         }
         __syncthreads();                                           // (the other list's readers are a chunk behind this barrier)
-        for (int r = warp; r < kRounds; r += kExpandThreads / 32) {
-            const int o = r / (kRounds / 2), x = r % (kRounds / 2);                  // octet, round
+        for (int r0 = warp; r0 < kRounds * kTurn; r0 += kExpandThreads / 32) {
+            const int r = r0 % kRounds, o = r / (kRounds / 2), x = r % (kRounds / 2);     // octet, round
+            const int tc = tc0 + r0 / kRounds;
+            if (tc >= total) continue;
             const unsigned word = unsigned((x >> 3) * 32 + ((4 * ((x & 7) + kidx) + sub) & 31));
-            const unsigned list = lists + parity * (16u * TNC * 2u) + unsigned((o * 8 + kidx) * TNC) * 2u;
+            const unsigned list = lists + (parity * kTurn + unsigned(r0 / kRounds)) * (16u * TNC * 2u) + unsigned((o * 8 + kidx) * TNC) * 2u;
             unsigned v[TNC];
 #pragma unroll
             for (int s4 = 0; s4 < TNC / 8; ++s4) {
@@ -856,6 +861,7 @@ struct XParams {
     const int *acode, *bcode;   // sums of codes (or NULL) and what they enter the total with: 128 for a centred table, less
     int a_coef, b_coef;         // the zero points of a quantised call
     int splits, chunks_per_split;
+    int group;                  // units that a CTA takes one after the other: neighbouring pixels, the same channels and part of K
     long long units;            // pixel tiles x channel tiles x splits
 };
 
@@ -922,20 +928,30 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
 
     // unit number -> split of K, channel tile, first pixel, chunks
     auto coords = [&](unsigned u, int &nt, int &m0, int &c_begin, int &c_end) {
-        const unsigned u2 = u / unsigned(P.splits), sp = u - u2 * unsigned(P.splits), mt = u2 / unsigned(g.tiles_n);
+        const unsigned v = kSmall ? u / unsigned(P.group) : u, sub = kSmall ? u - v * unsigned(P.group) : 0u;
+        const unsigned u2 = v / unsigned(P.splits), sp = v - u2 * unsigned(P.splits), mt = u2 / unsigned(g.tiles_n);
         nt = int(u2 - mt * unsigned(g.tiles_n));
-        m0 = int(mt) * kPix;
+        m0 = int(kSmall ? mt * unsigned(P.group) + sub : mt) * kPix;
         c_begin = int(sp) * P.chunks_per_split;
         c_end = min(g.chunks, c_begin + P.chunks_per_split);
     };
 
-    // ---- codes: this warp's pixels, 16 elements of K at a time, one chunk ahead --------------------------------------
+    const unsigned first_unit = kSmall ? blockIdx.x * unsigned(P.group) : blockIdx.x;
+    auto after = [&](unsigned u) {                                 // the unit that this CTA takes after unit u
+        if (!kSmall) return u + gridDim.x;
+        return (u + 1u) % unsigned(P.group) != 0u ? u + 1u : u + 1u + (gridDim.x - 1u) * unsigned(P.group);
+    };
+
+    // ---- codes: this warp's pixels, 16 elements of K at a time ---------------------------------------------------------
+    // Asked for kAhead chunks before they are used: a chunk of a small tile is over before memory has answered.
+    constexpr int kAhead = !kTables ? 1 : NB <= 8 ? 4 : NB == 16 ? 2 : 1;
+    unsigned chunk = 0;                                            // chunks of this CTA so far
     constexpr int PPL = (NB * 8 + 31) / 32;                        // pixels per lane
     const int pieces = g.im2col ? g.M : g.N * g.H * g.W;           // distance of the 16-byte pieces of one pixel
     const int eh = g.im2col ? 1 : g.H, ew = g.im2col ? 1 : g.W;
     const unsigned my_codes = kCodes + unsigned(warp) * (NB * 8 * 16u);
     int f_base[PPL], f_yx[PPL];                                    // pixel number of the patch origin, its row and column
-    unsigned f_unit = blockIdx.x;
+    unsigned f_unit = first_unit;
     int f_left = 0, f_cc = 0, f_ky = 0, f_kx = 0;
     auto fetch_unit = [&]() {
         int nt, m0, c_begin, c_end;
@@ -972,7 +988,7 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
     auto fetch_begin = [&]() {
         f_active = false;
         if (f_left == 0) {
-            f_unit += gridDim.x;
+            f_unit = after(f_unit);
             if (f_unit >= units) return;
             fetch_unit();
         }
@@ -1002,26 +1018,30 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
     const int kidx = lane & 7, sub = lane >> 3;
     const int hf = kBytes ? sub & 1 : 0;
     unsigned raw[8];
-    unsigned b_unit = blockIdx.x;
+    unsigned b_unit = first_unit;
     int b_left = 0;                                                // octets left to build in b_unit
     const uint4 *b_rows = nullptr;
-    uint4 wq = make_uint4(0, 0, 0, 0), wq_next = wq;               // row lists of the octet being built and of the one after it
+    constexpr int kLists = NB < 32 ? 2 : 1;                        // row lists asked for ahead (the largest tiles have no registers to spare)
+    uint4 wq = make_uint4(0, 0, 0, 0), wq_next[2] = {wq, wq};      // of the octet being built and of those after it
     auto build_unit = [&]() {
         int nt, m0, c_begin, c_end;
         coords(b_unit, nt, m0, c_begin, c_end);
         b_left = 2 * (c_end - c_begin);
         b_rows = reinterpret_cast<const uint4 *>(P.wrow) + (((size_t)nt * g.chunks + c_begin) * 16 + kidx) * HV + hf;
     };
-    auto build_next = [&]() {                                      // take the next octet's row list, request the one after it
-        wq = wq_next;
+    auto build_ask = [&](int h) {                                  // request the next octet's row list (octet h of a chunk)
         if (b_left == 0) {
-            b_unit += gridDim.x;
+            if (b_rows) b_unit = after(b_unit);
             if (b_unit >= units) return;
             build_unit();
         }
-        if (AXC_SCRATCH_OK(P, b_rows, 16, 312u)) wq_next = __ldg(b_rows);
+        if (AXC_SCRATCH_OK(P, b_rows, 16, 312u)) wq_next[h & (kLists - 1)] = __ldg(b_rows);
         b_rows += 8 * HV;
         --b_left;
+    };
+    auto build_next = [&](int h) {                                 // take an octet's row list, request the next one that has not been
+        wq = wq_next[h & (kLists - 1)];
+        build_ask(h);
     };
     // Words of a row that the lane works on: 32 r + (4 (warp + kidx) + sub) mod 32 in round r (8-bit entries: 32 (r / 2) + .. with
     // the two lanes that share a piece's channels swapped in odd rounds), so that a round is a constant offset.
@@ -1063,12 +1083,12 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
     };
 
     // ---- expanded tables from global memory: two chunks in flight, issued by one thread ------------------------------------
-    unsigned x_unit = blockIdx.x;
+    unsigned x_unit = first_unit;
     int x_left = 0;
     const unsigned char *x_src = nullptr;
     auto copy_table = [&](unsigned buf) {                          // the next chunk's table into buffer `buf`
         if (x_left == 0) {
-            if (x_src) x_unit += gridDim.x;
+            if (x_src) x_unit = after(x_unit);
             if (x_unit >= units) return;
             int nt, m0, c_begin, c_end;
             coords(x_unit, nt, m0, c_begin, c_end);
@@ -1132,7 +1152,8 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
         request(0, x[0]);
         if (h == 0) fetch_begin();
         else {
-            asm volatile("cp.async.wait_all;" ::: "memory");
+            if (kAhead > 1) asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
+            else asm volatile("cp.async.wait_all;" ::: "memory");
             __syncwarp();
         }
 #pragma unroll
@@ -1149,10 +1170,10 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
             if (h == 0) {
 #pragma unroll
                 for (int f = 0; f < PPL; ++f)
-                    if (n == f * kSteps / PPL) fetch_pixel(f, my_codes);
+                    if (n == f * kSteps / PPL) fetch_pixel(f, kAhead > 1 ? my_codes + (chunk & (kAhead - 1)) * (kPix * 16u) : my_codes);
             } else if (n & 1) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) cw[2 * (n - 1) + e] = lds32(code_src + unsigned(2 * (n - 1) + e) * 128u);
+                for (int e = 0; e < 4; ++e) cw[2 * (n - 1) + e] = lds32((kAhead > 1 ? code_src + ((chunk + 1u) & (kAhead - 1)) * (kPix * 16u) : code_src) + unsigned(2 * (n - 1) + e) * 128u);
             }
             if (PRE && h == 0 && n == 1 && tid == 0 && oct > 0) {
                 // the other buffer's readers finished the chunk before this one: ask for the chunk after this one
@@ -1162,7 +1183,7 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
             }
             if (kBuild && kSmall && more) {                            // oct: chunk; octet h of the next one, in two rounds
                 if (n == 0) {
-                    build_next();
+                    build_next(h);
                     // the place's last readers worked on the chunk before this one
                     if (h == 0 && oct > 0) mbar_wait(tab_empty + ((oct + 1u) & 1u) * 8, ((oct - 1u) >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
                     build_rows();
@@ -1178,7 +1199,7 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
                 for (int r = 0; r < 4; ++r) {
                     if (n == r * kSteps / 4) {
                         if (r == 0) {
-                            build_next();
+                            build_next(h ^ 1);
                             // the stage's last readers worked on the octet before this one
                             if (oct > 0) mbar_wait(tab_empty + (st ^ 1u) * 8, ((oct - 1) >> 1) & 1u, ok, AXC_WAIT_POLLS(1));
                             build_rows();
@@ -1189,6 +1210,7 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
                 }
             }
         }
+        if (kAhead > 1 && h == 0) asm volatile("cp.async.commit_group;" ::: "memory");
         __syncwarp();                                              // also: every lane has the codes before the next are asked for
         if (lane == 0) {
             if (kBuild && kSmall) {
@@ -1203,13 +1225,13 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
 
     unsigned oct = 0, oct_total = 0;                               // octets of this CTA so far, and all of them
     constexpr int kBufs = kTables ? 1 : 4;                         // code buffers (only exact products: latency is all there is)
-    if (blockIdx.x < units) {
+    if (first_unit < units) {
         fetch_unit();
 #pragma unroll
-        for (int k = 0; k < (kTables ? 1 : kBufs - 1); ++k) fetch_chunk(my_codes + unsigned(k) * (kPix * 16u));
+        for (int k = 0; k < (kTables ? kAhead : kBufs - 1); ++k) fetch_chunk(my_codes + unsigned(k) * (kPix * 16u));
     }
-    if (kTables && blockIdx.x < units) {
-        for (unsigned u = blockIdx.x; u < units; u += gridDim.x) {
+    if (kTables && first_unit < units) {
+        for (unsigned u = first_unit; u < units; u = after(u)) {
             int nt, m0, c_begin, c_end;
             coords(u, nt, m0, c_begin, c_end);
             oct_total += 2u * unsigned(c_end - c_begin);
@@ -1219,12 +1241,13 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
             copy_table(1u);
         }
         if (kBuild) {
-            build_unit();
-            build_next();
+            build_ask(0);
+            if (kLists > 1) build_ask(1);
             mbar_wait(rows_full, 0u, ok, AXC_WAIT_POLLS(1));
             if (kSmall) {
+#pragma unroll
                 for (unsigned o = 0; o < 2u; ++o) {                       // a chunk
-                    build_next();
+                    build_next(int(o));
                     build_rows();
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
@@ -1233,7 +1256,7 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
                     }
                 }
             } else {
-                build_next();
+                build_next(0);
                 build_rows();
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
@@ -1242,21 +1265,26 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
                 }
             }
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
         __syncwarp();
         if (kBuild && lane == 0) mbar_arrive(tab_full);
 #pragma unroll
         for (int i = 0; i < NB; ++i) cw[i] = lds32(code_src + unsigned(i) * 128u);
         __syncwarp();
     }
-    unsigned chunk = 0;
-    for (unsigned u = blockIdx.x; u < units; u += gridDim.x) {
+    for (unsigned u = first_unit; u < units; u = after(u)) {
         int nt, m0, c_begin, c_end;
         coords(u, nt, m0, c_begin, c_end);
 #pragma unroll
         for (int i = 0; i < kAcc; ++i)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][e] = 0;
+        if (P.residual && !P.partial) {
+            // the shortcut is read at the tile's end, four loads at a time: from L2 by then
+#pragma unroll 1
+            for (int p = warp * (NB * 8) + lane; p < (warp + 1) * (NB * 8) && m0 + p < g.M; p += 32)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(P.residual + (size_t)(m0 + p) * g.Cout + nt * TNC));
+        }
         const uint2 *wbp = P.wb + ((size_t)nt * g.chunks + c_begin) * 32 + lane;
         uint2 wb_next = make_uint2(0, 0);
         if (MODE != kXtabFull && AXC_SCRATCH_OK(P, wbp, 8, 316u)) wb_next = __ldg(wbp);
@@ -1561,7 +1589,7 @@ bool xgeom(const Geom &g, XGeom *x)
 }
 
 struct Config {
-    int nb, splits, chunks_per_split;
+    int nb, splits, chunks_per_split;          // blocks of 8 pixels per warp; kXtabByte64: of a tile of 64 * nb pixels by two CTAs
     bool pre;
 };
 
@@ -1577,25 +1605,66 @@ size_t xt_size(const XGeom &x, int mode) { return size_t((x.Cout + (mode == kXta
 //   1x1 64 -> 256 at 56x56, 64 images, one byte       249 (2048, global) / 249 (1024, global) / 680
 //   3x3 64 -> 96 at 28x28, 64 images, two digits      259 (1024, global) / 331 (2048, global) / 836
 //   3x3 64 -> 64 at 56x56, 64 images, two digits      679 (1024, global) / 660 (2048, global) / 2232
+// The same where the rows repeat: two CTAs of four warps to an SM, each with a half of a tile (of 2048 pixels: in two runs of 512,
+// since 1024 pixels at a time have no registers left - 265 us against 222 on 1x1 64 -> 256 at 56x56, 64 images).  In clocks per octet of
+// both CTAs: 2.18 per pixel of a half (also for a CTA that has the SM to itself, whose four warps wait for their loads), 250 for
+// the waits around a table, 590 for building one.  Against all others forced (one B200, us per call, chosen / best / worst):
+//   3x3 512 -> 512 at 7x7, 1 image                    70 (256, K in 9) / 70 / 1110
+//   3x3 512 -> 512 at 7x7, 8 images                   103 (1024, K in 9) / 103 / 1139
+//   1x1 512 -> 2048 at 7x7, 8 images                  55 (1024, K in 2) / 56 / 144
+//   3x3 256 -> 256 at 14x14, 8 images                 90 (2048, K in 9, global) / 90 / 576
+//   1x1 512 -> 128 at 28x28, 8 images                 45 (512, global) / 46 / 139
+//   3x3 64 -> 64 at 56x56, 8 images                   66 (1024, K in 3, global) / 66 / 155
+//   3x3 256 -> 256 at 14x14, 128 images               644 (1024, K in 3, global) / 644 / 1612
+//   1x1 64 -> 256 at 56x56, 64 images                 232 (2048, global) / 232 / 559
+//   3x3 32 -> 8 at 97x97, 20 images                   81 (2048, K in 3, global) / 76 (512, global) / 120
+Config choose_halves(const XGeom &x, int sms, bool may_split, size_t xt_bytes)
+{
+    const int tiles_n = (x.Cout + 15) / 16, slots = 2 * sms;
+    Config best = {16, 1, x.chunks, false};
+    double best_cost = 1e300;
+    for (int pre = 0; pre < 2; ++pre) {
+        if (pre && xt_size(x, kXtabByte64) > xt_bytes) continue;
+        for (int nb = 32; nb >= (pre ? 8 : 4); nb >>= 1) {
+            const int group = nb == 32 ? 2 : 1, pix = 32 * nb / group;
+            const long long tiles = ((long long)x.M + 32 * nb - 1) / (32 * nb) * tiles_n;
+            // no split; as many as fill one to four rounds; two or three where there are rounds enough without and K is long
+            const bool many = tiles >= slots;
+            for (int r = 0; r <= 4; ++r) {
+                if (r > 0 && (!may_split || (many && (r > 2 || x.chunks < 32)))) break;
+                const long long fill = r == 0 ? 1 : many ? r + 1 : r * (long long)slots / tiles;
+                const int sp = int(fill < x.chunks ? fill : x.chunks), cps = (x.chunks + sp - 1) / sp, spe = (x.chunks + cps - 1) / cps;
+                const long long rounds = (tiles * spe + slots - 1) / slots;
+                const double octet = 2.18 * pix + (pre ? 250.0 : 840.0), end = (pix == 512 ? 10.0 : 13.0) * pix;
+                const double cost = double(rounds) * (group * (2.0 * cps * octet + end) + 2000.0) + (spe > 1 ? 7000.0 + double(x.M) * x.Cout / 300.0 : 0.0) +
+                                    (pre ? double(xt_size(x, kXtabByte64)) / 1600.0 + 8600.0 : 3000.0);
+                if (cost < best_cost) { best_cost = cost; best = {nb, spe, cps, pre != 0}; }
+            }
+        }
+    }
+    return best;
+}
+
 Config choose_config(int mode, const XGeom &x, int sms, bool may_split, size_t xt_bytes)
 {
+    if (mode == kXtabByte64) return choose_halves(x, sms, may_split, xt_bytes);
     const int tiles_n = (x.Cout + (mode == kXtabFull ? 7 : 15)) / (mode == kXtabFull ? 8 : 16);
     Config best = {32, 1, x.chunks, false};
     double best_cost = 1e300;
     for (int pre = 0; pre < 2; ++pre) {
         if (pre && (mode == kXtabExact || xt_size(x, mode) > xt_bytes)) continue;
-        for (int nb = mode == kXtabFull && pre ? 48 : 32; nb >= (!pre ? 4 : mode == kXtabByte64 ? 8 : 16); nb = nb == 48 ? 32 : nb >> 1) {
+        for (int nb = mode == kXtabFull && pre ? 48 : 32; nb >= (pre ? 16 : 4); nb = nb == 48 ? 32 : nb >> 1) {
             const int pix = kWarps * 8 * nb;
             const long long tiles = ((long long)x.M + pix - 1) / pix * tiles_n;
-            const double octet = mode == kXtabExact ? 0.30 * pix + 100.0 : 1.09 * pix + (pre ? 130.0 : mode == kXtabByte64 ? 400.0 : 850.0);
+            const double octet = mode == kXtabExact ? 0.30 * pix + 100.0 : 1.09 * pix + (pre ? 130.0 : 850.0);
             for (int r = 0; r <= 4; ++r) {                         // no split, or as many as fill one to four rounds
                 if (r > 0 && (!may_split || tiles >= sms)) break;
                 const int sp = r == 0 ? 1 : int(r * (long long)sms / tiles < x.chunks ? r * (long long)sms / tiles : x.chunks);
                 const int cps = (x.chunks + sp - 1) / sp;
                 const int spe = (x.chunks + cps - 1) / cps;
                 const long long rounds = (tiles * spe + sms - 1) / sms;
-                double cost = double(rounds) * (2.0 * cps * octet + 2000.0 + 3.0 * pix) + (spe > 1 ? 6000.0 : 0.0);
-                cost += pre ? double(xt_size(x, mode)) / 2300.0 + (mode == kXtabByte64 ? 4700.0 : 8000.0) : 3000.0;
+                double cost = double(rounds) * (2.0 * cps * octet + 2000.0 + 3.0 * pix * (spe > 1 && mode == kXtabFull ? 2.0 : 1.0)) + (spe > 1 ? 6000.0 : 0.0);
+                cost += pre ? double(xt_size(x, mode)) / 2300.0 + 8000.0 : 3000.0;
                 if (cost < best_cost) { best_cost = cost; best = {nb, spe, cps, pre != 0}; }
             }
         }
@@ -1635,7 +1704,7 @@ int launch_variant(const XParams &P, const DeviceInfo &di, cudaStream_t stream)
     constexpr bool kHalf = MODE == kXtabByte64;                    // two CTAs to an SM, each a half of the tiles
     const int smem = kHalf ? int(kWindowHalf - di.smem_base) : di.max_smem_optin, slots = kHalf ? 2 * di.sm_count : di.sm_count;
     AXC_CUDA(cudaFuncSetAttribute(xtab_kernel<MODE, NB, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const long long grid = P.units < slots ? P.units : slots;
+    const long long turns = kHalf ? P.units / P.group : P.units, grid = turns < slots ? turns : slots;
     return launch_dependent(xtab_kernel<MODE, NB, PRE>, unsigned(grid), kWarpsOf<MODE> * 32, size_t(smem), stream, P);
 }
 
@@ -1644,12 +1713,12 @@ int launch_mode(const Config &cf, const XParams &P, const DeviceInfo &di, cudaSt
 {
     constexpr bool kPre = MODE != kXtabExact;
     if (cf.pre) {
-        if (cf.nb == 48) return launch_variant<MODE, MODE == kXtabFull ? 48 : 32, kPre>(P, di, stream);
+        if (cf.nb == 48) return launch_variant<MODE, MODE == kXtabFull ? 48 : 16, kPre>(P, di, stream);
         if (cf.nb == 8) return launch_variant<MODE, MODE == kXtabByte64 ? 8 : 16, kPre>(P, di, stream);
-        return cf.nb == 32 ? launch_variant<MODE, 32, kPre>(P, di, stream) : launch_variant<MODE, 16, kPre>(P, di, stream);
+        return cf.nb == 32 && MODE != kXtabByte64 ? launch_variant<MODE, MODE == kXtabByte64 ? 16 : 32, kPre>(P, di, stream) : launch_variant<MODE, 16, kPre>(P, di, stream);
     }
     switch (cf.nb) {
-    case 32: return launch_variant<MODE, 32, false>(P, di, stream);
+    case 32: return launch_variant<MODE, MODE == kXtabByte64 ? 16 : 32, false>(P, di, stream);
     case 16: return launch_variant<MODE, 16, false>(P, di, stream);
     case 8: return launch_variant<MODE, 8, false>(P, di, stream);
     default: return launch_variant<MODE, 4, false>(P, di, stream);
@@ -1659,10 +1728,10 @@ int launch_mode(const Config &cf, const XParams &P, const DeviceInfo &di, cudaSt
 template <int MODE>
 int launch_expand(const ExpandParams &E, const DeviceInfo &di, cudaStream_t stream)
 {
-    constexpr size_t smem = MODE == kXtabFull ? 257 * 512 + 2 * 16 * 8 * 2 + 16 : 257 * (MODE == kXtabByte ? 256 : 128) + 2 * 16 * 16 * 2 + 16;
-    constexpr int per_sm = 1;
+    constexpr size_t smem = MODE == kXtabFull ? 257 * 512 + 2 * 16 * 8 * 2 + 16 : 257 * (MODE == kXtabByte ? 256 : 128) + (MODE == kXtabByte ? 2 : 4) * 16 * 16 * 2 + 16;
     AXC_CUDA(cudaFuncSetAttribute(xexpand_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const int total = E.g.tiles_n * E.g.chunks, grid = total < di.sm_count * per_sm ? total : di.sm_count * per_sm;
+    const int total = E.g.tiles_n * E.g.chunks, turns = MODE == kXtabByte64 ? (total + 1) / 2 : total, slots = di.sm_count * (MODE == kXtabByte64 ? 2 : 1);
+    const int grid = turns < slots ? turns : slots;
     return launch_dependent(xexpand_kernel<MODE>, unsigned(grid), kExpandThreads, smem, stream, E);
 }
 
@@ -1760,7 +1829,8 @@ int launch_xtab(const uint16_t *lut_dev, int mode, int centred, int e_min, const
     if (mode == kXtabRef) return launch_ref(P, di, stream);
     P.splits = cf.splits; P.chunks_per_split = cf.chunks_per_split;
     const int tile = (mode == kXtabByte64 ? kWarpsOf<kXtabByte64> : kWarps) * 8 * cf.nb;
-    P.units = ((long long)x.M + tile - 1) / tile * x.tiles_n * cf.splits;
+    P.group = mode == kXtabByte64 && cf.nb == 32 ? 2 : 1;
+    P.units = ((long long)x.M + tile - 1) / tile * x.tiles_n * cf.splits * P.group;
     if (P.units >= (1ll << 31)) return AXC_INTERNAL;
     P.plain = ((output != nullptr) != (P.acc_out != nullptr) && !P.partial &&
                ((reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(P.acc_out) | reinterpret_cast<uintptr_t>(g.ep.residual)) & 15u) == 0) ? 1 : 0;
