@@ -277,14 +277,15 @@ class GpuRunner:
             e0 = self.torch.cuda.Event(enable_timing=True)
             e1 = self.torch.cuda.Event(enable_timing=True)
             e0.record()
-        # a shortcut (with its ReLU) is added by the library's one-pass kernel right after the convolution - outside the
-        # convolution's event pair, so that the per-layer times stay those of the table convolution
+        # a shortcut (with its ReLU) is added at the end of the convolution; where the layers are timed, by the library's
+        # one-pass kernel outside the convolution's event pair, so that their times stay those of the table convolution
+        apart = residual is not None and self.conv_events is not None
         y = fn(x, self.filters[i], lo, hi, self.f_ranges[i][0], self.f_ranges[i][1],
-               [1, spec.stride, spec.stride, 1], 8, table, "SAME", input_relu=input_relu, relu=relu and residual is None)
+               [1, spec.stride, spec.stride, 1], 8, table, "SAME", input_relu=input_relu, relu=relu and not apart, residual=None if apart else residual)
         if self.conv_events is not None:
             e1.record()
             self.conv_events.append((i, e0, e1))
-        if residual is not None:
+        if apart:
             self.ax.ops.add_residual_(y, residual, relu=relu)
         return y
 
