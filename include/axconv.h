@@ -48,8 +48,8 @@ enum { AXC_FORMAT_NHWC = 0, AXC_FORMAT_NCHW = 1 };
  *   total (tf2/src/approx_nn_conv_kernels.cpp:245-246), which rounds once a partial sum passes 2^24.  Output
  *   bits equal the reference's CPU kernel for every K.  Where the table and K prove that no partial sum can
  *   round (K * largest entry <= 2^24 * the power of two dividing every entry) the fast integer kernel serves
- *   the call, since both give the same bits; otherwise a kernel that walks K in order does (a quarter
- *   to half of the speed).  Depthwise calls ignore the field (K = kh*kw never rounds). */
+ *   the call, since both give the same bits; otherwise a kernel that walks K in order does (half of the speed on
+ *   expanded tables, with a buffer of axc_conv2d_fast_workspace_bytes; else a quarter).  Depthwise calls ignore the field (K = kh*kw never rounds). */
 enum { AXC_ACCUM_EXACT_I32 = 0, AXC_ACCUM_REFERENCE_F32 = 1 };
 /* Whether the dense op prepares a per-filter lookup plan (kept in the workspace, built in 3-90 ms, reused while the
  * filter is unchanged) or serves the call without one.
@@ -140,7 +140,7 @@ int axc_conv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc 
 enum {
     AXC_ROUTE_NONE = 0,      /* nothing to do, or a buffer that the call refuses (AXC_INTERNAL) */
     AXC_ROUTE_PLAN = 1,      /* lookups scheduled by the plan in the buffer */
-    AXC_ROUTE_COMMON_K = 2,  /* all lanes at the same K index, no plan */
+    AXC_ROUTE_COMMON_K = 2,  /* all lanes at the same K index, no plan; and every call whose sum is taken in the reference's order */
     AXC_ROUTE_EXPANDED = 3   /* expanded tables */
 };
 int axc_conv2d_route(const axc_table *table, const axc_conv_desc *desc, size_t workspace_bytes, int32_t out4[4]);

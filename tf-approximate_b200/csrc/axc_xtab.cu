@@ -12,7 +12,7 @@
 // What is looked up (whole numbers throughout, so the total is the same):
 //   8-bit entries    where the table differs from the exact product by values that span at most 255: that distance less its
 //                    minimum.  The exact products are added by further MMAs on the codes themselves (one per 16 K elements,
-//                    8 pixels and 16 channels).
+//                    8 pixels and 16 channels).  Where that distance is the same for a and a + 64 the table has 64 rows.
 //   16-bit entries   two digits to the base 255, so that one MMA with the weights 1 and 255 adds both into a single
 //                    accumulator (256 does not fit a u8 operand; low and high bytes in accumulators of their own would
 //                    halve the pixels a tile can hold).  A table that reaches past 65279 is stored less 128 (a + b) and its
@@ -50,6 +50,8 @@ namespace {
 //   [65536, 131072)       two expanded tables, interleaved: row a of stage s at a*256 + s*128, so that an address is
 //                         {offset in the row, a, 1, 0} and one byte permute puts the activation in
 //   [131072, 232960)      transposed table, the other rows (8-bit entries: all 257 rows)
+// 64 rows, two CTAs to an SM: codes [3072, 19456), transposed table [19456, 52352), tables of two chunks [65536, 98304), 64 rows of
+// 256 bytes each, a chunk's two octets interleaved; the place in the ring is bit 6 of the row.
 // With expanded tables from global memory: codes from 3072 up to 52224, tables of two chunks at 65536 and 131072, a chunk's
 // two octets interleaved like the two stages above.
 constexpr unsigned kCodes = 3072u;
