@@ -1533,8 +1533,9 @@ bool prep_tile(const Geom &g, int vec, bool im2col, bool sums, PrepTile *out)
         last = parts >= g.OW;
         const int tw = last ? 1 : (g.OW + parts - 1) / parts;
         if (tw > kPrepThreads) continue;
+        if (tw < 8 && g.OW >= 16 && best < 1e300) break;           // (the search itself is host time of every call)
         const size_t rw = region_w(tw);
-        for (int th = 1; th <= g.OH && th * tw <= kPrepThreads; th += th < 8 ? 1 : 2) {
+        for (int th = 1; th <= g.OH && th * tw <= kPrepThreads; th += th < 8 ? 1 : th < 16 ? 2 : 4) {
             const size_t rh = region_h(th), bytes = smem(rh, rw);
             if (bytes > kPrepSmemMax) break;
             const size_t block = (bytes < kSumSmem ? kSumSmem : bytes) + 1024;
