@@ -29,17 +29,17 @@ SM_COUNT = 148
 SMEM_BYTES_PER_CLK_PER_SM = 128   # shared-memory bandwidth: what bounds the table lookups
 
 
-def call_bytes(spec, in_hw, batch, group):
+def call_bytes(spec, in_hw, batch, group, rows_of_table=256):
     """Bytes that a dense call on the expanded tables moves between its kernels and memory, from their layout: the fp32 tensors
-    once; the 8-bit codes, the patch sums and - with `group` channels each, 0: not in memory - the expanded tables written by one kernel and
-    read once by the next.  (Further reads of a table by other pixel tiles are expected to hit L2.)"""
+    once; the 8-bit codes, the patch sums and - with `group` channels each, 0: not in memory; 256 rows, or 64 where they repeat - the expanded
+    tables written by one kernel and read once by the next.  (Further reads of a table by other pixel tiles are expected to hit L2.)"""
     from tf_approximate_b200 import workloads as W
     o = W.out_hw(in_hw, spec.stride)
     pixels, taps, pieces = batch * o * o, spec.k * spec.k, -(-spec.cin // 16)
     rows = -(-taps * spec.cin // 16)
     im2col = taps * pieces * 8 > rows * 9
     codes = 16 * (pixels * rows if im2col else batch * in_hw * in_hw * pieces)
-    tables = 65536 * (rows if im2col else taps * pieces) * -(-spec.cout // group) if group else 0
+    tables = 256 * rows_of_table * (rows if im2col else taps * pieces) * -(-spec.cout // group) if group else 0
     return W.conv_io_bytes(spec, in_hw, batch) + 2 * (codes + 4 * pixels + tables)
 
 
@@ -396,7 +396,9 @@ def run_gpu(args):
         if not s.depthwise:
             table = runner.tables[i % len(runner.tables)]
             r = ax.ops.dense_route((batch, h, h, s.cin), (s.k, s.k, s.cin, s.cout), (1, s.stride, s.stride, 1), "SAME", table)
-            traffic += call_bytes(s, h, batch, (16 if entry_bytes == 1 else 8) if r["tables_in_global_memory"] else 0) / dense_launches
+            lut = table.numpy().astype(np.int64).reshape(256, 256) - np.arange(256)[:, None] * np.arange(256)[None, :]
+            repeat = 64 if entry_bytes == 1 and np.array_equal(lut[64:], lut[:-64]) else 256
+            traffic += call_bytes(s, h, batch, (16 if entry_bytes == 1 else 8) if r["tables_in_global_memory"] else 0, repeat) / dense_launches
     slowest = sorted(per_layer.items(), key=lambda kv: -kv[1])[:3]
     roofline = {
         "kernel": "xtab_kernel (table convolution, %d convolution calls per step)" % dense_launches,
