@@ -58,14 +58,46 @@ class _FakeQuantFn(torch.autograd.Function):
         return grad, None
 
 
+class _ColumnSumsFn(torch.autograd.Function):
+    """Sums over all but the last dimension, as autograd sees them: linear, so that the gradient of a bias has derivatives."""
+
+    @staticmethod
+    def forward(ctx, x):
+        ctx.shape = x.shape
+        return ops.column_sums(x)
+
+    @staticmethod
+    def backward(ctx, grad):
+        return grad.expand(ctx.shape)
+
+    @staticmethod
+    def jvp(ctx, tangent):
+        return ops.column_sums(tangent)
+
+
+def _bias_gradient(grad):
+    if not torch._C._has_storage(grad):                    # batched gradients: no memory that a kernel could be given
+        return grad.sum(tuple(range(grad.dim() - 1)))
+    if torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0:
+        return _ColumnSumsFn.apply(grad)
+    return ops.column_sums(grad)                           # an ordinary backward pass: nobody differentiates it
+
+
 class _ApproxConvFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, bias, ranges, strides, padding, mul_map_file, num_bits, dilations, plan, workspace):
         ctx.save_for_backward(x, w)
         ctx.cfg = (strides, padding, dilations)
-        return approx_conv2d_with_min_max_vars(x, w, None, None, None, None, strides=strides, num_bits=num_bits,
-                                               mul_map_file=mul_map_file, padding=padding, dilations=dilations,
-                                               plan=plan, workspace=workspace, ranges=ranges, bias=bias)
+        y = approx_conv2d_with_min_max_vars(x, w, None, None, None, None, strides=strides, num_bits=num_bits,
+                                            mul_map_file=mul_map_file, padding=padding, dilations=dilations,
+                                            plan=plan, workspace=workspace, ranges=ranges, bias=bias)
+        ctx.oshape = y.shape
+        return y
+
+    @staticmethod
+    def jvp(ctx, x, w, bias, *_):
+        # only a bias has a tangent here: operands with one are refused by their quantisation, which has no forward mode
+        return bias.expand(ctx.oshape).contiguous()
 
     @staticmethod
     def backward(ctx, grad):
@@ -79,23 +111,24 @@ class _ApproxConvFn(torch.autograd.Function):
             ph = max((oh - 1) * sh + (kh - 1) * dh + 1 - x.shape[1], 0)
             pw = max((ow - 1) * sw + (kw - 1) * dw + 1 - x.shape[2], 0)
         need_x, need_w, need_b = ctx.needs_input_grad[:3]
-        gx = gw = None
-        with torch.no_grad():
-            if need_x or need_w:
-                # the exact convolution's two gradients, asked for as such: no forward convolution to differentiate, and a padded
-                # copy only where the padding is not the same on both sides
-                xc, even = x.permute(0, 3, 1, 2), ph % 2 == 0 and pw % 2 == 0
-                if not even:
-                    xc = torch.nn.functional.pad(xc, (pw // 2, pw - pw // 2, ph // 2, ph - ph // 2))
-                gx, gw, _ = torch.ops.aten.convolution_backward(
-                    grad.permute(0, 3, 1, 2), xc, w.permute(3, 2, 0, 1), None, (sh, sw), (ph // 2, pw // 2) if even else (0, 0), (dh, dw),
-                    False, (0, 0), 1, (need_x, need_w, False))
-                if need_x:
-                    gx = gx if even else gx[:, :, ph // 2:ph // 2 + x.shape[1], pw // 2:pw // 2 + x.shape[2]]
-                    gx = gx.permute(0, 2, 3, 1)
-                if need_w:
-                    gw = gw.permute(2, 3, 1, 0)
-            gb = ops.column_sums(grad) if need_b else None
+        gx = gw = gb = None
+        # every step is one that autograd can differentiate again: a penalty on any of the gradients has its own gradients
+        if need_x or need_w:
+            # the exact convolution's two gradients, asked for as such: no forward convolution to differentiate, and a padded
+            # copy only where the padding is not the same on both sides
+            xc, even = x.permute(0, 3, 1, 2), ph % 2 == 0 and pw % 2 == 0
+            if not even:
+                xc = torch.nn.functional.pad(xc, (pw // 2, pw - pw // 2, ph // 2, ph - ph // 2))
+            gx, gw, _ = torch.ops.aten.convolution_backward(
+                grad.permute(0, 3, 1, 2), xc, w.permute(3, 2, 0, 1), None, (sh, sw), (ph // 2, pw // 2) if even else (0, 0), (dh, dw),
+                False, (0, 0), 1, (need_x, need_w, False))
+            if need_x:
+                gx = gx if even else gx[:, :, ph // 2:ph // 2 + x.shape[1], pw // 2:pw // 2 + x.shape[2]]
+                gx = gx.permute(0, 2, 3, 1)
+            if need_w:
+                gw = gw.permute(2, 3, 1, 0)
+        if need_b:
+            gb = _bias_gradient(grad)
         return gx, gw, gb, None, None, None, None, None, None, None, None
 
 
