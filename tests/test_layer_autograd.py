@@ -23,6 +23,8 @@ def conv(x, w, strides, padding, dilations):
 def cpu_op(monkeypatch):
     def op(x, w, *_, strides, padding, dilations, bias=None, **__):
         y = conv(x, w, strides, padding, dilations).contiguous()
+        if bias is not None and (bias.dtype != torch.float32 or tuple(bias.shape) != y.shape[3:]):
+            raise ops.InvalidArgumentError("bias")         # (as the op does)
         return y if bias is None else y + bias
     monkeypatch.setattr(layers, "approx_conv2d_with_min_max_vars", op)
     monkeypatch.setattr(ops, "column_sums", lambda x: torch.from_numpy(x.detach().numpy().reshape(-1, x.shape[-1]).sum(0)))
@@ -139,3 +141,19 @@ def test_tangents_of_the_operands_are_refused(cpu_op):
     layer, x = make()
     with fwAD.dual_level(), pytest.raises(NotImplementedError):
         layer(fwAD.make_dual(x, torch.randn_like(x)))
+
+
+@pytest.mark.parametrize("shape", [(1,), (), (1, 5), (9, 1), (8, 9, 5)], ids=str)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16])
+def test_biases_that_are_broadcast(cpu_op, shape, dtype):
+    layer, x = make()
+    bias = torch.randn(shape).to(dtype)
+    layer.bias = torch.nn.Parameter(bias)
+    y = layer(x)
+    y.square().sum().backward()
+    ref = [t.detach().double().requires_grad_(True) for t in (layer.kernel, bias)]
+    y64 = in_float64(layer, x.double(), *ref)
+    y64.square().sum().backward()
+    assert close(y.detach(), y64.detach()) and close(layer.kernel.grad, ref[0].grad)
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-5      # the gradient has the bias's type
+    assert torch.allclose(layer.bias.grad.double(), ref[1].grad, rtol=tol, atol=tol * float(ref[1].grad.abs().max()))

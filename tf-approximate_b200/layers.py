@@ -196,12 +196,13 @@ class FakeApproxConv2D(torch.nn.Module):
         q_k = _FakeQuantFn.apply(self.kernel, ranges[2:4])
         # while the weights are being trained they change every step: no lookup plan then (nothing to rebuild)
         plan = "none" if (self.training and self.kernel.requires_grad) else "keep"
-        # the op adds a bias that it can take in the same pass
-        fused = self.bias if self.bias is not None and self.bias.dtype == torch.float32 and self.bias.device == inputs.device and self.bias.dim() == 1 else None
+        # the op adds an fp32 bias per filter in the same pass; any other is added as torch broadcasts it
+        b = self.bias
+        fused = b if b is not None and b.dtype == torch.float32 and b.device == inputs.device and b.shape == self.kernel.shape[3:] else None
         y = _ApproxConvFn.apply(q_in, q_k, fused, ranges, strides4, self.padding, table, self.num_bits, dilations4,
                                 plan, workspace)
-        if self.bias is not None and fused is None:
-            y = y + self.bias
+        if b is not None and fused is None:
+            y = y + b
         if self.activation is not None:
             y = self.activation(y)
         return y
