@@ -140,8 +140,8 @@ int axc_conv2d_fast_workspace_bytes(const axc_table *table, const axc_conv_desc 
 enum {
     AXC_ROUTE_NONE = 0,      /* nothing to do, or a buffer that the call refuses (AXC_INTERNAL) */
     AXC_ROUTE_PLAN = 1,      /* lookups scheduled by the plan in the buffer */
-    AXC_ROUTE_COMMON_K = 2,  /* all lanes at the same K index, no plan; and every call whose sum is taken in the reference's order */
-    AXC_ROUTE_EXPANDED = 3   /* expanded tables */
+    AXC_ROUTE_COMMON_K = 2,  /* all lanes at the same K index, no plan */
+    AXC_ROUTE_EXPANDED = 3   /* expanded tables, whichever order the sum is taken in */
 };
 int axc_conv2d_route(const axc_table *table, const axc_conv_desc *desc, size_t workspace_bytes, int32_t out4[4]);
 /* Reads back {rebuilt in the last call, fallback kernel in use, kernel status (0 = fine), schedule steps per

@@ -132,12 +132,13 @@ int describe_route(const axc_table *table, const Geom &g, size_t bytes, size_t g
     const Route r = choose_route(table, g, bytes, general);
     if (g.M * g.Cout == 0 || !r.enough) return AXC_OK;
     const bool ref_order = sums_in_reference_order(table, g);
-    if (!r.expanded || ref_order) {
+    if (!r.expanded) {
         out4[0] = plan_serves(g, ref_order) ? AXC_ROUTE_PLAN : AXC_ROUTE_COMMON_K;
         return AXC_OK;
     }
     int mode, centred, e_min;
     table_form(table, &mode, &centred, &e_min);
+    if (ref_order) mode = kXtabRef;
     out4[0] = AXC_ROUTE_EXPANDED;
     xtab_config(g, mode, out4 + 1);
     return AXC_OK;

@@ -1757,6 +1757,10 @@ void xtab_config(const Geom &g, int mode, int32_t out3[3])
 {
     XGeom x;
     xgeom(g, &x);
+    if (mode == kXtabRef) {
+        out3[0] = xref_tile(x, kModelSms); out3[1] = 1; out3[2] = 0;
+        return;
+    }
     const Config cf = choose_config(mode, x, kModelSms, size_t(g.M) * g.Cout * 4 <= kPartialMax, xlayout(g, x, mode).xt_bytes);
     out3[0] = kWarps * 8 * cf.nb; out3[1] = cf.splits; out3[2] = cf.pre ? 1 : 0;
 }
