@@ -230,7 +230,7 @@ struct PrepParams {
     int blocks_sum, blocks_w, blocks_t;      // first blocks, last but one and last; the rest are input tiles
     int TH, TW, tiles_y, tiles_x, RH, RW, pitch, vec;
     int sums;                                 // patch and filter sums are asked for (a quantised call has none)
-    int bytes_at, bytes_pitch;                // im2col: codes of the staged taps behind the taps, bytes per region row
+    int bytes_at, bytes_pitch;                // im2col: codes of the staged taps behind the taps (-1: none), bytes per region row
 };
 
 __host__ __device__ __forceinline__ bool two_bytes(int mode) { return mode == kXtabFull || mode == kXtabRef; }
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) xprep_kernel(const PrepParams
                 v[u] = max_keep_nan(v[u], P.in_floor);
                 const int at = ry * P.RW * P.pitch + e + (P.pitch != g.C ? int(__umulhi(unsigned(e), per_c)) : 0);
                 if (staged_ok(at, 1, 333u)) prep_smem[at] = v[u];
-                if (g.im2col && staged_ok(P.bytes_at / 4 + (ry * P.bytes_pitch + e) / 4, 1, 334u)) code_bytes[ry * P.bytes_pitch + e] = (unsigned char)code_of(v[u], q.in_off, q.in_inv);
+                if (P.bytes_at >= 0 && staged_ok(P.bytes_at / 4 + (ry * P.bytes_pitch + e) / 4, 1, 334u)) code_bytes[ry * P.bytes_pitch + e] = (unsigned char)code_of(v[u], q.in_off, q.in_inv);
             }
         }
         if (!g.im2col) {
@@ -694,6 +694,18 @@ __global__ void __launch_bounds__(kPrepThreads, 2) xprep_kernel(const PrepParams
                 if (AXC_SCRATCH_OK(P, dst, 16, 344u)) *dst = make_uint4(w[0] ^ zz, w[1] ^ zz, w[2] ^ zz, w[3] ^ zz);
                 dst += g.M;
             };
+            if (P.bytes_at < 0) {
+                // a region that leaves no room for its codes: every tap's is computed again for each pixel that it belongs to
+                for (int ky = 0; ky < g.KH; ++ky)
+                    for (int kx = 0; kx < g.KW; ++kx) {
+                        const float *src = prep_smem + (first + ky * g.dh * P.RW + kx * g.dw) * P.pitch;
+                        if (!staged_ok(src - prep_smem, g.C, 346u)) continue;
+                        for (int c = 0; c < g.C; ++c) {
+                            pending |= code_of(src[c], q.in_off, q.in_inv) << bits;
+                            if ((bits += 8) == 32) { put(pending); pending = 0; bits = 0; }
+                        }
+                    }
+            } else
             for (int ky = 0; ky < g.KH; ++ky)
                 for (int kx = 0; kx < runs_x; ++kx) {
                     const unsigned at = src0 + unsigned(ky * g.dh * P.bytes_pitch + kx * g.dw * g.C), shift = (at & 3u) * 8u;
@@ -1524,8 +1536,11 @@ bool prep_tile(const Geom &g, int vec, bool im2col, bool sums, PrepTile *out)
     else t.pitch = im2col ? g.C : g.C | 1;
     auto region_h = [&](int th) { return size_t(th - 1) * g.sh + size_t(g.KH - 1) * g.dh + 1; };
     auto region_w = [&](int tw) { return size_t(tw - 1) * g.sw + size_t(g.KW - 1) * g.dw + 1; };
-    // per pixel: the staged taps, then its code sum or (im2col) its codes
-    auto smem = [&](size_t rh, size_t rw) { return (rh * rw * (size_t(t.pitch) * 4 + (im2col ? size_t(g.C) : 4)) + 8 + 15) & ~size_t(15); };
+    // per pixel: the staged taps, then its code sum or (im2col) its codes - these not where one output pixel's region fills the
+    // shared memory without them (a wide window with a wide dilation)
+    bool bytes = im2col;
+    auto smem = [&](size_t rh, size_t rw) { return (rh * rw * (size_t(t.pitch) * 4 + (bytes ? size_t(g.C) : im2col ? 0 : 4)) + (bytes ? 8 : 0) + 15) & ~size_t(15); };
+    if (smem(region_h(1), region_w(1)) > kPrepSmemMax) bytes = false;
     if (smem(region_h(1), region_w(1)) > kPrepSmemMax) return false;
     if (!out) return true;
     double best = 1e300;
@@ -1536,9 +1551,9 @@ bool prep_tile(const Geom &g, int vec, bool im2col, bool sums, PrepTile *out)
         if (tw < 8 && g.OW >= 16 && best < 1e300) break;           // (the search itself is host time of every call)
         const size_t rw = region_w(tw);
         for (int th = 1; th <= g.OH && th * tw <= kPrepThreads; th += th < 8 ? 1 : th < 16 ? 2 : 4) {
-            const size_t rh = region_h(th), bytes = smem(rh, rw);
-            if (bytes > kPrepSmemMax) break;
-            const size_t block = (bytes < kSumSmem ? kSumSmem : bytes) + 1024;
+            const size_t rh = region_h(th), need = smem(rh, rw);
+            if (need > kPrepSmemMax) break;
+            const size_t block = (need < kSumSmem ? kSumSmem : need) + 1024;
             const int ctas = block * 2 <= 228 * 1024 ? 2 : 1;
             const long long tiles = (long long)g.N * ((g.OH + th - 1) / th) * ((g.OW + tw - 1) / tw), slots = kModelSms * ctas;
             const long long taps = (long long)rh * (long long)rw * g.C, per_batch = kPrepThreads * (vec ? 16 : 8);
@@ -1555,7 +1570,7 @@ bool prep_tile(const Geom &g, int vec, bool im2col, bool sums, PrepTile *out)
         }
     }
     t.smem = smem(size_t(t.RH), size_t(t.RW));
-    t.bytes_at = t.RH * t.RW * t.pitch * 4;
+    t.bytes_at = bytes ? t.RH * t.RW * t.pitch * 4 : -1;
     t.bytes_pitch = t.RW * g.C;
     if (t.smem < kSumSmem) t.smem = kSumSmem;
     *out = t;
