@@ -156,46 +156,68 @@ extern "C" int axc_fake_quant(const float *x, size_t count, const float *range2,
 }
 
 // ------------------------------------------------------------------------------------------------
-// Sums of a matrix's columns: the gradient of a bias.  Bound by reading the matrix once.  Lanes take neighbouring columns, warps and
-// blocks share the rows evenly, so that no sum is a chain of more than rows / (8 blocks) additions; a second kernel adds the
-// blocks' sums, a block per 32 columns.  25088 x 128: 4.6 us, of which the second kernel 2 (a library reduction over the same rows: 39).
+// Sums of a matrix's columns: the gradient of a bias.  Bound by reading the matrix once, and below some megabytes by the launches.
+// Lanes take neighbouring columns (or groups of four); a matrix narrower than a warp's 32 has the next rows in the lanes left over, a
+// wider one more blocks.  The rows are shared evenly by up to 296 blocks and the threads' rows of a block, so that a sum is a chain
+// of at most rows / 2368 additions in a thread, a tree of 8 in its block, and 45 in the second kernel, which adds the blocks' sums.
+// Up to 256 rows one block takes them all (a chain of 32) and there is no second kernel.
+// us per call, with all columns in turn in every block and idle lanes beside narrow rows / so / a library reduction:
+//   1 x 100000     266 / 3.5 / 2.7        64 x 30000     88 / 3.6 / 3.5         49 x 2048    8.7 / 3.1 / 4.9
+//   3211264 x 1    67 / 7.1 / 10.2        1048576 x 16   45 / 15.5 / 33         25088 x 128  7.3 / 8.4 / 36
+//   802816 x 64    96 / 87 / 116          200704 x 256   61 / 48 / 149
 // ------------------------------------------------------------------------------------------------
 namespace axc {
 namespace {
 
 constexpr int kColumnBlocks = 296;             // AXC_COLUMN_SUM_ROWS of the header
 
+// lanes: threads next to one another along a row
 template <int V>
-__global__ void __launch_bounds__(256) column_sums_kernel(const float *__restrict__ x, long long rows, int cols, float *__restrict__ part)
+__global__ void __launch_bounds__(256) column_sums_kernel(const float *__restrict__ x, long long rows, int cols, int lanes, float *__restrict__ part)
 {
-    __shared__ float sums[8][32 * V];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long begin = rows * blockIdx.x / gridDim.x, end = rows * (blockIdx.x + 1) / gridDim.x;
-    for (int c0 = 0; c0 < cols; c0 += 32 * V) {
-        const int c = c0 + lane * V;
-        float a[V];
+    __shared__ float sums[256 * V];
+    const int tid = threadIdx.x, r0 = tid / lanes, groups = 256 / lanes;
+    const long long c = ((long long)blockIdx.x * lanes + (tid - r0 * lanes)) * V;
+    const long long begin = rows * blockIdx.y / gridDim.y, end = rows * (blockIdx.y + 1) / gridDim.y;
+    float a[V];
 #pragma unroll
-        for (int e = 0; e < V; ++e) a[e] = 0.0f;
-        if (c < cols) {
-#pragma unroll 4
-            for (long long r = begin + warp; r < end; r += 8) {
-                if (V == 4) {
-                    const float4 v = __ldg(reinterpret_cast<const float4 *>(x + r * cols + c));
-                    a[0] += v.x; a[1 % V] += v.y; a[2 % V] += v.z; a[3 % V] += v.w;
-                } else a[0] += __ldg(x + r * cols + c);
+    for (int e = 0; e < V; ++e) a[e] = 0.0f;
+    if (r0 < groups && c < cols) {
+        constexpr int kBatch = 8;                              // loads in flight, also in the last round
+        const float *from = x + (begin + r0) * cols + c;
+        const long long step = (long long)groups * cols;
+        for (long long left = end - begin - r0; left > 0; left -= kBatch * groups, from += kBatch * step) {
+            float v[kBatch][V];
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+#pragma unroll
+                for (int e = 0; e < V; ++e) v[u][e] = 0.0f;
+                if (u * groups < left) {
+                    if (V == 4) {
+                        const float4 w = __ldg(reinterpret_cast<const float4 *>(from + u * step));
+                        v[u][0] = w.x; v[u][1 % V] = w.y; v[u][2 % V] = w.z; v[u][3 % V] = w.w;
+                    } else v[u][0] = __ldg(from + u * step);
+                }
             }
-        }
 #pragma unroll
-        for (int e = 0; e < V; ++e) sums[warp][lane * V + e] = a[e];
-        __syncthreads();
-        for (int i = threadIdx.x; i < 32 * V && c0 + i < cols; i += 256) {
-            float s = 0.0f;
+            for (int u = 0; u < kBatch; ++u)
 #pragma unroll
-            for (int w = 0; w < 8; ++w) s += sums[w][i];
-            part[(long long)blockIdx.x * cols + c0 + i] = s;
+                for (int e = 0; e < V; ++e) a[e] += v[u][e];
         }
-        __syncthreads();
     }
+#pragma unroll
+    for (int e = 0; e < V; ++e) sums[e * 256 + tid] = a[e];
+    for (int left = groups; left > 1;) {
+        const int half = (left + 1) >> 1;
+        __syncthreads();
+        if (r0 + half < left)
+#pragma unroll
+            for (int e = 0; e < V; ++e) sums[e * 256 + tid] += sums[e * 256 + tid + half * lanes];
+        left = half;
+    }
+    if (r0 == 0 && c < cols)
+#pragma unroll
+        for (int e = 0; e < V; ++e) part[(long long)blockIdx.y * cols + c + e] = sums[e * 256 + tid];
 }
 
 __global__ void __launch_bounds__(256) column_total_kernel(const float *__restrict__ part, int count, int cols, float *__restrict__ out)
@@ -231,14 +253,18 @@ extern "C" int axc_column_sums(const float *x, size_t rows, int cols, float *scr
     rc = with_device(device, &prev);
     if (rc) return rc;
     cudaStream_t s = cudaStream_t(stream);
-    const unsigned blocks = unsigned((rows + 7) / 8 < size_t(kColumnBlocks) ? (rows + 7) / 8 : size_t(kColumnBlocks));
-    if (blocks > 0) {
-        if (cols % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) column_sums_kernel<4><<<blocks, 256, 0, s>>>(x, (long long)rows, cols, scratch);
-        else column_sums_kernel<1><<<blocks, 256, 0, s>>>(x, (long long)rows, cols, scratch);
+    const int wide = cols % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 ? 4 : 1, groups = cols / wide, lanes = groups < 32 ? groups : 32;
+    const size_t fill = (rows + size_t(256 / lanes) * 4 - 1) / (size_t(256 / lanes) * 4);       // blocks that have four rows per thread
+    const unsigned blocks = unsigned(rows <= 256 || fill < 2 ? 1 : fill < size_t(kColumnBlocks) ? fill : size_t(kColumnBlocks));
+    const dim3 grid(unsigned((groups + lanes - 1) / lanes), blocks);
+    float *part = blocks > 1 ? scratch : out;
+    if (wide == 4) column_sums_kernel<4><<<grid, 256, 0, s>>>(x, (long long)rows, cols, lanes, part);
+    else column_sums_kernel<1><<<grid, 256, 0, s>>>(x, (long long)rows, cols, lanes, part);
+    count_launch();
+    if (blocks > 1) {
+        column_total_kernel<<<unsigned((cols + 31) / 32), 256, 0, s>>>(scratch, int(blocks), cols, out);
         count_launch();
     }
-    column_total_kernel<<<unsigned((cols + 31) / 32), 256, 0, s>>>(scratch, int(blocks), cols, out);
-    count_launch();
     const cudaError_t e = cudaGetLastError();
     if (prev != device) cudaSetDevice(prev);
     return e == cudaSuccess ? AXC_OK : cuda_failed(e);
