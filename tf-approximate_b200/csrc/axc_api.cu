@@ -108,10 +108,16 @@ size_t expanded_scratch_bytes(const axc_table *table, const Geom &g)
     return xtab_scratch_bytes(g, mode);
 }
 
+// Whether the expanded tables, where they can serve the call, are the quicker kernels for it.
+static bool expanded_pays(const axc_table *table, const Geom &g)
+{
+    return !table || !sums_in_reference_order(table, g) || xtab_ref_pays(g);
+}
+
 Route choose_route(const axc_table *table, const Geom &g, size_t bytes, size_t general)
 {
     const size_t fast = expanded_scratch_bytes(table, g);
-    if (fast > 0) {
+    if (fast > 0 && (bytes < general || expanded_pays(table, g))) {
         if (g.plan == AXC_PLAN_NONE || bytes < general) {
             if (bytes >= fast) return {true, true, 0};
         } else if (bytes - general >= fast) return {true, true, general};
@@ -121,7 +127,7 @@ Route choose_route(const axc_table *table, const Geom &g, size_t bytes, size_t g
 
 size_t fast_buffer_bytes(const axc_table *table, const Geom &g, size_t general)
 {
-    const size_t fast = expanded_scratch_bytes(table, g);
+    const size_t fast = expanded_pays(table, g) ? expanded_scratch_bytes(table, g) : 0;
     return fast == 0 || fast < general || g.plan == AXC_PLAN_NONE ? fast : general + fast;
 }
 

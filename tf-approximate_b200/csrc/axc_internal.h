@@ -165,7 +165,8 @@ struct Route {
     size_t scratch;         // where the expanded-table kernels' scratch starts
 };
 Route choose_route(const axc_table *table, const Geom &g, size_t bytes, size_t general);
-// Smallest buffer with which choose_route takes the expanded tables, 0 where none does.
+// Smallest buffer with which choose_route takes the expanded tables, 0 where none does or they would be the slower kernels (a buffer
+// that is too small for the others takes them all the same).
 size_t fast_buffer_bytes(const axc_table *table, const Geom &g, size_t general);
 // Body of axc_conv2d_route / axc_qconv2d_route.
 int describe_route(const axc_table *table, const Geom &g, size_t bytes, size_t general, int32_t out4[4]);

@@ -247,6 +247,21 @@ int xref_tile(const XGeom &x, int sms)
     return best;
 }
 
+// The other kernel for this order (dense_kernel<WN, true>: a tile of 64 pixels x 64 channels, or 128 x 32, per SM and round) goes round
+// less often where there are few pixels and many channels.  In us, fitted to 57 layers (within 16 %, the other within 10 % from
+// K = 256 on), 148 SMs; expanded tables / the other, measured:
+//   1x1 2048 -> 4096, one pixel             889 / 405    (4 rounds / 1)        1x1 2048 -> 512 at 7x7, 4 images       252 / 409    (1 / 1)
+//   1x1 512 -> 2048 at 7x7, 4 images        137 / 111    (2 / 1)               1x1 512 -> 2048 at 7x7, 16 images      242 / 293    (2 / 3)
+//   1x1 1024 -> 2048 s2 at 14x14, 4 images  270 / 214    (2 / 1)               3x3 256 -> 256 at 14x14, 16 images     506 / 862    (1 / 2)
+bool xref_pays(const XGeom &x)
+{
+    constexpr long long sms = kModelSms;
+    const long long tile = xref_tile(x, kModelSms), units = (x.M + tile - 1) / tile * ((x.Cout + 7) / 8), rounds = (units + sms - 1) / sms;
+    const int tn = x.Cout <= 32 ? 32 : 64, tm = 4096 / tn;
+    const long long others = (x.M + tm - 1ll) / tm * ((x.Cout + tn - 1) / tn), other_rounds = (others + sms - 1) / sms;
+    return double(rounds) * ((2.0 * x.chunks + 1.0) * (0.86 + 0.0011 * double(tile)) + 0.0136 * double(tile)) <= x.K * (0.172 * double(other_rounds) + 0.033);
+}
+
 template <int PXL>
 int launch_ref_variant(const RefParams &R, const DeviceInfo &di, cudaStream_t stream)
 {

@@ -1768,6 +1768,12 @@ size_t xtab_scratch_bytes(const Geom &g, int mode)
     return xlayout(g, x, mode).total;
 }
 
+bool xtab_ref_pays(const Geom &g)
+{
+    XGeom x;
+    return xgeom(g, &x) && xref_pays(x);
+}
+
 void xtab_config(const Geom &g, int mode, int32_t out3[3])
 {
     XGeom x;

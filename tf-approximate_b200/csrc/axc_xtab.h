@@ -18,6 +18,8 @@ inline bool window_ok(const DeviceInfo &di) { return di.max_smem_optin >= 232448
 // Scratch bytes of the expanded-table route for this shape and a table kept as `mode` (kXtabAny: enough for every table); 0
 // where the plan-based kernels serve the call.
 size_t xtab_scratch_bytes(const Geom &g, int mode);
+// Whether a call in the reference's order of additions is quicker on expanded tables.
+bool xtab_ref_pays(const Geom &g);
 // {pixels per tile, splits of K, tables from global memory} of a call that these kernels serve, on 148 SMs (diagnostics).
 void xtab_config(const Geom &g, int mode, int32_t out3[3]);
 
