@@ -1045,7 +1045,7 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
     };
     auto build_ask = [&](int h) {                                  // request the next octet's row list (octet h of a chunk)
         if (b_left == 0) {
-            if (b_rows) b_unit = after(b_unit);
+            b_unit = after(b_unit);
             if (b_unit >= units) return;
             build_unit();
         }
@@ -1255,6 +1255,7 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
             copy_table(1u);
         }
         if (kBuild) {
+            build_unit();
             build_ask(0);
             if (kLists > 1) build_ask(1);
             mbar_wait(rows_full, 0u, ok, AXC_WAIT_POLLS(1));
@@ -1293,8 +1294,8 @@ __global__ void __launch_bounds__(kWarpsOf<MODE> * 32, MODE == kXtabByte64 ? 2 :
         for (int i = 0; i < kAcc; ++i)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][e] = 0;
-        if (P.residual && !P.partial) {
-            // the shortcut is read at the tile's end, four loads at a time: from L2 by then
+        // the shortcut is read at the tile's end, four loads at a time: from L2 by then (not in the form that spills registers as it is)
+        if (!(MODE == kXtabByte && NB == 32 && kBuild) && P.residual && !P.partial) {
 #pragma unroll 1
             for (int p = warp * (NB * 8) + lane; p < (warp + 1) * (NB * 8) && m0 + p < g.M; p += 32)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(P.residual + (size_t)(m0 + p) * g.Cout + nt * TNC));
