@@ -1615,16 +1615,24 @@ struct Config {
 
 size_t xt_size(const XGeom &x, int mode) { return size_t((x.Cout + (mode == kXtabFull ? 7 : 15)) / (mode == kXtabFull ? 8 : 16)) * x.chunks * (mode == kXtabByte64 ? 16384u : 65536u); }
 
-// Pixels per tile, splits of K, and where the expanded tables are made.  In clocks per octet: lookups and codes 1.09 per pixel,
-// about 130 for the waits around a table, 720 for building one (512 of them on the shared-memory pipe); a start and an end that
-// do not shrink with the tile; tables from global memory cost their writes (2.3 KiB per clock over the chip) and a launch.
-// Against every other tile, split and place forced (one B200, us per call, chosen / best of the others / worst):
-//   3x3 512 -> 512 at 7x7, 1 image, one byte          186 (256 pixels, K in 9) / 194 (K in 13) / 1306
-//   3x3 256 -> 256 at 14x14, 8 images, one byte       140 (2048, K in 9) / 151 (1024) / 664
-//   3x3 256 -> 256 at 14x14, 128 images, one byte     786 (1024, global) / 976 (2048, global) / 2362
-//   1x1 64 -> 256 at 56x56, 64 images, one byte       249 (2048, global) / 249 (1024, global) / 680
-//   3x3 64 -> 96 at 28x28, 64 images, two digits      259 (1024, global) / 331 (2048, global) / 836
-//   3x3 64 -> 64 at 56x56, 64 images, two digits      679 (1024, global) / 660 (2048, global) / 2232
+// Pixels per tile, splits of K, and where the expanded tables are made, by the clocks of all rounds (TileClocks below: per octet, lookups
+// and codes per pixel, the waits around a table or building one; a start and an end; tables from global memory cost their writes and
+// a launch).  Against every other tile, split and place forced (one B200, us per call, chosen / best / worst):
+//   two digits                                        3x3 64 -> 96 at 28x28, 64 images    259 (1024, global) / 259 / 836
+//                                                     3x3 64 -> 64 at 56x56, 64 images    679 (1024, global) / 660 (2048, global) / 2232
+//   one byte, 256 rows (errors drawn from 0 .. 156)   3x3 512 -> 512 at 7x7, 1 image      126 (256, K in 9) / 126 / 1265
+//                                                     3x3 64 -> 64 at 56x56, 1 image      28 (1024, K in 9, global) / 28 / 74
+//                                                     3x3 64 -> 64 at 56x56, 8 images     69 (1024, global) / 69 / 176
+//                                                     1x1 256 -> 1024 at 14x14, 8 images  56 (1024) / 56 / 119
+//                                                     3x3 256 -> 256 at 14x14, 8 images   99 (2048, K in 9) / 99 / 384
+//                                                     the same, 64 images                 451 (1024, K in 2, global) / 451 / 1221
+//                                                     1x1 64 -> 256 at 56x56, 64 images   226 (1024, global) / 226 / 337
+//                                                     1x1 1024 -> 2048 s2, 14x14, 64 im.  604 (2048) / 604 / 1120
+//   exact products                                    3x3 512 -> 512 at 7x7, 1 image      51 (256, K in 9) / 51 / 202
+//                                                     3x3 256 -> 256 at 14x14, 64 images  126 (1024, K in 2) / 119 (2048) / 203
+// Fitted over 74 layers each, 0.4 % (one byte) and 0.6 % (exact) above the best on average; with the clocks of two-digit entries for
+// all three it was 3.2 % and 2.4 %, up to 31 %.  A pixel of a 2048-pixel tile of bytes costs more (its registers spill), and so does a split
+// of bytes: its sums are added one by one, and a pass over all of them follows.
 // The same where the rows repeat: two CTAs of four warps to an SM, each with a half of a tile (of 2048 pixels: in two runs of 512,
 // since 1024 pixels at a time have no registers left - 265 us against 222 on 1x1 64 -> 256 at 56x56, 64 images).  In clocks per octet of
 // both CTAs: 2.18 per pixel of a half (also for a CTA that has the SM to itself, whose four warps wait for their loads), 250 for
@@ -1665,26 +1673,39 @@ Config choose_halves(const XGeom &x, int sms, bool may_split, size_t xt_bytes)
     return best;
 }
 
+// Clocks of a tile: per pixel and octet of K (tiles of 4, 8, 16, 32 and 48 blocks per warp), around a table that comes from global
+// memory or is built, a start, the end per pixel (plain / K split), a split's last pass and its sums, tables in global memory.
+struct TileClocks {
+    double pixel[5], copied, built, start, end, end_split, split, per_sum, tables, per_byte, own;
+};
+constexpr TileClocks kClocksFull = {{1.09, 1.09, 1.09, 1.09, 1.09}, 130, 850, 2000, 3.0, 6.0, 6000, 0.0, 8000, 1.0 / 2300, 3000};
+constexpr TileClocks kClocksByte = {{1.13, 1.09, 1.055, 1.23, 0.0}, 110, 1010, 1000, 3.4, 16.0, 5500, 1.0 / 2150, 3150, 1.0 / 1430, 3000};
+constexpr TileClocks kClocksExact = {{0.328, 0.30, 0.30, 0.333, 0.0}, 0, 118, 900, 5.6, 6.6, 2600, 1.0 / 356, 0, 0.0, 3000};
+
 Config choose_config(int mode, const XGeom &x, int sms, bool may_split, size_t xt_bytes)
 {
     if (mode == kXtabByte64) return choose_halves(x, sms, may_split, xt_bytes);
+    const TileClocks &t = mode == kXtabFull ? kClocksFull : mode == kXtabByte ? kClocksByte : kClocksExact;
     const int tiles_n = (x.Cout + (mode == kXtabFull ? 7 : 15)) / (mode == kXtabFull ? 8 : 16);
     Config best = {32, 1, x.chunks, false};
     double best_cost = 1e300;
     for (int pre = 0; pre < 2; ++pre) {
         if (pre && (mode == kXtabExact || xt_size(x, mode) > xt_bytes)) continue;
         for (int nb = mode == kXtabFull && pre ? 48 : 32; nb >= (pre ? 16 : 4); nb = nb == 48 ? 32 : nb >> 1) {
-            const int pix = kWarps * 8 * nb;
+            const int pix = kWarps * 8 * nb, size = nb == 48 ? 4 : nb == 32 ? 3 : nb == 16 ? 2 : nb == 8 ? 1 : 0;
             const long long tiles = ((long long)x.M + pix - 1) / pix * tiles_n;
-            const double octet = mode == kXtabExact ? 0.30 * pix + 100.0 : 1.09 * pix + (pre ? 130.0 : 850.0);
-            for (int r = 0; r <= 4; ++r) {                         // no split, or as many as fill one to four rounds
-                if (r > 0 && (!may_split || tiles >= sms)) break;
-                const int sp = r == 0 ? 1 : int(r * (long long)sms / tiles < x.chunks ? r * (long long)sms / tiles : x.chunks);
+            const double octet = t.pixel[size] * pix + (pre ? t.copied : t.built);
+            // no split, or as many as fill one to four rounds; two or three (not with two digits) where there are rounds enough without and K is long
+            const bool many = tiles >= sms;
+            for (int r = 0; r <= 4; ++r) {
+                if (r > 0 && (!may_split || (many && (mode == kXtabFull || r > 2 || x.chunks < 32)))) break;
+                const long long fill = r == 0 ? 1 : many ? r + 1 : r * (long long)sms / tiles;
+                const int sp = int(fill < x.chunks ? fill : x.chunks);
                 const int cps = (x.chunks + sp - 1) / sp;
                 const int spe = (x.chunks + cps - 1) / cps;
                 const long long rounds = (tiles * spe + sms - 1) / sms;
-                double cost = double(rounds) * (2.0 * cps * octet + 2000.0 + 3.0 * pix * (spe > 1 && mode == kXtabFull ? 2.0 : 1.0)) + (spe > 1 ? 6000.0 : 0.0);
-                cost += pre ? double(xt_size(x, mode)) / 2300.0 + 8000.0 : 3000.0;
+                double cost = double(rounds) * (2.0 * cps * octet + t.start + pix * (spe > 1 ? t.end_split : t.end)) + (spe > 1 ? t.split + double(x.M) * x.Cout * t.per_sum : 0.0);
+                cost += pre ? double(xt_size(x, mode)) * t.per_byte + t.tables : t.own;
                 if (cost < best_cost) { best_cost = cost; best = {nb, spe, cps, pre != 0}; }
             }
         }
