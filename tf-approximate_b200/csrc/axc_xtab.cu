@@ -1528,7 +1528,8 @@ struct PrepTile {
 // memory and registers (two) allow, each loading its region (20 bytes per clock and SM, a batch of loads 700, a piece 100) and then
 // adding K taps per pixel in a chain (4.5 clocks each, 32 taps per clock and SM at most).  Tiles of at most 72 KiB, as many as
 // fill it, left 14 of 256 threads adding at 14x14x256.  Widths down to 7 pixels: without them 1x1 512 -> 128 at 28x28, 64 images, exact
-// table, had tiles of 28 pixels in a row and took 113 us, with 7x7 95 (4 rows at least: few narrow pixels gain nothing).  out == NULL: only whether there is such a tile.
+// table, had tiles of 28 pixels in a row and took 113 us, with 7x7 95 (only where there are several rounds: else
+// they gain nothing).  out == NULL: only whether there is such a tile.
 bool prep_tile(const Geom &g, int vec, bool im2col, bool sums, PrepTile *out)
 {
     PrepTile t = {};
@@ -1546,13 +1547,15 @@ bool prep_tile(const Geom &g, int vec, bool im2col, bool sums, PrepTile *out)
     if (smem(region_h(1), region_w(1)) > kPrepSmemMax) return false;
     if (!out) return true;
     double best = 1e300;
+    const bool few = g.OW < 16 || g.M < 49 * 2 * kModelSms;        // one round whatever the tile
     for (int parts = 1, last = 0; !last; parts = parts < 4 ? parts + 1 : parts == 4 ? 7 : parts == 7 ? 8 : parts * 2) {
         last = parts >= g.OW;
         const int tw = last ? 1 : (g.OW + parts - 1) / parts;
         if (tw > kPrepThreads) continue;
-        if (tw < 7 && g.OW >= 14 && best < 1e300) break;           // (the search itself is host time of every call)
+        if (tw < 8 && g.OW >= 16 && best < 1e300 && (few || tw < 7)) break;      // (the search itself is host time of every call)
+        if (parts == 7 && few) continue;
         const size_t rw = region_w(tw);
-        for (int th = (parts == 7 || parts == 8) && g.OW >= 14 ? 4 : 1; th <= g.OH && th * tw <= kPrepThreads; th += th < 8 ? 1 : th < 16 ? 2 : 4) {
+        for (int th = 1; th <= g.OH && th * tw <= kPrepThreads; th += th < 8 ? 1 : th < 16 ? 2 : 4) {
             const size_t rh = region_h(th), need = smem(rh, rw);
             if (need > kPrepSmemMax) break;
             const size_t block = (need < kSumSmem ? kSumSmem : need) + 1024;
