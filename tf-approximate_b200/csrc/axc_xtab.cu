@@ -463,8 +463,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) xprep_kernel(const PrepParams
             const int v = w < 256 ? int(__ldg(P.lut + a * 256 + w)) - less : 0;
             if (!AXC_SCRATCH_OK(P, P.tt + x * (two_bytes(P.mode) ? 2 : 1), two_bytes(P.mode) ? 2 : 1, 326u)) continue;
             if (P.mode == kXtabRef) reinterpret_cast<uint16_t *>(P.tt)[x] = w < 256 ? __ldg(P.lut + a * 256 + w) : 0;
-            else
-            if (P.mode == kXtabFull) reinterpret_cast<uint16_t *>(P.tt)[x] = uint16_t(v % 255 + (v / 255) * 256);
+            else if (P.mode == kXtabFull) reinterpret_cast<uint16_t *>(P.tt)[x] = uint16_t(v % 255 + (v / 255) * 256);
             else P.tt[x] = (unsigned char)v;
         }
         return;
@@ -759,7 +758,8 @@ struct ExpandParams {
 // xt[channel tile][chunk][row a][piece kk][16 bytes], kk = octet * 8 + k; 64 rows where they repeat, else 256.  The table's rows (one per weight) lie in shared memory.
 // A lane reads the same word (two or four a) of the rows of its piece's 8 or 16 weights, transposes in registers and writes
 // whole pieces; the 32 lanes (8 k x 4 words) read 32 different banks whatever the weights are, and write 128-byte runs.
-// Bound by the writes, 64 KiB per chunk (gathering entry by entry with random banks took 12 700 clocks per chunk, this 1500).
+// Bound by the writes, 64 KiB per chunk (gathering entry by entry with random banks took 12 700 clocks per chunk, this 1500); with 64 rows
+// 16 KiB, so that two chunks share a turn of the CTA.
 template <int MODE>
 __global__ void __launch_bounds__(kExpandThreads, 1) xexpand_kernel(const ExpandParams P)
 {
@@ -861,7 +861,7 @@ struct XParams {
     const unsigned char *codes, *tt;
     const uint16_t *wrow;
     const uint2 *wb;
-    const unsigned char *xt;    // expanded tables [channel tile][chunk][256][2 octets][8][16], or NULL: built by the CTAs
+    const unsigned char *xt;    // expanded tables [channel tile][chunk][256 or 64 rows][2 octets][8][16], or NULL: built by the CTAs
     const float *asum, *bsum;
     const PlanHeader *hdr;
     long long scratch_bytes;
@@ -889,8 +889,8 @@ __device__ __forceinline__ float dequantise(const DevQuant &Q, int total, float 
 // Warp w holds the sums of pixels [w*8*NB, (w+1)*8*NB) x all channels of the tile in 2*NB (16-bit entries) or 4*NB registers
 // per lane.  Lane (g, t) = (lane / 4, lane % 4) looks pixel g of a block up at k = t and t + 4 of an octet; even and odd g take
 // the two in opposite order, so that a quarter warp covers all 8 k at once.
-// All warps are alike: each builds an eighth of the next octet's expanded table, in four rounds between its own lookups, and
-// fetches the codes of its own pixels.  Eight warps with 255 registers rather than sixteen with 128: the loads of the next two
+// All warps are alike: each builds an eighth of the next octet's expanded table, in four rounds between its own lookups (64 rows: four
+// warps, a quarter each in two rounds), and fetches the codes of its own pixels.  Eight warps with 255 registers rather than sixteen with 128: the loads of the next two
 // block pairs are in flight while the MMAs of the last two run.
 // PRE: the expanded tables come from global memory (xexpand_kernel) by bulk copies, 64 KiB per 16 elements of K, which cost the
 // shared-memory pipe next to nothing (measured: 2 to 4 % beside a stream of LDS.128 + MMA); otherwise they are built here.
@@ -1632,8 +1632,9 @@ size_t xt_size(const XGeom &x, int mode) { return size_t((x.Cout + (mode == kXta
 //                                                     1x1 64 -> 256 at 56x56, 64 images   226 (1024, global) / 226 / 337
 //                                                     1x1 1024 -> 2048 s2, 14x14, 64 im.  604 (2048) / 604 / 1120
 //   exact products                                    3x3 512 -> 512 at 7x7, 1 image      51 (256, K in 9) / 51 / 202
-//                                                     3x3 256 -> 256 at 14x14, 64 images  126 (1024, K in 2) / 119 (2048) / 203
-// Fitted over 74 layers each, 0.4 % (one byte) and 0.6 % (exact) above the best on average; with the clocks of two-digit entries for
+//                                                     3x3 256 -> 256 at 14x14, 64 images  119 (2048) / 119 / 203
+//                                                     3x3 192 -> 96 at 72x71, 12 images   171 (1024; K in 2 187) / 171 / 206
+// Fitted over 74 layers each, 0.4 % (one byte) and 0.7 % (exact) above the best on average (0.8 % and 1.1 % over 40 drawn others); with the clocks of two-digit entries for
 // all three it was 3.2 % and 2.4 %, up to 31 %.  A pixel of a 2048-pixel tile of bytes costs more (its registers spill), and so does a split
 // of bytes: its sums are added one by one, and a pass over all of them follows.
 // The same where the rows repeat: two CTAs of four warps to an SM, each with a half of a tile (of 2048 pixels: in two runs of 512,
@@ -1698,10 +1699,10 @@ Config choose_config(int mode, const XGeom &x, int sms, bool may_split, size_t x
             const int pix = kWarps * 8 * nb, size = nb == 48 ? 4 : nb == 32 ? 3 : nb == 16 ? 2 : nb == 8 ? 1 : 0;
             const long long tiles = ((long long)x.M + pix - 1) / pix * tiles_n;
             const double octet = t.pixel[size] * pix + (pre ? t.copied : t.built);
-            // no split, or as many as fill one to four rounds; two or three (not with two digits) where there are rounds enough without and K is long
+            // no split, or as many as fill one to four rounds; with bytes two or three where there are rounds enough without and K is long
             const bool many = tiles >= sms;
             for (int r = 0; r <= 4; ++r) {
-                if (r > 0 && (!may_split || (many && (mode == kXtabFull || r > 2 || x.chunks < 32)))) break;
+                if (r > 0 && (!may_split || (many && (mode != kXtabByte || r > 2 || x.chunks < 32)))) break;
                 const long long fill = r == 0 ? 1 : many ? r + 1 : r * (long long)sms / tiles;
                 const int sp = int(fill < x.chunks ? fill : x.chunks);
                 const int cps = (x.chunks + sp - 1) / sp;
